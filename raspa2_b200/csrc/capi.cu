@@ -64,7 +64,7 @@ struct rgpu_system {
   cudaStream_t st;
   int kw;
   /* device buffers */
-  double4 *fw64;
+  double4 *fw64, *fw64t;
   int4 *fw32;
   TileRec *tiles_d;
   char4 *kvec;
@@ -82,7 +82,12 @@ struct rgpu_system {
   void *rec64;
   /* per-call scratch */
   double *io_xyz, *io_out, *io_q;
-  int *io_atom, *io_excl, *io_ov;
+  /* results of a per-call evaluation: mapped host memory that its kernel
+   * writes, so that a call costs a launch and a wait */
+  struct CallOut {
+    double e[4 * RGPU_MAX_POS];
+    int ov[RGPU_MAX_POS];
+  } *h_call;
   /* host mirrors */
   RgpuState h_state;          /* initial state at creation; last state read */
   std::vector<double> h_xyz;  /* [nmol*natom*3] */
@@ -178,11 +183,12 @@ static bool plan_group(const rgpu_engine *e, int lo, int hi, int cluster, Engine
 static void sys_free(rgpu_system *s)
 {
   if (!s) return;
-  void *ptrs[] = {s->d_uc, s->d_sys, s->fw64, s->fw32, s->tiles_d, s->kvec, s->kfactor, s->sk_fw, s->sk_ads, s->ds, s->ads_xyz,
+  void *ptrs[] = {s->d_uc, s->d_sys, s->fw64, s->fw64t, s->fw32, s->tiles_d, s->kvec, s->kfactor, s->sk_fw, s->sk_ads, s->ds, s->ads_xyz,
                   s->state, s->rec32, s->rec64, s->io_xyz,
-                  s->io_out, s->io_q, s->io_atom, s->io_excl, s->io_ov};
+                  s->io_out, s->io_q};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  if (s->h_call) cudaFreeHost(s->h_call);
   if (s->st) cudaStreamDestroy(s->st);
   delete s;
 }
@@ -456,6 +462,7 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
    * The two low bits of the z coordinate carry the atom's segment
    * (pseudo-atom type), an offset of at most 3 * L / 2^32 (< 1e-8 A). */
   std::vector<TileRec> tiles;
+  std::vector<double4> fw64t;
   {
     std::vector<int> seg_of(d->nfw);
     std::vector<double> fr((size_t)d->nfw * 3);
@@ -518,6 +525,7 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
       }
     }
     fw32.assign((size_t)ntile * RGPU_TILE, make_int4(0, 0, 0, 0));
+    fw64t.assign((size_t)ntile * RGPU_TILE, make_double4(0, 0, 0, 0));
     tiles.resize(ntile);
     for (int o = 0; o < ntile && tri; o++) {
       /* triclinic tile: fractional extents about the first atom (each
@@ -546,6 +554,7 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
         int qb;
         memcpy(&qb, &qf, 4);
         fw32[(size_t)RGPU_TILE * o + j] = make_int4(v[0], v[1], v[2], qb);
+        fw64t[(size_t)RGPU_TILE * o + j] = fw64[idx];
       }
       double cen[3], half[3], rad = 0.0;
       for (int c = 0; c < 3; c++) {
@@ -599,6 +608,7 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
         int qb;
         memcpy(&qb, &qf, 4);
         fw32[(size_t)RGPU_TILE * o + j] = make_int4(v[0], v[1], v[2], qb);
+        fw64t[(size_t)RGPU_TILE * o + j] = fw64[idx];
       }
       TileRec tr;
       double cen[3];
@@ -626,6 +636,18 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   }
   h.rc2 = d->cutoff * d->cutoff;
   h.rc2f = (float)h.rc2;
+  {
+    /* FP32 rounding and the fixed-point grid move a coordinate difference by
+     * less than 1e-6 of the box, a tile's box by less than 1e-5 A more */
+    double len = 0.0;
+    for (int c = 0; c < 3; c++) {
+      double l = d->box[c];
+      if (tri) l = fabs(h.hm[3 * c]) + fabs(h.hm[3 * c + 1]) + fabs(h.hm[3 * c + 2]);
+      len = std::max(len, l);
+    }
+    const double rp = d->cutoff + 1e-4 + 1e-6 * len;
+    h.rc2_pre = (float)(rp * rp * (1.0 + 1e-6));
+  }
   h.overlap = d->overlap;
   h.beta = d->beta;
   h.coulomb = d->coulomb;
@@ -727,6 +749,7 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   ALLOC(s->d_sys, sizeof(RgpuSys));
   if (tri) ALLOC(s->d_uc, sizeof(double) * 36);
   ALLOC(s->fw64, sizeof(double4) * d->nfw);
+  ALLOC(s->fw64t, sizeof(double4) * RGPU_TILE * (size_t)h.ntile);
   ALLOC(s->fw32, sizeof(int4) * RGPU_TILE * (size_t)h.ntile);
   ALLOC(s->tiles_d, sizeof(TileRec) * (size_t)h.ntile);
   ALLOC(s->kvec, sizeof(char4) * nk1);
@@ -748,11 +771,13 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   ALLOC(s->io_xyz, sizeof(double) * 3 * io_n);
   ALLOC(s->io_q, sizeof(double) * io_n);
   ALLOC(s->io_out, sizeof(double) * 4 * RGPU_MAX_POS);
-  ALLOC(s->io_atom, sizeof(int) * RGPU_MAX_POS);
-  ALLOC(s->io_excl, sizeof(int) * RGPU_MAX_POS);
-  ALLOC(s->io_ov, sizeof(int) * RGPU_MAX_POS);
 #undef ALLOC
+  if (cudaHostAlloc((void **)&s->h_call, sizeof(*s->h_call), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    sys_free(s);
+    return fail(RGPU_E_CUDA, "cudaHostAlloc");
+  }
   h.fw64 = s->fw64;
+  h.fw64t = s->fw64t;
   h.fw32 = s->fw32;
   h.tiles = s->tiles_d;
   h.kvec = s->kvec;
@@ -770,6 +795,7 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   int rc = RGPU_SUCCESS;
   do {
     if (cudaMemcpyAsync(s->fw64, fw64.data(), sizeof(double4) * d->nfw, cudaMemcpyHostToDevice, st) ||
+        cudaMemcpyAsync(s->fw64t, fw64t.data(), sizeof(double4) * RGPU_TILE * (size_t)h.ntile, cudaMemcpyHostToDevice, st) ||
         cudaMemcpyAsync(s->fw32, fw32.data(), sizeof(int4) * RGPU_TILE * (size_t)h.ntile, cudaMemcpyHostToDevice, st) ||
         cudaMemcpyAsync(s->tiles_d, tiles.data(), sizeof(TileRec) * (size_t)h.ntile, cudaMemcpyHostToDevice, st) ||
         cudaMemcpyAsync(s->state, &s->h_state, sizeof(RgpuState), cudaMemcpyHostToDevice, st) ||
@@ -916,16 +942,17 @@ extern "C" int rgpu_remove_molecule(rgpu_system *s, int m)
 static int bead_batch(rgpu_system *s, int precision, int n, const double *xyz, const int *atom, const int *excl,
                       int pair_check, double *out, int *ov)
 {
-  CK(cudaMemcpyAsync(s->io_xyz, xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s->st));
-  CK(cudaMemcpyAsync(s->io_atom, atom, sizeof(int) * n, cudaMemcpyHostToDevice, s->st));
-  CK(cudaMemcpyAsync(s->io_excl, excl, sizeof(int) * n, cudaMemcpyHostToDevice, s->st));
-  const int mixed = precision == RGPU_MIXED;
+  RgpuPoints in;
+  memcpy(in.xyz, xyz, sizeof(double) * 3 * n);
+  memcpy(in.atom, atom, sizeof(int) * n);
+  memcpy(in.excl, excl, sizeof(int) * n);
+  const int mixed = precision == RGPU_MIXED, grid = s->fw_model == RGPU_FRAMEWORK_GRID;
   const void *ads = mixed ? (const void *)s->rec32 : (const void *)s->rec64;
-  CK(rgpu_point_energies_launch(mixed, s->d_sys, ads, s->h_nmol * s->d.natom, s->io_xyz, s->io_atom, s->io_excl, n,
-                                pair_check, s->fw_model == RGPU_FRAMEWORK_GRID, s->io_out, s->io_ov, s->st));
-  CK(cudaMemcpyAsync(out, s->io_out, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, s->st));
-  if (ov) CK(cudaMemcpyAsync(ov, s->io_ov, sizeof(int) * n, cudaMemcpyDeviceToHost, s->st));
+  CK(rgpu_points_launch(mixed, s->d_sys, ads, s->h_nmol * s->d.natom, in, n, grid ? 0 : s->h.ntile, pair_check, grid,
+                        s->h_call->e, s->h_call->ov, s->st));
   CK(cudaStreamSynchronize(s->st));
+  memcpy(out, s->h_call->e, sizeof(double) * 4 * n);
+  if (ov) memcpy(ov, s->h_call->ov, sizeof(int) * n);
   return RGPU_SUCCESS;
 }
 

@@ -81,6 +81,15 @@ enum {
 /* NINT of src/utils.h:60 */
 __device__ __forceinline__ double rgpu_nint(double x) { return (double)(int)(x >= 0.0 ? x + 0.5 : x - 0.5); }
 
+/* x rounded to the nearest integer (ties to even; |x| < 2^51) by two
+ * additions: the minimum image of a pair at exactly half a box, where it and
+ * rgpu_nint differ, has the same distance */
+__device__ __forceinline__ double rgpu_round(double x)
+{
+  const double m = 6755399441055744.0;   /* 1.5 * 2^52 */
+  return (x + m) - m;
+}
+
 /* fixed-point form of a fractional coordinate f: f mod 1 in units of 2^-32 */
 __host__ __device__ inline int rgpu_fix_frac(double f)
 {
@@ -286,7 +295,7 @@ struct EvalPlan {
 
 /* nfw: framework items of the slice (tiles or atoms), nads: adsorbate atoms of
  * the slice, minitems: smallest worthwhile chunk of framework items */
-__device__ __forceinline__ EvalPlan eval_plan(int P, int nfw, int nads, int nwarps, int max_units, int minitems)
+__host__ __device__ __forceinline__ EvalPlan eval_plan(int P, int nfw, int nads, int nwarps, int max_units, int minitems)
 {
   EvalPlan pl;
   int target = nwarps;
@@ -695,6 +704,151 @@ __device__ __forceinline__ void unit_fw_fp64(const RgpuSys &S, const double4 *fw
   }
 }
 
+/* Whether tile `tr` can hold an atom closer than sqrt(rc2) to bead b (FP32;
+ * the tile's extents carry the margin for the rounding) */
+template <bool TRI>
+__device__ __forceinline__ bool tile_visible(const RgpuSys &S, const TileRec &tr, const BeadPos &b, float rc2)
+{
+  const int ix = tr.c.x - b.xi, iy = tr.c.y - b.yi, iz = tr.c.z - b.zi;
+  if (!TRI) {
+    const float dx = fmaxf(fabsf(__int2float_rn(ix) * S.fix_scale[0]) - tr.h.x, 0.0f);
+    const float dy = fmaxf(fabsf(__int2float_rn(iy) * S.fix_scale[1]) - tr.h.y, 0.0f);
+    const float dz = fmaxf(fabsf(__int2float_rn(iz) * S.fix_scale[2]) - tr.h.z, 0.0f);
+    return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < rc2;
+  }
+  /* triclinic tile: h = fractional half extents, h.w = Cartesian radius.
+   * Every atom's wrapped fractional offset along axis r is at least
+   * |t_r| - h_r, so it lies at least that many perpendicular widths away;
+   * when no atom can wrap differently from the centre (|t_r| + h_r < 1/2 on
+   * every axis), it also lies at least the centre's distance minus the
+   * radius away. */
+  const float tx = fabsf(__int2float_rn(ix) * 2.3283064365386963e-10f);
+  const float ty = fabsf(__int2float_rn(iy) * 2.3283064365386963e-10f);
+  const float tz = fabsf(__int2float_rn(iz) * 2.3283064365386963e-10f);
+  const float m = fmaxf(fmaxf((tx - tr.h.x) * S.wperp[0], (ty - tr.h.y) * S.wperp[1]), (tz - tr.h.z) * S.wperp[2]);
+  bool vis = !(m > 0.0f && m * m >= rc2);
+  if (vis && tx + tr.h.x < 0.5f && ty + tr.h.y < 0.5f && tz + tr.h.z < 0.5f) {
+    float dx, dy, dz;
+    rgpu_fix_to_cart_tri(S, ix, iy, iz, dx, dy, dz);
+    const float e = fmaxf(sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - tr.h.w, 0.0f);
+    vis = e * e < rc2;
+  }
+  return vis;
+}
+
+/* The LJ + real-space term of one preselected framework atom, FP64: entry =
+ * atom of the tiled order << 2 | segment */
+template <bool TRI>
+__device__ __forceinline__ void pair_fp64_queued(const RgpuSys &S, const double4 *fwd, int entry, const BeadPos &b,
+                                                 bool charged, double qa, bool check, double &av, double &ac, int &ov,
+                                                 int &nin, int &nch)
+{
+  const double4 f = fwd[entry >> 2];
+  double dx = b.x - f.x, dy = b.y - f.y, dz = b.z - f.z;
+  if (!TRI) {
+    dx -= S.box[0] * rgpu_round(dx * S.inv_box[0]);
+    dy -= S.box[1] * rgpu_round(dy * S.inv_box[1]);
+    dz -= S.box[2] * rgpu_round(dz * S.inv_box[2]);
+  } else {
+    rgpu_min_image_tri(S, dx, dy, dz);
+  }
+  const double r2 = dx * dx + dy * dy + dz * dz;
+  if (r2 < S.rc2) {
+    nin++;
+    const RgpuLJ P = S.lj_bf[b.atom][entry & 3];
+    double ri = 0.0, ir2;
+    if (charged) {
+      ri = rsqrt(r2);
+      ir2 = ri * ri;
+    } else {
+      ir2 = 1.0 / r2;
+    }
+    double s6 = P.sig2 * ir2;
+    s6 = s6 * s6 * s6;
+    const double u = P.eps4 * (s6 * (s6 - 1.0)) - P.shift;
+    av += u;
+    if (check && u >= S.overlap) ov = 1;
+    if (charged) {
+      nch++;
+      const double uc = qa * f.w * (erfc(S.alpha * (r2 * ri)) * ri);
+      ac += uc;
+      if (check && uc >= S.overlap) ov = 1;
+    }
+  }
+}
+
+/* Framework tiles [t0, t1) for bead b, FP64 path (warp-wide). Lanes cull 32
+ * tiles at once and visit the surviving ones two at a time, as
+ * unit_tiles_mixed does; an atom's FP32 fixed-point distance, tested against
+ * the cut-off with a margin, decides whether it is queued, and 32 queued
+ * atoms at a time get the FP64 distance, the exact cut-off test and the pair
+ * terms. So FP64 instructions are issued for atoms at the cut-off or inside
+ * it only, with every lane busy. queue: 64 ints of this warp, used as a
+ * ring. */
+template <bool TRI>
+__device__ __forceinline__ void unit_tiles_fp64(const RgpuSys &S, const int4 *fw, const double4 *fwd,
+                                                const TileRec *tiles, int t0, int t1, const BeadPos &b, bool check,
+                                                double &av, double &ac, int &ov, int &nin, int &nch, int &nvis,
+                                                int *queue)
+{
+  const int lane = threadIdx.x & 31;
+  const float sx = S.fix_scale[0], sy = S.fix_scale[1], sz = S.fix_scale[2];
+  const float rc2 = S.rc2_pre;
+  const double qa = S.mol_q[b.atom] * S.coulomb;
+  const bool charged = S.fw_charged && qa != 0.0;
+  const int half = lane >> 4, hl = lane & 15;
+  int head = 0, n = 0;                 /* ring: entries head .. head + n - 1 (mod 64) */
+  for (int tb = t0; tb < t1; tb += 32) {
+    bool vis = false;
+    int tn = 0;                        /* atoms of this lane's tile */
+    if (tb + lane < t1) {
+      const TileRec tr = tiles[tb + lane];
+      tn = tr.c.w;
+      vis = tile_visible<TRI>(S, tr, b, rc2);
+    }
+    unsigned m = __ballot_sync(RGPU_FULL, vis);
+    while (m) {
+      const int i1 = __ffs(m) - 1;
+      m &= m - 1;
+      const int i2 = m ? __ffs(m) - 1 : -1;
+      m &= m - 1;
+      const int n1 = __shfl_sync(RGPU_FULL, tn, i1);
+      const int n2s = __shfl_sync(RGPU_FULL, tn, i2 >= 0 ? i2 : 0);
+      const int n2 = i2 >= 0 ? n2s : 0;
+      nvis += n1 + n2;
+      const int a = (tb + (half ? i2 : i1)) * RGPU_TILE + hl;
+      bool in = false;
+      int seg = 0;
+      if (hl < (half ? n2 : n1)) {
+        const int4 f = fw[a];
+        seg = f.z & 3;
+        float dx, dy, dz;
+        if (!TRI) {
+          dx = __int2float_rn(f.x - b.xi) * sx;
+          dy = __int2float_rn(f.y - b.yi) * sy;
+          dz = __int2float_rn(f.z - b.zi) * sz;
+        } else {
+          rgpu_fix_to_cart_tri(S, f.x - b.xi, f.y - b.yi, f.z - b.zi, dx, dy, dz);
+        }
+        in = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < rc2;
+      }
+      const unsigned bal = __ballot_sync(RGPU_FULL, in);
+      if (in) queue[(head + n + __popc(bal & ((1u << lane) - 1u))) & 63] = a << 2 | seg;
+      n += __popc(bal);
+      __syncwarp();
+      if (n >= 32) {
+        pair_fp64_queued<TRI>(S, fwd, queue[(head + lane) & 63], b, charged, qa, check, av, ac, ov, nin, nch);
+        head = (head + 32) & 63;
+        n -= 32;
+        __syncwarp();
+      }
+    }
+  }
+  if (lane < n)
+    pair_fp64_queued<TRI>(S, fwd, queue[(head + lane) & 63], b, charged, qa, check, av, ac, ov, nin, nch);
+  __syncwarp();
+}
+
 template <bool TRI>
 __device__ __forceinline__ void unit_ads_mixed(const RgpuSys &S, const int4 *ads, const BeadPos &b, int lo,
                                                int hi, int exclude, bool check, float &av, float &ac, int &ov,
@@ -952,31 +1106,6 @@ __device__ __forceinline__ EvalPlan eval_units(const RgpuSys &S, const EvalSlice
     }
   }
   return pl;
-}
-
-/* Evaluates P bead positions over the slice; all threads of the block must
- * call it. Writes this slice's partial results to res/ovf. */
-template <int MIXED>
-__device__ void eval_positions(const RgpuSys &S, const EvalSlice &sl, const BeadPos *pos, int P, int pair_check,
-                               double (*res)[4], int *ovf, EvalScratch sc, int max_units)
-{
-  const EvalPlan pl = eval_units<MIXED>(S, sl, pos, P, pair_check, sc, max_units);
-  const int per = pl.cf + pl.ca;
-  __syncthreads();
-  if (threadIdx.x == 0) *sc.next = 0;
-  for (int p = threadIdx.x; p < P; p += blockDim.x) {
-    double hv = 0.0, hc = 0.0, av = 0.0, ac = 0.0;
-    int ov = 0;
-    for (int c = 0; c < per; c++) {
-      int u = p * per + c;
-      if (c < pl.cf) { hv += sc.uv[u]; hc += sc.uc[u]; }
-      else { av += sc.uv[u]; ac += sc.uc[u]; }
-      ov |= sc.uo[u];
-    }
-    res[p][0] = hv; res[p][1] = hc; res[p][2] = av; res[p][3] = ac;
-    ovf[p] = ov;
-  }
-  __syncthreads();
 }
 
 /* ------------------------------------------------------------------------ */

@@ -19,9 +19,9 @@ cudaError_t rgpu_engine_prepare(int mixed, bool wide, bool flex, size_t smem);
 cudaError_t rgpu_engine_launch(int mixed, RgpuSys *d_systems, int nsys, long long nsteps, int kw,
                                int max_ads_atoms, int fw_items, int tile_items, int k_items, int cluster,
                                int threads, bool wide, bool flex, cudaStream_t st);
-cudaError_t rgpu_point_energies_launch(int mixed, const RgpuSys *d_sys, const void *d_ads, int nads,
-                                       const double *d_xyz, const int *d_atom, const int *d_excl, int P,
-                                       int pair_check, int fw_grid, double *d_out, int *d_ov, cudaStream_t st);
+/* per-call entry points (percall.cu); d_out and d_ov in mapped host memory */
+cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ads, int nads, const RgpuPoints &in, int P,
+                               int ntile, int pair_check, int fw_grid, double *d_out, int *d_ov, cudaStream_t st);
 cudaError_t rgpu_ewald_delta_launch(int mixed, const RgpuSys *d_sys, const double *d_xyz, const double *d_q, int ns,
                                     double2 *d_ds, double *d_out, int kw, cudaStream_t st);
 cudaError_t rgpu_ewald_accept_launch(const RgpuSys *d_sys, const double2 *d_ds, int nk, cudaStream_t st);

@@ -104,6 +104,13 @@ typedef struct {
   float4 h;
 } TileRec;
 
+/* the positions of one per-call evaluation, passed by value to its kernel */
+typedef struct {
+  double xyz[RGPU_MAX_POS][3];
+  int atom[RGPU_MAX_POS];     /* index of the bead in the molecule */
+  int excl[RGPU_MAX_POS];     /* adsorbate molecule left out (-1: none) */
+} RgpuPoints;
+
 /* geometry of an energy grid: npts cells per axis over `size` from `shift`,
  * spanning a unit cell of lengths `cell`; a triclinic unit cell (tri = 1)
  * has its matrix (columns a, b, c; row-major) and then its inverse in
@@ -128,6 +135,8 @@ typedef struct RgpuSys {
   double hm[9], hinv[9];
   float hmf[9];
   float rc2f;
+  float rc2_pre;              /* rc2 with a margin for FP32 arithmetic on fixed-point positions: the FP64 path
+                               * culls and preselects with it, then tests its FP64 distance against rc2 */
   double rc2;                 /* VDW and real-space cut-off squared (equal) */
   double overlap;             /* EnergyOverlapCriteria */
   double beta;
@@ -179,6 +188,7 @@ typedef struct RgpuSys {
   const float *coul_grid;     /* Coulomb grid of a unit probe charge (rgpu_system_set_coulomb_grid) */
   /* device pointers */
   const double4 *fw64;        /* [nfw] x, y, z, q (sorted by type) */
+  const double4 *fw64t;       /* [ntile*RGPU_TILE] x, y, z, q in the order of fw32 */
   const int4 *fw32;           /* [ntile*RGPU_TILE] tiled: fixed-point x, y, z (low 2 bits of z = segment), float bits of q */
   const TileRec *tiles;       /* [ntile] */
   int ntile;

@@ -1,0 +1,61 @@
+"""Per-call kernels at the sizes where their work split changes, against the
+oracle: frameworks of one atom, one tile, a tile and an atom and more tiles
+than warps; one position up to the largest call; few and many adsorbates;
+orthorhombic and triclinic boxes.
+
+FP64: within 1e-9 of the result (the per-call parity bound) plus 1e-12 of the
+sum of the absolute pair terms (FP64 rounding of at most ~1e4 terms that
+cancel). Mixed (accuracy: test_gpu_parity): the same bits for a position in
+any call of five positions or more.
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from raspa2_b200 import native, systems
+
+pytestmark = pytest.mark.gpu
+
+
+def co2_box(atoms, tri):
+    s = systems.co2_system(seed=5, n_atoms=atoms, cell=26.5, kmax=3, layout="uniform")
+    if tri:
+        s = dataclasses.replace(s, unit_cell=np.array([29.0, 28.0, 30.0]), cell_angles=(80.0, 95.0, 110.0))
+    return s
+
+
+def molecules(rng, s, n):
+    u = rng.normal(size=(n, 1, 3))
+    u /= np.linalg.norm(u, axis=2, keepdims=True)
+    z = np.array([1.16, 0.0, -1.16])[None, :, None]
+    return s.box_point(rng.random((n, 1, 3))) + z * u
+
+
+@pytest.mark.parametrize("tri", [False, True])
+@pytest.mark.parametrize("atoms,nmol,n", [(1, 0, 1), (16, 1, 2), (17, 11, 7), (300, 90, 9), (700, 3, 19), (1100, 40, 64),
+                                          (33, 200, 33)])
+def test_points_at_split_edges(cuda, atoms, nmol, n, tri):
+    s = co2_box(atoms, tri)
+    rng = np.random.default_rng(atoms + n)
+    mols = molecules(rng, s, nmol)
+    g = native.GpuSystem(s, maxmol=256)
+    g.set_adsorbates(mols)
+    o = O.Oracle.from_system(s, maxmol=256)
+    o.set_molecules(mols)
+    # positions in and around the box, some in their neighbouring images
+    xyz = s.box_point(rng.uniform(-1.0, 2.0, (n, 3)))
+    atom = rng.integers(0, 3, n)
+    excl = rng.integers(-1, max(nmol, 1), n)
+    t, q = s.molecule_types(), s.molecule.charges()
+    ref = np.array([o.point(int(t[a]), float(q[a]), x, int(e)) for a, x, e in zip(atom, xyz, excl)])
+    scale = np.array([o.point_abs(int(t[a]), float(q[a]), x, int(e)) for a, x, e in zip(atom, xyz, excl)])
+    got = g.bead_energies(xyz, atom, excl, native.RGPU_FP64)
+    assert np.all(np.abs(got - ref) <= 1e-9 * np.abs(ref) + 1e-12 * scale + 1e-8)
+    # mixed: from five positions on a position's FP32 sums do not depend on the others of its call
+    if n >= 10:
+        got = g.bead_energies(xyz, atom, excl, native.RGPU_MIXED)
+        h = n // 2
+        parts = [g.bead_energies(xyz[k], atom[k], excl[k], native.RGPU_MIXED) for k in (slice(0, h), slice(h, n))]
+        np.testing.assert_array_equal(got, np.concatenate(parts))
