@@ -1263,6 +1263,14 @@ extern "C" int rgpu_total_energy(rgpu_system *s, double *out)
 }
 
 /* ---------------------------------------------------------------------- */
+/* smallest perpendicular width of the box less the cut-off */
+static double grid_reach(const rgpu_system *s)
+{
+  double w[3] = {s->d.box[0], s->d.box[1], s->d.box[2]};
+  if (s->h.triclinic) perpendicular_widths(s->h.hm, w);
+  return std::min(w[0], std::min(w[1], w[2])) - s->d.cutoff;
+}
+
 extern "C" int rgpu_grid_build(rgpu_system *s, int type, const int npts[3], const double size[3], const double shift[3],
                                float *d_grid)
 {
@@ -1279,7 +1287,7 @@ extern "C" int rgpu_grid_build(rgpu_system *s, int type, const int npts[3], cons
     lj[sg].sig2 = s->lj_sig2[ij];
     lj[sg].shift = s->lj_shift[ij];
   }
-  CK(rgpu_grid_build_launch_lj(s->d_sys, lj, npts, size, shift, d_grid, s->st));
+  CK(rgpu_grid_build_launch(s->d_sys, lj, grid_reach(s), npts, size, shift, d_grid, s->st));
   CK(cudaStreamSynchronize(s->st));
   return RGPU_SUCCESS;
 }
@@ -1292,7 +1300,7 @@ extern "C" int rgpu_grid_build_coulomb(rgpu_system *s, const int npts[3], const 
   if (!s->h.ewald) return fail(RGPU_E_INVALID, "a Coulomb grid needs Ewald summation");
   for (int c = 0; c < 3; c++)
     if (npts[c] < 1) return fail(RGPU_E_INVALID, "npts");
-  CK(rgpu_grid_build_launch_coulomb(s->d_sys, npts, size, shift, d_grid, s->st));
+  CK(rgpu_grid_build_launch(s->d_sys, nullptr, grid_reach(s), npts, size, shift, d_grid, s->st));
   CK(cudaStreamSynchronize(s->st));
   return RGPU_SUCCESS;
 }

@@ -5,8 +5,9 @@
  * LJ branch of PotentialThirdDerivative (src/potentials.c:10959-10990),
  * computed in FP64 and stored as FP32 like the reference. One thread per grid
  * point; a block covers a 4x8x8 tile and stages, chunk by chunk, only the
- * framework atoms within cutoff + tile radius of the tile centre in shared
- * memory, so each thread visits ~1/7 of the framework at 0.1 A spacing.
+ * images of framework atoms within cutoff + tile radius of the tile centre in
+ * shared memory, so each thread visits ~1/7 of the framework at 0.1 A spacing
+ * and forms no minimum image.
  *
  * Device layout is point-major: grid[((i*(ny+1) + j)*(nz+1) + k)*8 + m], so
  * the 8 values of a corner are one 32-byte sector and a lookup gathers eight
@@ -39,18 +40,143 @@ struct GridParams {
   RgpuLJ lj[RGPU_MAX_FWTYPES];
 };
 
+#define GRID_STAGE (2 * GRID_THREADS)   /* staged images of one round of atoms */
+
+/* 1/x by two Newton iterations from the hardware's approximation (relative
+ * error 2^-20 or better, squared by each); below 1e-60, where a grid point
+ * sits on an atom, by the division */
+__device__ __forceinline__ double grid_reciprocal(double x)
+{
+  if (x < 1e-60) return 1.0 / x;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+/* Staged images: position and framework charge (Coulomb) or LJ shift, and
+ * the LJ parameters 4 eps, sigma^2 */
+struct GridStage {
+  double4 xyz[GRID_STAGE];
+  double2 lj[GRID_STAGE];
+  int wcount[GRID_THREADS / 32];
+};
+
+/* Stages the images of atoms base .. base + GRID_THREADS within reach of the
+ * tile about (cx, cy, cz), those numbered s0 .. s0 + GRID_STAGE in thread
+ * order; returns how many there are in all. Contains a block barrier; the
+ * caller puts one before the stage is read. */
+template <bool COUL, bool IMAGES>
+__device__ __forceinline__ int grid_stage(const RgpuSys &S, const GridParams &gp, GridStage &st, int base, int s0,
+                                          double cx, double cy, double cz, double rcut2)
+{
+  const int a = base + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  /* this thread's atom: the images within reach, as a mask over the 8
+   * choices of nearest or next image along the cell vectors */
+  unsigned keep = 0;
+  double4 f = make_double4(0, 0, 0, 0);
+  double d[3] = {0, 0, 0}, step[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+  if (a < S.nfw) {
+    f = S.fw64[a];
+    if (!IMAGES) {
+      keep = 1;
+    } else {
+      const double c[3] = {cx - f.x, cy - f.y, cz - f.z};
+      if (!S.triclinic) {
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          d[r] = c[r] - S.box[r] * rgpu_round(c[r] * S.inv_box[r]);
+          step[r][r] = d[r] > 0.0 ? -S.box[r] : S.box[r];
+        }
+      } else {
+        double t[3];
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          const double u = S.hinv[3 * r] * c[0] + S.hinv[3 * r + 1] * c[1] + S.hinv[3 * r + 2] * c[2];
+          t[r] = u - rgpu_round(u);
+        }
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          d[r] = S.hm[3 * r] * t[0] + S.hm[3 * r + 1] * t[1] + S.hm[3 * r + 2] * t[2];
+#pragma unroll
+          for (int q = 0; q < 3; q++) step[q][r] = t[q] > 0.0 ? -S.hm[3 * r + q] : S.hm[3 * r + q];
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 8; m++) {
+        double r2 = 0.0;
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          const double v = d[r] + (m & 1 ? step[0][r] : 0.0) + (m & 2 ? step[1][r] : 0.0) + (m & 4 ? step[2][r] : 0.0);
+          r2 += v * v;
+        }
+        if (r2 < rcut2) keep |= 1u << m;
+      }
+    }
+  }
+  const int mine = __popc(keep);
+  int incl = mine;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const int y = __shfl_up_sync(RGPU_FULL, incl, s);
+    if (lane >= s) incl += y;
+  }
+  if (lane == 31) st.wcount[w] = incl;
+  __syncthreads();
+  int pos = incl - mine - s0, nsel = 0;
+#pragma unroll
+  for (int q = 0; q < GRID_THREADS / 32; q++) {
+    if (q < w) pos += st.wcount[q];
+    nsel += st.wcount[q];
+  }
+  if (keep) {
+    int seg = 0;
+    while (seg + 1 < S.nseg && a >= S.seg_start[seg + 1]) seg++;
+    const double2 lj = make_double2(gp.lj[seg].eps4, gp.lj[seg].sig2);
+    const double v = COUL ? f.w : gp.lj[seg].shift;
+    for (unsigned m = keep; m; m &= m - 1, pos++) {
+      if (pos < 0 || pos >= GRID_STAGE) continue;
+      const int c = __ffs(m) - 1;
+      double4 g = make_double4(f.x, f.y, f.z, v);
+      if (IMAGES) {
+        g.x = cx - (d[0] + (c & 1 ? step[0][0] : 0.0) + (c & 2 ? step[1][0] : 0.0) + (c & 4 ? step[2][0] : 0.0));
+        g.y = cy - (d[1] + (c & 1 ? step[0][1] : 0.0) + (c & 2 ? step[1][1] : 0.0) + (c & 4 ? step[2][1] : 0.0));
+        g.z = cz - (d[2] + (c & 1 ? step[0][2] : 0.0) + (c & 2 ? step[1][2] : 0.0) + (c & 4 ? step[2][2] : 0.0));
+      }
+      st.xyz[pos] = g;
+      if (!COUL) st.lj[pos] = lj;
+    }
+  }
+  return nsel;
+}
+
 /* COUL = false: the LJ grid of one probe pseudo-atom (gp.lj by framework
  * segment). COUL = true: the real-space Ewald (Coulomb) grid of a unit probe
  * charge, CalculateDerivativesAtPositionReal (src/framework_hessian.c:111-180)
  * with the framework charges, capped where the value exceeds the overlap
- * criterion or a framework atom is closer than 1 A (src/grids.c:656-668). */
-template <bool COUL>
-__global__ void __launch_bounds__(GRID_THREADS) k_grid_build(const RgpuSys *sysp, GridParams gp, float *grid)
+ * criterion or a framework atom is closer than 1 A (src/grids.c:656-668).
+ *
+ * The kernel is bound by FP64 instructions, one (point, staged image) pair at a
+ * time, so a pair is kept short: the images are staged about the tile's centre
+ * (no rounding to the nearest image per pair), LJ has one reciprocal by
+ * Newton's iteration, the Coulomb term one rsqrt and one exponential, which
+ * its erfc = exp(-x^2) erfcx(x) shares. 64 and 80 registers keep 32 and 24
+ * warps on an SM; with the compiler's choice (94, 116) there were 16 and the
+ * dependent FP64 instructions left the pipe half idle. 102^3 points over 4096
+ * atoms in a 40 A cell, LJ: 2.28 ms, 12.9 TFLOP/s at 60 FLOP a pair inside the
+ * cut-off (5.78 ms with a rounding per pair and axis and four divisions; 3.06
+ * at 94 registers). 78^3 points over 1536 atoms, Coulomb: 4.02 ms (6.76; 4.71).
+ * IMAGES: every image of an atom within reach of the tile is, along each cell
+ * vector, its nearest to the tile's centre or the next one
+ * (cutoff + tile radius below every perpendicular width); all of those within
+ * reach are staged, and at most one of an atom's is inside the cut-off of a
+ * point, because the widths are at least twice the cut-off. Otherwise (grids
+ * coarser than about 2 A) the atoms are staged as they are and each pair takes
+ * its minimum image. */
+template <bool COUL, bool IMAGES>
+__global__ void __launch_bounds__(GRID_THREADS, COUL ? 3 : 4) k_grid_build(const RgpuSys *sysp, GridParams gp, float *grid)
 {
-  __shared__ double4 fwc[GRID_THREADS];
-  __shared__ int segc[GRID_THREADS];
-  __shared__ int wcount[GRID_THREADS / 32];
-  __shared__ int nsel;
+  __shared__ GridStage st;
   const RgpuSys &S = *sysp;
   const int nx = gp.npts[0] + 1, ny = gp.npts[1] + 1, nz = gp.npts[2] + 1;
   const int tilesz = (nz + GRID_TZ - 1) / GRID_TZ, tilesy = (ny + GRID_TY - 1) / GRID_TY;
@@ -71,95 +197,71 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid_build(const RgpuSys *sysp
   const double hx = 0.5 * (GRID_TX - 1) * gp.delta[0], hy = 0.5 * (GRID_TY - 1) * gp.delta[1],
                hz = 0.5 * (GRID_TZ - 1) * gp.delta[2];
   const double rcut = sqrt(S.rc2) + sqrt(hx * hx + hy * hy + hz * hz) + 1e-6;
-  const double rcut2 = rcut * rcut;
-  const double Lx = S.box[0], Ly = S.box[1], Lz = S.box[2];
-  const double ix = S.inv_box[0], iy = S.inv_box[1], iz = S.inv_box[2];
+  const double rc2 = S.rc2;
   double o[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   double rmin2 = 1e300;
-  const double a2 = S.alpha * S.alpha, two_a_sqrtpi = 2.0 * S.alpha / sqrt(M_PI);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int base = 0; base < S.nfw; base += GRID_THREADS) {
-    const int a = base + threadIdx.x;
-    int keep = 0;
-    double4 f = make_double4(0, 0, 0, 0);
-    int seg = 0;
-    if (a < S.nfw) {
-      f = S.fw64[a];
-      if (S.triclinic) {
-        /* a triclinic box: every atom is staged (its minimum image may
-         * differ across the tile's points near half a cell vector) */
-        keep = 1;
-      } else {
-        double dx = cx - f.x, dy = cy - f.y, dz = cz - f.z;
-        dx -= Lx * rgpu_nint(dx * ix);
-        dy -= Ly * rgpu_nint(dy * iy);
-        dz -= Lz * rgpu_nint(dz * iz);
-        keep = dx * dx + dy * dy + dz * dz < rcut2;
-      }
-      while (seg + 1 < S.nseg && a >= S.seg_start[seg + 1]) seg++;
-    }
-    unsigned m = __ballot_sync(RGPU_FULL, keep);
-    if (lane == 0) wcount[w] = __popc(m);
+  const double alpha = S.alpha, a2 = alpha * alpha, two_a_sqrtpi = 2.0 * alpha / sqrt(M_PI), coulomb = S.coulomb;
+  const int nfw = S.nfw;
+  int s0 = 0;
+  for (int base = 0; base < nfw;) {
+    const int nsel = grid_stage<COUL, IMAGES>(S, gp, st, base, s0, cx, cy, cz, rcut * rcut);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int s = 0;
-      for (int q = 0; q < GRID_THREADS / 32; q++) { int c = wcount[q]; wcount[q] = s; s += c; }
-      nsel = s;
-    }
-    __syncthreads();
-    if (keep) {
-      int pos = wcount[w] + __popc(m & ((1u << lane) - 1u));
-      fwc[pos] = f;
-      segc[pos] = seg;
-    }
-    __syncthreads();
-    if (valid) {
-      for (int q = 0; q < nsel; q++) {
-        const double4 g = fwc[q];
-        double dx = px - g.x, dy = py - g.y, dz = pz - g.z;
+    const int n = min(nsel - s0, GRID_STAGE);
+    for (int q = 0; valid && q < n; q++) {
+      const double4 g = st.xyz[q];
+      double dx = px - g.x, dy = py - g.y, dz = pz - g.z;
+      if (!IMAGES) {
         if (S.triclinic) {
           rgpu_min_image_tri(S, dx, dy, dz);
         } else {
-          dx -= Lx * rgpu_nint(dx * ix);
-          dy -= Ly * rgpu_nint(dy * iy);
-          dz -= Lz * rgpu_nint(dz * iz);
+          dx -= S.box[0] * rgpu_round(dx * S.inv_box[0]);
+          dy -= S.box[1] * rgpu_round(dy * S.inv_box[1]);
+          dz -= S.box[2] * rgpu_round(dz * S.inv_box[2]);
         }
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 < S.rc2) {
-          double U, DF, DDF, DDDF;
-          if (COUL) {
-            /* f(r) = K q erfc(a r) / r; DF = f'/r, DDF = (f'' - f'/r)/r^2,
-             * DDDF = the r-part of the mixed third derivative */
-            rmin2 = fmin(rmin2, r2);
-            const double r = sqrt(r2), kq = S.coulomb * g.w;
-            const double e = erfc(S.alpha * r), gr = two_a_sqrtpi * r * exp(-a2 * r2);
-            const double ar2 = a2 * r2;
-            U = kq * e / r;
-            DF = -kq * (gr + e) / (r * r2);
-            DDF = kq * (gr * (3.0 + 2.0 * ar2) + 3.0 * e) / (r2 * r2 * r);
-            DDDF = -kq * (gr * (15.0 + 10.0 * ar2 + 4.0 * ar2 * ar2) + 15.0 * e) / (r2 * r2 * r2 * r);
-          } else {
-            const RgpuLJ P = gp.lj[segc[q]];
-            const double eps = 0.25 * P.eps4;
-            double r3 = P.sig2 / r2;
-            r3 = r3 * r3 * r3;
-            U = 4.0 * eps * (r3 * (r3 - 1.0)) - P.shift;
-            DF = 24.0 * eps * (r3 * (1.0 - 2.0 * r3)) / r2;
-            DDF = 96.0 * eps * (r3 * (7.0 * r3 - 2.0)) / (r2 * r2);
-            DDDF = 384.0 * eps * (r3 * (5.0 - 28.0 * r3)) / (r2 * r2 * r2 * r2);
-          }
-          o[0] += U;
-          o[1] += dx * DF;
-          o[2] += dy * DF;
-          o[3] += dz * DF;
-          o[4] += DDF * dx * dy;
-          o[5] += DDF * dx * dz;
-          o[6] += DDF * dy * dz;
-          o[7] += DDDF * dx * dy * dz;
+      }
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      if (r2 < rc2) {
+        double U, DF, DDF, DDDF;
+        if (COUL) {
+          /* f(r) = K q erfc(a r) / r; DF = f'/r, DDF = (f'' - f'/r)/r^2,
+           * DDDF = the r-part of the mixed third derivative */
+          rmin2 = fmin(rmin2, r2);
+          const double ri = rsqrt(r2), r = r2 * ri, ri2 = ri * ri, ar2 = a2 * r2;
+          const double x2 = exp(-ar2), e = x2 * erfcx(alpha * r), gr = two_a_sqrtpi * r * x2;
+          const double c1 = coulomb * g.w * ri, c3 = c1 * ri2, c5 = c3 * ri2;
+          U = c1 * e;
+          DF = -c3 * (gr + e);
+          DDF = c5 * (gr * (3.0 + 2.0 * ar2) + 3.0 * e);
+          DDDF = -c5 * ri2 * (gr * (15.0 + ar2 * (10.0 + 4.0 * ar2)) + 15.0 * e);
+        } else {
+          const double2 P = st.lj[q];
+          const double i2 = grid_reciprocal(r2), i4 = i2 * i2;
+          double r3 = P.y * i2;
+          r3 = r3 * r3 * r3;
+          const double v = P.x * r3;
+          U = v * (r3 - 1.0) - g.w;
+          DF = v * i2 * (6.0 - 12.0 * r3);
+          DDF = v * i4 * (168.0 * r3 - 48.0);
+          DDDF = v * (i4 * i4) * (480.0 - 2688.0 * r3);
         }
+        const double xy = dx * dy;
+        o[0] += U;
+        o[1] += dx * DF;
+        o[2] += dy * DF;
+        o[3] += dz * DF;
+        o[4] += DDF * xy;
+        o[5] += DDF * (dx * dz);
+        o[6] += DDF * (dy * dz);
+        o[7] += DDDF * (xy * dz);
       }
     }
     __syncthreads();
+    /* as a rule one pass a round; more where it has more images than the stage holds */
+    s0 += GRID_STAGE;
+    if (s0 >= nsel) {
+      s0 = 0;
+      base += GRID_THREADS;
+    }
   }
   if (!valid) return;
   /* cap, src/grids.c:546-563 (Coulomb: also within 1 A of an atom, :656-668) */
@@ -180,29 +282,12 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid_build(const RgpuSys *sysp
   dst[1] = v1;
 }
 
-/* lj[s]: LJ parameters of the probe pseudo-atom with framework segment s */
-cudaError_t rgpu_grid_build_launch_lj(const RgpuSys *d_sys, const RgpuLJ *lj, const int npts[3], const double size[3],
-                                      const double shift[3], float *d_grid, cudaStream_t st)
-{
-  GridParams gp;
-  for (int c = 0; c < 3; c++) {
-    gp.npts[c] = npts[c];
-    gp.size[c] = size[c];
-    gp.shift[c] = shift[c];
-    gp.delta[c] = size[c] / (double)npts[c];
-  }
-  for (int s = 0; s < RGPU_MAX_FWTYPES; s++) gp.lj[s] = lj[s];
-  const int nx = npts[0] + 1, ny = npts[1] + 1, nz = npts[2] + 1;
-  const long long blocks = (long long)((nx + GRID_TX - 1) / GRID_TX) * ((ny + GRID_TY - 1) / GRID_TY) *
-                           ((nz + GRID_TZ - 1) / GRID_TZ);
-  if (blocks > 2147483647LL) return cudaErrorInvalidValue;
-  k_grid_build<false><<<(unsigned)blocks, GRID_THREADS, 0, st>>>(d_sys, gp, d_grid);
-  return cudaGetLastError();
-}
-
-/* the Coulomb grid of a unit probe charge */
-cudaError_t rgpu_grid_build_launch_coulomb(const RgpuSys *d_sys, const int npts[3], const double size[3],
-                                           const double shift[3], float *d_grid, cudaStream_t st)
+/* lj[s]: LJ parameters of the probe pseudo-atom with framework segment s;
+ * nullptr: the Coulomb grid of a unit probe charge. reach: the box's smallest
+ * perpendicular width less the cut-off, the largest tile radius for which
+ * atoms are staged as images. */
+cudaError_t rgpu_grid_build_launch(const RgpuSys *d_sys, const RgpuLJ *lj, double reach, const int npts[3],
+                                   const double size[3], const double shift[3], float *d_grid, cudaStream_t st)
 {
   GridParams gp = {};
   for (int c = 0; c < 3; c++) {
@@ -211,11 +296,21 @@ cudaError_t rgpu_grid_build_launch_coulomb(const RgpuSys *d_sys, const int npts[
     gp.shift[c] = shift[c];
     gp.delta[c] = size[c] / (double)npts[c];
   }
+  for (int s = 0; lj && s < RGPU_MAX_FWTYPES; s++) gp.lj[s] = lj[s];
   const int nx = npts[0] + 1, ny = npts[1] + 1, nz = npts[2] + 1;
   const long long blocks = (long long)((nx + GRID_TX - 1) / GRID_TX) * ((ny + GRID_TY - 1) / GRID_TY) *
                            ((nz + GRID_TZ - 1) / GRID_TZ);
   if (blocks > 2147483647LL) return cudaErrorInvalidValue;
-  k_grid_build<true><<<(unsigned)blocks, GRID_THREADS, 0, st>>>(d_sys, gp, d_grid);
+  const double h[3] = {0.5 * (GRID_TX - 1) * gp.delta[0], 0.5 * (GRID_TY - 1) * gp.delta[1],
+                       0.5 * (GRID_TZ - 1) * gp.delta[2]};
+  const bool images = sqrt(h[0] * h[0] + h[1] * h[1] + h[2] * h[2]) < reach - 1e-3;
+  if (lj) {
+    if (images) k_grid_build<false, true><<<(unsigned)blocks, GRID_THREADS, 0, st>>>(d_sys, gp, d_grid);
+    else k_grid_build<false, false><<<(unsigned)blocks, GRID_THREADS, 0, st>>>(d_sys, gp, d_grid);
+  } else {
+    if (images) k_grid_build<true, true><<<(unsigned)blocks, GRID_THREADS, 0, st>>>(d_sys, gp, d_grid);
+    else k_grid_build<true, false><<<(unsigned)blocks, GRID_THREADS, 0, st>>>(d_sys, gp, d_grid);
+  }
   return cudaGetLastError();
 }
 

@@ -66,3 +66,37 @@ def test_interpolation_matches_reference(grid):
     pts = np.array(c["interp_points"])
     got = native.grid_interpolate(buf.data_ptr(), m["n"], m["size"], m["shift"], m["cell"], pts)
     np.testing.assert_allclose(got, c["interp_ref"], rtol=2e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("tri", [False, True])
+@pytest.mark.parametrize("npts,coulomb", [((1, 1, 1), False), ((3, 9, 17), False), ((24, 5, 31), True), ((15, 40, 23), False),
+                                          ((2, 3, 2), True)])
+def test_grid_build_paths_match_oracle(cuda, npts, coulomb, tri):
+    """Grids from one cell to fine ones, over staged images and (tile radius beyond the box's reach) over minimum
+    images, in the smallest box the cut-off allows, against the oracle's derivatives at every point: FP32 storage
+    (6e-8 relative of a value; twice for the products with the FP32 spacings), and where terms cancel 1e-6 of an
+    internal energy unit plus 1e-13 of the plane's largest value (FP64 rounding of its terms)."""
+    import dataclasses
+    import torch
+    s = systems.co2_system(seed=9, n_atoms=150, cell=24.0001, kmax=3, layout="uniform")
+    size, shift = np.array([24.0001] * 3), np.zeros(3)
+    if tri:
+        s = dataclasses.replace(s, unit_cell=np.array([26.5, 26.4, 25.0]), cell_angles=(80.0, 95.0, 110.0))
+        m = s.unit_cell_matrix
+        size, shift = np.abs(m).sum(axis=1), np.minimum(m, 0.0).sum(axis=1)
+    g = native.GpuSystem(s, maxmol=4)
+    o = O.Oracle.from_system(s, maxmol=4)
+    n = np.array(npts, np.int32)
+    buf = torch.zeros(int(np.prod(n + 1)) * 8, dtype=torch.float32, device="cuda")
+    t = systems.TYPE_ORDER.index("O_co2")
+    if coulomb:
+        g.grid_build_coulomb(n, size, shift, buf.data_ptr())
+        ref = o.grid_build_coulomb(n, size, shift)
+    else:
+        g.grid_build(t, n, size, shift, buf.data_ptr())
+        ref = o.grid_build(t, n, size, shift)
+    torch.cuda.synchronize()
+    got = np.moveaxis(buf.cpu().numpy().reshape(tuple(n + 1) + (8,)), 3, 0).reshape(8, -1).astype(np.float64)
+    ref = np.asarray(ref, np.float64).reshape(8, -1)
+    top = np.abs(ref).max(axis=1, keepdims=True)
+    assert np.all(np.abs(got - ref) <= 2e-7 * np.abs(ref) + 1e-6 + 1e-13 * top)
