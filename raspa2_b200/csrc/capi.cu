@@ -80,13 +80,14 @@ struct rgpu_system {
   int *status;
   int4 *rec32;
   void *rec64;
-  /* per-call scratch */
-  double *io_xyz, *io_out, *io_q;
+  double *io_xyz, *io_q;      /* the framework as the caller orders it, for S_fw(k) */
   /* results of a per-call evaluation: mapped host memory that its kernel
    * writes, so that a call costs a launch and a wait */
   struct CallOut {
     double e[4 * RGPU_MAX_POS];
     int ov[RGPU_MAX_POS];
+    double total[5 * RGPU_TOTAL_CTAS];
+    double fourier[2 * 128];   /* blocks of 256 wave vectors; kmax <= 20 has under 20000 */
   } *h_call;
   /* host mirrors */
   RgpuState h_state;          /* initial state at creation; last state read */
@@ -184,8 +185,7 @@ static void sys_free(rgpu_system *s)
 {
   if (!s) return;
   void *ptrs[] = {s->d_uc, s->d_sys, s->fw64, s->fw64t, s->fw32, s->tiles_d, s->kvec, s->kfactor, s->sk_fw, s->sk_ads, s->ds, s->ads_xyz,
-                  s->state, s->rec32, s->rec64, s->io_xyz,
-                  s->io_out, s->io_q};
+                  s->state, s->rec32, s->rec64, s->io_xyz, s->io_q};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (s->h_call) cudaFreeHost(s->h_call);
@@ -268,7 +268,7 @@ static void kvectors(const rgpu_system_desc *d, std::vector<char4> &kv, std::vec
 static int upload_records(rgpu_system *s)
 {
   const int nads = s->h_nmol * s->d.natom;
-  CK(rgpu_records_launch(s->d_sys, nads, s->rec32, s->rec64, s->st));
+  CK(rgpu_records_launch(s->d_sys, nads, -1, s->rec32, s->rec64, s->st));
   s->records_stale = 0;
   return RGPU_SUCCESS;
 }
@@ -767,10 +767,8 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   s->status = &s->state->status;
   ALLOC(s->rec32, sizeof(int4) * nads);
   ALLOC(s->rec64, 32 * nads);
-  const size_t io_n = std::max((size_t)RGPU_MAX_POS, std::max((size_t)d->nfw, nads));
-  ALLOC(s->io_xyz, sizeof(double) * 3 * io_n);
-  ALLOC(s->io_q, sizeof(double) * io_n);
-  ALLOC(s->io_out, sizeof(double) * 4 * RGPU_MAX_POS);
+  ALLOC(s->io_xyz, sizeof(double) * 3 * d->nfw);
+  ALLOC(s->io_q, sizeof(double) * d->nfw);
 #undef ALLOC
   if (cudaHostAlloc((void **)&s->h_call, sizeof(*s->h_call), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
     sys_free(s);
@@ -831,23 +829,6 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   return RGPU_SUCCESS;
 }
 
-static int recompute_sk_ads(rgpu_system *s)
-{
-  const int nads = s->h_nmol * s->d.natom;
-  if (!s->h.nk) return RGPU_SUCCESS;
-  if (nads == 0) {
-    CK(cudaMemsetAsync(s->sk_ads, 0, sizeof(double2) * s->h.nk, s->st));
-    return RGPU_SUCCESS;
-  }
-  std::vector<double> q(nads);
-  for (int i = 0; i < nads; i++) q[i] = s->h.mol_q[i % s->d.natom];
-  CK(cudaMemcpyAsync(s->io_xyz, s->h_xyz.data(), sizeof(double) * 3 * nads, cudaMemcpyHostToDevice, s->st));
-  CK(cudaMemcpyAsync(s->io_q, q.data(), sizeof(double) * nads, cudaMemcpyHostToDevice, s->st));
-  CK(rgpu_structure_factor_launch(s->d_sys, s->io_xyz, s->io_q, nads, s->h.nk, s->sk_ads, s->st));
-  CK(cudaStreamSynchronize(s->st));
-  return RGPU_SUCCESS;
-}
-
 extern "C" int rgpu_set_adsorbates(rgpu_system *s, int nmol, const double *xyz)
 {
   if (!s || nmol < 0 || (nmol > 0 && !xyz)) return fail(RGPU_E_INVALID, "bad argument");
@@ -855,14 +836,12 @@ extern "C" int rgpu_set_adsorbates(rgpu_system *s, int nmol, const double *xyz)
   const size_t n = (size_t)nmol * s->d.natom * 3;
   s->h_xyz.assign(xyz, xyz + n);
   s->h_nmol = nmol;
-  if (n) CK(cudaMemcpyAsync(s->ads_xyz, s->h_xyz.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
-  CK(cudaMemcpyAsync(s->nmol, &s->h_nmol, sizeof(int), cudaMemcpyHostToDevice, s->st));
   s->net_ads = nmol * s->h.mol_charge;
   s->pending_dq = 0.0;
-  int rc = upload_records(s);
-  if (rc) return rc;
-  rc = recompute_sk_ads(s);
-  if (rc) return rc;
+  if (n) CK(cudaMemcpyAsync(s->ads_xyz, s->h_xyz.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
+  CK(rgpu_records_launch(s->d_sys, nmol * s->d.natom, nmol, s->rec32, s->rec64, s->st));
+  s->records_stale = 0;
+  CK(rgpu_structure_factor_launch(s->d_sys, s->ads_xyz, nullptr, nmol * s->d.natom, s->h.nk, s->sk_ads, s->st));
   CK(cudaStreamSynchronize(s->st));
   return RGPU_SUCCESS;
 }
@@ -880,12 +859,17 @@ extern "C" int rgpu_get_adsorbates(rgpu_system *s, int *nmol, double *xyz, int c
   return RGPU_SUCCESS;
 }
 
+/* puts xyz in molecule slot m (none for m < 0) and the molecule count h_nmol
+ * on the device, with the slot's records */
 static int write_molecule(rgpu_system *s, int m, const double *xyz)
 {
   const int na = s->d.natom;
-  memcpy(&s->h_xyz[(size_t)m * na * 3], xyz, sizeof(double) * 3 * na);
-  CK(cudaMemcpyAsync(s->ads_xyz + (size_t)m * na * 3, &s->h_xyz[(size_t)m * na * 3], sizeof(double) * 3 * na,
-                     cudaMemcpyHostToDevice, s->st));
+  RgpuSites in;
+  if (m >= 0) {
+    memcpy(&s->h_xyz[(size_t)m * na * 3], xyz, sizeof(double) * 3 * na);
+    memcpy(in.xyz, xyz, sizeof(double) * 3 * na);
+  }
+  CK(rgpu_set_molecule_launch(s->d_sys, in, m, s->h_nmol, s->rec32, s->rec64, s->st));
   return RGPU_SUCCESS;
 }
 
@@ -895,9 +879,7 @@ extern "C" int rgpu_update_molecule(rgpu_system *s, int m, const double *xyz)
   int rc = refresh_from_device(s);
   if (rc) return rc;
   if (m < 0 || m >= s->h_nmol) return fail(RGPU_E_INVALID, "molecule %d", m);
-  rc = write_molecule(s, m, xyz);
-  if (rc) return rc;
-  return upload_records(s);
+  return write_molecule(s, m, xyz);
 }
 
 extern "C" int rgpu_insert_molecule(rgpu_system *s, const double *xyz)
@@ -907,11 +889,8 @@ extern "C" int rgpu_insert_molecule(rgpu_system *s, const double *xyz)
   if (rc) return rc;
   if (s->h_nmol >= s->d.maxmol) return fail(RGPU_E_CAPACITY, "maxmol %d reached", s->d.maxmol);
   s->h_xyz.resize((size_t)(s->h_nmol + 1) * s->d.natom * 3);
-  rc = write_molecule(s, s->h_nmol, xyz);
-  if (rc) return rc;
   s->h_nmol++;
-  CK(cudaMemcpyAsync(s->nmol, &s->h_nmol, sizeof(int), cudaMemcpyHostToDevice, s->st));
-  rc = upload_records(s);
+  rc = write_molecule(s, s->h_nmol - 1, xyz);
   if (rc) return rc;
   CK(cudaStreamSynchronize(s->st));
   return RGPU_SUCCESS;
@@ -924,16 +903,12 @@ extern "C" int rgpu_remove_molecule(rgpu_system *s, int m)
   if (rc) return rc;
   if (m < 0 || m >= s->h_nmol) return fail(RGPU_E_INVALID, "molecule %d", m);
   const int na = s->d.natom, last = s->h_nmol - 1;
-  if (m != last) {
-    std::vector<double> tmp(&s->h_xyz[(size_t)last * na * 3], &s->h_xyz[(size_t)last * na * 3] + 3 * na);
-    rc = write_molecule(s, m, tmp.data());
-    if (rc) return rc;
-  }
+  double x[3 * RGPU_MAX_ATOMS];
+  memcpy(x, &s->h_xyz[(size_t)last * na * 3], sizeof(double) * 3 * na);
   s->h_nmol--;
-  s->h_xyz.resize((size_t)s->h_nmol * na * 3);
-  CK(cudaMemcpyAsync(s->nmol, &s->h_nmol, sizeof(int), cudaMemcpyHostToDevice, s->st));
-  rc = upload_records(s);
+  rc = write_molecule(s, m != last ? m : -1, x);
   if (rc) return rc;
+  s->h_xyz.resize((size_t)s->h_nmol * na * 3);
   CK(cudaStreamSynchronize(s->st));
   return RGPU_SUCCESS;
 }
@@ -1030,7 +1005,7 @@ extern "C" int rgpu_ewald_fourier_difference(rgpu_system *s, int precision, int 
   if (!s->h.ewald || !s->h.nk) return RGPU_SUCCESS;
   if (old_mol >= s->h_nmol) return fail(RGPU_E_INVALID, "molecule %d", old_mol);
   const int na = s->d.natom;
-  double xyz[2 * RGPU_MAX_ATOMS * 3], q[2 * RGPU_MAX_ATOMS];
+  RgpuSites in;
   int ns = 0;
   double ex_old = 0.0, ex_new = 0.0;
   int dn = 0;
@@ -1038,8 +1013,8 @@ extern "C" int rgpu_ewald_fourier_difference(rgpu_system *s, int precision, int 
     const double *o = &s->h_xyz[(size_t)old_mol * na * 3];
     for (int a = 0; a < na; a++) {
       if (s->h.mol_q[a] == 0.0) continue;
-      for (int c = 0; c < 3; c++) xyz[3 * ns + c] = o[3 * a + c];
-      q[ns++] = -s->h.mol_q[a];
+      for (int c = 0; c < 3; c++) in.xyz[ns][c] = o[3 * a + c];
+      in.q[ns++] = -s->h.mol_q[a];
     }
     ex_old = exclusion_energy(s, o);
     dn--;
@@ -1047,20 +1022,18 @@ extern "C" int rgpu_ewald_fourier_difference(rgpu_system *s, int precision, int 
   if (new_xyz) {
     for (int a = 0; a < na; a++) {
       if (s->h.mol_q[a] == 0.0) continue;
-      for (int c = 0; c < 3; c++) xyz[3 * ns + c] = new_xyz[3 * a + c];
-      q[ns++] = s->h.mol_q[a];
+      for (int c = 0; c < 3; c++) in.xyz[ns][c] = new_xyz[3 * a + c];
+      in.q[ns++] = s->h.mol_q[a];
     }
     ex_new = exclusion_energy(s, new_xyz);
     dn++;
   }
   double e[2] = {0.0, 0.0};
   if (ns) {
-    CK(cudaMemcpyAsync(s->io_xyz, xyz, sizeof(double) * 3 * ns, cudaMemcpyHostToDevice, s->st));
-    CK(cudaMemcpyAsync(s->io_q, q, sizeof(double) * ns, cudaMemcpyHostToDevice, s->st));
-    CK(rgpu_ewald_delta_launch(precision == RGPU_MIXED, s->d_sys, s->io_xyz, s->io_q, ns, s->ds, s->io_out, s->kw,
-                               s->st));
-    CK(cudaMemcpyAsync(e, s->io_out, sizeof(double) * 2, cudaMemcpyDeviceToHost, s->st));
+    CK(rgpu_ewald_delta_launch(precision == RGPU_MIXED, s->d_sys, in, ns, s->h.nk, s->ds, s->h_call->e, s->kw, s->st));
     CK(cudaStreamSynchronize(s->st));
+    e[0] = s->h_call->e[0];
+    e[1] = s->h_call->e[1];
   } else {
     CK(cudaMemsetAsync(s->ds, 0, sizeof(double2) * s->h.nk, s->st));
   }
@@ -1211,42 +1184,28 @@ extern "C" int rgpu_total_energy(rgpu_system *s, double *out)
   if (!s || !out) return fail(RGPU_E_INVALID, "bad argument");
   int rc = refresh_from_device(s);
   if (rc) return rc;
-  const int na = s->d.natom, nads = s->h_nmol * na;
-  double hv = 0, hc = 0, av = 0, ac = 0;
-  std::vector<int> atom(RGPU_MAX_POS), excl(RGPU_MAX_POS);
-  std::vector<double> res(4 * RGPU_MAX_POS);
-  for (int base = 0; base < nads; base += RGPU_MAX_POS) {
-    int b = std::min(RGPU_MAX_POS, nads - base);
-    for (int i = 0; i < b; i++) {
-      atom[i] = (base + i) % na;
-      excl[i] = (base + i) / na;
-    }
-    rc = bead_batch(s, RGPU_FP64, b, &s->h_xyz[(size_t)base * 3], atom.data(), excl.data(), 0, res.data(), nullptr);
-    if (rc) return rc;
-    for (int i = 0; i < b; i++) {
-      hv += res[4 * i];
-      hc += res[4 * i + 1];
-      av += res[4 * i + 2];
-      ac += res[4 * i + 3];
-    }
-  }
-  double hf = 0.0, af = 0.0;
+  const int nads = s->h_nmol * s->d.natom;
   const RgpuSys &h = s->h;
-  if (h.ewald && h.nk) {
-    rc = recompute_sk_ads(s);
-    if (rc) return rc;
-    std::vector<double2> sa(h.nk), sf(h.nk);
-    std::vector<double> kf(h.nk);
-    CK(cudaMemcpyAsync(sa.data(), s->sk_ads, sizeof(double2) * h.nk, cudaMemcpyDeviceToHost, s->st));
-    CK(cudaMemcpyAsync(sf.data(), s->sk_fw, sizeof(double2) * h.nk, cudaMemcpyDeviceToHost, s->st));
-    CK(cudaMemcpyAsync(kf.data(), s->kfactor, sizeof(double) * h.nk, cudaMemcpyDeviceToHost, s->st));
-    CK(cudaStreamSynchronize(s->st));
-    for (int k = 0; k < h.nk; k++) {
-      af += kf[k] * (sa[k].x * sa[k].x + sa[k].y * sa[k].y);
-      hf += kf[k] * (sf[k].x * sa[k].x + sf[k].y * sa[k].y);
+  const bool fourier = h.ewald && h.nk;
+  int ctas = 0, blocks = 0;
+  CK(rgpu_total_pairs_launch(s->d_sys, s->rec64, nads, s->fw_model == RGPU_FRAMEWORK_GRID, s->h_call->total, &ctas, s->st));
+  if (fourier)
+    CK(rgpu_ads_fourier_launch(s->d_sys, s->ads_xyz, nads, h.nk, s->sk_ads, s->h_call->fourier, &blocks, s->st));
+  CK(cudaStreamSynchronize(s->st));
+  double hv = 0, hc = 0, av = 0, ac = 0, ex = 0, hf = 0, af = 0;
+  for (int c = 0; c < ctas; c++) {
+    const double *t = s->h_call->total + 5 * c;
+    hv += t[0];
+    hc += t[1];
+    av += t[2];
+    ac += t[3];
+    ex += t[4];
+  }
+  if (fourier) {
+    for (int c = 0; c < blocks; c++) {
+      af += s->h_call->fourier[2 * c];
+      hf += s->h_call->fourier[2 * c + 1];
     }
-    double ex = 0.0;
-    for (int m = 0; m < s->h_nmol; m++) ex += exclusion_energy(s, &s->h_xyz[(size_t)m * na * 3]);
     const double net = s->h_nmol * h.mol_charge;
     af -= ex + s->h_nmol * h.self_mol;
     af += h.uion * net * net;
@@ -1997,7 +1956,7 @@ extern "C" int rgpu_engine_set_adsorbates(rgpu_engine *e, const int *nmol, const
   int max_nk = 0;
   for (int i = 0; i < n; i++) {
     rgpu_system *s = e->sys[i];
-    CK(rgpu_records_launch(s->d_sys, nmol[i] * s->d.natom, s->rec32, s->rec64, e->st));
+    CK(rgpu_records_launch(s->d_sys, nmol[i] * s->d.natom, -1, s->rec32, s->rec64, e->st));
     s->records_stale = 0;
     max_nk = std::max(max_nk, s->h.nk);
   }

@@ -13,8 +13,7 @@
  *    (translation, rotation, CBMC insertion, CBMC deletion: src/mc_moves.c:1529,
  *    :2636, :6941, :7150) without returning to the host; FP64 and mixed runs
  *    see identical random streams.
- *  - per-call kernels behind the reference-named C entry points: batched
- *    bead energies, Ewald Fourier difference and accept, structure factors.
+ *  - the batched state transfer of an engine's systems.
  */
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -1943,100 +1942,6 @@ cudaError_t rgpu_engine_launch(int mixed, RgpuSys *d_systems, int nsys, long lon
                             fw_items, tile_items, k_items);
 }
 
-/* Ewald Fourier difference of ns signed sites (FP64 xyz + charges), writing
- * dS(k) of the candidate into d_ds (for a later accept) and {e_ads, e_host}. */
-template <int MIXED>
-__global__ void __launch_bounds__(256) k_ewald_delta(const RgpuSys *sysp, const double *xyz, const double *q, int ns,
-                                                     double2 *d_ds, double *out, int kw)
-{
-  __shared__ RgpuSys S;
-  __shared__ EwSite sites[2 * RGPU_MAX_ATOMS];
-  /* phase tables of the FP64 path; the mixed path forms its phases directly */
-  __shared__ typename PhaseT<MIXED>::T tab[MIXED == 1 ? 1 : 2 * RGPU_MAX_ATOMS * 3 * 41];
-  __shared__ double red[72];
-  load_sys(&S, sysp);
-  for (int s = threadIdx.x; s < ns; s += blockDim.x) {
-    bead_set(sites[s].b, S, xyz[3 * s], xyz[3 * s + 1], xyz[3 * s + 2], 0, -1);
-    sites[s].q = q[s];
-  }
-  __syncthreads();
-  ewald_phases<MIXED>(S, sites, ns, tab, kw);
-  __syncthreads();
-  double ea = 0.0, eh = 0.0;
-  for (int k = threadIdx.x; k < S.nk; k += blockDim.x) {
-    double2 d = ewald_dS<MIXED>(tab, kw, sites, ns, S.kvec[k]);
-    double2 so = S.sk_ads[k];
-    double2 sf = S.sk_fw[k];
-    double kf = S.kfactor[k];
-    ea += kf * (2.0 * (so.x * d.x + so.y * d.y) + d.x * d.x + d.y * d.y);
-    eh += kf * (sf.x * d.x + sf.y * d.y);
-    if (d_ds) d_ds[k] = d;
-  }
-  block_sum2(ea, eh, red);
-  if (threadIdx.x == 0) { out[0] = ea; out[1] = eh; }
-}
-
-__global__ void k_ewald_accept(const RgpuSys *sysp, const double2 *d_ds)
-{
-  const RgpuSys *S = sysp;
-  int nk = S->nk;
-  double2 *sk = S->sk_ads;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nk; k += gridDim.x * blockDim.x) {
-    double2 a = sk[k], d = d_ds[k];
-    sk[k] = make_double2(a.x + d.x, a.y + d.y);
-  }
-}
-
-cudaError_t rgpu_ewald_delta_launch(int mixed, const RgpuSys *d_sys, const double *d_xyz, const double *d_q, int ns,
-                                    double2 *d_ds, double *d_out, int kw, cudaStream_t st)
-{
-  if (ns > 2 * RGPU_MAX_ATOMS || kw > 41) return cudaErrorInvalidValue;
-  if (mixed) k_ewald_delta<true><<<1, 256, 0, st>>>(d_sys, d_xyz, d_q, ns, d_ds, d_out, kw);
-  else k_ewald_delta<false><<<1, 256, 0, st>>>(d_sys, d_xyz, d_q, ns, d_ds, d_out, kw);
-  return cudaGetLastError();
-}
-
-cudaError_t rgpu_ewald_accept_launch(const RgpuSys *d_sys, const double2 *d_ds, int nk, cudaStream_t st)
-{
-  int blocks = (nk + 255) / 256;
-  if (blocks < 1) blocks = 1;
-  k_ewald_accept<<<blocks, 256, 0, st>>>(d_sys, d_ds);
-  return cudaGetLastError();
-}
-
-/* S(k) = sum_i q_i exp(i k.r_i) over n sites (FP64), one thread per k */
-__global__ void k_structure_factor(const RgpuSys *sysp, const double *xyz, const double *q, int n, double2 *sk)
-{
-  const RgpuSys *S = sysp;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= S->nk) return;
-  char4 kv = S->kvec[k];
-  double re = 0.0, im = 0.0;
-  for (int i = 0; i < n; i++) {
-    const double *x = xyz + 3 * i;
-    double a;
-    if (!S->triclinic)
-      a = 2.0 * (kv.x * x[0] * S->inv_box[0] + kv.y * x[1] * S->inv_box[1] + kv.z * x[2] * S->inv_box[2]);
-    else
-      a = 2.0 * (kv.x * rgpu_frac(*S, 0, x[0], x[1], x[2]) + kv.y * rgpu_frac(*S, 1, x[0], x[1], x[2]) +
-                 kv.z * rgpu_frac(*S, 2, x[0], x[1], x[2]));
-    double sn, cs;
-    sincospi(a, &sn, &cs);
-    re += q[i] * cs;
-    im += q[i] * sn;
-  }
-  sk[k] = make_double2(re, im);
-}
-
-cudaError_t rgpu_structure_factor_launch(const RgpuSys *d_sys, const double *d_xyz, const double *d_q, int n,
-                                         int nk, double2 *d_sk, cudaStream_t st)
-{
-  int blocks = (nk + 127) / 128;
-  if (blocks < 1) blocks = 1;
-  k_structure_factor<<<blocks, 128, 0, st>>>(d_sys, d_xyz, d_q, n, d_sk);
-  return cudaGetLastError();
-}
-
 /* Batched state transfer of an engine's systems through one staging buffer:
  * system i's region starts at off[i] (8-byte aligned) and holds its state
  * block (RgpuState; for an upload only its nmol field is read), then
@@ -2064,41 +1969,6 @@ __global__ void k_scatter_positions(const RgpuSys *systems, const unsigned long 
   if (threadIdx.x == 0) *S.nmol = nmol;
 }
 
-/* S_ads(k) of every system of an engine from its positions (the batched
- * upload): block (x, y) = wave vectors x*128.. of system y; the same sum, in
- * the same order, as k_structure_factor with the molecule's charges. */
-__global__ void k_upload_sk(const RgpuSys *systems)
-{
-  const RgpuSys &S = systems[blockIdx.y];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= S.nk) return;
-  const int n = *S.nmol * S.natom;
-  const char4 kv = S.kvec[k];
-  double re = 0.0, im = 0.0;
-  for (int i = 0; i < n; i++) {
-    const double *x = S.ads_xyz + 3 * i;
-    const double q = S.mol_q[i % S.natom];
-    double a;
-    if (!S.triclinic)
-      a = 2.0 * (kv.x * x[0] * S.inv_box[0] + kv.y * x[1] * S.inv_box[1] + kv.z * x[2] * S.inv_box[2]);
-    else
-      a = 2.0 * (kv.x * rgpu_frac(S, 0, x[0], x[1], x[2]) + kv.y * rgpu_frac(S, 1, x[0], x[1], x[2]) +
-                 kv.z * rgpu_frac(S, 2, x[0], x[1], x[2]));
-    double sn, cs;
-    sincospi(a, &sn, &cs);
-    re += q * cs;
-    im += q * sn;
-  }
-  S.sk_ads[k] = make_double2(re, im);
-}
-
-cudaError_t rgpu_upload_sk_launch(const RgpuSys *d_systems, int n, int max_nk, cudaStream_t st)
-{
-  if (n <= 0 || max_nk <= 0) return cudaSuccess;
-  k_upload_sk<<<dim3((unsigned)((max_nk + 127) / 128), (unsigned)n), 128, 0, st>>>(d_systems);
-  return cudaGetLastError();
-}
-
 cudaError_t rgpu_gather_states_launch(const RgpuSys *d_systems, int n, const unsigned long long *d_off,
                                       unsigned char *d_buf, cudaStream_t st)
 {
@@ -2112,28 +1982,5 @@ cudaError_t rgpu_scatter_positions_launch(const RgpuSys *d_systems, int n, const
 {
   if (n <= 0) return cudaSuccess;
   k_scatter_positions<<<n, 256, 0, st>>>(d_systems, d_off, d_buf);
-  return cudaGetLastError();
-}
-
-/* adsorbate records (fixed-point and FP64) from the authoritative positions */
-__global__ void k_build_records(const RgpuSys *sysp, int nads, int4 *rec32, AdsRec64 *rec64)
-{
-  const RgpuSys *S = sysp;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nads) return;
-  const int m = i / S->natom, a = i - m * S->natom;
-  const double x = S->ads_xyz[3 * i], y = S->ads_xyz[3 * i + 1], z = S->ads_xyz[3 * i + 2];
-  int xi, yi, zi;
-  rgpu_fix3(*S, x, y, z, xi, yi, zi);
-  rec32[i] = make_int4(xi, yi, zi, m * 16 + a);
-  AdsRec64 r;
-  r.x = x; r.y = y; r.z = z; r.tag = m * 16 + a;
-  rec64[i] = r;
-}
-
-cudaError_t rgpu_records_launch(const RgpuSys *d_sys, int nads, int4 *d_rec32, void *d_rec64, cudaStream_t st)
-{
-  if (nads <= 0) return cudaSuccess;
-  k_build_records<<<(nads + 127) / 128, 128, 0, st>>>(d_sys, nads, d_rec32, (AdsRec64 *)d_rec64);
   return cudaGetLastError();
 }

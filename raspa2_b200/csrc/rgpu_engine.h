@@ -22,12 +22,22 @@ cudaError_t rgpu_engine_launch(int mixed, RgpuSys *d_systems, int nsys, long lon
 /* per-call entry points (percall.cu); d_out and d_ov in mapped host memory */
 cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ads, int nads, const RgpuPoints &in, int P,
                                int ntile, int pair_check, int fw_grid, double *d_out, int *d_ov, cudaStream_t st);
-cudaError_t rgpu_ewald_delta_launch(int mixed, const RgpuSys *d_sys, const double *d_xyz, const double *d_q, int ns,
-                                    double2 *d_ds, double *d_out, int kw, cudaStream_t st);
+/* d_out[5 * *ctas]; *ctas <= RGPU_TOTAL_CTAS */
+cudaError_t rgpu_total_pairs_launch(const RgpuSys *d_sys, const void *d_ads, int nads, int fw_grid, double *d_out,
+                                    int *ctas, cudaStream_t st);
+/* S_ads(k) of n adsorbate atoms into d_sk, and the Fourier sums into
+ * d_out[2 * *blocks], *blocks = (nk + 255) / 256 */
+cudaError_t rgpu_ads_fourier_launch(const RgpuSys *d_sys, const double *d_xyz, int n, int nk, double2 *d_sk, double *d_out,
+                                    int *blocks, cudaStream_t st);
+cudaError_t rgpu_ewald_delta_launch(int mixed, const RgpuSys *d_sys, const RgpuSites &in, int ns, int nk, double2 *d_ds,
+                                    double *d_out, int kw, cudaStream_t st);
 cudaError_t rgpu_ewald_accept_launch(const RgpuSys *d_sys, const double2 *d_ds, int nk, cudaStream_t st);
+/* d_q: charge of each atom; nullptr: the molecule's, by atom */
 cudaError_t rgpu_structure_factor_launch(const RgpuSys *d_sys, const double *d_xyz, const double *d_q, int n,
                                          int nk, double2 *d_sk, cudaStream_t st);
-cudaError_t rgpu_records_launch(const RgpuSys *d_sys, int nads, int4 *d_rec32, void *d_rec64, cudaStream_t st);
+cudaError_t rgpu_records_launch(const RgpuSys *d_sys, int nads, int nmol, int4 *d_rec32, void *d_rec64, cudaStream_t st);
+cudaError_t rgpu_set_molecule_launch(const RgpuSys *d_sys, const RgpuSites &in, int m, int nmol, int4 *d_rec32,
+                                     void *d_rec64, cudaStream_t st);
 
 /* grids (grid.cu) */
 cudaError_t rgpu_grid_build_launch(const RgpuSys *d_sys, const RgpuLJ *lj, double reach, const int npts[3],

@@ -111,6 +111,15 @@ typedef struct {
   int excl[RGPU_MAX_POS];     /* adsorbate molecule left out (-1: none) */
 } RgpuPoints;
 
+/* charged sites of an Ewald difference, or a molecule's positions, passed by
+ * value to the kernel */
+typedef struct {
+  double xyz[2 * RGPU_MAX_ATOMS][3];
+  double q[2 * RGPU_MAX_ATOMS];
+} RgpuSites;
+
+#define RGPU_TOTAL_CTAS 592    /* CTAs of a total-energy evaluation: 4 on each of 148 SMs */
+
 /* geometry of an energy grid: npts cells per axis over `size` from `shift`,
  * spanning a unit cell of lengths `cell`; a triclinic unit cell (tri = 1)
  * has its matrix (columns a, b, c; row-major) and then its inverse in

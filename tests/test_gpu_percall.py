@@ -59,3 +59,50 @@ def test_points_at_split_edges(cuda, atoms, nmol, n, tri):
         h = n // 2
         parts = [g.bead_energies(xyz[k], atom[k], excl[k], native.RGPU_MIXED) for k in (slice(0, h), slice(h, n))]
         np.testing.assert_array_equal(got, np.concatenate(parts))
+
+
+@pytest.mark.parametrize("tri", [False, True])
+@pytest.mark.parametrize("atoms,nmol,kmax", [(1, 1, 1), (16, 5, 2), (40, 6, 6), (300, 43, 10), (96, 210, 4)])
+def test_totals_and_fourier_at_split_edges(cuda, atoms, nmol, kmax, tri):
+    """Total energies, Fourier differences (insertion, deletion, displacement), acceptance and molecule updates
+    where the split over CTAs changes: fewer wave vectors than a block and more than a cluster's, fewer atoms than
+    a phase table and more, one position to more positions than CTAs. FP64 bounds as above; the sums of absolute
+    terms are those of the oracle."""
+    s = dataclasses.replace(co2_box(atoms, tri), kmax=(kmax, kmax, kmax))
+    rng = np.random.default_rng(atoms + nmol + kmax)
+    mols = molecules(rng, s, nmol + 1)
+    mols, extra = mols[:-1], mols[-1]
+    g = native.GpuSystem(s, maxmol=256)
+    g.set_adsorbates(mols)
+    o = O.Oracle.from_system(s, maxmol=256)
+
+    def totals(x):
+        o.set_molecules(x)
+        ref = np.array(o.total_energy())[:6]
+        t, q = s.molecule_types(), s.molecule.charges()
+        pair = sum(o.point_abs(int(t[a]), float(q[a]), m[a], i) for i, m in enumerate(x) for a in range(3))
+        e = np.asarray(g.total_energy())
+        scale = np.array([pair[0], pair[2], pair[1], pair[3], 0.0, 0.0])
+        scale[4:] = np.abs(np.array(o.ewald_delta_abs(new=extra)))[:2].max() * (len(x) + 1) ** 2
+        assert np.all(np.abs(e - ref) <= 1e-9 * np.abs(ref) + 1e-12 * scale + 1e-7), (e, ref)
+
+    totals(mols)
+    new = mols[0] + rng.uniform(-0.3, 0.3, 3)
+    for old, x in ((-1, extra), (nmol - 1, None), (0, new)):
+        got = g.ewald_difference(old, x)
+        prev = None if old < 0 else mols[old]
+        ref, size = np.array(o.ewald_delta(old=prev, new=x)[0]), np.abs(np.array(o.ewald_delta_abs(old=prev, new=x)))
+        assert np.all(np.abs(got[:2] - ref[:2]) <= 1e-9 * np.abs(ref[:2]) + 1e-12 * size[:2].max() + 1e-8)
+    g.ewald_accept()                       # the displacement
+    g.update_molecule(0, new)
+    moved = mols.copy()
+    moved[0] = new
+    np.testing.assert_array_equal(g.adsorbates(), moved)
+    o.set_molecules(moved)
+    got, ref = g.ewald_difference(-1, extra), np.array(o.ewald_delta(new=extra)[0])
+    size = np.abs(np.array(o.ewald_delta_abs(new=extra)))[:2].max()
+    assert np.all(np.abs(got[:2] - ref[:2]) <= 1e-9 * np.abs(ref[:2]) + 1e-12 * size + 1e-8)
+    g.insert_molecule(extra)
+    totals(np.concatenate([moved, extra[None]]))
+    g.remove_molecule(0)
+    totals(np.concatenate([extra[None], moved[1:]]))
