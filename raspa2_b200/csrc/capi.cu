@@ -107,7 +107,7 @@ struct rgpu_system {
 struct rgpu_engine {
   std::vector<rgpu_system *> sys;
   RgpuSys *d_systems;
-  int mixed, threads, kw, max_ads, cluster, fw_items, tile_items, k_items;
+  int mixed, threads, kw, max_ads, cluster, fw_items, fwd_items, tile_items, k_items;
   bool wide;                  /* 64-register build of the mixed kernel */
   bool flex;                  /* build with flexible-chain moves and energy grids */
   size_t smem;
@@ -133,7 +133,7 @@ struct rgpu_engine {
   RgpuSys *h_slots;
   std::vector<cudaEvent_t> slot_ev;
   int smem_max;
-  int nsplit, cluster_b, fw_items_b, tile_items_b, k_items_b;
+  int nsplit, cluster_b, fw_items_b, fwd_items_b, tile_items_b, k_items_b;
   size_t smem_b;
   cudaStream_t st_b;
   cudaEvent_t ev_fork, ev_join;
@@ -143,38 +143,34 @@ struct rgpu_engine {
  * size: each CTA's share of the framework (tiles) and of the wave vectors,
  * staged in shared memory as far as it fits, in order of preference:
  * framework share and wave vectors, framework only, wave vectors only,
- * neither. Returns false when not even the adsorbates fit. */
+ * neither. The FP64 path's share holds each atom twice (fixed point, for
+ * the preselection of every visited atom, and FP64, for those selected);
+ * where both do not fit, the FP64 positions stay in global memory (L2).
+ * Returns false when not even the adsorbates fit. */
 struct EngineGroup {
-  int fw_items, tile_items, k_items;
+  int fw_items, fwd_items, tile_items, k_items;
   size_t smem;
 };
 
 static bool plan_group(const rgpu_engine *e, int lo, int hi, int cluster, EngineGroup &g)
 {
-  int maxfw = 0, maxtile = 0, maxk = 0;
+  int maxtile = 0, maxk = 0;
   bool all_grids = true;
   for (int j = lo; j < hi; j++) {
     const rgpu_system *s = e->sys[e->order[j]];
     all_grids = all_grids && s->h.use_grid;
-    maxfw = std::max(maxfw, (s->d.nfw + cluster - 1) / cluster);
     maxtile = std::max(maxtile, (s->h.ntile + cluster - 1) / cluster);
     if (s->h.ewald) maxk = std::max(maxk, (s->h.nk + cluster - 1) / cluster);
   }
-  int fw = e->mixed ? maxtile * RGPU_TILE : maxfw, tiles = e->mixed ? maxtile : 0;
-  if (all_grids) {
-    /* no framework pairs are evaluated: nothing of the framework to stage */
-    fw = 0;
-    tiles = 0;
-  }
-  const int fw_try[4] = {fw, fw, 0, 0}, tile_try[4] = {tiles, tiles, 0, 0}, k_try[4] = {maxk, 0, maxk, 0};
-  for (int t = 0; t < 4; t++) {
-    const size_t b = rgpu_engine_smem_bytes(e->mixed, fw_try[t], tile_try[t], e->max_ads, e->kw, k_try[t],
-                                            e->threads, e->flex);
+  if (all_grids) maxtile = 0;   /* no framework pairs are evaluated: nothing of the framework to stage */
+  for (int t = 0; t < 6; t++) {
+    const int level = 2 - t / 2;                 /* 2: both forms of the atoms, 1: fixed point, 0: none */
+    if (level == 2 && e->mixed) continue;
+    const int tiles = level > 0 ? maxtile : 0, fw = tiles * RGPU_TILE, fwd = level == 2 ? fw : 0;
+    const int k = t % 2 == 0 ? maxk : 0;
+    const size_t b = rgpu_engine_smem_bytes(e->mixed, fw, fwd, tiles, e->max_ads, e->kw, k, e->threads, e->flex);
     if (b <= (size_t)e->smem_max) {
-      g.fw_items = fw_try[t];
-      g.tile_items = tile_try[t];
-      g.k_items = k_try[t];
-      g.smem = b;
+      g = {fw, fwd, tiles, k, b};
       return true;
     }
   }
@@ -1526,16 +1522,17 @@ extern "C" int rgpu_grid_interpolate_noalloc(const float *d_grid, const int npts
 /* The device slots: d_systems[j] = system order[j], its framework staged in
  * shared memory when its launch group stages it; d_off (once the staging
  * buffer exists) in the same slot order. */
-/* whether system s, in the first launch (second = false) or the second,
- * has its framework share staged in shared memory: the engine stages when
- * its plan holds a framework share and the system's share fits it */
-static bool slot_smem_fw(const rgpu_engine *e, const rgpu_system *s, bool second)
+/* what of system s's framework share, in the first launch (second = false) or
+ * the second, is staged in shared memory (RgpuSys.smem_fw): the engine stages
+ * what its plan has room for and the system's share fits */
+static int slot_smem_fw(const rgpu_engine *e, const rgpu_system *s, bool second)
 {
   const int c = second ? e->cluster_b : e->cluster;
   const int fw_items = second ? e->fw_items_b : e->fw_items, tile_items = second ? e->tile_items_b : e->tile_items;
-  const int share_tiles = (s->h.ntile + c - 1) / c, share_fw = (s->d.nfw + c - 1) / c;
-  return fw_items > 0 && (e->mixed ? share_tiles * RGPU_TILE <= fw_items && share_tiles <= tile_items
-                                   : share_fw <= fw_items);
+  const int fwd_items = second ? e->fwd_items_b : e->fwd_items;
+  const int share = (s->h.ntile + c - 1) / c, atoms = share * RGPU_TILE;
+  if (fw_items <= 0 || atoms > fw_items || share > tile_items) return 0;
+  return atoms <= fwd_items ? 2 : 1;
 }
 
 static cudaError_t upload_slots(rgpu_engine *e)
@@ -1636,12 +1633,13 @@ extern "C" int rgpu_engine_create_ex(rgpu_engine **out, rgpu_system *const *syst
     return fail(RGPU_E_INVALID, "adsorbate capacity does not fit in shared memory");
   }
   e->fw_items = g.fw_items;
+  e->fwd_items = g.fwd_items;
   e->tile_items = g.tile_items;
   e->k_items = g.k_items;
   e->smem = g.smem;
   e->nsplit = 0;
   e->cluster_b = 0;
-  e->fw_items_b = e->tile_items_b = e->k_items_b = 0;
+  e->fw_items_b = e->fwd_items_b = e->tile_items_b = e->k_items_b = 0;
   e->smem_b = 0;
   e->st_b = nullptr;
   e->ev_fork = e->ev_join = nullptr;
@@ -1715,7 +1713,7 @@ extern "C" int rgpu_engine_set_split(rgpu_engine *e, const int *second, int nsec
   for (int k = 0; k < nsecond; k++) order.push_back(second[k]);
   const std::vector<int> old_order = e->order;
   e->order = order;
-  EngineGroup ga, gb = {0, 0, 0, 0};
+  EngineGroup ga, gb = {0, 0, 0, 0, 0};
   if (!plan_group(e, 0, n - nsecond, e->cluster, ga) || (nsecond > 0 && !plan_group(e, n - nsecond, n, cluster_b, gb))) {
     e->order = old_order;
     return fail(RGPU_E_INVALID, "adsorbate capacity does not fit in shared memory");
@@ -1731,12 +1729,14 @@ extern "C" int rgpu_engine_set_split(rgpu_engine *e, const int *second, int nsec
   /* launches and staging kernels in flight (on any stream) read the old slots */
   CK(cudaDeviceSynchronize());
   e->fw_items = ga.fw_items;
+  e->fwd_items = ga.fwd_items;
   e->tile_items = ga.tile_items;
   e->k_items = ga.k_items;
   e->smem = ga.smem;
   e->nsplit = nsecond;
   e->cluster_b = nsecond > 0 ? cluster_b : 0;
   e->fw_items_b = gb.fw_items;
+  e->fwd_items_b = gb.fwd_items;
   e->tile_items_b = gb.tile_items;
   e->k_items_b = gb.k_items;
   e->smem_b = gb.smem;
@@ -1760,11 +1760,11 @@ static cudaError_t engine_launch_all(rgpu_engine *e, long long nsteps, cudaStrea
     if ((err = cudaEventRecord(e->ev_fork, st)) != cudaSuccess) return err;
     if ((err = cudaStreamWaitEvent(e->st_b, e->ev_fork, 0)) != cudaSuccess) return err;
   }
-  err = rgpu_engine_launch(e->mixed, e->d_systems, na, nsteps, e->kw, e->max_ads, e->fw_items, e->tile_items,
+  err = rgpu_engine_launch(e->mixed, e->d_systems, na, nsteps, e->kw, e->max_ads, e->fw_items, e->fwd_items, e->tile_items,
                            e->k_items, e->cluster, e->threads, e->wide, e->flex, st);
   if (e->nsplit > 0) {
     cudaError_t eb = rgpu_engine_launch(e->mixed, e->d_systems + na, e->nsplit, nsteps, e->kw, e->max_ads,
-                                        e->fw_items_b, e->tile_items_b, e->k_items_b, e->cluster_b, e->threads,
+                                        e->fw_items_b, e->fwd_items_b, e->tile_items_b, e->k_items_b, e->cluster_b, e->threads,
                                         e->wide, e->flex, e->st_b);
     if (err == cudaSuccess) err = eb;
     cudaError_t ej = cudaEventRecord(e->ev_join, e->st_b);

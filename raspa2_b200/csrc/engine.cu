@@ -5,14 +5,16 @@
  *    the wave vectors are split between the CTAs of the cluster (each stages
  *    its share, with its share of S(k), in shared memory); every CTA keeps a
  *    full copy of the adsorbate records, draws the same counter-based random
- *    numbers and takes the same decisions. Each energy evaluation leaves
- *    this CTA's per-position sums in shared memory; after one cluster barrier
- *    the lanes that need a total read the sums of every CTA through
- *    distributed shared memory in rank order, so all CTAs see bitwise
- *    identical totals. Each cluster advances its box by `nsteps` MC moves
- *    (translation, rotation, CBMC insertion, CBMC deletion: src/mc_moves.c:1529,
- *    :2636, :6941, :7150) without returning to the host; FP64 and mixed runs
- *    see identical random streams.
+ *    numbers and takes the same decisions. The step loop is a sequence of
+ *    stages, each one energy evaluation: all threads place its positions, all
+ *    warps evaluate (one place in the code, whatever the move), one cluster
+ *    barrier makes every CTA's per-position sums readable, all threads add
+ *    them up in rank order through distributed shared memory, so all CTAs see
+ *    bitwise identical totals, and warp 0 of every CTA does the bookkeeping of
+ *    the move and describes the next stage. Each cluster advances its box by `nsteps` MC
+ *    moves (translation, rotation, CBMC insertion, CBMC deletion:
+ *    src/mc_moves.c:1529, :2636, :6941, :7150) without returning to the host;
+ *    FP64 and mixed runs see identical random streams.
  *  - the batched state transfer of an engine's systems.
  */
 #include <cooperative_groups.h>
@@ -30,28 +32,22 @@
 
 namespace cg = cooperative_groups;
 
-#define RGPU_MAX_UNITS 512
+/* eval_plan makes at most max(warps, positions) <= 64 framework units and no
+ * more adsorbate units than that */
+#define RGPU_MAX_UNITS 128
 #define RGPU_MAX_WARPS 32
-#define RGPU_RND 192          /* random slots drawn per MC step */
-#define RGPU_CTL_BYTES 6144   /* shared-memory slot of the control block */
+#define RGPU_RND 64           /* random slots tabulated per MC step (the trial orientations are drawn on their own) */
+#define RGPU_FIXED_BYTES 26624 /* shared-memory slot of the fixed block */
 
 /* ------------------------------------------------------------------------ */
 /* shared-memory plan of the engine (offsets in bytes from the dynamic base).
- * fw_items: framework records of this CTA's share (atoms; tiles*RGPU_TILE on the
- * mixed path), tiles: tile records of the share (mixed only), k_items: wave
- * vectors of the share staged with their S(k) (0: read from global memory). */
+ * fw_items: framework records of this CTA's share (tiles * RGPU_TILE), fwd_items:
+ * their FP64 positions (FP64 path only), tiles: tile records of the share, k_items: wave
+ * vectors of the share staged with their S(k) (0: read from global memory). The
+ * block whose size is fixed (Fixed) comes first. */
 struct EngineLayout {
-  size_t sys, fw, tiles, ads, pos, uv, uc, uo, part, q, sites, tab, red, kvec, kf, skfw, skads, ctl, ang, total;
+  size_t fw, fwd, tiles, ads, q, tab, kvec, kf, skfw, skads, ang, total;
 };
-
-/* this CTA's sums for one position of an evaluation: host VDW, host real,
- * adsorbate VDW, adsorbate real, overlap flag. 16-byte aligned (48 bytes) so
- * that v[0..1] and v[2..3] are read as double2. */
-struct __align__(16) PosSum {
-  double v[4];
-  int ov, pad;
-};
-static_assert(sizeof(PosSum) % 16 == 0, "PosSum must keep 16-byte alignment in arrays");
 
 __host__ __device__ inline size_t rgpu_align(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -62,160 +58,257 @@ __host__ __device__ inline size_t rgpu_align(size_t x) { return (x + 255) & ~(si
 #define RGPU_ANG_TABLE (RGPU_ANG_STRIDE * (RGPU_MAX_ATOMS - 2) * RGPU_MAX_TRIALS)
 #define RGPU_ANG_DOUBLES (RGPU_ANG_TABLE + RGPU_MAX_ATOMS)   /* + the bend angle of each bead (chain_scheme 0) */
 
-__host__ __device__ inline EngineLayout engine_layout(int mixed, int fw_items, int tiles, int max_ads_atoms, int kw,
-                                                      int k_items, int nwarps, int flex)
+__host__ __device__ inline EngineLayout engine_layout(int mixed, int fw_items, int fwd_items, int tiles, int max_ads_atoms,
+                                                      int kw, int k_items, int nwarps, int flex)
 {
   EngineLayout L;
-  size_t o = 0;
-  L.sys = o; o = rgpu_align(o + sizeof(RgpuSys));
-  L.fw = o; o = rgpu_align(o + (size_t)fw_items * (mixed ? sizeof(int4) : sizeof(double4)));
+  size_t o = RGPU_FIXED_BYTES;
+  L.fw = o; o = rgpu_align(o + (size_t)fw_items * sizeof(int4));
+  L.fwd = o; o = rgpu_align(o + (size_t)fwd_items * sizeof(double4));
   L.tiles = o; o = rgpu_align(o + (size_t)tiles * sizeof(TileRec));
   L.ads = o; o = rgpu_align(o + (size_t)max_ads_atoms * (mixed ? sizeof(int4) : sizeof(AdsRec64)));
-  L.pos = o; o = rgpu_align(o + RGPU_MAX_POS * sizeof(BeadPos));
-  L.uv = o; o = rgpu_align(o + RGPU_MAX_UNITS * sizeof(double));
-  L.uc = o; o = rgpu_align(o + RGPU_MAX_UNITS * sizeof(double));
-  L.uo = o; o = rgpu_align(o + RGPU_MAX_UNITS * sizeof(int));
-  L.part = o; o = rgpu_align(o + 2 * RGPU_MAX_POS * sizeof(PosSum));   /* double-buffered */
-  /* per-warp pair queues: r2 (FP32, or FP64 for mixed = 2), charge, type */
-  L.q = o; o = rgpu_align(o + (mixed ? (size_t)nwarps * 64 * (mixed == 2 ? 16 : 12) : 0));
-  L.sites = o; o = rgpu_align(o + 2 * RGPU_MAX_ATOMS * sizeof(EwSite));
+  /* per-warp pair queues: r2 (FP32, or FP64 for mixed = 2), charge, type; the
+   * FP64 path queues atom indices */
+  L.q = o; o = rgpu_align(o + (size_t)nwarps * 64 * (mixed == 2 ? 16 : (mixed ? 12 : 4)));
   /* per-site phase tables (none on the mixed path) */
   L.tab = o; o = rgpu_align(o + (mixed == 1 ? 0 : (size_t)2 * RGPU_MAX_ATOMS * 3 * kw * sizeof(double2)));
-  L.red = o; o = rgpu_align(o + 2 * 2 * RGPU_MAX_WARPS * sizeof(double));
   L.kvec = o; o = rgpu_align(o + (size_t)k_items * sizeof(char4));
   L.kf = o; o = rgpu_align(o + (size_t)k_items * sizeof(double));
   L.skfw = o; o = rgpu_align(o + (size_t)k_items * sizeof(double2));
   L.skads = o; o = rgpu_align(o + (size_t)k_items * sizeof(double2));
-  L.ctl = o; o = rgpu_align(o + RGPU_CTL_BYTES);
   L.ang = o; o = rgpu_align(o + (flex ? 2 * RGPU_ANG_DOUBLES * sizeof(double) : 0));   /* growth, retrace */
   L.total = o;
   return L;
 }
 
-size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int tiles, int max_ads_atoms, int kw, int k_items,
+size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int fwd_items, int tiles, int max_ads_atoms, int kw, int k_items,
                               int threads, int flex)
 {
-  return engine_layout(mixed, fw_items, tiles, max_ads_atoms, kw, k_items, threads / 32, flex).total;
+  return engine_layout(mixed, fw_items, fwd_items, tiles, max_ads_atoms, kw, k_items, threads / 32, flex).total;
 }
+
+/* The bookkeeping between evaluations is straight-line code that one warp runs
+ * once per stage: it is bound by instruction fetch (compiled inline at each
+ * use, with an evaluation in each move, the kernel had 520 to 800 KB of code,
+ * several times an SM's instruction cache, and an addition cost about 30
+ * cycles there). So one evaluation is inlined, into the loop; what is used
+ * more than once beside it is a function of its own; and the work that can be
+ * spread over threads (placing positions, adding up CTAs' sums) is done by all
+ * of them between barriers, which cost some 500 cycles. Code now 120 to 270
+ * KB. Measured (upload, moves, states read back): 64 mixed CO2 boxes, 1000
+ * moves each, 21.9 ms (27.4 before); one FP64 CO2 box, 200 moves, 3.28 ms
+ * (4.27); 32 hexane boxes over grids, 100 moves, 4.29 ms (4.42). */
+#define RGPU_COLD __noinline__
+
+/* floor(2^32 / n) + 1 (less one for powers of two: 2^32 / n) for 2 <= n <= 64, 0
+ * for n <= 1: x / n is the high half of its product with x, for x < 2^26 */
+#define M1(n) ((unsigned)((4294967296ULL + (n) - 1) / (n)))
+#define M8(n) M1(n), M1(n + 1), M1(n + 2), M1(n + 3), M1(n + 4), M1(n + 5), M1(n + 6), M1(n + 7)
+static __constant__ unsigned c_magic[66] = {0, 0, M8(2), M8(10), M8(18), M8(26), M8(34), M8(42), M8(50), M8(58)};
+#undef M8
+#undef M1
+
+/* One evaluation stage of the step loop, written by warp 0 and read by every
+ * thread after the barrier that opens the stage. */
+struct __align__(16) Stage {
+  int ph;                     /* PH_*: what the stage evaluates, and what warp 0 does with it */
+  int P, check;               /* bead positions to evaluate, how many of them test single pairs for overlap */
+  int ns, xs;                 /* Ewald sites to sum (0: none); sites buffer of these, or of the latest ones */
+  int ap, xa;                 /* accepted sites still to be added to S_ads(k), in sites buffer xa (0: none) */
+  int db;                     /* buffer to draw step dstep's random numbers into (-1: none) */
+  unsigned long long dstep;
+  int sample;                 /* the step before ended: its state enters the ensemble sums */
+  int first;                  /* the first stage of a step: the move is counted */
+  /* the move: its type, molecule, whether a deletion takes one evaluation,
+   * the buffer of the step's random numbers, steps done in this launch */
+  int mv, m, one, buf;
+  long long it;
+  int ci, k;                  /* chains: bead of the growth and its trials */
+  int r0, r1, rP;             /* chains: retrace beads of the stage, and their positions */
+  int alo, ahi;               /* this CTA's adsorbate atoms */
+  unsigned mf, ma;            /* chunk bounds: floor(2^32 / cf) + 1 and the same of ca (0 for one chunk) */
+  int plan[8];                /* cf | ca << 16: the chunks of a position in each CTA of the cluster */
+};
+enum {
+  PH_END, PH_SKIP,            /* launch done; step without an evaluation */
+  PH_DISP,                    /* translation, rotation */
+  PH_SWAP1, PH_SWAP2, PH_SWAPEW,     /* rigid insertion, deletion, Widom: first bead, orientations, Ewald sum */
+  PH_REINS1, PH_REINS2, PH_REINSEW,  /* rigid reinsertion */
+  PH_TABLE, PH_GROW, PH_RETRACE, PH_CHAINEND   /* flexible chains */
+};
+
+/* outcome of a set of CBMC trials (cbmc_trials) */
+struct Trials {
+  double w_sum, w_sel;        /* sum of the weights, the selected trial's weight */
+  double e[4];                /* the selected trial's energies */
+  int sel, any;               /* the selected trial; whether any is valid */
+};
 
 /* broadcast/control block in shared memory */
 struct Ctl {
-  double rnd[2][RGPU_RND];    /* uniforms by slot, double-buffered by step parity */
+  Stage st[3];                /* the current stage c, and the next: c + 1 as warp 0 describes it, c + 2 as warp 1
+                               * does ahead of it (mod 3) */
+  int which;                  /* which of them the next stage is */
+  int cur;                    /* the current stage, for warp 0 */
+  double rnd[3][RGPU_RND];    /* uniforms by slot, of three steps (step index mod 3) */
+  double csn[3][2];           /* cos, sin of the step's rotation move */
+  int mvn[3];                 /* move type of the step */
+  long long it;               /* steps done in this launch */
   double energy[RGPU_NE];     /* running energies (written back by rank 0) */
   long long cnt[RGPU_NCNT];   /* move counters [0, RGPU_CNT_PAIRS) and reinsertion counters (rank 0's written back) */
-  BeadPos first;              /* chosen first bead */
+  Trials tr[2];
   double u[4];                /* energies of the chosen configuration */
   double uo[4];               /* energies of the retraced old configuration (reinsertion) */
   double rosen;
   double rosen_old;
+  double first[3];            /* chosen first bead */
   /* flexible chains: chosen bead positions of the configuration being grown
-   * or retraced (cp) and of a reinsertion's new one (cpn), intramolecular
-   * energies of the configurations */
+   * or retraced, intramolecular energy */
   double cp[RGPU_MAX_ATOMS][3];
-  double cpn[RGPU_MAX_ATOMS][3];
-  double ub[RGPU_MAX_TRIALS];  /* bonded energies of the current bead's trials */
+  double ub[2][RGPU_MAX_TRIALS];  /* bonded energies of a bead's trials, by bead parity */
   /* a retrace's beads: trial weight sum, the old bead's host VDW, adsorbate
    * VDW, intramolecular LJ and bonded energy, any valid trial */
   double rb[RGPU_MAX_ATOMS][6];
   double co[RGPU_MAX_ATOMS][3];  /* the old beads of a reinsertion's retrace */
-  double uintra, uintra_old;
-  double dl[4];
+  double uintra;
+  __align__(16) double ewt[2][2];   /* this CTA's Ewald sums {e_ads, e_host}, by buffer */
+  double ew[2];               /* the cluster's, of the stage */
   int nmol;
   int fail;
-  int accept;
+  int accept;                 /* accepted Ewald sites (0: none) */
   int sel;
   int nads;                   /* adsorbate atoms = nmol * natom */
   int status;                 /* RGPU_ERR_* bits */
-  /* work done: pairs visited, in cut-off, charged in cut-off, k x site, k */
-  unsigned long long work[5];
+  unsigned long long work[2]; /* work done: (k, site) products, k terms */
   long long cyc[2];           /* clock cycles in evaluations and Ewald sums */
   double sums[RGPU_NSUM];     /* ensemble sums of this launch */
   int next;                   /* unit counter of eval_units */
-  double ewt[2][2];           /* this CTA's Ewald sums {e_ads, e_host}, by buffer */
-  double gv[RGPU_MAX_POS];    /* grid host VDW of the positions of the current evaluation */
-  double gq[RGPU_MAX_POS];    /* grid host real-space charge energy of the positions */
+  int nextk, ewdone;          /* shares of the wave vectors taken, and summed */
+  int ov;                     /* an overlap in the stage, in any CTA */
+  int ovf[2];                 /* overlap flag of this CTA's evaluation, by buffer */
+  int done[RGPU_MAX_POS];     /* units done of each position */
+  unsigned long long wcnt[RGPU_MAX_WARPS][3];   /* pairs visited, in cut-off, charged in cut-off, by warp */
 };
-static_assert(sizeof(Ctl) <= RGPU_CTL_BYTES, "control block exceeds its shared-memory slot");
+static_assert(sizeof(Stage) % 16 == 0, "stages are 16-byte aligned");
 
+/* The part of shared memory whose size does not depend on the systems, at its
+ * start: the bookkeeping reaches it with addresses known to the compiler,
+ * without pointers (which, in functions of their own, would be generic ones:
+ * a dependent load each, and slower loads behind them). */
+struct __align__(256) Fixed {
+  RgpuSys S;
+  Ctl C;
+  BeadPos pos[RGPU_MAX_POS];
+  double2 u[RGPU_MAX_UNITS];
+  double4 part[2][RGPU_MAX_POS];   /* this CTA's sums {host VDW, host real, adsorbate VDW, adsorbate real} of each
+                                    * position, by buffer */
+  double4 tot[RGPU_MAX_POS];       /* the cluster's, of the stage */
+  EwSite sites[2][2 * RGPU_MAX_ATOMS];   /* by sites buffer */
+  double red[2 * RGPU_MAX_WARPS];
+  double rot[3][2][RGPU_MAX_TRIALS][4];  /* quaternions of the orientation trials (new, retrace), of three steps */
+  uint64_t step0;                  /* first MC step of the launch */
+  unsigned ads, ang;               /* offsets of the adsorbate records and of the chain trial trigonometry
+                                    * ([2][RGPU_ANG_DOUBLES]: of a growth and of a retrace stage) */
+  int rank, csize;
+};
+static_assert(sizeof(Fixed) <= RGPU_FIXED_BYTES, "fixed block exceeds its shared-memory slot");
+
+__device__ __forceinline__ unsigned char *smem_at(unsigned offset)
+{
+  extern __shared__ __align__(256) unsigned char smem[];
+  return smem + offset;
+}
+__device__ __forceinline__ Fixed &fx() { return *(Fixed *)smem_at(0); }
+__device__ __forceinline__ double *fx_ang() { return (double *)smem_at(fx().ang); }
+
+/* selects the build of a function of the bookkeeping */
+template <int MIXED, bool FLEX>
+struct Build {};
+
+/* what the evaluation keeps in registers */
 template <int MIXED, bool FLEX>
 struct Eng {
-  RgpuSys *S;
   EvalSlice sl;
-  void *ads;                 /* int4[] or AdsRec64[] (full copy) */
-  BeadPos *pos;
-  double *uv, *uc;           /* [RGPU_MAX_UNITS] unit partials */
-  int *uo;
-  PosSum *part;              /* [2][RGPU_MAX_POS] position sums of this CTA */
   EvalScratch sc;
-  EwSite *sites;
   typename PhaseT<MIXED>::T *tab;
   int kw;
   int k0, k1;                /* this CTA's wave vectors */
-  double *red;               /* [2][2*RGPU_MAX_WARPS] */
-  double *ang;               /* [2][RGPU_ANG_DOUBLES] chain trial trigonometry of a growth and of a retrace
-                              * stage (flexible-chain builds) */
-  Ctl *ctl;
-  const double *rnd;         /* this step's uniforms */
-  uint64_t step;             /* index of the current MC step */
+  uint64_t step0;            /* first MC step of the launch */
   int rank, csize;
-  int xb;                    /* exchange buffer (same sequence in every thread and CTA) */
+  int xb;                    /* buffer of the next evaluation (same sequence in every thread and CTA) */
 };
 
 /* Position of atom a of molecule m. FP64 records carry the position; on the
  * mixed path the FP64 positions stay in global memory (ads_xyz), which every
  * CTA of the cluster writes with the same values on each accepted move. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void atom_xyz(const Eng<MIXED, FLEX> &E, int m, int a, double *p)
+__device__ __forceinline__ void atom_xyz(Build<MIXED, FLEX> E, int m, int a, double *p)
 {
-  const int idx = m * E.S->natom + a;
+  const int idx = m * fx().S.natom + a;
   if (MIXED) {
-    const double *x = E.S->ads_xyz + 3 * idx;
+    const double *x = fx().S.ads_xyz + 3 * idx;
     p[0] = x[0]; p[1] = x[1]; p[2] = x[2];
   } else {
-    const AdsRec64 &r = ((const AdsRec64 *)E.ads)[idx];
+    const AdsRec64 &r = ((const AdsRec64 *)smem_at(fx().ads))[idx];
     p[0] = r.x; p[1] = r.y; p[2] = r.z;
   }
 }
 
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void atom_store(const Eng<MIXED, FLEX> &E, int m, int a, const double *p)
+__device__ RGPU_COLD void atom_store(Build<MIXED, FLEX> E, int m, int a, const double *p)
 {
-  const RgpuSys &S = *E.S;
+  const RgpuSys &S = fx().S;
   const int idx = m * S.natom + a;
   if (MIXED) {
-    double *x = E.S->ads_xyz + 3 * idx;
+    double *x = fx().S.ads_xyz + 3 * idx;
     x[0] = p[0]; x[1] = p[1]; x[2] = p[2];
     int xi, yi, zi;
     rgpu_fix3(S, p[0], p[1], p[2], xi, yi, zi);
-    ((int4 *)E.ads)[idx] = make_int4(xi, yi, zi, m * 16 + a);
+    ((int4 *)smem_at(fx().ads))[idx] = make_int4(xi, yi, zi, m * 16 + a);
   } else {
     AdsRec64 r;
     r.x = p[0]; r.y = p[1]; r.z = p[2]; r.tag = m * 16 + a;
-    ((AdsRec64 *)E.ads)[idx] = r;
+    ((AdsRec64 *)smem_at(fx().ads))[idx] = r;
   }
 }
 
-/* RotationAround{X,Y,Z}Axis, src/utils.c:876-936 */
-__device__ __forceinline__ void rotate_axis(double *c, int axis, double th)
+/* RotationAround{X,Y,Z}Axis, src/utils.c:876-936; cs, sn of the angle */
+__device__ __forceinline__ void rotate_axis(double *c, int axis, double cs, double sn)
 {
-  double cs, sn;
-  sincos(th, &sn, &cs);
   double x = c[0], y = c[1], z = c[2];
   if (axis == 0) { c[1] = cs * y + sn * z; c[2] = -sn * y + cs * z; }
   else if (axis == 1) { c[0] = cs * x - sn * z; c[2] = sn * x + cs * z; }
   else { c[0] = cs * x + sn * y; c[1] = -sn * x + cs * y; }
 }
 
-/* RandomArrayRotationMatrix (Shoemake), src/utils.c:835-874 */
-__device__ __forceinline__ void random_rotation(double x0, double y1, double y2, double R[3][3])
+__device__ RGPU_COLD double2 cold_sincos(double x)
+{
+  double sn, cs;
+  sincos(x, &sn, &cs);
+  return make_double2(sn, cs);
+}
+
+__device__ RGPU_COLD double2 cold_uniforms(const RgpuSys &S, uint64_t step, uint32_t blk)
+{
+  double u[2];
+  rgpu_uniform_pair(S.seed, S.sys_id, step, blk, u);
+  return make_double2(u[0], u[1]);
+}
+
+/* RandomArrayRotationMatrix (Shoemake), src/utils.c:835-874, in two parts:
+ * the quaternion, which needs the trigonometry, and its matrix */
+__device__ __forceinline__ void random_quaternion(double x0, double y1, double y2, double *u)
 {
   y1 *= 2.0 * M_PI;
   y2 *= 2.0 * M_PI;
   double r1 = sqrt(1.0 - x0), r2 = sqrt(x0);
-  double s1, c1, s2, c2;
-  sincos(y1, &s1, &c1);
-  sincos(y2, &s2, &c2);
-  double u0 = c2 * r2, u1 = s1 * r1, u2 = c1 * r1, u3 = s2 * r2;
+  const double2 a = cold_sincos(y1), b = cold_sincos(y2);   /* {sin, cos} */
+  u[0] = b.y * r2; u[1] = a.x * r1; u[2] = a.y * r1; u[3] = b.x * r2;
+}
+
+__device__ __forceinline__ void rotation_matrix(const double *u, double R[3][3])
+{
+  const double u0 = u[0], u1 = u[1], u2 = u[2], u3 = u[3];
   double ci = 2.0 * u0 * u0 - 1.0, ce = 2.0 * u0;
   R[0][0] = ci + 2.0 * u1 * u1;
   R[1][1] = ci + 2.0 * u2 * u2;
@@ -236,307 +329,575 @@ __device__ __forceinline__ void share(int n, int r, int c, int &lo, int &hi)
   hi = n * (r + 1) / c;
 }
 
-/* Pair evaluation of P positions on this CTA's share, then one cluster
- * barrier; the totals are read with gather(). All threads call. */
+__device__ __forceinline__ bool has_ewald(const RgpuSys &S) { return S.ewald && S.mol_charged; }
+
+/* ------------------------------------------------------------------------ */
+/* Random numbers, move type, rotation of a displacement and quaternions
+ * of the orientation trials of MC step `step`, into buffer db, by
+ * threads t0, t0 + nt, .... All of it depends on the step alone. The warps
+ * that wait for warp 0's bookkeeping draw it two steps ahead (a step's tables
+ * have to be visible when warp 0 starts it, in the same section in which it
+ * ends the step before), so it costs the step loop no time of its own. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void engine_eval(Eng<MIXED, FLEX> &E, int P, int pair_check, int ew_ns = 0)
+__device__ RGPU_COLD void draw_step(Build<MIXED, FLEX> E, uint64_t step, int db, int t0, int nt)
 {
-  Ctl &C = *E.ctl;
-  const long long t0 = clock64();
-  if (ew_ns) {
-    /* the Ewald sum of sites E.sites[0..ew_ns) rides along (a displacement,
-     * whose sites are known up front): phase tables now, each warp's share
-     * of the wave vectors right after its pair units, so it fills the
-     * units' tail; the CTA total goes to C.ewt[E.xb] as engine_ewald does */
-    ewald_phases<MIXED>(*E.S, E.sites, ew_ns, E.tab, E.kw);
-    if (threadIdx.x == 0) {
-      C.work[3] += (unsigned long long)(E.k1 - E.k0) * ew_ns;
-      C.work[4] += (unsigned long long)(E.k1 - E.k0);
+  const RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  /* thread i < nr: block i of the table; nr + j, j < 16: orientation trial j;
+   * j < 32: retrace orientation j - 16 of a reinsertion; j = 32: the move */
+  const int nr = RGPU_RND / 2;
+#pragma unroll 1
+  for (int i = t0; i < nr + 33; i += nt) {
+    const int j = i - nr, t = j & 15, old = j >> 4;
+    const uint32_t slot = (old ? SLOT_ORIENT_OLD : SLOT_ORIENT) + 4 * t;
+    double2 u = cold_uniforms(S, step, j < 0 ? (uint32_t)i : 0u);
+    if (j < 0) {
+      C.rnd[db][2 * i] = u.x;
+      C.rnd[db][2 * i + 1] = u.y;
+      continue;
     }
-    __syncthreads();
+    int mv = 0;
+    while (mv < 5 && u.x >= S.cum[mv]) mv++;
+    const bool turn = j == 32 && mv == 1;
+    if (j == 32) C.mvn[db] = mv;
+    else if (mv < 2 || t >= S.ntrial || S.natom == 1 || (old && mv != 4) || (FLEX && S.flexible)) continue;
+    u = cold_uniforms(S, step, j == 32 ? SLOT_VNEW >> 1 : slot >> 1);
+    if (turn) {
+      const double2 sc = cold_sincos((2.0 * u.x - 1.0) * S.max_rotation);
+      C.csn[db][0] = sc.y;
+      C.csn[db][1] = sc.x;
+    }
+    if (j == 32) continue;
+    const double2 v = cold_uniforms(S, step, (slot >> 1) + 1);
+    random_quaternion(u.x, u.y, v.x, fx().rot[db][old][t]);
   }
-  if (FLEX && E.S->use_grid && E.rank == 0) {
+}
+
+static_assert(SLOT_VNEW % 2 == 0 && SLOT_MOVE == 0 && SLOT_ORIENT % 2 == 0 && SLOT_ORIENT_OLD % 2 == 0,
+              "draw_step takes the first uniform of a block");
+
+/* ------------------------------------------------------------------------ */
+/* Placing a stage's positions and Ewald sites: thread i < P places position i,
+ * thread P + j site j (the moves' drivers below say what they are). */
+
+/* bead j of orientation trial t about o, with the trials' quaternions Q;
+ * keep >= 0: trial 0 is molecule keep's own orientation */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ int orientation_bead(Build<MIXED, FLEX> E, const double *o, const double (*Q)[4], int i,
+                                                int keep, double *p)
+{
+  const RgpuSys &S = fx().S;
+  const int nb = S.natom - 1, sb = S.start_bead;
+  const int t = small_div(i, nb), j = i - t * nb, a = j < sb ? j : j + 1;
+  if (t == 0 && keep >= 0) {
+    atom_xyz(E, keep, a, p);
+    return a;
+  }
+  const double c[3] = {S.mol_ref[a][0] - S.mol_ref[sb][0], S.mol_ref[a][1] - S.mol_ref[sb][1],
+                       S.mol_ref[a][2] - S.mol_ref[sb][2]};
+  double R[3][3];
+  rotation_matrix(Q[t], R);
+  p[0] = o[0] + c[0] * R[0][0] + c[1] * R[0][1] + c[2] * R[0][2];
+  p[1] = o[1] + c[0] * R[1][0] + c[1] * R[1][1] + c[2] * R[1][2];
+  p[2] = o[2] + c[0] * R[2][0] + c[1] * R[2][1] + c[2] * R[2][2];
+  return a;
+}
+
+/* atom a of the configuration chosen among the last evaluation's trials */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void chosen_atom(Build<MIXED, FLEX> E, int a, double *p)
+{
+  const RgpuSys &S = fx().S;
+  const Ctl &C = fx().C;
+  const int sb = S.start_bead;
+  if (a == sb) {
+    p[0] = C.first[0]; p[1] = C.first[1]; p[2] = C.first[2];
+  } else {
+    const BeadPos &b = fx().pos[C.sel * (S.natom - 1) + (a < sb ? a : a - 1)];
+    p[0] = b.x; p[1] = b.y; p[2] = b.z;
+  }
+}
+
+/* position of trial t of bead i of a chain grown onto beads x[0..i-1], with
+ * the stage's table of trial angles */
+template <int MIXED, bool FLEX>
+__device__ RGPU_COLD void chain_position(Build<MIXED, FLEX> E, uint64_t step, int stage, int i, int t,
+                                               const double (*x)[3], const double *ang, double *p)
+{
+  const RgpuSys &S = fx().S;
+  if (i == 0) {
+    rgpu_box_point(S, rgpu_uniform(S.seed, S.sys_id, step, chain_slot(stage, 0, t, 0)),
+                   rgpu_uniform(S.seed, S.sys_id, step, chain_slot(stage, 0, t, 1)),
+                   rgpu_uniform(S.seed, S.sys_id, step, chain_slot(stage, 0, t, 2)), p);
+  } else if (i == 1) {
+    chain_trial(S, x, i, [&](int d) { return rgpu_uniform(S.seed, S.sys_id, step, chain_slot(stage, i, t, d)); }, p);
+  } else {
+    const double *a = ang + RGPU_ANG_STRIDE * ((i - 2) * RGPU_MAX_TRIALS + t);
+    chain_place_trig(i >= 3 ? x[i - 3] : nullptr, x[i - 2], x[i - 1], S.bond, a[0], a[1], a[2], a[3], p);
+  }
+}
+
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void place(Build<MIXED, FLEX> E, const Stage &g, int i)
+{
+  const RgpuSys &S = fx().S;
+  const Ctl &C = fx().C;
+  const int na = S.natom, sb = S.start_bead, nf = S.ntrial_first, buf = g.buf, ph = g.ph, m = g.m;
+  const double *R = C.rnd[buf];
+  const bool site = i >= g.P;
+  const int j = site ? i - g.P : i;
+  double p[3], q = 0.0;
+  int a = 0, excl = m;
+  if (ph == PH_DISP) {
+    /* the new positions, then the old ones; the sites are the same with
+     * charges of opposite sign */
+    a = j < na ? j : j - na;
+    q = j < na ? S.mol_q[a] : -S.mol_q[a];
+    atom_xyz(E, m, a, p);
+    if (j < na) {
+      const double vnew = 2.0 * R[SLOT_VNEW] - 1.0;
+      int axis = (int)(3.0 * R[SLOT_AXIS]);
+      if (axis > 2) axis = 2;
+      if (g.mv == 0) {
+        const double d = vnew * S.max_translation;
+        if (axis == 0) p[0] += d;
+        else if (axis == 1) p[1] += d;
+        else p[2] += d;
+      } else {
+        double o[3];
+        atom_xyz(E, m, sb, o);
+        double c[3] = {p[0] - o[0], p[1] - o[1], p[2] - o[2]};
+        rotate_axis(c, axis, C.csn[buf][0], C.csn[buf][1]);
+        p[0] = c[0] + o[0]; p[1] = c[1] + o[1]; p[2] = c[2] + o[2];
+      }
+    }
+  } else if (FLEX && (ph == PH_GROW || ph == PH_RETRACE)) {
+    const uint64_t step = fx().step0 + (uint64_t)g.it;
+    if (j < g.k) {
+      a = g.ci;
+      excl = g.mv == 4 ? m : -1;
+      chain_position(E, step, 0, a, j, C.cp, fx_ang(), p);
+    } else {
+      /* retrace trials: bead a of the group, trial t in growth order; trial
+       * 0 of each bead is the old bead */
+      const double (*old)[3] = ph == PH_GROW ? C.co : C.cp;
+      const int nt = S.ntrial;
+      int t = j - g.k;
+      a = g.r0;
+      while (t >= (a == 0 ? nf : nt)) {
+        t -= a == 0 ? nf : nt;
+        a++;
+      }
+      if (t == 0) {
+        p[0] = old[a][0]; p[1] = old[a][1]; p[2] = old[a][2];
+      } else {
+        chain_position(E, step, 1, a, t, old, fx_ang() + (ph == PH_GROW ? RGPU_ANG_DOUBLES : 0), p);
+      }
+    }
+  } else if (ph == PH_SWAPEW || ph == PH_REINSEW) {
+    /* the chosen configuration, then a reinsertion's old one */
+    a = j < na ? j : j - na;
+    q = j < na && g.mv != 3 ? S.mol_q[a] : -S.mol_q[a];
+    if (j < na) chosen_atom(E, a, p);
+    else atom_xyz(E, m, a, p);
+  } else if (site) {
+    /* a one-evaluation deletion's removed molecule */
+    a = j;
+    q = -S.mol_q[a];
+    atom_xyz(E, m, a, p);
+  } else {
+    const bool insert = ph <= PH_SWAPEW && g.mv != 3, second = ph == PH_SWAP2 || ph == PH_REINS2;
+    const int n1 = second ? 0 : (ph == PH_REINS1 ? nf + 1 : nf);   /* first-bead positions */
+    if (insert) excl = -1;
+    if (j < n1) {
+      a = sb;
+      /* new first-bead trials; the old first bead is a deletion's trial 0
+       * and the position after a reinsertion's trials */
+      if (ph == PH_REINS1 ? j == nf : (!insert && j == 0)) atom_xyz(E, m, sb, p);
+      else rgpu_box_point(S, R[SLOT_FIRST + 3 * j + 2], R[SLOT_FIRST + 3 * j + 1], R[SLOT_FIRST + 3 * j + 0], p);
+    } else {
+      double o[3];
+      if (second) { o[0] = C.first[0]; o[1] = C.first[1]; o[2] = C.first[2]; }
+      else atom_xyz(E, m, sb, o);
+      a = orientation_bead(E, o, fx().rot[buf][ph == PH_REINS1], j - n1, insert || ph == PH_REINS2 ? -1 : m, p);
+    }
+  }
+  BeadPos b;
+  bead_set(b, S, p[0], p[1], p[2], a, excl);
+  if (!site) fx().pos[j] = b;
+  if (g.ns && (site || ph == PH_DISP)) {
+    EwSite &t = fx().sites[g.xs][j];
+    t.b = b;
+    t.q = q;
+  }
+}
+
+/* ------------------------------------------------------------------------ */
+/* The evaluation of a stage: pair sums of its positions on this CTA's share,
+ * the pending S_ads(k) update and the Ewald sum of its sites on this CTA's
+ * wave vectors, one cluster barrier; then the cluster's totals of every
+ * position (fx().tot) and of the Ewald sum (C.ew), each CTA's part added in rank
+ * order, and a block barrier. All threads call.
+ *
+ * The Ewald work follows the pair units and fills their tail (with a fixed
+ * share per warp a stage waited for the warps that had two pair units before
+ * theirs). On the mixed path it needs no phase table; the other paths build one
+ * per stage, after the pending update has used the last. */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void eval_stage(Eng<MIXED, FLEX> &E, const Stage &g)
+{
+  Ctl &C = fx().C;
+  RgpuSys &S = fx().S;
+  cg::cluster_group cl = cg::this_cluster();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const long long t0 = clock64();
+  const EwSite *sites = fx().sites[g.xs], *acc = fx().sites[g.xa & 1];
+  if (MIXED != 1) {
+    if (g.ap) {
+      ewald_apply_share<MIXED>(S, E.tab, E.kw, acc, g.ap, E.k0, E.k1, w);
+      if (g.ns) __syncthreads();
+    }
+    if (g.ns) {
+      ewald_phases<MIXED>(S, sites, g.ns, E.tab, E.kw);
+      __syncthreads();
+    }
+  }
+  if (g.ns && threadIdx.x == 0) {
+    C.work[0] += (unsigned long long)(E.k1 - E.k0) * g.ns;
+    C.work[1] += (unsigned long long)(E.k1 - E.k0);
+  }
+  double4 *part = fx().part[E.xb];
+  if (FLEX && S.use_grid && E.rank == 0) {
     /* host VDW from the bead types' energy grids (one CTA of the cluster):
      * 8 lanes per position, 4 positions per warp, before the pair units */
-    const int lane = threadIdx.x & 31;
-    for (int base = (threadIdx.x >> 5) * 4; base < P; base += (blockDim.x >> 5) * 4) {
+#pragma unroll 1
+    for (int base = w * 4; base < g.P; base += nw * 4) {
       const int p = base + (lane >> 3);
-      const bool live = p < P;
-      const double x[3] = {live ? E.pos[p].x : 0.0, live ? E.pos[p].y : 0.0, live ? E.pos[p].z : 0.0};
-      const double g = rgpu_grid_value8(E.S->grid[live ? E.pos[p].atom : 0], E.S->grid_geom, x, lane & 7, live);
-      if (live && (lane & 7) == 0) C.gv[p] = g;
-      if (E.S->use_coul_grid) {
+      const bool live = p < g.P;
+      const double x[3] = {live ? fx().pos[p].x : 0.0, live ? fx().pos[p].y : 0.0, live ? fx().pos[p].z : 0.0};
+      const double v = rgpu_grid_value8(S.grid[live ? fx().pos[p].atom : 0], S.grid_geom, x, lane & 7, live);
+      double vq = 0.0;
+      if (S.use_coul_grid) {
         /* real-space charge energy: the bead charge times the unit-charge
          * Coulomb grid (InterpolateCoulombGrid, src/grids.c:1200) */
-        const double q = live ? E.S->mol_q[E.pos[p].atom] : 0.0;
-        const double gq = rgpu_grid_value8(E.S->coul_grid, E.S->coul_geom, x, lane & 7, live && q != 0.0, false);
-        if (live && (lane & 7) == 0) C.gq[p] = q * gq;
+        const double q = live ? S.mol_q[fx().pos[p].atom] : 0.0;
+        vq = q * rgpu_grid_value8(S.coul_grid, S.coul_geom, x, lane & 7, live && q != 0.0, false);
+      }
+      if (live && (lane & 7) == 0) {
+        part[p].x = v;
+        part[p].y = vq;
+        if (p < g.check && v >= S.overlap) C.ovf[E.xb] = 1;
       }
     }
   }
-  const EvalPlan pl = eval_units<MIXED>(*E.S, E.sl, E.pos, P, pair_check, E.sc, RGPU_MAX_UNITS);
-  const int per = pl.cf + pl.ca;
-  double *ewred = E.red + E.xb * 2 * RGPU_MAX_WARPS;
-  if (ew_ns) ewald_energy_warps<MIXED>(*E.S, E.tab, E.kw, E.sites, ew_ns, E.k0, E.k1, ewred);
-  __syncthreads();
-  if (threadIdx.x == 0) C.next = 0;      /* unit counter of the next evaluation */
-  if (ew_ns && threadIdx.x < 32) {
-    /* this CTA's Ewald total (warp 0, fixed reduction order) */
-    const int nw = blockDim.x >> 5;
-    double a = 0.0, h = 0.0;
-    if (threadIdx.x < nw) {
-      a = ewred[2 * threadIdx.x];
-      h = ewred[2 * threadIdx.x + 1];
-    }
-    a = warp_sum(a);
-    h = warp_sum(h);
-    if (threadIdx.x == 0) {
-      C.ewt[E.xb][0] = a;
-      C.ewt[E.xb][1] = h;
+  if (g.P) {
+    E.sc.ovf = &C.ovf[E.xb];
+    E.sc.part = part;
+    E.sl.ads_lo = g.alo;
+    E.sl.ads_hi = g.ahi;
+    const int pl = g.plan[E.rank];
+    eval_units<MIXED>(S, E.sl, fx().pos, g.P, g.check, E.sc, pl & 0xffff, pl >> 16, g.mf, g.ma);
+  }
+  if (g.ns || (MIXED == 1 && g.ap)) {
+    /* the shares of the wave vectors, one per warp of the block, taken as the
+     * warps run out of pair units; the last to finish adds them up in order */
+    for (;;) {
+      int u = 0;
+      if (lane == 0) u = atomicAdd(&C.nextk, 1);
+      u = __shfl_sync(RGPU_FULL, u, 0);
+      if (u >= nw) break;
+      if (MIXED == 1 && g.ap) ewald_apply_share<MIXED>(S, E.tab, E.kw, acc, g.ap, E.k0, E.k1, u);
+      if (!g.ns) continue;
+      ewald_energy_share<MIXED>(S, E.tab, E.kw, sites, g.ns, E.k0, E.k1, u, fx().red);
+      int d = 0;
+      if (lane == 0) {
+        __threadfence_block();
+        d = atomicAdd(&C.ewdone, 1);
+        __threadfence_block();
+      }
+      if (__shfl_sync(RGPU_FULL, d, 0) == nw - 1) {
+        const double ea = warp_sum(lane < nw ? fx().red[2 * lane] : 0.0), eh = warp_sum(lane < nw ? fx().red[2 * lane + 1] : 0.0);
+        if (lane == 0) {
+          C.ewt[E.xb][0] = ea;
+          C.ewt[E.xb][1] = eh;
+          C.ewdone = 0;
+        }
+      }
     }
   }
-  /* this CTA's sum per position, units in order */
-  PosSum *ps = E.part + E.xb * RGPU_MAX_POS;
-  for (int p = threadIdx.x; p < P; p += blockDim.x) {
-    double hv = 0.0, hc = 0.0, av = 0.0, ac = 0.0;
-    int ov = 0;
-    for (int c = 0; c < per; c++) {
-      const int u = p * per + c;
-      if (c < pl.cf) { hv += E.uv[u]; hc += E.uc[u]; }
-      else { av += E.uv[u]; ac += E.uc[u]; }
-      ov |= E.uo[u];
+  cl.sync();
+  /* term k of position p: thread 4 p + k */
+  const bool grids = FLEX && S.use_grid;
+#pragma unroll 1
+  for (int e = threadIdx.x; e < 4 * g.P; e += blockDim.x) {
+    const double *own = (const double *)part + e;
+    const bool host = (e & 2) == 0;
+    double t = 0.0;
+#pragma unroll 1
+    for (int q0 = 0; q0 < E.csize; q0 += 8) {
+      double v[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int q = q0 + j;
+        v[j] = 0.0;
+        if (q < E.csize) {
+          const int pl = g.plan[q];
+          if (host ? (grids ? q == 0 : (pl & 0xffff) != 0) : (pl >> 16) != 0)
+            v[j] = E.csize > 1 ? *cl.map_shared_rank(own, q) : *own;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) t += v[j];
     }
-    if (FLEX && E.S->use_grid && E.rank == 0) {
-      const double g = C.gv[p];
-      hv += g;
-      ov |= g >= E.S->overlap;
-      if (E.S->use_coul_grid) hc += C.gq[p];
+    ((double *)fx().tot)[e] = t;
+  }
+  if (w == nw - 1) {
+    /* the last warp: Ewald totals (lane q: CTA q's) and the overlap flag */
+    double2 t = make_double2(0.0, 0.0);
+    int o = 0;
+    if (lane < E.csize) {
+      const double2 *ow = (const double2 *)C.ewt[E.xb];
+      const int *of = &C.ovf[E.xb];
+      if (E.csize > 1) {
+        ow = cl.map_shared_rank(ow, lane);
+        of = cl.map_shared_rank(of, lane);
+      }
+      if (g.ns) t = *ow;
+      o = *of;
     }
-    ps[p].v[0] = hv; ps[p].v[1] = hc; ps[p].v[2] = av; ps[p].v[3] = ac;
-    ps[p].ov = ov;
+    o = __any_sync(RGPU_FULL, o);
+    double ea = 0.0, eh = 0.0;
+#pragma unroll 1
+    for (int q = 0; g.ns && q < E.csize; q++) {
+      ea += __shfl_sync(RGPU_FULL, t.x, q);
+      eh += __shfl_sync(RGPU_FULL, t.y, q);
+    }
+    if (lane == 0) {
+      C.ew[0] = ea;
+      C.ew[1] = eh;
+      C.ov = o;
+    }
   }
-  cg::this_cluster().sync();
-  if (threadIdx.x == 0) C.cyc[0] += clock64() - t0;
-}
-
-/* Totals of position p of the last evaluation (buffer b): the CTAs' sums
- * added in rank order. */
-template <int MIXED, bool FLEX>
-__device__ __forceinline__ void gather(const Eng<MIXED, FLEX> &E, int b, int p, double *r, int &ov)
-{
-  cg::cluster_group cl = cg::this_cluster();
-  const PosSum *own = E.part + b * RGPU_MAX_POS + p;
-  r[0] = r[1] = r[2] = r[3] = 0.0;
-  ov = 0;
-  for (int q = 0; q < E.csize; q++) {
-    const PosSum *ps = E.csize > 1 ? cl.map_shared_rank(own, q) : own;
-    const double2 a = *(const double2 *)&ps->v[0], c = *(const double2 *)&ps->v[2];
-    r[0] += a.x; r[1] += a.y; r[2] += c.x; r[3] += c.y;
-    ov |= ps->ov;
-  }
-}
-
-/* Ewald sum over this CTA's wave vectors for the sites in E.sites[0..ns),
- * warp partials left in E.red[b]; one cluster barrier. All threads call. */
-template <int MIXED, bool FLEX>
-__device__ __forceinline__ void engine_ewald(Eng<MIXED, FLEX> &E, int ns)
-{
-  Ctl &C = *E.ctl;
-  const long long t0 = clock64();
-  ewald_phases<MIXED>(*E.S, E.sites, ns, E.tab, E.kw);
   if (threadIdx.x == 0) {
-    C.work[3] += (unsigned long long)(E.k1 - E.k0) * ns;
-    C.work[4] += (unsigned long long)(E.k1 - E.k0);
+    C.next = C.nextk = 0;       /* counters of the next evaluation */
+    C.ovf[E.xb ^ 1] = 0;        /* read last before this stage's cluster barrier */
+    C.cyc[g.P ? 0 : 1] += clock64() - t0;
   }
+  E.xb ^= 1;
   __syncthreads();
-  double *red = E.red + E.xb * 2 * RGPU_MAX_WARPS;
-  ewald_energy_warps<MIXED>(*E.S, E.tab, E.kw, E.sites, ns, E.k0, E.k1, red);
-  __syncthreads();
-  /* this CTA's total (warp 0, fixed reduction order) */
-  if (threadIdx.x < 32) {
-    const int nw = blockDim.x >> 5;
-    double a = 0.0, h = 0.0;
-    if (threadIdx.x < nw) {
-      a = red[2 * threadIdx.x];
-      h = red[2 * threadIdx.x + 1];
-    }
-    a = warp_sum(a);
-    h = warp_sum(h);
-    if (threadIdx.x == 0) {
-      C.ewt[E.xb][0] = a;
-      C.ewt[E.xb][1] = h;
-    }
-  }
-  cg::this_cluster().sync();
-  if (threadIdx.x == 0) C.cyc[1] += clock64() - t0;
 }
 
-/* cluster total of the last Ewald sum (buffer b) */
+/* The functions from here to end_stage are run by warp 0 of every CTA, all
+ * lanes converged, where they do not say otherwise. E is the handle's copy in
+ * shared memory, which warp 0 alone updates. Every CTA of the cluster holds
+ * the same totals and takes the same decisions. */
+
+__device__ __forceinline__ int stage_after(int c, int n) { return c + n >= 3 ? c + n - 3 : c + n; }
+
+/* the stage just evaluated */
+__device__ __forceinline__ const Stage &cur() { return fx().C.st[fx().C.cur]; }
+
+/* Describes stage n, which follows stage c: what it evaluates, and the chunks
+ * of a position in every CTA (lane q: CTA q). ns > 0: its Ewald sites take the
+ * buffer that the last sites, whose S(k) update may be pending, do not use. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void gather_ewald(const Eng<MIXED, FLEX> &E, int b, double &ea, double &eh)
+__device__ RGPU_COLD void fill_stage(Build<MIXED, FLEX> E, Stage &n, const Stage &c, int ph, int P, int check, int ns)
 {
-  cg::cluster_group cl = cg::this_cluster();
-  ea = eh = 0.0;
-  const double *own = &E.ctl->ewt[b][0];
-  for (int q = 0; q < E.csize; q++) {
-    const double *t = E.csize > 1 ? cl.map_shared_rank(own, q) : own;
-    ea += t[0];
-    eh += t[1];
+  const RgpuSys &S = fx().S;
+  const int lane = threadIdx.x & 31, q = lane;
+  if (P && q < fx().csize) {
+    const unsigned mc = c_magic[fx().csize];
+    const int nads = fx().C.nads;
+    int t0 = S.ntile * q, t1 = S.ntile * (q + 1), a0 = nads * q, a1 = nads * (q + 1);
+    if (fx().csize > 1) {
+      t0 = (int)__umulhi((unsigned)t0, mc);
+      t1 = (int)__umulhi((unsigned)t1, mc);
+      a0 = (int)__umulhi((unsigned)a0, mc);
+      a1 = (int)__umulhi((unsigned)a1, mc);
+    }
+    if (FLEX && S.use_grid) t1 = t0;
+    const EvalPlan pl = eval_plan(P, t1 - t0, a1 - a0, blockDim.x >> 5, RGPU_MAX_UNITS, 2);
+    n.plan[q] = pl.cf | pl.ca << 16;
+    if (q == fx().rank) {
+      n.alo = a0;
+      n.ahi = a1;
+      n.mf = c_magic[pl.cf];
+      n.ma = c_magic[pl.ca];
+    }
+  }
+  if (lane == 0) {
+    n.ph = ph;
+    n.P = P;
+    n.check = check;
+    n.ns = ns;
+    n.xs = ns ? c.xs ^ 1 : c.xs;
+    n.db = -1;
+    n.first = 0;
+    n.k = n.rP = 0;
+    n.mv = c.mv;
+    n.m = c.m;
+    n.one = c.one;
+    n.buf = c.buf;
+    n.it = c.it;
   }
 }
 
-/* Warp 0: Rosenbluth bookkeeping of n trials (lane t = trial t, nb beads each
- * at positions t*nb + j of buffer b). First bead (nb = 1, first = true):
- * overlap when any energy reaches the criterion (src/cbmc.c:699-701);
- * orientations: when a bead's host VDW energy does (src/cbmc.c:1210-1215).
- * LJ biasing (src/cbmc.c:734-735, :1432-1436). Selection as
- * SelectTrialPosition (src/cbmc.c:563-599). Lane 0 leaves the weight sum
- * (w_sum = sum exp(bf)), the selected trial and its energies in Ctl. */
+/* the stage that follows in the same move */
+__device__ __forceinline__ Stage &next_of() { return fx().C.st[stage_after(fx().C.cur, 1)]; }
+
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void cbmc_trials(const Eng<MIXED, FLEX> &E, int b, int n, int nb, bool first, bool select, double usel,
-                            double &w_sum, int &sel, double *usum, int &any, int off = 0, double *w_sel = nullptr)
+__device__ __forceinline__ void next_stage(Build<MIXED, FLEX> E, int ph, int P, int check, int ns)
+{
+  fill_stage(E, next_of(), cur(), ph, P, check, ns);
+}
+
+/* an accepted move's sites are added to S_ads(k) in the next stage (end_stage
+ * passes them on) */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void accept_sites(Build<MIXED, FLEX> E, int ns)
+{
+  if (has_ewald(fx().S) && threadIdx.x == 0) fx().C.accept = ns;
+}
+
+__device__ RGPU_COLD double cold_exp(double x) { return exp(x); }
+
+/* exp(x) and exp(y), by two lanes */
+__device__ __forceinline__ void exp_pair(double x, double y, double &ex, double &ey)
+{
+  const double r = cold_exp((threadIdx.x & 1) ? y : x);
+  ex = __shfl_sync(RGPU_FULL, r, 0);
+  ey = __shfl_sync(RGPU_FULL, r, 1);
+}
+
+/* inclusive sum over the lanes up to each one */
+__device__ __forceinline__ double warp_scan(double v)
 {
   const int lane = threadIdx.x & 31;
-  const RgpuSys &S = *E.S;
-  double e[4] = {0.0, 0.0, 0.0, 0.0};
-  int ov = 0;
-  double bf = 0.0;
-  if (lane < n) {
-    for (int j = 0; j < nb; j++) {
-      double r[4];
-      int o;
-      gather(E, b, off + lane * nb + j, r, o);
-      if (first) ov |= (r[0] >= S.overlap || r[1] >= S.overlap || r[2] >= S.overlap || r[3] >= S.overlap);
-      else ov |= (r[0] >= S.overlap);
-      for (int k = 0; k < 4; k++) e[k] += r[k];
-    }
-    bf = -S.beta * (e[0] + e[2]);
-  }
-  const bool valid = lane < n && !ov;
-  const double w = valid ? exp(bf) : 0.0;
-  double largest = valid ? bf : -DBL_MAX;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) largest = fmax(largest, __shfl_xor_sync(RGPU_FULL, largest, o));
-  const double ws = valid ? exp(bf - largest) : 0.0;
-  const unsigned okmask = __ballot_sync(RGPU_FULL, valid);
-  any = okmask != 0u;
-  /* the sums run in trial order, as the reference's loops do */
-  double wsum = 0.0, shsum = 0.0;
-  for (int t = 0; t < n; t++) {
-    wsum += __shfl_sync(RGPU_FULL, w, t);
-    shsum += __shfl_sync(RGPU_FULL, ws, t);
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(RGPU_FULL, v, o);
+    if (lane >= o) v += y;
   }
+  return v;
+}
+
+/* SelectTrialPosition (src/cbmc.c:563-599) among the weights w of lanes < n,
+ * cum their sums up to each lane: the first trial whose cumulative weight
+ * reaches u times their sum */
+__device__ __forceinline__ int select_trial(double w, double cum, int n, double u)
+{
+  const int lane = threadIdx.x & 31;
+  const double target = u * __shfl_sync(RGPU_FULL, cum, 31);
+  const unsigned hit = __ballot_sync(RGPU_FULL, lane < n && w > 0.0 && !(cum < target));
+  return hit ? __ffs(hit) - 1 : n - 1;
+}
+
+/* Rosenbluth bookkeeping of n trials (lane t = trial t, nb beads each at
+ * positions off + t*nb + j) into out. First bead (nb = 1, first = true):
+ * overlap when any energy reaches the criterion (src/cbmc.c:699-701);
+ * orientations: when a bead's host VDW energy does (src/cbmc.c:1210-1215).
+ * LJ biasing (src/cbmc.c:734-735, :1432-1436). select: a trial is chosen with
+ * usel, else trial 0 is. */
+template <int MIXED, bool FLEX>
+__device__ RGPU_COLD void cbmc_trials(Build<MIXED, FLEX> E, int off, int n, int nb, bool first, bool select, double usel,
+                                      Trials *out)
+{
+  const int lane = threadIdx.x & 31;
+  const RgpuSys &S = fx().S;
+  double4 e = make_double4(0.0, 0.0, 0.0, 0.0);
+  int ov = lane >= n;
+  if (lane < n)
+#pragma unroll 1
+    for (int j = 0; j < nb; j++) {
+      const double4 r = fx().tot[off + lane * nb + j];
+      ov |= r.x >= S.overlap || (first && (r.y >= S.overlap || r.z >= S.overlap || r.w >= S.overlap));
+      e.x += r.x; e.y += r.y; e.z += r.z; e.w += r.w;
+    }
+  const double bf = -S.beta * (e.x + e.z);
+  const double w = ov ? 0.0 : cold_exp(bf);
+  const bool any = __any_sync(RGPU_FULL, !ov);
+  const double cum = warp_scan(w), w_sum = __shfl_sync(RGPU_FULL, cum, 31);
   int s = 0;
   if (select && any) {
-    const double target = usel * shsum;
-    double cum = __shfl_sync(RGPU_FULL, ws, 0);
-    while (cum < target && s < n - 1) {
-      s++;
-      cum += __shfl_sync(RGPU_FULL, ws, s);
+    if (w_sum > 1e-200 && w_sum < 1e200) {
+      s = select_trial(w, cum, n, usel);
+    } else {
+      /* the weights leave FP64's range: relative to the largest, as
+       * SelectTrialPosition forms them */
+      double largest = ov ? -DBL_MAX : bf;
+#pragma unroll 1
+      for (int o = 16; o > 0; o >>= 1) largest = fmax(largest, __shfl_xor_sync(RGPU_FULL, largest, o));
+      const double ws = ov ? 0.0 : cold_exp(bf - largest);
+      s = select_trial(ws, warp_scan(ws), n, usel);
     }
   }
-  w_sum = wsum;
-  sel = s;
-  for (int k = 0; k < 4; k++) usum[k] = __shfl_sync(RGPU_FULL, e[k], s);
-  const double ws_sel = __shfl_sync(RGPU_FULL, w, s);
-  if (w_sel) *w_sel = ws_sel;
+  if (lane == s) {
+    out->w_sum = w_sum;
+    out->w_sel = w;
+    out->e[0] = e.x; out->e[1] = e.y; out->e[2] = e.z; out->e[3] = e.w;
+    out->sel = s;
+    out->any = any;
+  }
+  __syncwarp();
+}
+
+/* adds sgn times the energies u and the Fourier terms to the running totals
+ * (lane 0) */
+__device__ __forceinline__ void add_energies(Ctl &C, double sgn, const double *u, double d_host, double d_ads)
+{
+  C.energy[RGPU_E_HOST_VDW] += sgn * u[0];
+  C.energy[RGPU_E_HOST_REAL] += sgn * u[1];
+  C.energy[RGPU_E_ADS_VDW] += sgn * u[2];
+  C.energy[RGPU_E_ADS_REAL] += sgn * u[3];
+  C.energy[RGPU_E_HOST_FOURIER] += d_host;
+  C.energy[RGPU_E_ADS_FOURIER] += d_ads;
 }
 
 /* ------------------------------------------------------------------------ */
 /* translation (mv=0) and rotation (mv=1):
- * TranslationMoveAdsorbate src/mc_moves.c:1529-1762, RotationMoveAdsorbate :2636 */
+ * TranslationMoveAdsorbate src/mc_moves.c:1529-1762, RotationMoveAdsorbate :2636.
+ * One stage: the na new positions, the na old ones, the Ewald sum. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void step_displace(Eng<MIXED, FLEX> &E, int mv)
+__device__ __forceinline__ void end_displace(Build<MIXED, FLEX> E, int buf)
 {
-  RgpuSys &S = *E.S;
-  Ctl &C = *E.ctl;
-  const double *R = E.rnd;
-  const int na = S.natom, nmol = C.nmol;
-  int m = (int)(R[SLOT_MOLECULE] * nmol);
-  if (m >= nmol) m = nmol - 1;
-  const double vnew = 2.0 * R[SLOT_VNEW] - 1.0;
-  int axis = (int)(3.0 * R[SLOT_AXIS]);
-  if (axis > 2) axis = 2;
-  if (threadIdx.x < na) {
-    const int a = threadIdx.x;
-    double o[3], n[3];
-    atom_xyz(E, m, a, o);
-    if (mv == 0) {
-      n[0] = o[0]; n[1] = o[1]; n[2] = o[2];
-      n[axis] += vnew * S.max_translation;
-    } else {
-      double sb[3];
-      atom_xyz(E, m, S.start_bead, sb);
-      double c[3] = {o[0] - sb[0], o[1] - sb[1], o[2] - sb[2]};
-      rotate_axis(c, axis, vnew * S.max_rotation);
-      n[0] = c[0] + sb[0]; n[1] = c[1] + sb[1]; n[2] = c[2] + sb[2];
-    }
-    bead_set(E.pos[a], S, n[0], n[1], n[2], a, m);
-    bead_set(E.pos[na + a], S, o[0], o[1], o[2], a, m);
-    E.sites[a].b = E.pos[a];
-    E.sites[a].q = S.mol_q[a];
-    E.sites[na + a].b = E.pos[na + a];
-    E.sites[na + a].q = -S.mol_q[a];
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int na = S.natom, lane = threadIdx.x;
+  if (C.ov) {
+    if (lane == 0) C.cnt[RGPU_CNT_OVERLAP]++;
+    return;
   }
-  __syncthreads();
-  const bool ew = S.ewald && S.mol_charged;
-  engine_eval(E, 2 * na, na, ew ? 2 * na : 0);
-  const int be = E.xb;
-  E.xb ^= 1;
-  if (threadIdx.x < 32) {
-    /* lane a: totals of new position a and old position a (a < na <= 8) */
-    const int a = threadIdx.x;
-    double rn[4] = {0.0, 0.0, 0.0, 0.0}, ro[4] = {0.0, 0.0, 0.0, 0.0};
-    int o1 = 0, o2 = 0;
-    if (a < na) {
-      gather(E, be, a, rn, o1);
-      gather(E, be, na + a, ro, o2);
-    }
-    const int ov = __any_sync(RGPU_FULL, o1);
-    double dl[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int j = 0; j < na; j++)
-      for (int k = 0; k < 4; k++)
-        dl[k] += __shfl_sync(RGPU_FULL, rn[k], j) - __shfl_sync(RGPU_FULL, ro[k], j);
-    if (a == 0) {
-      C.fail = ov;
-      for (int k = 0; k < 4; k++) C.dl[k] = dl[k];
-      if (ov) C.cnt[RGPU_CNT_OVERLAP]++;
-    }
+  /* lane k < 4: change of energy term k */
+  const double *tot = (const double *)fx().tot + (lane & 3);
+  double dl = 0.0;
+#pragma unroll 1
+  for (int j = 0; j < na; j++) dl += tot[4 * j] - tot[4 * (na + j)];
+  double d_ads = 0.0, d_host = 0.0;
+  if (has_ewald(S)) {
+    /* the exclusion energy of a rigid molecule is the same before and
+     * after the displacement (the reference's difference of the two is
+     * zero up to rounding) */
+    ewald_finish(S, C.ew[0], C.ew[1], S.excl_mol, S.excl_mol, 0, 0.0, d_ads, d_host);
   }
-  __syncthreads();
-  if (C.fail) return;
-  if (threadIdx.x == 0) {
-    double d_ads = 0.0, d_host = 0.0;
-    if (ew) {
-      double ea, eh;
-      gather_ewald(E, be, ea, eh);
-      /* the exclusion energy of a rigid molecule is the same before and
-       * after the displacement (the reference's difference of the two is
-       * zero up to rounding) */
-      ewald_finish(S, ea, eh, S.excl_mol, S.excl_mol, 0, 0.0, d_ads, d_host);
-    }
-    double du = C.dl[0] + C.dl[1] + C.dl[2] + C.dl[3] + d_ads + d_host;
-    double pacc = exp(-S.beta * du);
+  double u[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) u[k] = __shfl_sync(RGPU_FULL, dl, k);
+  const double du = u[0] + u[1] + u[2] + u[3] + d_ads + d_host;
+  const double pacc = cold_exp(-S.beta * du);
+  const bool accept = C.rnd[buf][SLOT_ACCEPT] < pacc;
+  if (lane == 0) {
     if (!isfinite(du)) C.status |= RGPU_ERR_NONFINITE;
-    C.accept = R[SLOT_ACCEPT] < pacc;
-    if (C.accept) {
-      C.cnt[RGPU_CNT_ACCEPT + mv]++;
-      C.energy[RGPU_E_HOST_VDW] += C.dl[0];
-      C.energy[RGPU_E_HOST_REAL] += C.dl[1];
-      C.energy[RGPU_E_ADS_VDW] += C.dl[2];
-      C.energy[RGPU_E_ADS_REAL] += C.dl[3];
-      C.energy[RGPU_E_HOST_FOURIER] += d_host;
-      C.energy[RGPU_E_ADS_FOURIER] += d_ads;
+    if (accept) {
+      C.cnt[RGPU_CNT_ACCEPT + cur().mv]++;
+      add_energies(C, 1.0, u, d_host, d_ads);
     }
   }
-  __syncthreads();
-  if (C.accept) {
-    if (threadIdx.x < na) {
-      double p[3] = {E.pos[threadIdx.x].x, E.pos[threadIdx.x].y, E.pos[threadIdx.x].z};
-      atom_store(E, m, threadIdx.x, p);
+  if (accept) {
+    if (lane < na) {
+      const double p[3] = {fx().pos[lane].x, fx().pos[lane].y, fx().pos[lane].z};
+      atom_store(E, cur().m, lane, p);
     }
-    if (ew) ewald_apply<MIXED>(S, E.tab, E.kw, E.sites, 2 * na, E.k0, E.k1);
-    __syncthreads();
+    accept_sites(E, 2 * na);
   }
 }
 
@@ -548,237 +909,134 @@ __device__ __forceinline__ void step_displace(Eng<MIXED, FLEX> &E, int mv)
  * HandleFirstBead :623-795, Rosen/RosenOld :2762-2926, the rigid-group branch
  * of GenerateTrialOrientationsSimpleSphere :1480-1578 and
  * ComputeExternalEnergies :1154-1478, LJ biasing; acceptance of
- * SwapAddAdsorbateMove src/mc_moves.c:7016 and SwapRemoveAdsorbateMove :7228. */
+ * SwapAddAdsorbateMove src/mc_moves.c:7016 and SwapRemoveAdsorbateMove :7228.
+ * Stages: first-bead trials, orientation trials, Ewald sum. A deletion retraces
+ * the old molecule: its first bead and orientation are trial 0 of each stage,
+ * known up front, so both stages' trials and the Ewald sum of the removed
+ * molecule go into one evaluation (first-bead trials at positions 0..nf,
+ * orientation t's beads at nf + t*nb + j) when they fit. */
+/* acceptance of an insertion, deletion or Widom sample whose weight and
+ * energies stand in C */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void step_swap(Eng<MIXED, FLEX> &E, bool insert, bool widom = false)
+__device__ RGPU_COLD void accept_swap(Build<MIXED, FLEX> E, int buf)
 {
-  RgpuSys &S = *E.S;
-  Ctl &C = *E.ctl;
-  if (widom && threadIdx.x == 0) C.sums[RGPU_SUM_WIDOM_N] += 1.0;   /* overlap samples count with weight 0 */
-  const int na = S.natom, sb = S.start_bead, nmol = C.nmol;
-  const int nf = S.ntrial_first, nt = S.ntrial;
-  int m = nmol;
-  if (!insert) {
-    m = (int)(E.rnd[SLOT_MOLECULE] * nmol);
-    if (m >= nmol) m = nmol - 1;
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int mv = cur().mv, nmol = C.nmol, na = S.natom, m = cur().m;
+  const bool insert = mv != 3, widom = mv == 5;
+  /* LJ-biasing correction, src/cbmc.c:3171-3178 / :3044-3051 */
+  double d_ads = 0.0, d_host = 0.0, lj, f;
+  if (has_ewald(S)) {
+    const double ex = S.excl_mol;      /* rigid molecule */
+    const double net = nmol * S.mol_charge;
+    if (insert) ewald_finish(S, C.ew[0], C.ew[1], ex, 0.0, 1, net, d_ads, d_host);
+    else ewald_finish(S, C.ew[0], C.ew[1], 0.0, ex, -1, net, d_ads, d_host);
   }
-  const int exclude = insert ? -1 : m;
-  const int nb = na - 1;   /* beads grown per orientation trial */
-  const bool ew = S.ewald && S.mol_charged;
-  /* a deletion retraces the old molecule: its first bead and orientation
-   * are trial 0 of each stage, known up front, so both stages' trials and
-   * the Ewald sum of the removed molecule go into one evaluation (first-bead
-   * trials at positions 0..nf, orientation t's beads at nf + t*nb + j) */
-  const bool one = !insert && nf + (na > 1 ? nt * nb : 0) <= RGPU_MAX_POS;
-  /* first-bead trials */
-  if (threadIdx.x < nf) {
-    const int i = threadIdx.x;
-    double p[3];
-    if (!insert && i == 0) {
-      atom_xyz(E, m, sb, p);
-    } else {
-      rgpu_box_point(S, E.rnd[SLOT_FIRST + 3 * i + 2], E.rnd[SLOT_FIRST + 3 * i + 1], E.rnd[SLOT_FIRST + 3 * i + 0],
-                     p);
-    }
-    bead_set(E.pos[i], S, p[0], p[1], p[2], sb, exclude);
-  }
-  if (one) {
-    /* the retrace orientations about the old first bead (trial 0: the old
-     * one) and the removed molecule's Ewald sites (nf, nt <= 16, na <= 8;
-     * blocks have at least 64 threads) */
-    if (na > 1 && threadIdx.x >= 32 && threadIdx.x < 32 + nt) {
-      const int t = threadIdx.x - 32;
-      double o[3];
-      atom_xyz(E, m, sb, o);
-      double R[3][3];
-      if (t > 0)
-        random_rotation(E.rnd[SLOT_ORIENT + 4 * t + 0], E.rnd[SLOT_ORIENT + 4 * t + 1],
-                        E.rnd[SLOT_ORIENT + 4 * t + 2], R);
-      int j = 0;
-      for (int a = 0; a < na; a++) {
-        if (a == sb) continue;
-        double p[3];
-        if (t == 0) {
-          atom_xyz(E, m, a, p);
-        } else {
-          const double c[3] = {S.mol_ref[a][0] - S.mol_ref[sb][0], S.mol_ref[a][1] - S.mol_ref[sb][1],
-                               S.mol_ref[a][2] - S.mol_ref[sb][2]};
-          p[0] = o[0] + c[0] * R[0][0] + c[1] * R[0][1] + c[2] * R[0][2];
-          p[1] = o[1] + c[0] * R[1][0] + c[1] * R[1][1] + c[2] * R[1][2];
-          p[2] = o[2] + c[0] * R[2][0] + c[1] * R[2][1] + c[2] * R[2][2];
-        }
-        bead_set(E.pos[nf + t * nb + j], S, p[0], p[1], p[2], a, exclude);
-        j++;
-      }
-    }
-    if (threadIdx.x >= 48 && threadIdx.x < 48 + na) {
-      const int a = threadIdx.x - 48;
-      double p[3];
-      atom_xyz(E, m, a, p);
-      bead_set(E.sites[a].b, S, p[0], p[1], p[2], a, exclude);
-      E.sites[a].q = -S.mol_q[a];
-    }
-  }
-  __syncthreads();
-  engine_eval(E, one ? nf + (na > 1 ? nt * nb : 0) : nf, 0, one && ew ? na : 0);
-  int b1 = E.xb;
-  E.xb ^= 1;
-  if (threadIdx.x < 32) {
-    double wsum, u[4];
-    int sel, any;
-    cbmc_trials(E, b1, nf, 1, true, insert, E.rnd[SLOT_FIRST_SELECT], wsum, sel, u, any);
-    if (threadIdx.x == 0) {
-      C.rosen = wsum / (double)nf;
-      C.fail = !any || (insert && C.rosen < 1e-150);
-      C.sel = sel;
-      for (int k = 0; k < 4; k++) C.u[k] = u[k];
-      C.first = E.pos[sel];
-      if (C.fail) C.cnt[RGPU_CNT_OVERLAP]++;
-    }
-    if (one && na > 1 && any) {
-      /* the retrace orientations (trial 0 is the old one, not selected) */
-      cbmc_trials(E, b1, nt, nb, false, false, E.rnd[SLOT_ORIENT_SELECT], wsum, sel, u, any, nf);
-      if (threadIdx.x == 0) {
-        if (!any) C.fail = 1;
-        else {
-          C.rosen *= wsum / (double)nt;
-          for (int k = 0; k < 4; k++) C.u[k] += u[k];
-        }
-        C.sel = sel;
-        if (C.fail) C.cnt[RGPU_CNT_OVERLAP]++;
-      }
-    }
-  }
-  __syncthreads();
-  if (C.fail) return;
-  if (na > 1 && !one) {
-    const BeadPos first = C.first;
-    if (threadIdx.x < nt) {
-      const int t = threadIdx.x;
-      if (!insert && t == 0) {
-        int j = 0;
-        for (int a = 0; a < na; a++) {
-          if (a == sb) continue;
-          double p[3];
-          atom_xyz(E, m, a, p);
-          bead_set(E.pos[t * nb + j], S, p[0], p[1], p[2], a, exclude);
-          j++;
-        }
-      } else {
-        double R[3][3];
-        random_rotation(E.rnd[SLOT_ORIENT + 4 * t + 0], E.rnd[SLOT_ORIENT + 4 * t + 1],
-                        E.rnd[SLOT_ORIENT + 4 * t + 2], R);
-        int j = 0;
-        for (int a = 0; a < na; a++) {
-          if (a == sb) continue;
-          double c[3] = {S.mol_ref[a][0] - S.mol_ref[sb][0], S.mol_ref[a][1] - S.mol_ref[sb][1],
-                         S.mol_ref[a][2] - S.mol_ref[sb][2]};
-          double p[3];
-          p[0] = first.x + c[0] * R[0][0] + c[1] * R[0][1] + c[2] * R[0][2];
-          p[1] = first.y + c[0] * R[1][0] + c[1] * R[1][1] + c[2] * R[1][2];
-          p[2] = first.z + c[0] * R[2][0] + c[1] * R[2][1] + c[2] * R[2][2];
-          bead_set(E.pos[t * nb + j], S, p[0], p[1], p[2], a, exclude);
-          j++;
-        }
-      }
-    }
-    __syncthreads();
-    engine_eval(E, nt * nb, 0);
-    const int b2 = E.xb;
-    E.xb ^= 1;
-    if (threadIdx.x < 32) {
-      double wsum, u[4];
-      int sel, any;
-      cbmc_trials(E, b2, nt, nb, false, insert, E.rnd[SLOT_ORIENT_SELECT], wsum, sel, u, any);
-      if (threadIdx.x == 0) {
-        if (!any) C.fail = 1;
-        else {
-          C.rosen *= wsum / (double)nt;
-          if (insert && C.rosen < 1e-150) C.fail = 1;
-          for (int k = 0; k < 4; k++) C.u[k] += u[k];
-        }
-        C.sel = sel;
-        if (C.fail) C.cnt[RGPU_CNT_OVERLAP]++;
-      }
-    }
-    __syncthreads();
-    if (C.fail) return;
-  }
-  int bw = b1;
-  if (!one) {
-    /* sites of the chosen configuration: first bead + beads of trial C.sel */
-    if (threadIdx.x < na) {
-      const int a = threadIdx.x;
-      BeadPos bp;
-      if (a == sb) bp = C.first;
-      else {
-        int j = a < sb ? a : a - 1;
-        bp = E.pos[C.sel * nb + j];
-      }
-      E.sites[a].b = bp;
-      E.sites[a].q = insert ? S.mol_q[a] : -S.mol_q[a];
-    }
-    __syncthreads();
-    if (ew) {
-      engine_ewald(E, na);
-      bw = E.xb;
-      E.xb ^= 1;
-    }
-  }
+  exp_pair(-S.beta * (C.u[1] + C.u[3]), (insert ? -S.beta : S.beta) * (d_ads + d_host), lj, f);
+  const double rosen = C.rosen * lj;
+  double pacc;
+  if (insert) pacc = rosen * f * S.fugacity_beta_v / (1.0 + nmol);
+  else pacc = (double)nmol / (rosen * f * S.fugacity_beta_v);
+  const bool accept = !widom && C.rnd[buf][SLOT_ACCEPT] < pacc;
+  __syncwarp();
   if (threadIdx.x == 0) {
-    /* LJ-biasing correction, src/cbmc.c:3171-3178 / :3044-3051 */
-    double rosen = C.rosen * exp(-S.beta * (C.u[1] + C.u[3]));
-    double d_ads = 0.0, d_host = 0.0;
-    if (ew) {
-      double ea, eh;
-      gather_ewald(E, bw, ea, eh);
-      const double ex = S.excl_mol;      /* rigid molecule */
-      double net = nmol * S.mol_charge;
-      if (insert) ewald_finish(S, ea, eh, ex, 0.0, 1, net, d_ads, d_host);
-      else ewald_finish(S, ea, eh, 0.0, ex, -1, net, d_ads, d_host);
-    }
-    double pacc;
-    if (insert) pacc = rosen * exp(-S.beta * (d_ads + d_host)) * S.fugacity_beta_v / (1.0 + nmol);
-    else pacc = (double)nmol / (rosen * exp(S.beta * (d_ads + d_host)) * S.fugacity_beta_v);
     if (!(pacc == pacc)) C.status |= RGPU_ERR_NONFINITE;
-    C.accept = !widom && E.rnd[SLOT_ACCEPT] < pacc;
-    if (widom) C.sums[RGPU_SUM_WIDOM_W] += rosen * exp(-S.beta * (d_ads + d_host));
-    const int mv = insert ? 2 : 3;
-    if (C.accept) {
+    if (widom) C.sums[RGPU_SUM_WIDOM_W] += rosen * f;
+    if (accept) {
       C.cnt[RGPU_CNT_ACCEPT + mv]++;
-      double sgn = insert ? 1.0 : -1.0;
-      C.energy[RGPU_E_HOST_VDW] += sgn * C.u[0];
-      C.energy[RGPU_E_HOST_REAL] += sgn * C.u[1];
-      C.energy[RGPU_E_ADS_VDW] += sgn * C.u[2];
-      C.energy[RGPU_E_ADS_REAL] += sgn * C.u[3];
-      C.energy[RGPU_E_HOST_FOURIER] += d_host;
-      C.energy[RGPU_E_ADS_FOURIER] += d_ads;
-    }
-  }
-  __syncthreads();
-  if (C.accept) {
-    if (insert) {
-      if (threadIdx.x < na) {
-        double p[3] = {E.sites[threadIdx.x].b.x, E.sites[threadIdx.x].b.y, E.sites[threadIdx.x].b.z};
-        atom_store(E, nmol, threadIdx.x, p);
-      }
-    } else {
-      /* RemoveAdsorbateMolecule (src/molecule.c:3193): the last molecule
-       * takes the freed slot */
-      const int last = nmol - 1;
-      if (threadIdx.x < na && m != last) {
-        double p[3];
-        atom_xyz(E, last, threadIdx.x, p);
-        atom_store(E, m, threadIdx.x, p);
-      }
-    }
-    if (ew) ewald_apply<MIXED>(S, E.tab, E.kw, E.sites, na, E.k0, E.k1);
-    if (threadIdx.x == 0) {
+      add_energies(C, insert ? 1.0 : -1.0, C.u, d_host, d_ads);
       C.nmol = insert ? nmol + 1 : nmol - 1;
       C.nads = C.nmol * na;
     }
-    __syncthreads();
   }
+  if (accept) {
+    if (threadIdx.x < na) {
+      double p[3];
+      if (insert) {
+        chosen_atom(E, threadIdx.x, p);
+        atom_store(E, nmol, threadIdx.x, p);
+      } else if (m != nmol - 1) {
+        /* RemoveAdsorbateMolecule (src/molecule.c:3193): the last molecule
+         * takes the freed slot */
+        atom_xyz(E, nmol - 1, threadIdx.x, p);
+        atom_store(E, m, threadIdx.x, p);
+      }
+    }
+    accept_sites(E, na);
+  }
+}
+
+/* the configuration is chosen: its Ewald sum, or the acceptance. Returns
+ * whether the step is done. */
+template <int MIXED, bool FLEX>
+__device__ RGPU_COLD bool grown_swap(Build<MIXED, FLEX> E, int buf)
+{
+  if (has_ewald(fx().S)) {
+    next_stage(E, PH_SWAPEW, 0, 0, fx().S.natom);
+    return false;
+  }
+  accept_swap(E, buf);
+  return true;
+}
+
+/* after the first-bead trials (and, in a one-evaluation deletion, the
+ * retrace orientations); returns whether the step is done */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ bool end_swap1(Build<MIXED, FLEX> E, int buf)
+{
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const bool insert = cur().mv != 3, one = cur().one != 0;
+  const int na = S.natom, nf = S.ntrial_first, nt = S.ntrial, nb = na - 1;
+  const Trials &a = C.tr[0], &b = C.tr[1];
+  cbmc_trials(E, 0, nf, 1, true, insert, C.rnd[buf][SLOT_FIRST_SELECT], &C.tr[0]);
+  double rosen = a.w_sum / (double)nf;
+  bool fail = !a.any || (insert && rosen < 1e-150);
+  const bool both = !fail && one && na > 1;
+  if (both) {
+    /* the retrace orientations (trial 0 is the old one, not selected) */
+    cbmc_trials(E, nf, nt, nb, false, false, 0.0, &C.tr[1]);
+    fail = !b.any;
+    rosen *= b.w_sum / (double)nt;
+  }
+  if (threadIdx.x < 4) C.u[threadIdx.x] = both ? a.e[threadIdx.x] + b.e[threadIdx.x] : a.e[threadIdx.x];
+  if (threadIdx.x == 0) {
+    C.rosen = rosen;
+    C.sel = a.sel;
+    const BeadPos &p = fx().pos[a.sel];
+    C.first[0] = p.x; C.first[1] = p.y; C.first[2] = p.z;
+    if (fail) C.cnt[RGPU_CNT_OVERLAP]++;
+  }
+  __syncwarp();
+  if (fail) return true;
+  if (one) {
+    accept_swap(E, buf);
+    return true;
+  }
+  if (na == 1) return grown_swap(E, buf);
+  next_stage(E, PH_SWAP2, nt * nb, 0, 0);
+  return false;
+}
+
+/* the orientation trials enter C; returns whether the growth failed */
+template <int MIXED, bool FLEX>
+__device__ RGPU_COLD bool add_orientations(Build<MIXED, FLEX> E, bool grow, int buf)
+{
+  Ctl &C = fx().C;
+  const int nt = fx().S.ntrial;
+  const Trials &a = C.tr[0];
+  cbmc_trials(E, 0, nt, fx().S.natom - 1, false, grow, C.rnd[buf][SLOT_ORIENT_SELECT], &C.tr[0]);
+  const double rosen = C.rosen * (a.w_sum / (double)nt);
+  const bool fail = !a.any || (grow && rosen < 1e-150);
+  __syncwarp();
+  if (threadIdx.x < 4) C.u[threadIdx.x] += a.e[threadIdx.x];
+  if (threadIdx.x == 0) {
+    C.rosen = rosen;
+    C.sel = a.sel;
+    if (fail) C.cnt[RGPU_CNT_OVERLAP]++;
+  }
+  __syncwarp();
+  return fail;
 }
 
 /* ------------------------------------------------------------------------ */
@@ -789,189 +1047,90 @@ __device__ __forceinline__ void step_swap(Eng<MIXED, FLEX> &E, bool insert, bool
  * first-bead trials (src/cbmc.c:750-762), and the old orientation among
  * nt - 1 fresh ones. Accepted with probability
  * exp(-beta dU_Fourier) W(new) / W(old).
- * Evaluation 1 holds the nf new first-bead trials, the old first bead and
- * the retrace orientations (all known up front); evaluation 2 the new
- * orientations around the chosen first bead. */
+ * Stage 1 holds the nf new first-bead trials, the old first bead and the
+ * retrace orientations (all known up front); stage 2 the new orientations
+ * around the chosen first bead; stage 3 the Ewald sum of both. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void step_reinsert(Eng<MIXED, FLEX> &E)
+__device__ RGPU_COLD void accept_reinsert(Build<MIXED, FLEX> E, int buf)
 {
-  RgpuSys &S = *E.S;
-  Ctl &C = *E.ctl;
-  const int na = S.natom, sb = S.start_bead, nmol = C.nmol;
-  const int nf = S.ntrial_first, nt = S.ntrial, nb = na - 1;
-  int m = (int)(E.rnd[SLOT_MOLECULE] * nmol);
-  if (m >= nmol) m = nmol - 1;
-  const int old_first = nf;              /* position of the old first bead */
-  const int old_orient = nf + 1;         /* first position of the retrace orientations */
-  if (threadIdx.x < nf) {
-    const int i = threadIdx.x;
-    double p[3];
-    rgpu_box_point(S, E.rnd[SLOT_FIRST + 3 * i + 2], E.rnd[SLOT_FIRST + 3 * i + 1], E.rnd[SLOT_FIRST + 3 * i + 0], p);
-    bead_set(E.pos[i], S, p[0], p[1], p[2], sb, m);
-  } else if (threadIdx.x == nf) {
-    double p[3];
-    atom_xyz(E, m, sb, p);
-    bead_set(E.pos[old_first], S, p[0], p[1], p[2], sb, m);
-  }
-  if (na > 1 && threadIdx.x >= 32 && threadIdx.x < 32 + nt) {
-    const int t = threadIdx.x - 32;
-    double o[3];
-    atom_xyz(E, m, sb, o);
-    double R[3][3];
-    if (t > 0)
-      random_rotation(E.rnd[SLOT_ORIENT_OLD + 4 * t + 0], E.rnd[SLOT_ORIENT_OLD + 4 * t + 1],
-                      E.rnd[SLOT_ORIENT_OLD + 4 * t + 2], R);
-    int j = 0;
-    for (int a = 0; a < na; a++) {
-      if (a == sb) continue;
-      double p[3];
-      if (t == 0) {
-        atom_xyz(E, m, a, p);
-      } else {
-        const double c[3] = {S.mol_ref[a][0] - S.mol_ref[sb][0], S.mol_ref[a][1] - S.mol_ref[sb][1],
-                             S.mol_ref[a][2] - S.mol_ref[sb][2]};
-        for (int d = 0; d < 3; d++) p[d] = o[d] + c[0] * R[d][0] + c[1] * R[d][1] + c[2] * R[d][2];
-      }
-      bead_set(E.pos[old_orient + t * nb + j], S, p[0], p[1], p[2], a, m);
-      j++;
-    }
-  }
-  __syncthreads();
-  engine_eval(E, nf + 1 + (na > 1 ? nt * nb : 0), 0);
-  const int b1 = E.xb;
-  E.xb ^= 1;
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    double wsum, u[4], wsel;
-    int sel, any;
-    cbmc_trials(E, b1, nf, 1, true, true, E.rnd[SLOT_FIRST_SELECT], wsum, sel, u, any, 0, &wsel);
-    /* the old first bead */
-    double r[4];
-    int o;
-    gather(E, b1, old_first, r, o);
-    const bool ovo = r[0] >= S.overlap || r[1] >= S.overlap || r[2] >= S.overlap || r[3] >= S.overlap;
-    const double w_old1 = ovo ? 0.0 : exp(-S.beta * (r[0] + r[2]));
-    /* the retrace orientations (trial 0 = the old one) */
-    double wo = 0.0, uo[4] = {r[0], r[1], r[2], r[3]};
-    int anyo = 1;
-    if (na > 1) {
-      double uot[4];
-      int selo;
-      cbmc_trials(E, b1, nt, nb, false, false, 0.0, wo, selo, uot, anyo, old_orient);
-      for (int k = 0; k < 4; k++) uo[k] += uot[k];
-    }
-    if (lane == 0) {
-      C.rosen = wsum / (double)nf;
-      double rosen_old = (w_old1 + (wsum - wsel)) / (double)nf;
-      if (na > 1) rosen_old *= wo / (double)nt;
-      C.fail = !any || C.rosen < 1e-150 || ovo || !anyo;
-      C.rosen_old = rosen_old;
-      C.sel = sel;
-      for (int k = 0; k < 4; k++) {
-        C.u[k] = u[k];
-        C.uo[k] = uo[k];
-      }
-      C.first = E.pos[sel];
-      if (C.fail) C.cnt[RGPU_CNT_OVERLAP]++;
-    }
-  }
-  __syncthreads();
-  if (C.fail) return;
-  if (na > 1) {
-    const BeadPos first = C.first;
-    if (threadIdx.x < nt) {
-      const int t = threadIdx.x;
-      double R[3][3];
-      random_rotation(E.rnd[SLOT_ORIENT + 4 * t + 0], E.rnd[SLOT_ORIENT + 4 * t + 1],
-                      E.rnd[SLOT_ORIENT + 4 * t + 2], R);
-      int j = 0;
-      for (int a = 0; a < na; a++) {
-        if (a == sb) continue;
-        const double c[3] = {S.mol_ref[a][0] - S.mol_ref[sb][0], S.mol_ref[a][1] - S.mol_ref[sb][1],
-                             S.mol_ref[a][2] - S.mol_ref[sb][2]};
-        double p[3];
-        p[0] = first.x + c[0] * R[0][0] + c[1] * R[0][1] + c[2] * R[0][2];
-        p[1] = first.y + c[0] * R[1][0] + c[1] * R[1][1] + c[2] * R[1][2];
-        p[2] = first.z + c[0] * R[2][0] + c[1] * R[2][1] + c[2] * R[2][2];
-        bead_set(E.pos[t * nb + j], S, p[0], p[1], p[2], a, m);
-        j++;
-      }
-    }
-    __syncthreads();
-    engine_eval(E, nt * nb, 0);
-    const int b2 = E.xb;
-    E.xb ^= 1;
-    if (threadIdx.x < 32) {
-      double wsum, u[4];
-      int sel, any;
-      cbmc_trials(E, b2, nt, nb, false, true, E.rnd[SLOT_ORIENT_SELECT], wsum, sel, u, any);
-      if (threadIdx.x == 0) {
-        if (!any) C.fail = 1;
-        else {
-          C.rosen *= wsum / (double)nt;
-          if (C.rosen < 1e-150) C.fail = 1;
-          for (int k = 0; k < 4; k++) C.u[k] += u[k];
-        }
-        C.sel = sel;
-        if (C.fail) C.cnt[RGPU_CNT_OVERLAP]++;
-      }
-    }
-    __syncthreads();
-    if (C.fail) return;
-  }
-  /* Ewald sites: the new configuration (+q) and the old one (-q) */
-  if (threadIdx.x < na) {
-    const int a = threadIdx.x;
-    BeadPos bp;
-    if (a == sb) bp = C.first;
-    else bp = E.pos[C.sel * nb + (a < sb ? a : a - 1)];
-    E.sites[a].b = bp;
-    E.sites[a].q = S.mol_q[a];
-    double p[3];
-    atom_xyz(E, m, a, p);
-    bead_set(E.sites[na + a].b, S, p[0], p[1], p[2], a, m);
-    E.sites[na + a].q = -S.mol_q[a];
-  }
-  __syncthreads();
-  const bool ew = S.ewald && S.mol_charged;
-  int bw = 0;
-  if (ew) {
-    engine_ewald(E, 2 * na);
-    bw = E.xb;
-    E.xb ^= 1;
-  }
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int na = S.natom;
+  /* LJ-biasing corrections of both Rosenbluth weights, src/cbmc.c:3171-3178, :3044-3051 */
+  const double rosen_new = C.rosen * cold_exp(-S.beta * (C.u[1] + C.u[3]));
+  const double rosen_old = C.rosen_old * cold_exp(-S.beta * (C.uo[1] + C.uo[3]));
+  double d_ads = 0.0, d_host = 0.0;
+  if (has_ewald(S)) ewald_finish(S, C.ew[0], C.ew[1], S.excl_mol, S.excl_mol, 0, 0.0, d_ads, d_host);
+  const double pacc = cold_exp(-S.beta * (d_ads + d_host)) * rosen_new / rosen_old;
+  const bool accept = C.rnd[buf][SLOT_ACCEPT] < pacc;
   if (threadIdx.x == 0) {
-    /* LJ-biasing corrections of both Rosenbluth weights, src/cbmc.c:3171-3178, :3044-3051 */
-    const double rosen_new = C.rosen * exp(-S.beta * (C.u[1] + C.u[3]));
-    const double rosen_old = C.rosen_old * exp(-S.beta * (C.uo[1] + C.uo[3]));
-    double d_ads = 0.0, d_host = 0.0;
-    if (ew) {
-      double ea, eh;
-      gather_ewald(E, bw, ea, eh);
-      ewald_finish(S, ea, eh, S.excl_mol, S.excl_mol, 0, 0.0, d_ads, d_host);
-    }
-    const double pacc = exp(-S.beta * (d_ads + d_host)) * rosen_new / rosen_old;
     if (!(pacc == pacc)) C.status |= RGPU_ERR_NONFINITE;
-    C.accept = E.rnd[SLOT_ACCEPT] < pacc;
-    if (C.accept) {
+    if (accept) {
       C.cnt[RGPU_CNT_REINS_ACCEPT]++;
-      C.energy[RGPU_E_HOST_VDW] += C.u[0] - C.uo[0];
-      C.energy[RGPU_E_HOST_REAL] += C.u[1] - C.uo[1];
-      C.energy[RGPU_E_ADS_VDW] += C.u[2] - C.uo[2];
-      C.energy[RGPU_E_ADS_REAL] += C.u[3] - C.uo[3];
-      C.energy[RGPU_E_HOST_FOURIER] += d_host;
-      C.energy[RGPU_E_ADS_FOURIER] += d_ads;
+      double u[4];
+      for (int k = 0; k < 4; k++) u[k] = C.u[k] - C.uo[k];
+      add_energies(C, 1.0, u, d_host, d_ads);
     }
   }
-  __syncthreads();
-  if (C.accept) {
+  if (accept) {
     if (threadIdx.x < na) {
-      double p[3] = {E.sites[threadIdx.x].b.x, E.sites[threadIdx.x].b.y, E.sites[threadIdx.x].b.z};
-      atom_store(E, m, threadIdx.x, p);
+      double p[3];
+      chosen_atom(E, threadIdx.x, p);
+      atom_store(E, cur().m, threadIdx.x, p);
     }
-    if (ew) ewald_apply<MIXED>(S, E.tab, E.kw, E.sites, 2 * na, E.k0, E.k1);
-    __syncthreads();
+    accept_sites(E, 2 * na);
   }
+}
+
+/* the new configuration is chosen: its Ewald sum, or the acceptance */
+template <int MIXED, bool FLEX>
+__device__ RGPU_COLD bool grown_reinsert(Build<MIXED, FLEX> E, int buf)
+{
+  if (has_ewald(fx().S)) {
+    next_stage(E, PH_REINSEW, 0, 0, 2 * fx().S.natom);
+    return false;
+  }
+  accept_reinsert(E, buf);
+  return true;
+}
+
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ bool end_reinsert1(Build<MIXED, FLEX> E, int buf)
+{
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int na = S.natom, nf = S.ntrial_first, nt = S.ntrial, nb = na - 1;
+  const Trials &a = C.tr[0], &b = C.tr[1];
+  cbmc_trials(E, 0, nf, 1, true, true, C.rnd[buf][SLOT_FIRST_SELECT], &C.tr[0]);
+  /* the old first bead */
+  const double4 r = fx().tot[nf];
+  const bool ovo = r.x >= S.overlap || r.y >= S.overlap || r.z >= S.overlap || r.w >= S.overlap;
+  const double w_old1 = ovo ? 0.0 : cold_exp(-S.beta * (r.x + r.z));
+  /* the retrace orientations (trial 0 = the old one) */
+  if (na > 1) cbmc_trials(E, nf + 1, nt, nb, false, false, 0.0, &C.tr[1]);
+  const double rosen = a.w_sum / (double)nf;
+  double rosen_old = (w_old1 + (a.w_sum - a.w_sel)) / (double)nf;
+  if (na > 1) rosen_old *= b.w_sum / (double)nt;
+  const bool fail = !a.any || rosen < 1e-150 || ovo || (na > 1 && !b.any);
+  if (threadIdx.x == 0) {
+    const double ro[4] = {r.x, r.y, r.z, r.w};
+    C.rosen = rosen;
+    C.rosen_old = rosen_old;
+    C.sel = a.sel;
+#pragma unroll 1
+    for (int k = 0; k < 4; k++) {
+      C.u[k] = a.e[k];
+      C.uo[k] = na > 1 ? ro[k] + b.e[k] : ro[k];
+    }
+    const BeadPos &p = fx().pos[a.sel];
+    C.first[0] = p.x; C.first[1] = p.y; C.first[2] = p.z;
+    if (fail) C.cnt[RGPU_CNT_OVERLAP]++;
+  }
+  __syncwarp();
+  if (fail) return true;
+  if (na == 1) return grown_reinsert(E, buf);
+  next_stage(E, PH_REINS2, nt * nb, 0, 0);
+  return false;
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1021,18 +1180,6 @@ __device__ __forceinline__ void chain_angles_group(const RgpuSys &S, int i, int 
   }
 }
 
-/* CBMC growth (retrace = false) or retrace (retrace = true) of a flexible
- * chain, bead by bead from atom 0 (GrowMolecule / RetraceMolecule,
- * src/cbmc.c:2928-3181, for a linear chain): the first bead from nf trials
- * (random in the box; for a retrace trial 0 is the old bead), every other
- * bead from nt trials drawn by chain_trial (bonded Boltzmann factor built
- * in). The weight of a trial is exp(-beta (host VDW + adsorbate VDW + LJ
- * with the chain's beads four or more bonds back)); a trial overlaps when
- * one of them reaches the criterion. Leaves in Ctl the Rosenbluth weight
- * (product over beads of sum w / trials), the chosen beads (cp), their
- * host and adsorbate VDW (u[0], u[2]) and the intramolecular energy
- * (uintra: bonded + LJ), or fail. Molecule m is the one retraced; `exclude`
- * leaves a molecule out of the adsorbate sums. All threads call. */
 /* The bend angle shared by the trials of bead i >= 2 in the reference's
  * scheme (chain_scheme 0): a growth draws it from sin(theta) exp(-beta
  * U_bend) (proposals in the slots of trial RGPU_REF_THETA_TRIAL from
@@ -1212,27 +1359,27 @@ __device__ __noinline__ void chain_ref_trial(const RgpuSys &S, int i, int stage,
  * All threads of the cluster call; the caller's next barrier publishes the
  * table. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void chain_angles_table(Eng<MIXED, FLEX> &E, int stage, double *tab,
+__device__ __forceinline__ void chain_angles_table(Build<MIXED, FLEX> E, uint64_t step, int stage, double *tab,
                                                    const double (*old)[3])
 {
-  const RgpuSys &S = *E.S;
+  const RgpuSys &S = fx().S;
   const int na = S.natom, nt = S.ntrial;
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int ntask = na > 2 ? (na - 2) * nt : 0;
-  const int gw = E.rank * nw + (threadIdx.x >> 5), ngw = nw * E.csize;   /* warp of the cluster */
+  const int gw = fx().rank * nw + (threadIdx.x >> 5), ngw = nw * fx().csize;   /* warp of the cluster */
   const int per = S.chain_scheme == 0 ? 1 : 4;                           /* tasks a warp takes at once */
   if (S.chain_scheme == 0) {
     /* each bead's bend angle once (one warp per bead, in every CTA), then
      * one warp per (bead, trial); the angles sit after the table */
     double *theta = tab + RGPU_ANG_TABLE;
     for (int i = 2 + (threadIdx.x >> 5); i < na; i += nw) {
-      const double th = chain_ref_theta(S, i, stage, E.step, lane, old);
+      const double th = chain_ref_theta(S, i, stage, step, lane, old);
       if (lane == 0) theta[i] = th;
     }
     __syncthreads();
     for (int task = gw; task < ntask; task += ngw) {
       const int i = 2 + task / nt, t = task % nt;
-      chain_ref_trial<(MIXED != 0)>(S, i, stage, t, E.step, lane, old, theta[i],
+      chain_ref_trial<(MIXED != 0)>(S, i, stage, t, step, lane, old, theta[i],
                              tab + RGPU_ANG_STRIDE * ((i - 2) * RGPU_MAX_TRIALS + t));
     }
   } else {
@@ -1241,7 +1388,7 @@ __device__ __forceinline__ void chain_angles_table(Eng<MIXED, FLEX> &E, int stag
       const bool live = task < ntask;
       const int i = live ? 2 + task / nt : 2, t = live ? task % nt : 0;
       double th, ph;
-      chain_angles_group(S, i, stage, t, live, E.step, lane, th, ph);
+      chain_angles_group(S, i, stage, t, live, step, lane, th, ph);
       if (live && (lane & 7) == 0) {
         double *a = tab + RGPU_ANG_STRIDE * ((i - 2) * RGPU_MAX_TRIALS + t);
         a[0] = cos(th);
@@ -1252,12 +1399,12 @@ __device__ __forceinline__ void chain_angles_table(Eng<MIXED, FLEX> &E, int stag
       }
     }
   }
-  if (E.csize > 1) {
+  if (fx().csize > 1) {
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
     for (int task = threadIdx.x; task < ntask; task += blockDim.x) {
       const int owner = ((task / per) % ngw) / nw;
-      if (owner == E.rank) continue;
+      if (owner == fx().rank) continue;
       const int off = RGPU_ANG_STRIDE * ((task / nt) * RGPU_MAX_TRIALS + task % nt);
       const double *src = cl.map_shared_rank(tab, owner) + off;
       for (int d = 0; d < RGPU_ANG_STRIDE; d++) tab[off + d] = src[d];
@@ -1268,18 +1415,6 @@ __device__ __forceinline__ void chain_angles_table(Eng<MIXED, FLEX> &E, int stag
   }
 }
 
-/* Retrace of a flexible chain's configuration (RetraceMolecule,
- * src/cbmc.c:3056-3181, for a linear chain). The beads a retrace "chooses"
- * are the old ones, known before anything is evaluated, so the trial sets of
- * several beads are placed together and evaluated at once: beads are taken
- * in growth order in groups whose trials fit one evaluation (RGPU_MAX_POS
- * positions; for 6 beads of 16 trials and 8 first-bead trials, two
- * evaluations instead of six). Each bead's weights are summed by one warp in
- * trial order, and the Rosenbluth weight and the energies are combined bead
- * by bead in growth order, stopping at the first bead without a valid
- * trial, as the bead-by-bead retrace does. The trials draw the same random
- * numbers as that retrace (counter-based, by stage, bead and trial). All
- * threads call. */
 /* Beads of a retrace taken in one evaluation: from bead i0 on, as many as
  * fit `room` positions (at least one; room >= RGPU_MAX_TRIALS). */
 __device__ __forceinline__ int retrace_group_end(int i0, int na, int nf, int nt, int room, int &P)
@@ -1293,75 +1428,38 @@ __device__ __forceinline__ int retrace_group_end(int i0, int na, int nf, int nt,
   return i1;
 }
 
-/* Places the trials of retrace beads [i0, i0 + ...) at positions off ..
- * off + P, position j of the group being bead i, trial t in growth order;
- * trial 0 of each bead is the old bead old[i]. Threads t0, t0 + step, ...
- * of the block place. */
-template <int MIXED, bool FLEX>
-__device__ __forceinline__ void retrace_place(Eng<MIXED, FLEX> &E, int stage, int i0, int P, int off,
-                                              const double (*old)[3], const double *ang, int exclude, int t0,
-                                              int step)
-{
-  const RgpuSys &S = *E.S;
-  const int nf = S.ntrial_first, nt = S.ntrial;
-  for (int j = t0; j < P; j += step) {
-    int i = i0, t = j;
-    while (t >= (i == 0 ? nf : nt)) {
-      t -= i == 0 ? nf : nt;
-      i++;
-    }
-    double p[3];
-    if (t == 0) {
-      p[0] = old[i][0];
-      p[1] = old[i][1];
-      p[2] = old[i][2];
-    } else if (i == 0) {
-      rgpu_box_point(S, rgpu_uniform(S.seed, S.sys_id, E.step, chain_slot(stage, 0, t, 0)),
-                     rgpu_uniform(S.seed, S.sys_id, E.step, chain_slot(stage, 0, t, 1)),
-                     rgpu_uniform(S.seed, S.sys_id, E.step, chain_slot(stage, 0, t, 2)), p);
-    } else if (i == 1) {
-      const uint64_t stp = E.step;
-      chain_trial(S, old, i, [&](int d) { return rgpu_uniform(S.seed, S.sys_id, stp, chain_slot(stage, i, t, d)); },
-                  p);
-    } else {
-      const double *a = ang + RGPU_ANG_STRIDE * ((i - 2) * RGPU_MAX_TRIALS + t);
-      chain_place_trig(i >= 3 ? old[i - 3] : nullptr, old[i - 2], old[i - 1], S.bond, a[0], a[1], a[2], a[3], p);
-    }
-    bead_set(E.pos[off + j], S, p[0], p[1], p[2], i, exclude);
-  }
-}
-
 /* Bookkeeping of retrace beads [i0, i1) evaluated at positions off.. of
- * buffer b: warp w0 + g takes bead i0 + g (warps w0, w0 + 1, ... of the
- * block), sums its weights in trial order and leaves in C.rb[i] the sum,
+ * the last evaluation: warp w0 + g takes bead i0 + g (warps w0, w0 + 1, ... of the
+ * block), sums its weights and leaves in C.rb[i] the sum,
  * the old bead's host and adsorbate VDW, intramolecular LJ and bonded
  * energy, and whether any trial was valid. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void retrace_book(const Eng<MIXED, FLEX> &E, int b, int i0, int i1, int off,
+__device__ RGPU_COLD void retrace_book(Build<MIXED, FLEX> E, int i0, int i1, int off,
                                              const double (*old)[3], const double *ang, int w0)
 {
-  const RgpuSys &S = *E.S;
-  Ctl &C = *E.ctl;
+  const RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
   const int nf = S.ntrial_first, nt = S.ntrial;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (warp < w0) return;
   for (int g = warp - w0; g < i1 - i0; g += nw - w0) {
     const int i = i0 + g, k = i == 0 ? nf : nt;
     const int o0 = off + (i0 == 0 ? (i == 0 ? 0 : nf + (i - 1) * nt) : g * nt);
-    double r[4] = {0.0, 0.0, 0.0, 0.0}, lj = 0.0, bf = 0.0;
-    int o = 0, ov = 0;
+    double lj = 0.0, bf = 0.0;
+    int ov = 0;
+    const double4 rt = fx().tot[o0 + (lane < k ? lane : 0)];
+    const double r[4] = {rt.x, rt.y, rt.z, rt.w};
     if (lane < k) {
-      gather(E, b, o0 + lane, r, o);
-      const double p[3] = {E.pos[o0 + lane].x, E.pos[o0 + lane].y, E.pos[o0 + lane].z};
+      const BeadPos &q = fx().pos[o0 + lane];
+      const double p[3] = {q.x, q.y, q.z};
       lj = chain_intra_lj(S, old, i, p);
       ov = r[0] >= S.overlap || r[1] >= S.overlap || r[2] >= S.overlap || r[3] >= S.overlap || lj >= S.overlap;
       bf = -S.beta * (r[0] + r[2] + lj);
     }
     const bool valid = lane < k && !ov;
-    const double w = valid ? exp(bf) : 0.0;
+    const double w = valid ? cold_exp(bf) : 0.0;
     const bool any = __ballot_sync(RGPU_FULL, valid) != 0u;
-    double wsum = 0.0;
-    for (int t = 0; t < k; t++) wsum += __shfl_sync(RGPU_FULL, w, t);
+    const double wsum = warp_sum(w);
     if (lane == 0) {
       double *rb = C.rb[i];
       /* with the old trial's torsion Rosenbluth factor (1 for independent draws) */
@@ -1394,279 +1492,393 @@ __device__ __forceinline__ void retrace_combine(Ctl &C, int i0, int i1, int nf, 
   }
 }
 
-/* Retrace of a flexible chain's configuration (RetraceMolecule,
- * src/cbmc.c:3056-3181, for a linear chain). The beads a retrace "chooses"
- * are the old ones, known before anything is evaluated, so the trial sets of
- * several beads are placed together and evaluated at once: beads are taken
- * in growth order in groups whose trials fit one evaluation (RGPU_MAX_POS
- * positions; for 6 beads of 16 trials and 8 first-bead trials, two
- * evaluations instead of six). Each bead's weights are summed by one warp in
- * trial order, and the Rosenbluth weight and the energies are combined bead
- * by bead in growth order, stopping at the first bead without a valid
+/* ------------------------------------------------------------------------ */
+/* CBMC growth and retrace of a flexible chain, bead by bead from atom 0
+ * (GrowMolecule / RetraceMolecule, src/cbmc.c:2928-3181, for a linear chain):
+ * the first bead from nf trials (random in the box; for a retrace trial 0 is
+ * the old bead), every other bead from nt trials of the stage's angle table.
+ * The weight of a trial is exp(-beta (host VDW + adsorbate VDW + LJ with the
+ * chain's beads four or more bonds back)); a trial overlaps when one of them
+ * reaches the criterion. Ctl holds the Rosenbluth weight (product over beads
+ * of sum w / trials), the chosen beads (cp), their host and adsorbate VDW
+ * (u[0], u[2]) and the intramolecular energy (uintra: bonded + LJ).
+ *
+ * Growth: one stage per bead. Warp 0 selects a trial; meanwhile warp 1
+ * computes every trial's bonded energy, the chosen
+ * one's being added in the next stage.
+ *
+ * Retrace: the beads it "chooses" are the old ones, known before anything is
+ * evaluated, so the trial sets of several beads are placed together and
+ * evaluated at once: beads are taken in growth order in groups whose trials
+ * fit one evaluation (RGPU_MAX_POS positions; for 6 beads of 16 trials and 8
+ * first-bead trials, two evaluations instead of six). Each bead's weights are
+ * summed by one warp, and the Rosenbluth weight and the energies are combined
+ * bead by bead in growth order, stopping at the first bead without a valid
  * trial, as the bead-by-bead retrace does. The trials draw the same random
- * numbers as that retrace (counter-based, by stage, bead and trial). All
- * threads call. */
+ * numbers as that retrace (counter-based, by stage, bead and trial). A
+ * reinsertion's retrace rides along with its growth's first evaluations, one
+ * group each, in the positions after the growth's trials. */
+/* the angle tables of a chain move: its growth's, or its retrace's; a
+ * reinsertion's both. All threads call. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void retrace_chain(Eng<MIXED, FLEX> &E, int stage, int m, int exclude)
+__device__ RGPU_COLD void chain_tables(Build<MIXED, FLEX> E, const Stage &g)
 {
-  RgpuSys &S = *E.S;
-  Ctl &C = *E.ctl;
-  const int na = S.natom, nf = S.ntrial_first, nt = S.ntrial;
+  Ctl &C = fx().C;
+  const int mv = g.mv;
+  const uint64_t step = fx().step0 + (uint64_t)g.it;
+#pragma unroll 1
+  for (int t = 0; t < (mv == 4 ? 2 : 1); t++) {
+    const bool old = mv == 3 || t == 1;
+    double (*x)[3] = t ? C.co : C.cp;
+    if (old) {
+      if (threadIdx.x < fx().S.natom) atom_xyz(E, g.m, threadIdx.x, x[threadIdx.x]);
+      __syncthreads();          /* the old configuration, read by the table */
+    }
+    chain_angles_table(E, step, old ? 1 : 0, fx_ang() + t * RGPU_ANG_DOUBLES, old ? x : nullptr);
+  }
+}
+
+/* Stage for bead i of a growth (k trials), with
+ * the retrace beads from r0 on that ride along (r0 = natom: none) */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void grow_stage(Build<MIXED, FLEX> E, int i, int k, int r0)
+{
+  const RgpuSys &S = fx().S;
+  int r1 = r0, rP = 0;
+  if (r0 < S.natom) r1 = retrace_group_end(r0, S.natom, S.ntrial_first, S.ntrial, RGPU_MAX_POS - k, rP);
+  next_stage(E, PH_GROW, k + rP, 0, 0);
+  if (threadIdx.x == 0) {
+    Stage &n = next_of();
+    n.ci = i;
+    n.k = k;
+    n.r0 = r0;
+    n.r1 = r1;
+    n.rP = rP;
+  }
+}
+
+/* stage for the retrace group of a deletion from bead i0 on */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void retrace_stage(Build<MIXED, FLEX> E, int i0)
+{
+  const RgpuSys &S = fx().S;
+  int P;
+  const int i1 = retrace_group_end(i0, S.natom, S.ntrial_first, S.ntrial, RGPU_MAX_POS, P);
+  next_stage(E, PH_RETRACE, P, 0, 0);
+  if (threadIdx.x == 0) {
+    Stage &n = next_of();
+    n.r0 = i0;
+    n.r1 = i1;
+    n.rP = P;
+  }
+}
+
+/* warp 0, after the angle tables */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void end_table(Build<MIXED, FLEX> E)
+{
+  const RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int mv = cur().mv;
   if (threadIdx.x == 0) {
     C.rosen = 1.0;
     C.u[0] = C.u[1] = C.u[2] = C.u[3] = 0.0;
     C.uintra = 0.0;
     C.fail = 0;
   }
-  if (threadIdx.x < na) atom_xyz(E, m, threadIdx.x, C.cp[threadIdx.x]);
-  if (S.chain_scheme == 0) __syncthreads();   /* the old configuration, read by the table */
-  chain_angles_table(E, stage, E.ang, (const double(*)[3])C.cp);
-  __syncthreads();
-  for (int i0 = 0; i0 < na;) {
-    int P;
-    const int i1 = retrace_group_end(i0, na, nf, nt, RGPU_MAX_POS, P);
-    retrace_place(E, stage, i0, P, 0, C.cp, E.ang, exclude, threadIdx.x, blockDim.x);
-    __syncthreads();
-    engine_eval(E, P, 0);
-    const int b = E.xb;
-    E.xb ^= 1;
-    retrace_book(E, b, i0, i1, 0, C.cp, E.ang, 0);
-    __syncthreads();
-    if (threadIdx.x == 0) retrace_combine(C, i0, i1, nf, nt);
-    __syncthreads();
-    if (C.fail) return;
-    i0 = i1;
-  }
-}
-
-template <int MIXED, bool FLEX>
-__device__ __forceinline__ void grow_chain(Eng<MIXED, FLEX> &E, bool retrace, int stage, int m, int exclude,
-                                           bool ride = false)
-{
-  if (retrace) {
-    retrace_chain(E, stage, m, exclude);
+  if (mv == 3) {
+    retrace_stage(E, 0);
     return;
   }
-  RgpuSys &S = *E.S;
-  Ctl &C = *E.ctl;
-  const int na = S.natom, nf = S.ntrial_first, nt = S.ntrial;
-  if (threadIdx.x == 0) {
-    C.rosen = 1.0;
-    C.u[0] = C.u[1] = C.u[2] = C.u[3] = 0.0;
-    C.uintra = 0.0;
-    C.fail = 0;
-  }
-  /* the bend angles and dihedrals of beads 2.. of every trial, ahead of the
-   * first bead (the first barrier below publishes them) */
-  chain_angles_table(E, stage, E.ang, nullptr);
-  /* ride: a reinsertion's retrace (stage 1) of molecule m rides along with
-   * the first beads' evaluations, one group of retrace beads each, in the
-   * positions after the growth's trials; its beads' sums are left in C.rb */
-  double *ang_r = E.ang + RGPU_ANG_DOUBLES;
-  if (ride) {
-    if (threadIdx.x < na) atom_xyz(E, m, threadIdx.x, C.co[threadIdx.x]);
-    if (S.chain_scheme == 0) __syncthreads();   /* the old configuration, read by the table */
-    chain_angles_table(E, 1, ang_r, (const double(*)[3])C.co);
-  }
-  int r0 = ride ? 0 : na;   /* next retrace bead */
-  for (int i = 0; i < na; i++) {
-    const int k = i == 0 ? nf : nt;
-    int r1 = r0, rP = 0;
-    if (r0 < na) {
-      r1 = retrace_group_end(r0, na, nf, nt, RGPU_MAX_POS - k, rP);
-      if (i == 0) __syncthreads();   /* C.co and the retrace angles */
-      if (threadIdx.x >= 32) retrace_place(E, 1, r0, rP, k, C.co, ang_r, m, threadIdx.x - 32, blockDim.x - 32);
-    }
-    if (threadIdx.x < k) {
-      const int t = threadIdx.x;
-      double p[3];
-      if (retrace && t == 0) {
-        atom_xyz(E, m, i, p);
-      } else if (i == 0) {
-        rgpu_box_point(S, rgpu_uniform(S.seed, S.sys_id, E.step, chain_slot(stage, 0, t, 0)),
-                       rgpu_uniform(S.seed, S.sys_id, E.step, chain_slot(stage, 0, t, 1)),
-                       rgpu_uniform(S.seed, S.sys_id, E.step, chain_slot(stage, 0, t, 2)), p);
-      } else if (i == 1) {
-        const uint64_t step = E.step;
-        chain_trial(S, C.cp, i,
-                    [&](int d) { return rgpu_uniform(S.seed, S.sys_id, step, chain_slot(stage, i, t, d)); }, p);
-      } else {
-        const double *a = E.ang + RGPU_ANG_STRIDE * ((i - 2) * RGPU_MAX_TRIALS + t);
-        chain_place_trig(i >= 3 ? C.cp[i - 3] : nullptr, C.cp[i - 2], C.cp[i - 1], S.bond, a[0], a[1], a[2], a[3], p);
-      }
-      bead_set(E.pos[t], S, p[0], p[1], p[2], i, exclude);
-    }
-    __syncthreads();
-    engine_eval(E, k + rP, 0);
-    const int b = E.xb;
-    E.xb ^= 1;
-    if (r1 > r0) {
-      /* warps 1..: the retrace group's bookkeeping (warp 1 then goes on to
-       * this bead's bonded energies) */
-      retrace_book(E, b, r0, r1, k, C.co, ang_r, 1);
-      r0 = r1;
-    }
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
-      double r[4] = {0.0, 0.0, 0.0, 0.0}, lj = 0.0, bf = 0.0;
-      int o = 0, ov = 0;
-      if (lane < k) {
-        gather(E, b, lane, r, o);
-        const double p[3] = {E.pos[lane].x, E.pos[lane].y, E.pos[lane].z};
-        lj = chain_intra_lj(S, C.cp, i, p);
-        ov = r[0] >= S.overlap || r[1] >= S.overlap || r[2] >= S.overlap || r[3] >= S.overlap || lj >= S.overlap;
-        bf = -S.beta * (r[0] + r[2] + lj);
-      }
-      const bool valid = lane < k && !ov;
-      const double w = valid ? exp(bf) : 0.0;
-      const bool any = __ballot_sync(RGPU_FULL, valid) != 0u;
-      double wsum = 0.0;
-      for (int t = 0; t < k; t++) wsum += __shfl_sync(RGPU_FULL, w, t);
-      int sel = 0;
-      if (!retrace && any) {
-        /* SelectTrialPosition (src/cbmc.c:563-599) on the weights themselves */
-        const double target = rgpu_uniform(S.seed, S.sys_id, E.step, RGPU_SLOT_CHAIN_SEL + stage * 8 + i) * wsum;
-        double cum = __shfl_sync(RGPU_FULL, w, 0);
-        while (cum < target && sel < k - 1) {
-          sel++;
-          cum += __shfl_sync(RGPU_FULL, w, sel);
-        }
-      }
-      const double hv = __shfl_sync(RGPU_FULL, r[0], sel), av = __shfl_sync(RGPU_FULL, r[2], sel);
-      const double ljs = __shfl_sync(RGPU_FULL, lj, sel);
-      if (lane == 0) {
-        /* with the chosen trial's torsion Rosenbluth factor (src/cbmc.c:2793;
-         * 1 for independent draws) */
-        C.rosen *= wsum / (double)k * (i >= 2 ? E.ang[RGPU_ANG_STRIDE * ((i - 2) * RGPU_MAX_TRIALS + sel) + 4] : 1.0);
-        if (!any || (!retrace && C.rosen < 1e-150)) C.fail = 1;
-        C.u[0] += hv;
-        C.u[2] += av;
-        C.uintra += ljs;
-        C.sel = sel;
-        C.cp[i][0] = E.pos[sel].x;
-        C.cp[i][1] = E.pos[sel].y;
-        C.cp[i][2] = E.pos[sel].z;
-        if (C.fail) C.cnt[RGPU_CNT_OVERLAP]++;
-      }
-    } else if (i >= 2 && threadIdx.x < 32 + k) {
-      /* meanwhile warp 1: the trials' bonded energies (beads i-1.. of C.cp
-       * are fixed; warp 0 writes only C.cp[i]) */
-      const int t = threadIdx.x - 32;
-      const double p[3] = {E.pos[t].x, E.pos[t].y, E.pos[t].z};
-      C.ub[t] = chain_bonded_energy(S, C.cp, i, p);
-    }
-    __syncthreads();
-    /* the chosen trial's bonded energy; C.ub and C.sel stay untouched until
-     * the next bead's selection, several barriers on */
-    if (threadIdx.x == 0 && i >= 2) C.uintra += C.ub[C.sel];
-    if (C.fail) return;
-  }
+  grow_stage(E, 0, S.ntrial_first, mv == 4 ? 0 : S.natom);
 }
 
-/* CBMC insertion, deletion and Widom test insertion of a flexible chain
+/* warp 0, after the trials of bead g.ci: returns whether the step is done
+ * (the growth failed) */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ bool end_grow(Build<MIXED, FLEX> E, const Stage &g)
+{
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int na = S.natom, i = g.ci, k = g.k, lane = threadIdx.x;
+  double lj = 0.0, bf = 0.0;
+  int ov = 0;
+  const double4 rt = fx().tot[lane < k ? lane : 0];
+  const double r[4] = {rt.x, rt.y, rt.z, rt.w};
+  const BeadPos &q = fx().pos[lane];
+  if (lane < k) {
+    const double p[3] = {q.x, q.y, q.z};
+    lj = chain_intra_lj(S, C.cp, i, p);
+    ov = r[0] >= S.overlap || r[1] >= S.overlap || r[2] >= S.overlap || r[3] >= S.overlap || lj >= S.overlap;
+    bf = -S.beta * (r[0] + r[2] + lj);
+  }
+  const bool valid = lane < k && !ov;
+  const double w = valid ? cold_exp(bf) : 0.0;
+  const bool any = __any_sync(RGPU_FULL, valid);
+  const double cum = warp_scan(w), wsum = __shfl_sync(RGPU_FULL, cum, 31);
+  int sel = 0;
+  /* SelectTrialPosition (src/cbmc.c:563-599) on the weights themselves */
+  if (any) sel = select_trial(w, cum, k, rgpu_uniform(S.seed, S.sys_id, fx().step0 + (uint64_t)cur().it, RGPU_SLOT_CHAIN_SEL + i));
+  const double hv = __shfl_sync(RGPU_FULL, r[0], sel), av = __shfl_sync(RGPU_FULL, r[2], sel);
+  const double ljs = __shfl_sync(RGPU_FULL, lj, sel);
+  /* with the chosen trial's torsion Rosenbluth factor (src/cbmc.c:2793; 1
+   * for independent draws) */
+  const double rosen =
+      C.rosen * (wsum / (double)k * (i >= 2 ? fx_ang()[RGPU_ANG_STRIDE * ((i - 2) * RGPU_MAX_TRIALS + sel) + 4] : 1.0));
+  const bool fail = !any || rosen < 1e-150;
+  __syncwarp();
+  if (lane == sel) {
+    C.cp[i][0] = q.x;
+    C.cp[i][1] = q.y;
+    C.cp[i][2] = q.z;
+  }
+  if (lane == 0) {
+    if (i - 1 >= 2) C.uintra += C.ub[(i - 1) & 1][C.sel];   /* the last bead's bonded energy (warp 1) */
+    C.rosen = rosen;
+    C.u[0] += hv;
+    C.u[2] += av;
+    C.uintra += ljs;
+    C.sel = sel;
+    if (fail) C.cnt[RGPU_CNT_OVERLAP]++;
+  }
+  __syncwarp();
+  if (fail) return true;
+  if (i + 1 < na) {
+    grow_stage(E, i + 1, S.ntrial, g.r1);
+  } else {
+    next_stage(E, PH_CHAINEND, 0, 0, 0);
+  }
+  return false;
+}
+
+/* Acceptance of a chain insertion, deletion or Widom sample
  * (SwapAddAdsorbateMove src/mc_moves.c:7016, SwapRemoveAdsorbateMove :7228,
  * WidomAdsorbateMove :7844; uncharged chains, no Fourier part). */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void step_swap_chain(Eng<MIXED, FLEX> &E, bool insert, bool widom)
+__device__ RGPU_COLD void accept_swap_chain(Build<MIXED, FLEX> E, int buf)
 {
-  RgpuSys &S = *E.S;
-  Ctl &C = *E.ctl;
-  const int na = S.natom, nmol = C.nmol;
-  if (widom && threadIdx.x == 0) C.sums[RGPU_SUM_WIDOM_N] += 1.0;
-  int m = nmol;
-  if (!insert) {
-    m = (int)(E.rnd[SLOT_MOLECULE] * nmol);
-    if (m >= nmol) m = nmol - 1;
-  }
-  grow_chain(E, !insert, insert ? 0 : 1, m, insert ? -1 : m);
-  if (C.fail) return;
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int na = S.natom, nmol = C.nmol, m = cur().m, mv = cur().mv;
+  const bool insert = mv != 3, widom = mv == 5;
+  double pacc;
+  if (insert) pacc = C.rosen * S.fugacity_beta_v / (1.0 + nmol);
+  else pacc = (double)nmol / (C.rosen * S.fugacity_beta_v);
+  const bool accept = !widom && C.rnd[buf][SLOT_ACCEPT] < pacc;
+  __syncwarp();
   if (threadIdx.x == 0) {
-    double pacc;
-    if (insert) pacc = C.rosen * S.fugacity_beta_v / (1.0 + nmol);
-    else pacc = (double)nmol / (C.rosen * S.fugacity_beta_v);
     if (!(pacc == pacc)) C.status |= RGPU_ERR_NONFINITE;
-    C.accept = !widom && E.rnd[SLOT_ACCEPT] < pacc;
     if (widom) C.sums[RGPU_SUM_WIDOM_W] += C.rosen;
-    if (C.accept) {
-      C.cnt[RGPU_CNT_ACCEPT + (insert ? 2 : 3)]++;
+    if (accept) {
+      C.cnt[RGPU_CNT_ACCEPT + mv]++;
       const double sgn = insert ? 1.0 : -1.0;
       C.energy[RGPU_E_HOST_VDW] += sgn * C.u[0];
       C.energy[RGPU_E_ADS_VDW] += sgn * C.u[2];
       C.energy[RGPU_E_INTRA] += sgn * C.uintra;
-    }
-  }
-  __syncthreads();
-  if (C.accept) {
-    if (insert) {
-      if (threadIdx.x < na) atom_store(E, nmol, threadIdx.x, C.cp[threadIdx.x]);
-    } else {
-      const int last = nmol - 1;
-      if (threadIdx.x < na && m != last) {
-        double p[3];
-        atom_xyz(E, last, threadIdx.x, p);
-        atom_store(E, m, threadIdx.x, p);
-      }
-    }
-    if (threadIdx.x == 0) {
       C.nmol = insert ? nmol + 1 : nmol - 1;
       C.nads = C.nmol * na;
     }
-    __syncthreads();
+  }
+  if (accept && threadIdx.x < na) {
+    if (insert) {
+      atom_store(E, nmol, threadIdx.x, C.cp[threadIdx.x]);
+    } else if (m != nmol - 1) {
+      double p[3];
+      atom_xyz(E, nmol - 1, threadIdx.x, p);
+      atom_store(E, m, threadIdx.x, p);
+    }
   }
 }
 
 /* CBMC reinsertion of a flexible chain (ReinsertionAdsorbateMove,
  * src/mc_moves.c:4415): a new configuration grown with molecule m left out,
- * the old one retraced; accepted with W(new) / W(old). */
+ * the old one retraced; accepted with W(new) / W(old). The retrace's beads
+ * are combined after a successful growth, as a retrace run after it would. */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void step_reinsert_chain(Eng<MIXED, FLEX> &E)
+__device__ __forceinline__ void accept_reinsert_chain(Build<MIXED, FLEX> E, int buf)
 {
-  RgpuSys &S = *E.S;
-  Ctl &C = *E.ctl;
-  const int na = S.natom, nmol = C.nmol;
-  int m = (int)(E.rnd[SLOT_MOLECULE] * nmol);
-  if (m >= nmol) m = nmol - 1;
-  /* the retrace of the old configuration rides along with the growth's
-   * first evaluations (it does not depend on the new chain); its beads are
-   * combined after a successful growth, as a retrace run after it would */
-  grow_chain(E, false, 0, m, m, true);
-  if (C.fail) return;
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int na = S.natom;
+  bool accept = false;
   if (threadIdx.x == 0) {
-    C.rosen_old = C.rosen;     /* the new configuration's weight */
-    C.dl[0] = C.u[0];
-    C.dl[2] = C.u[2];
-    C.uintra_old = C.uintra;
-    for (int a = 0; a < na; a++)
-      for (int d = 0; d < 3; d++) C.cpn[a][d] = C.cp[a][d];
+    const double w_new = C.rosen, dl0 = C.u[0], dl2 = C.u[2], intra = C.uintra;
     C.rosen = 1.0;
     C.u[0] = C.u[1] = C.u[2] = C.u[3] = 0.0;
     C.uintra = 0.0;
     retrace_combine(C, 0, na, S.ntrial_first, S.ntrial);
-  }
-  __syncthreads();
-  if (C.fail) return;
-  if (threadIdx.x == 0) {
-    const double w_new = C.rosen_old, w_old = C.rosen;
-    const double pacc = w_new / w_old;
-    if (!(pacc == pacc)) C.status |= RGPU_ERR_NONFINITE;
-    C.accept = E.rnd[SLOT_ACCEPT] < pacc;
-    if (C.accept) {
-      C.cnt[RGPU_CNT_REINS_ACCEPT]++;
-      C.energy[RGPU_E_HOST_VDW] += C.dl[0] - C.u[0];
-      C.energy[RGPU_E_ADS_VDW] += C.dl[2] - C.u[2];
-      C.energy[RGPU_E_INTRA] += C.uintra_old - C.uintra;
+    if (!C.fail) {
+      const double pacc = w_new / C.rosen;
+      if (!(pacc == pacc)) C.status |= RGPU_ERR_NONFINITE;
+      accept = C.rnd[buf][SLOT_ACCEPT] < pacc;
+      if (accept) {
+        C.cnt[RGPU_CNT_REINS_ACCEPT]++;
+        C.energy[RGPU_E_HOST_VDW] += dl0 - C.u[0];
+        C.energy[RGPU_E_ADS_VDW] += dl2 - C.u[2];
+        C.energy[RGPU_E_INTRA] += intra - C.uintra;
+      }
     }
   }
-  __syncthreads();
-  if (C.accept) {
-    if (threadIdx.x < na) atom_store(E, m, threadIdx.x, C.cpn[threadIdx.x]);
-    __syncthreads();
+  accept = __shfl_sync(RGPU_FULL, accept, 0);
+  if (accept && threadIdx.x < na) atom_store(E, cur().m, threadIdx.x, C.cp[threadIdx.x]);
+}
+
+/* warp 0, after a growth's last bead */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void end_chain(Build<MIXED, FLEX> E, int buf)
+{
+  Ctl &C = fx().C;
+  const int last = fx().S.natom - 1;
+  if (last >= 2 && threadIdx.x == 0) C.uintra += C.ub[last & 1][C.sel];
+  __syncwarp();
+  if (cur().mv == 4) accept_reinsert_chain(E, buf);
+  else accept_swap_chain(E, buf);
+}
+
+/* warp 0, after a retrace group of a deletion: returns whether the step is
+ * done */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ bool end_retrace(Build<MIXED, FLEX> E, const Stage &g, int buf)
+{
+  RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  if (threadIdx.x == 0) retrace_combine(C, g.r0, g.r1, S.ntrial_first, S.ntrial);
+  __syncwarp();
+  if (C.fail) return true;
+  if (g.r1 < S.natom) {
+    retrace_stage(E, g.r1);
+    return false;
+  }
+  accept_swap_chain(E, buf);
+  return true;
+}
+
+/* ------------------------------------------------------------------------ */
+/* The state after a step enters the ensemble sums (one thread, in the stage
+ * that follows, before warp 0 changes it again) */
+__device__ __forceinline__ void sample_step(Ctl &C)
+{
+  const double n = (double)C.nmol;
+  const double u = C.energy[0] + C.energy[1] + C.energy[2] + C.energy[3] + C.energy[4] + C.energy[5] +
+                   C.energy[RGPU_E_INTRA];
+  C.sums[RGPU_SUM_SAMPLES] += 1.0;
+  C.sums[RGPU_SUM_N] += n;
+  C.sums[RGPU_SUM_N2] += n * n;
+  C.sums[RGPU_SUM_U] += u;
+  C.sums[RGPU_SUM_UN] += u * n;
+  C.sums[RGPU_SUM_U2] += u * u;
+}
+
+/* counts the move that stage g opens (the same thread) */
+__device__ __forceinline__ void count_step(Ctl &C, const Stage &g)
+{
+  const int mv = g.mv;
+  const bool skip = g.ph == PH_SKIP;
+  /* a displacement or reinsertion without a molecule is not counted (the
+   * reference returns before counting); a swap or Widom move always is */
+  if (skip && (mv <= 1 || mv == 4)) return;
+  C.cnt[RGPU_CNT_MOVES]++;
+  if (mv <= 3) C.cnt[RGPU_CNT_ATTEMPT + mv]++;
+  if (mv == 4) C.cnt[RGPU_CNT_REINS_ATTEMPT]++;
+  if (mv == 2 && skip) C.status |= RGPU_ERR_MAXMOL;
+  if (mv == 5) C.sums[RGPU_SUM_WIDOM_N] += 1.0;   /* overlap samples count with weight 0 */
+}
+
+/* Describes in n the first stage of step `it` (random numbers in buffer buf),
+ * which follows stage c, for the molecules there are now. One warp. */
+template <int MIXED, bool FLEX>
+__device__ RGPU_COLD void start_step(Build<MIXED, FLEX> E, Stage &n, const Stage &c, long long it, int buf, long long nsteps,
+                                     uint64_t step_end)
+{
+  const RgpuSys &S = fx().S;
+  const Ctl &C = fx().C;
+  const int na = S.natom, nf = S.ntrial_first, trials = S.ntrial * (na - 1);
+  const int mv = C.mvn[buf], nmol = C.nmol;
+  const bool end = !(it < nsteps && fx().step0 + (uint64_t)it < step_end);
+  const bool ew = has_ewald(S), one = mv == 3 && nf + trials <= RGPU_MAX_POS;
+  int ph, P = 0, check = 0, ns = 0, m = nmol;
+  if (mv != 2 && mv != 5) {
+    m = (int)(C.rnd[buf][SLOT_MOLECULE] * nmol);
+    if (m >= nmol) m = nmol - 1;
+  }
+  if (end) {
+    ph = PH_END;
+  } else if (mv <= 1 ? (nmol == 0 || (mv == 1 && na == 1)) : (mv == 2 ? nmol >= S.maxmol : mv != 5 && nmol == 0)) {
+    ph = PH_SKIP;
+  } else if (mv <= 1) {
+    ph = PH_DISP;
+    P = 2 * na;
+    check = na;
+    ns = ew ? 2 * na : 0;
+  } else if (FLEX && S.flexible) {
+    ph = PH_TABLE;       /* the chain moves begin with a stage that draws the angle tables */
+  } else if (mv == 4) {
+    ph = PH_REINS1;
+    P = nf + 1 + trials;
+  } else {
+    ph = PH_SWAP1;
+    P = one ? nf + trials : nf;
+    ns = one && ew ? na : 0;
+  }
+  fill_stage(E, n, c, ph, P, check, ns);
+  if ((threadIdx.x & 31) == 0) {
+    n.mv = mv;
+    n.m = m;
+    n.one = one;
+    n.buf = buf;
+    n.it = it;
+    n.first = !end;
+    n.db = end ? -1 : (buf == 0 ? 2 : buf - 1);          /* (it + 2) mod 3 */
+    n.dstep = fx().step0 + (uint64_t)it + 2;
+  }
+}
+
+/* Warp 0 after stage c: the bookkeeping of its move, then the next stage, of
+ * this step or of the next one. The latter warp 1 describes meanwhile for an
+ * unchanged number of molecules (start_step into stage c + 2); that stands
+ * unless the number has changed. */
+template <int MIXED, bool FLEX>
+__device__ RGPU_COLD void end_stage(Build<MIXED, FLEX> E, int c, long long nsteps, uint64_t step_end, uint64_t avg0)
+{
+  Ctl &C = fx().C;
+  const Stage &g = C.st[c];
+  const int ph = g.ph, buf = g.buf, nmol = C.nmol;
+  if (threadIdx.x == 0) {
+    C.cur = c;
+    C.accept = 0;
+  }
+  __syncwarp();
+  bool done = true;
+  if (ph == PH_DISP) end_displace(E, buf);
+  else if (ph == PH_SWAP1) done = end_swap1(E, buf);
+  else if (ph == PH_SWAP2) done = add_orientations(E, g.mv != 3, buf) || grown_swap(E, buf);
+  else if (ph == PH_SWAPEW) accept_swap(E, buf);
+  else if (ph == PH_REINS1) done = end_reinsert1(E, buf);
+  else if (ph == PH_REINS2) done = add_orientations(E, true, buf) || grown_reinsert(E, buf);
+  else if (ph == PH_REINSEW) accept_reinsert(E, buf);
+  else if (FLEX && ph == PH_TABLE) { end_table(E); done = false; }
+  else if (FLEX && ph == PH_GROW) done = end_grow(E, g);
+  else if (FLEX && ph == PH_RETRACE) done = end_retrace(E, g, buf);
+  else if (FLEX && ph == PH_CHAINEND) end_chain(E, buf);
+  __syncwarp();
+  int nx = stage_after(c, 1);
+  if (done) {
+    if (C.nmol == nmol) nx = stage_after(c, 2);
+    else start_step(E, C.st[nx], g, g.it + 1, buf == 2 ? 0 : buf + 1, nsteps, step_end);
+  }
+  if (threadIdx.x == 0) {
+    Stage &n = C.st[nx];
+    n.ap = C.accept;
+    n.xa = g.xs;
+    n.sample = done && fx().step0 + (uint64_t)g.it >= avg0;
+    if (done) C.it = g.it + 1;
+    C.which = nx;
   }
 }
 
 /* ------------------------------------------------------------------------ */
 /* Loads a descriptor copy into shared memory. */
-__device__ inline void load_sys(RgpuSys *dst, const RgpuSys *src)
+__device__ __forceinline__ void load_sys(RgpuSys *dst, const RgpuSys *src)
 {
   const uint32_t *s = (const uint32_t *)src;
   uint32_t *d = (uint32_t *)dst;
@@ -1683,7 +1895,7 @@ __device__ inline void load_sys(RgpuSys *dst, const RgpuSys *src)
 template <int MIXED, bool WIDE, bool FLEX>
 __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys *systems, int nsys, long long nsteps,
                                                                        int kw, int max_ads_atoms, int fw_items,
-                                                                       int tile_items, int k_items)
+                                                                       int fwd_items, int tile_items, int k_items)
 {
   extern __shared__ __align__(256) unsigned char smem[];
   cg::cluster_group cl = cg::this_cluster();
@@ -1691,59 +1903,68 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
   const int rank = (int)cl.block_rank();
   const int sysi = blockIdx.x / csize;
   const int nwarps = blockDim.x >> 5;
-  const EngineLayout L = engine_layout(MIXED, fw_items, tile_items, max_ads_atoms, kw, k_items, nwarps, FLEX);
+  const EngineLayout L = engine_layout(MIXED, fw_items, fwd_items, tile_items, max_ads_atoms, kw, k_items, nwarps, FLEX);
   if (sysi < nsys) {
     Eng<MIXED, FLEX> E;
+    const Build<MIXED, FLEX> B;
     E.rank = rank;
     E.csize = csize;
     E.xb = 0;
-    E.S = (RgpuSys *)(smem + L.sys);
-    E.ads = smem + L.ads;
-    E.pos = (BeadPos *)(smem + L.pos);
-    E.uv = (double *)(smem + L.uv);
-    E.uc = (double *)(smem + L.uc);
-    E.uo = (int *)(smem + L.uo);
-    E.part = (PosSum *)(smem + L.part);
-    E.sc.uv = E.uv;
-    E.sc.uc = E.uc;
-    E.sc.uo = E.uo;
+    E.sc.u = fx().u;
     E.sc.qr2 = (float *)(smem + L.q);
     E.sc.qq = E.sc.qr2 + nwarps * (MIXED == 2 ? 128 : 64);
-    E.sc.qt = (int *)(E.sc.qq + nwarps * 64);
-    E.sites = (EwSite *)(smem + L.sites);
+    E.sc.qt = MIXED ? (int *)(E.sc.qq + nwarps * 64) : (int *)(smem + L.q);
     E.tab = (typename PhaseT<MIXED>::T *)(smem + L.tab);
     E.kw = kw;
-    E.red = (double *)(smem + L.red);
-    E.ang = (double *)(smem + L.ang);
-    E.ctl = (Ctl *)(smem + L.ctl);
-    Ctl &C = *E.ctl;
-    E.sc.cnt = C.work;
+    Ctl &C = fx().C;
+    E.sc.cnt = &C.wcnt[0][0];
     E.sc.next = &C.next;
-    load_sys(E.S, &systems[sysi]);
-    RgpuSys &S = *E.S;
+    E.sc.done = C.done;
+    RgpuSys &S = fx().S;
+    load_sys(&S, &systems[sysi]);
     /* a system at its step limit (a finished job left in its slot) takes
      * no step in this launch: its CTAs leave before staging anything and
      * write nothing back. All CTAs of the cluster read the same limits, so
      * the whole cluster leaves and none waits at the cluster barrier below. */
     if (S.step[0] >= S.step[1]) return;
     double2 *sk_global = S.sk_ads;
-    if (threadIdx.x < 5) C.work[threadIdx.x] = 0ULL;
+    if (threadIdx.x < 3 * RGPU_MAX_WARPS) (&C.wcnt[0][0])[threadIdx.x] = 0ULL;
+    if (blockDim.x < 3 * RGPU_MAX_WARPS && threadIdx.x < 32) (&C.wcnt[0][0])[64 + threadIdx.x] = 0ULL;
+    if (threadIdx.x < RGPU_MAX_POS) C.done[threadIdx.x] = 0;   /* blocks have at least 64 threads */
     if (threadIdx.x < RGPU_NCNT) C.cnt[threadIdx.x] = 0;
     if (threadIdx.x < RGPU_NE) C.energy[threadIdx.x] = S.energy[threadIdx.x];
     if (threadIdx.x == 0) {
       C.cyc[0] = C.cyc[1] = 0;
+      C.work[0] = C.work[1] = 0ULL;
       C.status = 0;
       C.next = 0;
+      C.ovf[0] = C.ovf[1] = 0;
+      C.nextk = C.ewdone = 0;
+      Fixed &F = fx();
+      F.step0 = S.step[0];
+      F.ads = (unsigned)L.ads;
+      F.ang = (unsigned)L.ang;
+      F.rank = rank;
+      F.csize = csize;
+      C.it = 0;
+      C.cur = 0;
+      C.which = 0;
+      C.accept = 0;
+      C.st[2].xs = 0;
       for (int k = 0; k < RGPU_NSUM; k++) C.sums[k] = 0.0;
       C.nmol = *S.nmol;
       C.nads = C.nmol * S.natom;
     }
-    /* this CTA's framework share, staged in shared memory when it fits */
-    if (MIXED) {
+    /* this CTA's framework share, staged in shared memory when it fits
+     * (smem_fw 1: fixed-point atoms and tiles; 2: FP64 positions too) */
+    {
       int t0, t1;
       share(S.ntile, rank, csize, t0, t1);
       E.sl.fw_lo = t0;
       E.sl.fw_hi = t1;
+      E.sl.fw = S.fw32;
+      E.sl.tiles = S.tiles;
+      E.sl.fwd = MIXED ? nullptr : S.fw64t;
       if (S.smem_fw) {
         int4 *dfw = (int4 *)(smem + L.fw);
         TileRec *dt = (TileRec *)(smem + L.tiles);
@@ -1751,25 +1972,14 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
         for (int i = threadIdx.x; i < t1 - t0; i += blockDim.x) dt[i] = S.tiles[t0 + i];
         E.sl.fw = dfw - (size_t)t0 * RGPU_TILE;
         E.sl.tiles = dt - t0;
-      } else {
-        E.sl.fw = S.fw32;
-        E.sl.tiles = S.tiles;
       }
-    } else {
-      int a0, a1;
-      share(S.nfw, rank, csize, a0, a1);
-      E.sl.fw_lo = a0;
-      E.sl.fw_hi = a1;
-      E.sl.tiles = nullptr;
-      if (S.smem_fw) {
-        double4 *d = (double4 *)(smem + L.fw);
-        for (int i = threadIdx.x; i < a1 - a0; i += blockDim.x) d[i] = S.fw64[a0 + i];
-        E.sl.fw = d - a0;
-      } else {
-        E.sl.fw = S.fw64;
+      if (!MIXED && S.smem_fw > 1) {
+        double4 *d = (double4 *)(smem + L.fwd);
+        for (int i = threadIdx.x; i < (t1 - t0) * RGPU_TILE; i += blockDim.x) d[i] = S.fw64t[t0 * RGPU_TILE + i];
+        E.sl.fwd = d - (size_t)t0 * RGPU_TILE;
       }
     }
-    E.sl.ads = E.ads;
+    E.sl.ads = smem + L.ads;
     if (FLEX && S.use_grid) E.sl.fw_hi = E.sl.fw_lo;   /* host VDW from the grids: no framework pairs */
     /* this CTA's wave vectors with their prefactors and S(k) */
     if (S.ewald) share(S.nk, rank, csize, E.k0, E.k1);
@@ -1802,72 +2012,67 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
       if (MIXED) {
         int xi, yi, zi;
         rgpu_fix3(S, x[0], x[1], x[2], xi, yi, zi);
-        ((int4 *)E.ads)[i] = make_int4(xi, yi, zi, mm * 16 + a);
+        ((int4 *)(smem + L.ads))[i] = make_int4(xi, yi, zi, mm * 16 + a);
       } else
-        atom_store(E, mm, a, x);
+        atom_store(B, mm, a, x);
     }
     __syncthreads();
-    const uint64_t step0 = S.step[0], step_end = S.step[1], avg0 = S.step[2];
+    E.step0 = S.step[0];
+    const uint64_t step_end = S.step[1], avg0 = S.step[2];
     const long long t_start = clock64();
-    long long it = 0;
-    for (; it < nsteps && step0 + (uint64_t)it < step_end; it++) {
-      const uint64_t step = step0 + (uint64_t)it;
-      /* this step's random numbers, one Philox block per thread */
-      double *rb = C.rnd[it & 1];
-      for (int i = threadIdx.x; i < RGPU_RND / 2; i += blockDim.x) rgpu_uniform_pair(S.seed, S.sys_id, step, i, &rb[2 * i]);
-      __syncthreads();
-      E.rnd = rb;
-      E.step = step;
-      const double u0 = rb[SLOT_MOVE];
-      int mv = 0;
-      while (mv < 5 && u0 >= S.cum[mv]) mv++;
-      const int nmol = C.nmol;
-      share(C.nads, rank, csize, E.sl.ads_lo, E.sl.ads_hi);
-      if (mv <= 1) {
-        if (!(nmol == 0 || (mv == 1 && S.natom == 1))) {
-          if (threadIdx.x == 0) { C.cnt[RGPU_CNT_MOVES]++; C.cnt[RGPU_CNT_ATTEMPT + mv]++; }
-          step_displace(E, mv);
-        }
-      } else if (mv == 2) {
-        if (threadIdx.x == 0) { C.cnt[RGPU_CNT_MOVES]++; C.cnt[RGPU_CNT_ATTEMPT + 2]++; }
-        if (nmol >= S.maxmol) {
-          if (threadIdx.x == 0) C.status |= RGPU_ERR_MAXMOL;
-        } else if (FLEX && S.flexible) {
-          step_swap_chain(E, true, false);
-        } else {
-          step_swap(E, true);
-        }
-      } else if (mv == 3) {
-        if (threadIdx.x == 0) { C.cnt[RGPU_CNT_MOVES]++; C.cnt[RGPU_CNT_ATTEMPT + 3]++; }
-        if (nmol != 0) {
-          if (FLEX && S.flexible) step_swap_chain(E, false, false);
-          else step_swap(E, false);
-        }
-      } else if (mv == 4) {
-        /* the reference returns before counting when there is no molecule */
-        if (nmol != 0) {
-          if (threadIdx.x == 0) { C.cnt[RGPU_CNT_MOVES]++; C.cnt[RGPU_CNT_REINS_ATTEMPT]++; }
-          if (FLEX && S.flexible) step_reinsert_chain(E);
-          else step_reinsert(E);
-        }
-      } else {
-        if (threadIdx.x == 0) C.cnt[RGPU_CNT_MOVES]++;
-        if (FLEX && S.flexible) step_swap_chain(E, true, true);
-        else step_swap(E, true, true);
+    draw_step(B, E.step0, 0, threadIdx.x, blockDim.x);
+    draw_step(B, E.step0 + 1, 1, threadIdx.x, blockDim.x);
+    __syncthreads();
+    if (threadIdx.x < 32) start_step(B, C.st[0], C.st[2], 0, 0, nsteps, step_end);
+    if (threadIdx.x == 0) {
+      C.st[0].ap = 0;
+      C.st[0].sample = 0;
+    }
+    for (;;) {
+      __syncthreads();            /* the stage that warp 0 described */
+      const int c = C.which;
+      const Stage &g = C.st[c];
+      if (threadIdx.x == blockDim.x - 1) {
+        if (g.sample) sample_step(C);
+        if (g.first) count_step(C, g);
       }
-      /* ensemble sums after the step (thread 0 owns the running values) */
-      if (threadIdx.x == 0 && step >= avg0) {
-        const double n = (double)C.nmol;
-        const double u = C.energy[0] + C.energy[1] + C.energy[2] + C.energy[3] + C.energy[4] + C.energy[5] +
-                         C.energy[RGPU_E_INTRA];
-        C.sums[RGPU_SUM_SAMPLES] += 1.0;
-        C.sums[RGPU_SUM_N] += n;
-        C.sums[RGPU_SUM_N2] += n * n;
-        C.sums[RGPU_SUM_U] += u;
-        C.sums[RGPU_SUM_UN] += u * n;
-        C.sums[RGPU_SUM_U2] += u * u;
+      const int np = g.P + (g.ph == PH_DISP ? 0 : g.ns);
+      if (np) {
+        for (int i = threadIdx.x; i < np; i += blockDim.x) place(B, g, i);
+        __syncthreads();
+        eval_stage(E, g);
+      } else {
+        if (g.ap)
+          ewald_apply_share<MIXED>(S, E.tab, E.kw, fx().sites[g.xa & 1], g.ap, E.k0, E.k1, threadIdx.x >> 5);
+        if (g.ph == PH_END) break;
+        if (FLEX && g.ph == PH_TABLE) chain_tables(B, g);
+        __syncthreads();          /* also: every thread knows the stage before warp 0 names the next */
+      }
+      if (FLEX && g.ph == PH_RETRACE) {
+        retrace_book(B, g.r0, g.r1, 0, C.cp, fx_ang(), 0);
+        __syncthreads();
+      }
+      if (threadIdx.x < 32) {
+        end_stage(B, c, nsteps, step_end, avg0);
+      } else {
+        /* warp 1: the next step's first stage, should this stage end its step */
+        if (threadIdx.x < 64 && g.ph != PH_TABLE)
+          start_step(B, C.st[stage_after(c, 2)], g, g.it + 1, g.buf == 2 ? 0 : g.buf + 1, nsteps, step_end);
+        if (FLEX && g.ph == PH_GROW) {
+          /* a riding retrace group's bookkeeping; then warp 1: the bonded
+           * energies of this bead's trials (warp 0 writes only C.cp[ci]) */
+          if (g.r1 > g.r0) retrace_book(B, g.r0, g.r1, g.k, C.co, fx_ang() + RGPU_ANG_DOUBLES, 1);
+          const int t = threadIdx.x - 32;
+          if (g.ci >= 2 && t < g.k) {
+            const BeadPos &q = fx().pos[t];
+            const double p[3] = {q.x, q.y, q.z};
+            C.ub[g.ci & 1][t] = chain_bonded_energy(S, C.cp, g.ci, p);
+          }
+        }
+        if (g.db >= 0) draw_step(B, g.dstep, g.db, threadIdx.x - 32, blockDim.x - 32);
       }
     }
+    const long long it = C.it;
     __syncthreads();
     /* write back: positions, molecule count, energies, counters (rank 0);
      * this CTA's share of S(k) and its work counters (every CTA) */
@@ -1878,7 +2083,7 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
       for (int i = threadIdx.x; !MIXED && i < C.nads; i += blockDim.x) {
         const int mm = i / S.natom, a = i - mm * S.natom;
         double p[3];
-        atom_xyz(E, mm, a, p);
+        atom_xyz(B, mm, a, p);
         S.ads_xyz[3 * i] = p[0];
         S.ads_xyz[3 * i + 1] = p[1];
         S.ads_xyz[3 * i + 2] = p[2];
@@ -1886,7 +2091,7 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
       if (threadIdx.x < RGPU_NE) S.energy[threadIdx.x] = C.energy[threadIdx.x];
       if (threadIdx.x == 0) {
         *S.nmol = C.nmol;
-        S.step[0] = step0 + (uint64_t)it;
+        S.step[0] = E.step0 + (uint64_t)it;
         for (int k = 0; k < RGPU_NSUM; k++) S.sums[k] += C.sums[k];
         for (int c = 0; c < RGPU_CNT_PAIRS; c++) S.counters[c] += C.cnt[c];
         S.counters[RGPU_CNT_REINS_ATTEMPT] += C.cnt[RGPU_CNT_REINS_ATTEMPT];
@@ -1897,15 +2102,21 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
         S.counters[RGPU_CNT_CYC_EWALD] += C.cyc[1];
       }
     }
-    if (threadIdx.x == 0)
-      for (int c = 0; c < 5; c++) atomicAdd((unsigned long long *)&S.counters[RGPU_CNT_PAIRS + c], C.work[c]);
+    if (threadIdx.x < 5) {
+      unsigned long long v = 0;
+      if (threadIdx.x < 3)
+        for (int w = 0; w < nwarps; w++) v += C.wcnt[w][threadIdx.x];
+      else
+        v = C.work[threadIdx.x - 3];
+      atomicAdd((unsigned long long *)&S.counters[RGPU_CNT_PAIRS + threadIdx.x], v);
+    }
   }
   /* no CTA may leave while a peer can still read its shared memory */
   cl.sync();
 }
 
 /* the kernel build for (mixed, wide, flex) */
-using EngineKernel = void (*)(RgpuSys *, int, long long, int, int, int, int, int);
+using EngineKernel = void (*)(RgpuSys *, int, long long, int, int, int, int, int, int);
 static EngineKernel engine_kernel(int mixed, bool wide, bool flex)
 {
   if (mixed == 2) return wide ? rgpu_engine_kernel<2, true, false> : rgpu_engine_kernel<2, false, false>;
@@ -1920,10 +2131,10 @@ cudaError_t rgpu_engine_prepare(int mixed, bool wide, bool flex, size_t smem)
 }
 
 cudaError_t rgpu_engine_launch(int mixed, RgpuSys *d_systems, int nsys, long long nsteps, int kw,
-                               int max_ads_atoms, int fw_items, int tile_items, int k_items, int cluster,
+                               int max_ads_atoms, int fw_items, int fwd_items, int tile_items, int k_items, int cluster,
                                int threads, bool wide, bool flex, cudaStream_t st)
 {
-  size_t smem = rgpu_engine_smem_bytes(mixed, fw_items, tile_items, max_ads_atoms, kw, k_items, threads, flex);
+  size_t smem = rgpu_engine_smem_bytes(mixed, fw_items, fwd_items, tile_items, max_ads_atoms, kw, k_items, threads, flex);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nsys * cluster), 1, 1);
   cfg.blockDim = dim3((unsigned)threads, 1, 1);
@@ -1939,7 +2150,7 @@ cudaError_t rgpu_engine_launch(int mixed, RgpuSys *d_systems, int nsys, long lon
   /* the dynamic shared-memory limit is raised by rgpu_engine_prepare, outside
    * any stream capture */
   return cudaLaunchKernelEx(&cfg, engine_kernel(mixed, wide, flex), d_systems, nsys, nsteps, kw, max_ads_atoms,
-                            fw_items, tile_items, k_items);
+                            fw_items, fwd_items, tile_items, k_items);
 }
 
 /* Batched state transfer of an engine's systems through one staging buffer:

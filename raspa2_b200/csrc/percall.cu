@@ -153,8 +153,7 @@ __global__ void __launch_bounds__(64 * POINT_MIXED_WARPS) k_points_mixed(const R
 {
   __shared__ RgpuSys S;
   __shared__ BeadPos b;
-  __shared__ float qr2[2 * POINT_MIXED_WARPS * 64], qq[2 * POINT_MIXED_WARPS * 64];
-  __shared__ int qt[2 * POINT_MIXED_WARPS * 64];
+  __shared__ __align__(8) float queue[2 * POINT_MIXED_WARPS * RGPU_QUEUE_FLOATS];
   __shared__ double red[2 * POINT_MIXED_WARPS][2];
   __shared__ int rov[2 * POINT_MIXED_WARPS];
   const int p = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, per = pl.cf + pl.ca;
@@ -165,20 +164,19 @@ __global__ void __launch_bounds__(64 * POINT_MIXED_WARPS) k_points_mixed(const R
   if (w < per) {
     float av = 0.0f, ac = 0.0f;
     int o = 0, nin = 0, nch = 0, nvis = 0;
-    float *r2 = qr2 + 64 * w, *q = qq + 64 * w;
-    int *t = qt + 64 * w;
+    float *mem = queue + RGPU_QUEUE_FLOATS * w;
     if (w < pl.cf) {
       const int lo = (int)((unsigned)(S.ntile * w) / (unsigned)pl.cf);
       const int hi = (int)((unsigned)(S.ntile * (w + 1)) / (unsigned)pl.cf);
       if (S.triclinic)
-        unit_tiles_mixed<true>(S, S.fw32, S.tiles, lo, hi, b, check, av, ac, o, nin, nch, nvis, r2, q, t);
+        unit_tiles_mixed<true>(S, S.fw32, S.tiles, lo, hi, b, check, av, ac, o, nin, nch, nvis, mem);
       else
-        unit_tiles_mixed<false>(S, S.fw32, S.tiles, lo, hi, b, check, av, ac, o, nin, nch, nvis, r2, q, t);
+        unit_tiles_mixed<false>(S, S.fw32, S.tiles, lo, hi, b, check, av, ac, o, nin, nch, nvis, mem);
     } else {
       const int c = w - pl.cf;
       const int lo = (int)((unsigned)(nads * c) / (unsigned)pl.ca), hi = (int)((unsigned)(nads * (c + 1)) / (unsigned)pl.ca);
-      if (S.triclinic) unit_ads_mixed<true>(S, ads, b, lo, hi, b.excl, check, av, ac, o, nin, nch, nvis, r2, q, t);
-      else unit_ads_mixed<false>(S, ads, b, lo, hi, b.excl, check, av, ac, o, nin, nch, nvis, r2, q, t);
+      if (S.triclinic) unit_ads_mixed<true>(S, ads, b, lo, hi, b.excl, check, av, ac, o, nin, nch, nvis, mem);
+      else unit_ads_mixed<false>(S, ads, b, lo, hi, b.excl, check, av, ac, o, nin, nch, nvis, mem);
     }
     const double ev = (double)warp_sum(av), eq = (double)warp_sum(ac);
     o = warp_or(o);

@@ -262,9 +262,8 @@ __device__ inline void block_sum2(double &a, double &b, double *red)
  * early-out of the *EnergyDifference routines, e.g.
  * src/framework_energy.c:4988-4990).
  *
- * A call covers a slice of the framework ([fw_lo, fw_hi): tiles on the mixed
- * path, atoms on the FP64 path) and a slice of the adsorbate atoms, so that
- * the CTAs of a cluster can share one system. Work is split into
+ * A call covers a slice of the framework (tiles [fw_lo, fw_hi)) and a slice
+ * of the adsorbate atoms, so that the CTAs of a cluster can share one system. Work is split into
  * (position, slice chunk) units spread over the warps; a unit's lane sums are
  * warp-reduced and the per-position sums formed in FP64.
  *
@@ -277,29 +276,40 @@ __device__ inline void block_sum2(double &a, double &b, double *red)
  * with all lanes busy instead of under a divergent branch.
  */
 struct EvalScratch {
-  double *uv;     /* [max units] */
-  double *uc;
-  int *uo;
+  double2 *u;     /* [max units] {VDW, charge} sums of the units */
+  double4 *part;  /* [P] sums of each position, units in order */
+  int *done;      /* [P] units done of each position; 0 when an evaluation starts */
+  int *ovf;       /* set when a pair of a checked position reaches the overlap criterion */
   int *next;      /* unit counter of the dynamic schedule; 0 when an evaluation starts */
-  unsigned long long *cnt;   /* optional {pairs visited, in cut-off, charged in cut-off} */
-  float *qr2;     /* per-warp queue of in-cut-off pairs (mixed path): [nwarps][64], or
-                   * [nwarps][64] doubles for MIXED = 2 */
-  float *qq;
-  int *qt;
+  unsigned long long *cnt;   /* [nwarps][3] pairs visited, in cut-off, charged in cut-off, by warp */
+  float *qr2;     /* per-warp queues of in-cut-off pairs: [nwarps][RGPU_QUEUE_FLOATS]; MIXED = 2: the squared
+                   * distances, [nwarps][64] doubles */
+  float *qq;      /* MIXED = 2: charges and table indices, [nwarps][64] each */
+  int *qt;        /* also the FP64 path's queue of preselected atoms */
 };
+
+/* a / b for small integers (0 <= a < 2^12, 1 <= b < 2^12) */
+__host__ __device__ __forceinline__ int small_div(int a, int b)
+{
+#ifdef __CUDA_ARCH__
+  return (int)(((float)a + 0.5f) * __frcp_rn((float)b));
+#else
+  return a / b;
+#endif
+}
 
 struct EvalPlan {
   int cf, ca;     /* framework / adsorbate chunks per position */
   int nunits;
 };
 
-/* nfw: framework items of the slice (tiles or atoms), nads: adsorbate atoms of
- * the slice, minitems: smallest worthwhile chunk of framework items */
+/* nfw: framework tiles of the slice, nads: adsorbate atoms of
+ * the slice, minitems: smallest worthwhile chunk of tiles */
 __host__ __device__ __forceinline__ EvalPlan eval_plan(int P, int nfw, int nads, int nwarps, int max_units, int minitems)
 {
   EvalPlan pl;
   int target = nwarps;
-  int cf = target / P;                /* at most one framework unit per warp */
+  int cf = small_div(target, P);      /* at most one framework unit per warp */
   int maxcf = (nfw + minitems - 1) / minitems;
   if (cf > maxcf) cf = maxcf;
   if (cf < 1) cf = 1;
@@ -345,41 +355,49 @@ __device__ __forceinline__ void pair_mixed_queued(const RgpuLJf *P, float r2, fl
 /* Per-warp queue of pairs inside the cut-off (squared distance, partner
  * charge, LJ table index). Lanes append their pair when `in`; whenever 32 or
  * more pairs are queued, all lanes evaluate 32 of them at once, so the pair
- * arithmetic runs with every lane busy instead of under a divergent branch. */
+ * arithmetic runs with every lane busy instead of under a divergent branch.
+ * The 64 entries are a ring (head .. head + n - 1), so what is left after an
+ * evaluation stays where it is; entry j of the sequence goes to lane j mod 32. */
+#define RGPU_QUEUE_FLOATS 192   /* of one warp: 64 {r2, charge} pairs, 64 table indices */
+
 struct PairQueue {
-  float *r2, *q;
+  float2 *e;
   int *t;
-  int n;
+  int head, n;
+  unsigned below;               /* mask of the lanes below this one */
   const RgpuLJf *P;
   bool charged, check;
   float qa, alpha, thr;
 };
 
+__device__ __forceinline__ void queue_init(PairQueue &Q, float *mem)
+{
+  Q.e = (float2 *)mem;
+  Q.t = (int *)mem + 128;
+  Q.head = Q.n = 0;
+  Q.below = (1u << (threadIdx.x & 31)) - 1u;
+}
+
 __device__ __forceinline__ void queue_add(PairQueue &Q, bool in, float r2, float q, int t, float &av, float &ac,
                                           int &ov, int &nin, int &nch)
 {
-  const int lane = threadIdx.x & 31;
   const unsigned bal = __ballot_sync(RGPU_FULL, in);
   if (in) {
-    const int p = Q.n + __popc(bal & ((1u << lane) - 1u));
-    Q.r2[p] = r2;
-    Q.q[p] = q;
+    const int p = (Q.head + Q.n + __popc(bal & Q.below)) & 63;
+    Q.e[p] = make_float2(r2, q);
     Q.t[p] = t;
   }
   Q.n += __popc(bal);
   if (Q.n >= 32) {
     __syncwarp();
-    const float e_r2 = Q.r2[lane], e_q = Q.q[lane];
-    const int e_t = Q.t[lane];
-    float t_r2 = 0.0f, t_q = 0.0f;
-    int t_t = 0;
-    if (lane < Q.n - 32) { t_r2 = Q.r2[32 + lane]; t_q = Q.q[32 + lane]; t_t = Q.t[32 + lane]; }
+    const int p = (Q.head + (threadIdx.x & 31)) & 63;
+    const float2 e = Q.e[p];
+    const int et = Q.t[p];
     __syncwarp();
-    if (lane < Q.n - 32) { Q.r2[lane] = t_r2; Q.q[lane] = t_q; Q.t[lane] = t_t; }
-    nin++;
-    pair_mixed_queued(Q.P, e_r2, e_q, Q.charged, Q.qa, Q.alpha, Q.check, Q.thr, av, ac, ov, nch, e_t);
+    Q.head = (Q.head + 32) & 63;
     Q.n -= 32;
-    __syncwarp();
+    nin++;
+    pair_mixed_queued(Q.P, e.x, e.y, Q.charged, Q.qa, Q.alpha, Q.check, Q.thr, av, ac, ov, nch, et);
   }
 }
 
@@ -389,9 +407,10 @@ __device__ __forceinline__ void queue_drain(PairQueue &Q, float &av, float &ac, 
   const int lane = threadIdx.x & 31;
   __syncwarp();
   if (lane < Q.n) {
+    const int p = (Q.head + lane) & 63;
+    const float2 e = Q.e[p];
     nin++;
-    pair_mixed_queued(Q.P, Q.r2[lane], Q.q[lane], Q.charged, Q.qa, Q.alpha, Q.check, Q.thr, av, ac, ov, nch,
-                      Q.t[lane]);
+    pair_mixed_queued(Q.P, e.x, e.y, Q.charged, Q.qa, Q.alpha, Q.check, Q.thr, av, ac, ov, nch, Q.t[p]);
   }
   Q.n = 0;
   __syncwarp();
@@ -490,220 +509,6 @@ __device__ __forceinline__ double rgpu_fix_r2_d(const RgpuSys &S, int ix, int iy
   return dx * dx + dy * dy + dz * dz;
 }
 
-static_assert(RGPU_TILE == 16, "unit_tiles_mixed visits two tiles per warp pass, one per half warp");
-
-/* framework tiles [t0, t1) for bead b, FP32 path (warp-wide); TRI: the
- * box is triclinic (S.triclinic) */
-template <bool TRI>
-__device__ __forceinline__ void unit_tiles_mixed(const RgpuSys &S, const int4 *fw, const TileRec *tiles, int t0, int t1,
-                                                 const BeadPos &b, bool check, float &av, float &ac, int &ov,
-                                                 int &nin, int &nch, int &nvis, float *qr2, float *qq, int *qt)
-{
-  const int lane = threadIdx.x & 31;
-  const float sx = S.fix_scale[0], sy = S.fix_scale[1], sz = S.fix_scale[2];
-  const float rc2 = S.rc2f;
-  PairQueue Q;
-  Q.r2 = qr2; Q.q = qq; Q.t = qt; Q.n = 0;
-  Q.P = S.ljf_bf[b.atom];
-  Q.qa = S.mol_qf[b.atom] * S.coulombf;
-  Q.charged = S.fw_charged && Q.qa != 0.0f;
-  Q.check = check;
-  Q.alpha = S.alphaf;
-  Q.thr = (float)S.overlap;
-  const bool tri = TRI;
-  for (int tb = t0; tb < t1; tb += 32) {
-    const int t = tb + lane;
-    bool vis = false;
-    int tn = 0;                  /* atoms of this lane's tile */
-    if (t < t1) {
-      const TileRec tr = tiles[t];
-      tn = tr.c.w;
-      if (!tri) {
-        float dx = fmaxf(fabsf(__int2float_rn(tr.c.x - b.xi) * sx) - tr.h.x, 0.0f);
-        float dy = fmaxf(fabsf(__int2float_rn(tr.c.y - b.yi) * sy) - tr.h.y, 0.0f);
-        float dz = fmaxf(fabsf(__int2float_rn(tr.c.z - b.zi) * sz) - tr.h.z, 0.0f);
-        vis = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < rc2;
-      } else {
-        /* triclinic tile: h = fractional half extents, h.w = Cartesian
-         * radius. Every atom's wrapped fractional offset along axis r is at
-         * least |t_r| - h_r, so it lies at least that many perpendicular
-         * widths away; when no atom can wrap differently from the centre
-         * (|t_r| + h_r < 1/2 on every axis), it also lies at least the
-         * centre's distance minus the radius away. */
-        const int ix = tr.c.x - b.xi, iy = tr.c.y - b.yi, iz = tr.c.z - b.zi;
-        const float tx = fabsf(__int2float_rn(ix) * 2.3283064365386963e-10f);
-        const float ty = fabsf(__int2float_rn(iy) * 2.3283064365386963e-10f);
-        const float tz = fabsf(__int2float_rn(iz) * 2.3283064365386963e-10f);
-        const float m = fmaxf(fmaxf((tx - tr.h.x) * S.wperp[0], (ty - tr.h.y) * S.wperp[1]),
-                              (tz - tr.h.z) * S.wperp[2]);
-        vis = !(m > 0.0f && m * m >= rc2);
-        if (vis && tx + tr.h.x < 0.5f && ty + tr.h.y < 0.5f && tz + tr.h.z < 0.5f) {
-          float dx, dy, dz;
-          rgpu_fix_to_cart_tri(S, ix, iy, iz, dx, dy, dz);
-          const float e = fmaxf(sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - tr.h.w, 0.0f);
-          vis = e * e < rc2;
-        }
-      }
-    }
-    unsigned m = __ballot_sync(RGPU_FULL, vis);
-    /* two visible tiles per pass of the warp: lanes 0-15 take the atoms of
-     * the first, lanes 16-31 those of the second */
-    const int half = lane >> 4, hl = lane & 15;
-    while (m) {
-      const int i1 = __ffs(m) - 1;
-      m &= m - 1;
-      const int i2 = m ? __ffs(m) - 1 : -1;
-      m &= m - 1;
-      const int n1 = __shfl_sync(RGPU_FULL, tn, i1);
-      const int n2s = __shfl_sync(RGPU_FULL, tn, i2 >= 0 ? i2 : 0);
-      const int n2 = i2 >= 0 ? n2s : 0;
-      nvis += n1 + n2;
-      const int mine = half ? i2 : i1, nmine = half ? n2 : n1;
-      int4 f = make_int4(0, 0, 0, 0);
-      if (hl < nmine) f = fw[(tb + mine) * RGPU_TILE + hl];
-      float dx, dy, dz;
-      if (!tri) {
-        dx = __int2float_rn(f.x - b.xi) * sx;
-        dy = __int2float_rn(f.y - b.yi) * sy;
-        dz = __int2float_rn(f.z - b.zi) * sz;
-      } else {
-        rgpu_fix_to_cart_tri(S, f.x - b.xi, f.y - b.yi, f.z - b.zi, dx, dy, dz);
-      }
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      queue_add(Q, hl < nmine && r2 < rc2, r2, __int_as_float(f.w), f.z & 3, av, ac, ov, nin, nch);
-    }
-  }
-  queue_drain(Q, av, ac, ov, nin, nch);
-}
-
-/* unit_tiles_mixed for MIXED = 2: the same tile culling in FP32, then each
- * visited pair's distance and cut-off test in FP64 (queued as FP64), its LJ
- * term in FP32 and its real-space charge-charge term in FP64; qr2 holds 64
- * doubles */
-template <bool TRI>
-__device__ __forceinline__ void unit_tiles_cc64(const RgpuSys &S, const int4 *fw, const TileRec *tiles, int t0, int t1,
-                                                const BeadPos &b, bool check, float &av,
-                                                double &ac, int &ov, int &nin, int &nch, int &nvis, float *qr2,
-                                                float *qq, int *qt)
-{
-  const int lane = threadIdx.x & 31;
-  const float sx = S.fix_scale[0], sy = S.fix_scale[1], sz = S.fix_scale[2];
-  const float rc2 = S.rc2f;
-  PairQueueQ Q;
-  Q.r2 = reinterpret_cast<double *>(qr2); Q.q = qq; Q.t = qt; Q.n = 0;
-  Q.P = S.ljf_bf[b.atom];
-  Q.qa = S.mol_q[b.atom] * S.coulomb;
-  Q.alpha = S.alpha;
-  Q.charged = S.fw_charged && Q.qa != 0.0;
-  Q.check = check;
-  Q.thr = (float)S.overlap;
-  const bool tri = TRI;
-  for (int tb = t0; tb < t1; tb += 32) {
-    const int t = tb + lane;
-    bool vis = false;
-    int tn = 0;                  /* atoms of this lane's tile */
-    if (t < t1) {
-      const TileRec tr = tiles[t];
-      tn = tr.c.w;
-      if (!tri) {
-        float dx = fmaxf(fabsf(__int2float_rn(tr.c.x - b.xi) * sx) - tr.h.x, 0.0f);
-        float dy = fmaxf(fabsf(__int2float_rn(tr.c.y - b.yi) * sy) - tr.h.y, 0.0f);
-        float dz = fmaxf(fabsf(__int2float_rn(tr.c.z - b.zi) * sz) - tr.h.z, 0.0f);
-        vis = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < rc2;
-      } else {
-        /* triclinic tile: h = fractional half extents, h.w = Cartesian
-         * radius. Every atom's wrapped fractional offset along axis r is at
-         * least |t_r| - h_r, so it lies at least that many perpendicular
-         * widths away; when no atom can wrap differently from the centre
-         * (|t_r| + h_r < 1/2 on every axis), it also lies at least the
-         * centre's distance minus the radius away. */
-        const int ix = tr.c.x - b.xi, iy = tr.c.y - b.yi, iz = tr.c.z - b.zi;
-        const float tx = fabsf(__int2float_rn(ix) * 2.3283064365386963e-10f);
-        const float ty = fabsf(__int2float_rn(iy) * 2.3283064365386963e-10f);
-        const float tz = fabsf(__int2float_rn(iz) * 2.3283064365386963e-10f);
-        const float m = fmaxf(fmaxf((tx - tr.h.x) * S.wperp[0], (ty - tr.h.y) * S.wperp[1]),
-                              (tz - tr.h.z) * S.wperp[2]);
-        vis = !(m > 0.0f && m * m >= rc2);
-        if (vis && tx + tr.h.x < 0.5f && ty + tr.h.y < 0.5f && tz + tr.h.z < 0.5f) {
-          float dx, dy, dz;
-          rgpu_fix_to_cart_tri(S, ix, iy, iz, dx, dy, dz);
-          const float e = fmaxf(sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - tr.h.w, 0.0f);
-          vis = e * e < rc2;
-        }
-      }
-    }
-    unsigned m = __ballot_sync(RGPU_FULL, vis);
-    /* two visible tiles per pass of the warp: lanes 0-15 take the atoms of
-     * the first, lanes 16-31 those of the second */
-    const int half = lane >> 4, hl = lane & 15;
-    while (m) {
-      const int i1 = __ffs(m) - 1;
-      m &= m - 1;
-      const int i2 = m ? __ffs(m) - 1 : -1;
-      m &= m - 1;
-      const int n1 = __shfl_sync(RGPU_FULL, tn, i1);
-      const int n2s = __shfl_sync(RGPU_FULL, tn, i2 >= 0 ? i2 : 0);
-      const int n2 = i2 >= 0 ? n2s : 0;
-      nvis += n1 + n2;
-      const int mine = half ? i2 : i1, nmine = half ? n2 : n1;
-      int4 f = make_int4(0, 0, 0, 0);
-      if (hl < nmine) f = fw[(tb + mine) * RGPU_TILE + hl];
-      const double r2 = rgpu_fix_r2_d<TRI>(S, f.x - b.xi, f.y - b.yi, f.z - b.zi);
-      queue_add(Q, hl < nmine && r2 < S.rc2, r2, __int_as_float(f.w), f.z & 3, av, ac, ov, nin, nch);
-    }
-  }
-  queue_drain(Q, av, ac, ov, nin, nch);
-}
-
-/* framework atoms [lo, hi) of the type-sorted FP64 layout; TRI: the box is
- * triclinic (S.triclinic) */
-template <bool TRI>
-__device__ __forceinline__ void unit_fw_fp64(const RgpuSys &S, const double4 *fw, const BeadPos &b, int lo,
-                                             int hi, bool check, double &av, double &ac, int &ov, int &nin, int &nch,
-                                             int &nvis)
-{
-  const int lane = threadIdx.x & 31;
-  const double Lx = S.box[0], Ly = S.box[1], Lz = S.box[2];
-  const double ix = S.inv_box[0], iy = S.inv_box[1], iz = S.inv_box[2];
-  const double rc2 = S.rc2, thr = S.overlap;
-  const double qa = S.mol_q[b.atom] * S.coulomb;
-  const bool charged = S.fw_charged && qa != 0.0;
-  const double alpha = S.alpha;
-  nvis += hi - lo;
-  for (int s = 0; s < S.nseg; s++) {
-    int a0 = max(lo, S.seg_start[s]), a1 = min(hi, S.seg_start[s + 1]);
-    if (a0 >= a1) continue;
-    const RgpuLJ P = S.lj_bf[b.atom][s];
-    for (int j = a0 + lane; j < a1; j += 32) {
-      double4 f = fw[j];
-      double dx = b.x - f.x, dy = b.y - f.y, dz = b.z - f.z;
-      if (!TRI) {
-        dx -= Lx * rgpu_nint(dx * ix);
-        dy -= Ly * rgpu_nint(dy * iy);
-        dz -= Lz * rgpu_nint(dz * iz);
-      } else {
-        rgpu_min_image_tri(S, dx, dy, dz);
-      }
-      double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 < rc2) {
-        nin++;
-        double s6 = P.sig2 / r2;
-        s6 = s6 * s6 * s6;
-        double u = P.eps4 * (s6 * (s6 - 1.0)) - P.shift;
-        av += u;
-        if (check && u >= thr) ov = 1;
-        if (charged) {
-          nch++;
-          double r = sqrt(r2);
-          double uc = qa * f.w * (erfc(alpha * r) / r);
-          ac += uc;
-          if (check && uc >= thr) ov = 1;
-        }
-      }
-    }
-  }
-}
-
 /* Whether tile `tr` can hold an atom closer than sqrt(rc2) to bead b (FP32;
  * the tile's extents carry the margin for the rounding) */
 template <bool TRI>
@@ -734,6 +539,122 @@ __device__ __forceinline__ bool tile_visible(const RgpuSys &S, const TileRec &tr
     vis = e * e < rc2;
   }
   return vis;
+}
+
+static_assert(RGPU_TILE == 16, "unit_tiles_mixed visits two tiles per warp pass, one per half warp");
+
+/* unit_tiles_mixed for MIXED = 2: the same tile culling in FP32, then each
+ * visited pair's distance and cut-off test in FP64 (queued as FP64), its LJ
+ * term in FP32 and its real-space charge-charge term in FP64; qr2 holds 64
+ * doubles */
+template <bool TRI>
+__device__ __forceinline__ void unit_tiles_cc64(const RgpuSys &S, const int4 *fw, const TileRec *tiles, int t0, int t1,
+                                                const BeadPos &b, bool check, float &av,
+                                                double &ac, int &ov, int &nin, int &nch, int &nvis, float *qr2,
+                                                float *qq, int *qt)
+{
+  const int lane = threadIdx.x & 31;
+  const float rc2 = S.rc2f;
+  PairQueueQ Q;
+  Q.r2 = reinterpret_cast<double *>(qr2); Q.q = qq; Q.t = qt; Q.n = 0;
+  Q.P = S.ljf_bf[b.atom];
+  Q.qa = S.mol_q[b.atom] * S.coulomb;
+  Q.alpha = S.alpha;
+  Q.charged = S.fw_charged && Q.qa != 0.0;
+  Q.check = check;
+  Q.thr = (float)S.overlap;
+  for (int tb = t0; tb < t1; tb += 32) {
+    const int t = tb + lane;
+    bool vis = false;
+    int tn = 0;                  /* atoms of this lane's tile */
+    if (t < t1) {
+      const TileRec tr = tiles[t];
+      tn = tr.c.w;
+      vis = tile_visible<TRI>(S, tr, b, rc2);
+    }
+    unsigned m = __ballot_sync(RGPU_FULL, vis);
+    /* two visible tiles per pass of the warp: lanes 0-15 take the atoms of
+     * the first, lanes 16-31 those of the second */
+    const int half = lane >> 4, hl = lane & 15;
+    while (m) {
+      const int i1 = __ffs(m) - 1;
+      m &= m - 1;
+      const int i2 = m ? __ffs(m) - 1 : -1;
+      m &= m - 1;
+      const int n1 = __shfl_sync(RGPU_FULL, tn, i1);
+      const int n2s = __shfl_sync(RGPU_FULL, tn, i2 >= 0 ? i2 : 0);
+      const int n2 = i2 >= 0 ? n2s : 0;
+      const int mine = half ? i2 : i1, nmine = half ? n2 : n1;
+      int4 f = make_int4(0, 0, 0, 0);
+      if (hl < nmine) {
+        f = fw[(tb + mine) * RGPU_TILE + hl];
+        nvis++;
+      }
+      const double r2 = rgpu_fix_r2_d<TRI>(S, f.x - b.xi, f.y - b.yi, f.z - b.zi);
+      queue_add(Q, hl < nmine && r2 < S.rc2, r2, __int_as_float(f.w), f.z & 3, av, ac, ov, nin, nch);
+    }
+  }
+  queue_drain(Q, av, ac, ov, nin, nch);
+}
+
+/* framework tiles [t0, t1) for bead b, FP32 path (warp-wide); TRI: the
+ * box is triclinic (S.triclinic). mem: the warp's queue. Issue-bound (about
+ * 45 instructions a pass of two tiles, 90 per 32 queued pairs). */
+template <bool TRI>
+__device__ __forceinline__ void unit_tiles_mixed(const RgpuSys &S, const int4 *fw, const TileRec *tiles, int t0, int t1,
+                                                 const BeadPos &b, bool check, float &av, float &ac, int &ov,
+                                                 int &nin, int &nch, int &nvis, float *mem)
+{
+  const int lane = threadIdx.x & 31;
+  const float sx = S.fix_scale[0], sy = S.fix_scale[1], sz = S.fix_scale[2];
+  const float rc2 = S.rc2f;
+  const int bx = b.xi, by = b.yi, bz = b.zi;
+  PairQueue Q;
+  queue_init(Q, mem);
+  Q.P = S.ljf_bf[b.atom];
+  Q.qa = S.mol_qf[b.atom] * S.coulombf;
+  Q.charged = S.fw_charged && Q.qa != 0.0f;
+  Q.check = check;
+  Q.alpha = S.alphaf;
+  Q.thr = (float)S.overlap;
+  /* two visible tiles per pass of the warp: lanes 0-15 take the atoms of
+   * the first, lanes 16-31 those of the second */
+  const int half = lane >> 4, hl = lane & 15;
+  for (int tb = t0; tb < t1; tb += 32) {
+    bool vis = false;
+    int tn = 0;                  /* atoms of this lane's tile */
+    if (tb + lane < t1) {
+      const TileRec tr = tiles[tb + lane];
+      tn = tr.c.w;
+      vis = tile_visible<TRI>(S, tr, b, rc2);
+    }
+    unsigned m = __ballot_sync(RGPU_FULL, vis);
+    const int4 *row = fw + (size_t)tb * RGPU_TILE + hl;
+    while (m) {
+      const unsigned mm = m & (m - (unsigned)half);   /* the second half skips the first tile */
+      m &= m - 1;
+      m &= m - 1;
+      const int mine = __ffs(mm) - 1;                 /* -1: no second tile */
+      const int n = __shfl_sync(RGPU_FULL, tn, mine & 31);
+      const bool live = mine >= 0 && hl < n;
+      int4 f = make_int4(0, 0, 0, 0);
+      if (live) {
+        f = row[mine * RGPU_TILE];
+        nvis++;
+      }
+      float dx, dy, dz;
+      if (!TRI) {
+        dx = __int2float_rn(f.x - bx) * sx;
+        dy = __int2float_rn(f.y - by) * sy;
+        dz = __int2float_rn(f.z - bz) * sz;
+      } else {
+        rgpu_fix_to_cart_tri(S, f.x - bx, f.y - by, f.z - bz, dx, dy, dz);
+      }
+      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      queue_add(Q, live && r2 < rc2, r2, __int_as_float(f.w), f.z & 3, av, ac, ov, nin, nch);
+    }
+  }
+  queue_drain(Q, av, ac, ov, nin, nch);
 }
 
 /* The LJ + real-space term of one preselected framework atom, FP64: entry =
@@ -808,18 +729,16 @@ __device__ __forceinline__ void unit_tiles_fp64(const RgpuSys &S, const int4 *fw
     }
     unsigned m = __ballot_sync(RGPU_FULL, vis);
     while (m) {
-      const int i1 = __ffs(m) - 1;
+      const unsigned mm = m & (m - (unsigned)half);   /* the second half skips the first tile */
       m &= m - 1;
-      const int i2 = m ? __ffs(m) - 1 : -1;
       m &= m - 1;
-      const int n1 = __shfl_sync(RGPU_FULL, tn, i1);
-      const int n2s = __shfl_sync(RGPU_FULL, tn, i2 >= 0 ? i2 : 0);
-      const int n2 = i2 >= 0 ? n2s : 0;
-      nvis += n1 + n2;
-      const int a = (tb + (half ? i2 : i1)) * RGPU_TILE + hl;
+      const int mine = __ffs(mm) - 1;                 /* -1: no second tile */
+      const int nt = __shfl_sync(RGPU_FULL, tn, mine & 31);
+      const int a = (tb + mine) * RGPU_TILE + hl;
       bool in = false;
       int seg = 0;
-      if (hl < (half ? n2 : n1)) {
+      if (mine >= 0 && hl < nt) {
+        nvis++;
         const int4 f = fw[a];
         seg = f.z & 3;
         float dx, dy, dz;
@@ -852,20 +771,21 @@ __device__ __forceinline__ void unit_tiles_fp64(const RgpuSys &S, const int4 *fw
 template <bool TRI>
 __device__ __forceinline__ void unit_ads_mixed(const RgpuSys &S, const int4 *ads, const BeadPos &b, int lo,
                                                int hi, int exclude, bool check, float &av, float &ac, int &ov,
-                                               int &nin, int &nch, int &nvis, float *qr2, float *qq, int *qt)
+                                               int &nin, int &nch, int &nvis, float *mem)
 {
   const int lane = threadIdx.x & 31;
   const float sx = S.fix_scale[0], sy = S.fix_scale[1], sz = S.fix_scale[2];
   const float rc2 = S.rc2f;
   PairQueue Q;
-  Q.r2 = qr2; Q.q = qq; Q.t = qt; Q.n = 0;
+  queue_init(Q, mem);
   Q.P = S.ljf_bb[b.atom];
   Q.qa = S.mol_qf[b.atom] * S.coulombf;
   Q.charged = S.mol_charged && Q.qa != 0.0f;
   Q.check = check;
   Q.alpha = S.alphaf;
   Q.thr = (float)S.overlap;
-  nvis += hi - lo;
+  nvis += (hi - lo + 31 - lane) >> 5;   /* this lane's records */
+#pragma unroll 1
   for (int jb = lo; jb < hi; jb += 32) {
     const int j = jb + lane;
     bool in = false;
@@ -908,7 +828,8 @@ __device__ __forceinline__ void unit_ads_cc64(const RgpuSys &S, const int4 *ads,
   Q.charged = S.mol_charged && Q.qa != 0.0;
   Q.check = check;
   Q.thr = (float)S.overlap;
-  nvis += hi - lo;
+  nvis += (hi - lo + 31 - lane) >> 5;   /* this lane's records */
+#pragma unroll 1
   for (int jb = lo; jb < hi; jb += 32) {
     const int j = jb + lane;
     bool in = false;
@@ -941,7 +862,7 @@ __device__ __forceinline__ void unit_ads_fp64(const RgpuSys &S, const AdsRec64 *
   const double qa = S.mol_q[b.atom] * S.coulomb;
   const bool charged = S.mol_charged && qa != 0.0;
   const double alpha = S.alpha;
-  nvis += hi - lo;
+  nvis += (hi - lo + 31 - lane) >> 5;   /* this lane's records */
   for (int j = lo + lane; j < hi; j += 32) {
     AdsRec64 f = ads[j];
     int tag = (int)f.tag;
@@ -978,73 +899,69 @@ __device__ __forceinline__ void unit_ads_fp64(const RgpuSys &S, const AdsRec64 *
 
 /* Framework and adsorbate slices of one evaluation */
 struct EvalSlice {
-  const void *fw;          /* int4 atoms (mixed, tiled) or double4 atoms (FP64, type-sorted) */
-  const TileRec *tiles;    /* mixed only */
-  int fw_lo, fw_hi;        /* tiles (mixed) or atoms (FP64) */
+  const int4 *fw;          /* tiled atoms, fixed point */
+  const double4 *fwd;      /* the same atoms in FP64 (FP64 path only) */
+  const TileRec *tiles;
+  int fw_lo, fw_hi;        /* tiles */
   const void *ads;         /* int4 or AdsRec64 records */
   int ads_lo, ads_hi;
 };
 
-/* The (position, chunk) units of P positions over the slice: the unit of
- * position p and chunk c writes its FP64 sums and overlap flag to
- * sc.uv/uc/uo[p * (cf + ca) + c]. Warps take units dynamically from
- * *sc.next (framework chunks of every position first, then adsorbate
- * chunks), fetching the next index while they work on the current one, so
- * the warps of the block finish together. The stored sums do not depend on
- * which warp evaluated a unit. No block barrier; *sc.next is left past the
- * last unit (the caller resets it after its barrier). Returns the plan. */
+/* The (position, chunk) units of P positions over the slice, cut into cf
+ * framework and ca adsorbate chunks per position: the unit of position p and
+ * chunk c leaves its FP64 sums in sc.u[p * (cf + ca) + c] and sets *sc.ovf for
+ * an overlap; the warp that finishes the last unit of a position adds them up
+ * in order into sc.part[p] (.x, .y over the framework chunks if there are any,
+ * .z, .w over the adsorbate ones). Warps take units dynamically from *sc.next
+ * (framework chunks of every position first, then adsorbate chunks), fetching
+ * the next index while they work on the current one, so the warps of the
+ * block finish together. The sums do not depend on which warp evaluated a
+ * unit. No block barrier; *sc.next is left past the last unit (the caller
+ * resets it after its barrier). mf, ma: floor(2^32 / cf) + 1 and the same of
+ * ca, 0 for one chunk: chunk bounds n * c / cf are the high half of a product
+ * (exact for n * c < 2^26). */
 template <int MIXED>
-__device__ __forceinline__ EvalPlan eval_units(const RgpuSys &S, const EvalSlice &sl, const BeadPos *pos, int P, int pair_check,
-                               EvalScratch sc, int max_units)
+__device__ __forceinline__ void eval_units(const RgpuSys &S, const EvalSlice &sl, const BeadPos *pos, int P, int pair_check,
+                                           const EvalScratch &sc, int cf, int ca, unsigned mf, unsigned ma)
 {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nfw = sl.fw_hi - sl.fw_lo, nads = sl.ads_hi - sl.ads_lo;
-  const EvalPlan pl = eval_plan(P, nfw, nads, nw, max_units, MIXED ? 2 : 64);
-  const int per = pl.cf + pl.ca;
-  const int nfu = P * pl.cf;     /* framework units */
+  const int per = cf + ca;
+  const int nunits = P * per;
   /* work counts of this lane, summed over its units (statistics only) */
   int nin = 0, nch = 0, nvis = 0;
   int v = 0;
   if (lane == 0) v = atomicAdd(sc.next, 1);
   v = __shfl_sync(RGPU_FULL, v, 0);
-  while (v < pl.nunits) {
+  while (v < nunits) {
     int vn = 0;
     if (lane == 0) vn = atomicAdd(sc.next, 1);
     int p, c;
-    if (v < nfu) {
-      c = v / P;
-      p = v - c * P;
-    } else {
-      const int v2 = v - nfu;
-      const int ca = v2 / P;
-      p = v2 - ca * P;
-      c = pl.cf + ca;
-    }
+    c = small_div(v, P);           /* framework chunks 0 .. cf - 1, then the adsorbate ones */
+    p = v - c * P;
     const int u = p * per + c;
     const BeadPos b = pos[p];
     const bool check = p < pair_check;
     int ov = 0;
     double e_v, e_q;
     int lo, hi;
-    /* chunk bounds; item counts stay far below 2^31 / RGPU_MAX_UNITS */
-    if (c < pl.cf) {
-      lo = sl.fw_lo + (int)((unsigned)(nfw * c) / (unsigned)pl.cf);
-      hi = sl.fw_lo + (int)((unsigned)(nfw * (c + 1)) / (unsigned)pl.cf);
-    } else {
-      const int cc = c - pl.cf;
-      lo = sl.ads_lo + (int)((unsigned)(nads * cc) / (unsigned)pl.ca);
-      hi = sl.ads_lo + (int)((unsigned)(nads * (cc + 1)) / (unsigned)pl.ca);
+    {
+      const bool fw = c < cf;
+      const int n = fw ? nfw : nads, cc = fw ? c : c - cf, base = fw ? sl.fw_lo : sl.ads_lo;
+      const unsigned mm = fw ? mf : ma;
+      lo = base + (mm ? (int)__umulhi((unsigned)(n * cc), mm) : n * cc);
+      hi = base + (mm ? (int)__umulhi((unsigned)(n * (cc + 1)), mm) : n * (cc + 1));
     }
     if constexpr (MIXED == 2) {
       float av = 0.0f;
       double ac = 0.0;
       float *qr2 = sc.qr2 + 128 * w;   /* 64 FP64 squared distances per warp */
-      if (c < pl.cf) {
+      if (c < cf) {
         if (S.triclinic)
-          unit_tiles_cc64<true>(S, (const int4 *)sl.fw, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
+          unit_tiles_cc64<true>(S, sl.fw, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
                                 qr2, sc.qq + 64 * w, sc.qt + 64 * w);
         else
-          unit_tiles_cc64<false>(S, (const int4 *)sl.fw, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
+          unit_tiles_cc64<false>(S, sl.fw, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
                                  qr2, sc.qq + 64 * w, sc.qt + 64 * w);
       } else if (S.triclinic) {
         unit_ads_cc64<true>(S, (const int4 *)sl.ads, b, lo, hi, b.excl, check, av, ac, ov, nin, nch, nvis,
@@ -1057,29 +974,31 @@ __device__ __forceinline__ EvalPlan eval_units(const RgpuSys &S, const EvalSlice
       e_q = warp_sum(ac);
     } else if (MIXED) {
       float av = 0.0f, ac = 0.0f;
-      if (c < pl.cf) {
+      if (c < cf) {
         if (S.triclinic)
-          unit_tiles_mixed<true>(S, (const int4 *)sl.fw, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
-                                 sc.qr2 + 64 * w, sc.qq + 64 * w, sc.qt + 64 * w);
+          unit_tiles_mixed<true>(S, sl.fw, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
+                                 sc.qr2 + RGPU_QUEUE_FLOATS * w);
         else
-          unit_tiles_mixed<false>(S, (const int4 *)sl.fw, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
-                                  sc.qr2 + 64 * w, sc.qq + 64 * w, sc.qt + 64 * w);
+          unit_tiles_mixed<false>(S, sl.fw, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
+                                 sc.qr2 + RGPU_QUEUE_FLOATS * w);
       } else if (S.triclinic) {
         unit_ads_mixed<true>(S, (const int4 *)sl.ads, b, lo, hi, b.excl, check, av, ac, ov, nin, nch, nvis,
-                             sc.qr2 + 64 * w, sc.qq + 64 * w, sc.qt + 64 * w);
+                             sc.qr2 + RGPU_QUEUE_FLOATS * w);
       } else {
         unit_ads_mixed<false>(S, (const int4 *)sl.ads, b, lo, hi, b.excl, check, av, ac, ov, nin, nch, nvis,
-                              sc.qr2 + 64 * w, sc.qq + 64 * w, sc.qt + 64 * w);
+                             sc.qr2 + RGPU_QUEUE_FLOATS * w);
       }
       e_v = (double)warp_sum(av);
       e_q = (double)warp_sum(ac);
     } else {
       double av = 0.0, ac = 0.0;
-      if (c < pl.cf) {
+      if (c < cf) {
         if (S.triclinic)
-          unit_fw_fp64<true>(S, (const double4 *)sl.fw, b, lo, hi, check, av, ac, ov, nin, nch, nvis);
+          unit_tiles_fp64<true>(S, sl.fw, sl.fwd, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
+                                sc.qt + 64 * w);
         else
-          unit_fw_fp64<false>(S, (const double4 *)sl.fw, b, lo, hi, check, av, ac, ov, nin, nch, nvis);
+          unit_tiles_fp64<false>(S, sl.fw, sl.fwd, sl.tiles, lo, hi, b, check, av, ac, ov, nin, nch, nvis,
+                                 sc.qt + 64 * w);
       } else if (S.triclinic) {
         unit_ads_fp64<true>(S, (const AdsRec64 *)sl.ads, b, lo, hi, b.excl, check, av, ac, ov, nin, nch, nvis);
       } else {
@@ -1088,24 +1007,37 @@ __device__ __forceinline__ EvalPlan eval_units(const RgpuSys &S, const EvalSlice
       e_v = warp_sum(av);
       e_q = warp_sum(ac);
     }
-    ov = warp_or(ov);
+    if (check && __any_sync(RGPU_FULL, ov) && lane == 0) *sc.ovf = 1;
+    int d = 0;
     if (lane == 0) {
-      sc.uv[u] = e_v;
-      sc.uc[u] = e_q;
-      sc.uo[u] = ov;
+      sc.u[u] = make_double2(e_v, e_q);
+      __threadfence_block();
+      d = atomicAdd(&sc.done[p], 1);
+      __threadfence_block();
+    }
+    if (__shfl_sync(RGPU_FULL, d, 0) == per - 1) {
+      /* the position's last unit: lane k < 4 adds up term k */
+      if (lane < 4) {
+        const double *t = (const double *)(sc.u + p * per) + (lane & 1);
+        const int c0 = lane < 2 ? 0 : cf, c1 = lane < 2 ? cf : per;
+        double sum = 0.0;
+#pragma unroll 1
+        for (int q = c0; q < c1; q++) sum += t[2 * q];
+        if (c1 > c0) ((double *)(sc.part + p))[lane] = sum;
+      }
+      if (lane == 0) sc.done[p] = 0;
     }
     v = __shfl_sync(RGPU_FULL, vn, 0);
   }
-  if (sc.cnt) {
-    nin = __reduce_add_sync(RGPU_FULL, (unsigned)nin);
-    nch = __reduce_add_sync(RGPU_FULL, (unsigned)nch);
-    if (lane == 0) {
-      atomicAdd(&sc.cnt[0], (unsigned long long)nvis);
-      atomicAdd(&sc.cnt[1], (unsigned long long)nin);
-      atomicAdd(&sc.cnt[2], (unsigned long long)nch);
-    }
+  nvis = __reduce_add_sync(RGPU_FULL, (unsigned)nvis);
+  nin = __reduce_add_sync(RGPU_FULL, (unsigned)nin);
+  nch = __reduce_add_sync(RGPU_FULL, (unsigned)nch);
+  if (lane == 0) {
+    unsigned long long *c = sc.cnt + 3 * w;
+    c[0] += (unsigned long long)nvis;
+    c[1] += (unsigned long long)nin;
+    c[2] += (unsigned long long)nch;
   }
-  return pl;
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1176,6 +1108,7 @@ __device__ __forceinline__ double2 ewald_dS(const typename PhaseT<MIXED>::T *tab
      * bits, rotated to first order by its last 8 (at most 3.7e-7 rad);
      * q exp(ik.r) summed in FP64. No phase table. */
     double re = 0.0, im = 0.0;
+#pragma unroll 1
     for (int s = 0; s < ns; s++) {
       const BeadPos &b = sites[s].b;
       const int ang = (int)((unsigned)kv.x * (unsigned)b.xi + (unsigned)kv.y * (unsigned)b.yi +
@@ -1204,36 +1137,16 @@ __device__ __forceinline__ double2 ewald_dS(const typename PhaseT<MIXED>::T *tab
   }
 }
 
-/* Sum over wave vectors [k0, k1) of the energy change; every thread returns
- * {e_ads, e_host}:
- * e_ads = sum kf (|S+dS|^2 - |S|^2), e_host = sum kf Re(S_fw^* dS). */
+/* The energy change over share u of wave vectors [k0, k1): those of thread
+ * 32 u + lane of blockDim.x that stride through them; its {e_ads, e_host} go
+ * to red[2u], red[2u+1]. Warp-wide. */
 template <int MIXED>
-__device__ void ewald_energy_sum(const RgpuSys &S, const typename PhaseT<MIXED>::T *tab, int kw,
-                                 const EwSite *sites, int ns, int k0, int k1, double &e_ads, double &e_host,
-                                 double *red)
+__device__ __forceinline__ void ewald_energy_share(const RgpuSys &S, const typename PhaseT<MIXED>::T *tab, int kw,
+                                                   const EwSite *sites, int ns, int k0, int k1, int u, double *red)
 {
   double ea = 0.0, eh = 0.0;
-  for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-    double2 d = ewald_dS<MIXED>(tab, kw, sites, ns, S.kvec[k]);
-    double2 so = S.sk_ads[k];
-    double2 sf = S.sk_fw[k];
-    double kf = S.kfactor[k];
-    ea += kf * (2.0 * (so.x * d.x + so.y * d.y) + d.x * d.x + d.y * d.y);
-    eh += kf * (sf.x * d.x + sf.y * d.y);
-  }
-  block_sum2(ea, eh, red);
-  e_ads = ea;
-  e_host = eh;
-}
-
-/* As ewald_energy_sum, without block reduction: warp w leaves its partial
- * {e_ads, e_host} in red[2w], red[2w+1]. No block barrier. */
-template <int MIXED>
-__device__ __forceinline__ void ewald_energy_warps(const RgpuSys &S, const typename PhaseT<MIXED>::T *tab, int kw,
-                                   const EwSite *sites, int ns, int k0, int k1, double *red)
-{
-  double ea = 0.0, eh = 0.0;
-  for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+#pragma unroll 1
+  for (int k = k0 + 32 * u + (threadIdx.x & 31); k < k1; k += blockDim.x) {
     double2 d = ewald_dS<MIXED>(tab, kw, sites, ns, S.kvec[k]);
     double2 so = S.sk_ads[k];
     double2 sf = S.sk_fw[k];
@@ -1244,19 +1157,20 @@ __device__ __forceinline__ void ewald_energy_warps(const RgpuSys &S, const typen
   ea = warp_sum(ea);
   eh = warp_sum(eh);
   if ((threadIdx.x & 31) == 0) {
-    red[2 * (threadIdx.x >> 5)] = ea;
-    red[2 * (threadIdx.x >> 5) + 1] = eh;
+    red[2 * u] = ea;
+    red[2 * u + 1] = eh;
   }
 }
 
-/* S_ads(k) += dS(k) (AcceptEwaldAdsorbateMove, src/ewald.c:11732). The same
- * ewald_dS call as in the energy sum, so the stored sums are those the
- * accepted energy was computed with. */
+/* S_ads(k) += dS(k) (AcceptEwaldAdsorbateMove, src/ewald.c:11732) over share
+ * u of wave vectors [k0, k1). The same ewald_dS call as in the energy sum, so
+ * the stored sums are those the accepted energy was computed with. */
 template <int MIXED>
-__device__ __forceinline__ void ewald_apply(const RgpuSys &S, const typename PhaseT<MIXED>::T *tab, int kw, const EwSite *sites,
-                            int ns, int k0, int k1)
+__device__ __forceinline__ void ewald_apply_share(const RgpuSys &S, const typename PhaseT<MIXED>::T *tab, int kw,
+                                                  const EwSite *sites, int ns, int k0, int k1, int u)
 {
-  for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+#pragma unroll 1
+  for (int k = k0 + 32 * u + (threadIdx.x & 31); k < k1; k += blockDim.x) {
     double2 d = ewald_dS<MIXED>(tab, kw, sites, ns, S.kvec[k]);
     double2 so = S.sk_ads[k];
     S.sk_ads[k] = make_double2(so.x + d.x, so.y + d.y);

@@ -7,17 +7,17 @@
 
 #include "rgpu_types.h"
 
-/* fw_items / tile_items: framework records / tiles one CTA stages (0: the
- * framework is read from global memory); k_items: wave vectors one CTA
+/* fw_items / fwd_items / tile_items: framework atoms / their FP64 positions
+ * (FP64 path) / tiles one CTA stages (0: read from global memory); k_items: wave vectors one CTA
  * stages with their S(k) (0: read from global memory) */
-size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int tile_items, int max_ads_atoms, int kw, int k_items,
+size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int fwd_items, int tile_items, int max_ads_atoms, int kw, int k_items,
                               int threads, int flex);
 /* raises the kernel's dynamic shared-memory limit to `smem` (call before a
  * launch or a capture of one); flex selects the build with flexible-chain
  * moves and energy grids */
 cudaError_t rgpu_engine_prepare(int mixed, bool wide, bool flex, size_t smem);
 cudaError_t rgpu_engine_launch(int mixed, RgpuSys *d_systems, int nsys, long long nsteps, int kw,
-                               int max_ads_atoms, int fw_items, int tile_items, int k_items, int cluster,
+                               int max_ads_atoms, int fw_items, int fwd_items, int tile_items, int k_items, int cluster,
                                int threads, bool wide, bool flex, cudaStream_t st);
 /* per-call entry points (percall.cu); d_out and d_ov in mapped host memory */
 cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ads, int nads, const RgpuPoints &in, int P,

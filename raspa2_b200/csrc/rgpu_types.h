@@ -179,7 +179,8 @@ typedef struct RgpuSys {
   int ntrial_first, ntrial;
   uint64_t seed;
   uint32_t sys_id;
-  int smem_fw;                /* framework staged in shared memory by the engine */
+  int smem_fw;                /* framework staged in shared memory by the engine: 1 the fixed-point atoms and the
+                               * tiles, 2 the FP64 positions too (FP64 path) */
   /* flexible linear chain (rgpu_system_desc), grown from atom 0 */
   int flexible;
   int pad_flex;
