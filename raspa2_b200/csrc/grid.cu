@@ -314,12 +314,24 @@ cudaError_t rgpu_grid_build_launch(const RgpuSys *d_sys, const RgpuLJ *lj, doubl
   return cudaGetLastError();
 }
 
-__global__ void k_grid_interp(const float *grid, RgpuGridGeom ip, int n, const double *xyz, double *out)
+/* One thread per point. The block's positions come through shared memory, so
+ * that they are read once, in order, also from mapped host memory, where the
+ * kernel is bound by the 32 bytes a point that cross PCIe (else by the eight
+ * 32-byte corners). */
+#define INTERP_THREADS 256
+
+__global__ void __launch_bounds__(INTERP_THREADS) k_grid_interp(const float *grid, RgpuGridGeom ip, int n, const double *xyz,
+                                                              double *out)
 {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const double p[3] = {xyz[3 * q], xyz[3 * q + 1], xyz[3 * q + 2]};
-  out[q] = rgpu_grid_value(grid, ip, p);
+  __shared__ double sx[3 * INTERP_THREADS];
+  const int base = blockIdx.x * INTERP_THREADS, m = min(n - base, INTERP_THREADS);
+  for (int i = threadIdx.x; i < 3 * m; i += INTERP_THREADS) sx[i] = xyz[3 * (size_t)base + i];
+  __syncthreads();
+  const int q = threadIdx.x;
+  if (q < m) {
+    const double p[3] = {sx[3 * q], sx[3 * q + 1], sx[3 * q + 2]};
+    out[base + q] = rgpu_grid_value(grid, ip, p);
+  }
 }
 
 cudaError_t rgpu_grid_interp_launch(const float *d_grid, const int npts[3], const double size[3],
@@ -335,7 +347,7 @@ cudaError_t rgpu_grid_interp_launch(const float *d_grid, const int npts[3], cons
     ip.cell[c] = cell[c];
   }
   if (n <= 0) return cudaSuccess;
-  k_grid_interp<<<(n + 255) / 256, 256, 0, st>>>(d_grid, ip, n, d_xyz, d_out);
+  k_grid_interp<<<(n + INTERP_THREADS - 1) / INTERP_THREADS, INTERP_THREADS, 0, st>>>(d_grid, ip, n, d_xyz, d_out);
   return cudaGetLastError();
 }
 

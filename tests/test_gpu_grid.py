@@ -100,3 +100,30 @@ def test_grid_build_paths_match_oracle(cuda, npts, coulomb, tri):
     ref = np.asarray(ref, np.float64).reshape(8, -1)
     top = np.abs(ref).max(axis=1, keepdims=True)
     assert np.all(np.abs(got - ref) <= 2e-7 * np.abs(ref) + 1e-6 + 1e-13 * top)
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 16384, 16385, 131073])
+def test_interpolate_across_stage_edges(cuda, n):
+    """Lookups of one point, of blocks, staging chunks and the whole stage and one point more, from several threads
+    at once (one of them finds the stage in use), against single lookups through the static scratch: the same
+    kernel on the same values, so the same bits."""
+    import threading
+    import torch
+    rng = np.random.default_rng(n)
+    npts, size, shift = np.array([7, 9, 11], np.int32), np.array([10.0, 11.0, 12.0]), np.zeros(3)
+    grid = torch.rand(8 * 10 * 12 * 8, device="cuda")
+    xyz = rng.uniform(-20.0, 30.0, (n, 3))
+    got = [None] * 3
+
+    def look(i):
+        got[i] = native.grid_interpolate(grid.data_ptr(), npts, size, shift, size, xyz)
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=look, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    ref = np.concatenate([native.grid_interpolate_noalloc(grid.data_ptr(), npts, size, shift, size, xyz[i:i + 8192])
+                          for i in range(0, n, 8192)])
+    for g in got:
+        np.testing.assert_array_equal(g, ref)
