@@ -117,6 +117,34 @@ def _arr(a, dt):
     return np.ascontiguousarray(a, dtype=dt)
 
 
+_D1, _I1 = C.c_double * 1, C.c_int * 1
+
+
+def _dptr(a):
+    """`a`'s data as a double pointer argument. An array over its buffer costs
+    a seventh of ndarray.ctypes.data_as, of which a per-call routine makes up
+    to four; read-only and empty arrays take that."""
+    try:
+        return _D1.from_buffer(a)
+    except (TypeError, ValueError):
+        return a.ctypes.data_as(_dp)
+
+
+def _iptr(a):
+    """As _dptr, for an int32 array."""
+    try:
+        return _I1.from_buffer(a)
+    except (TypeError, ValueError):
+        return a.ctypes.data_as(_ip)
+
+
+def _per_bead(v, n):
+    """v for each of n beads, int32"""
+    if type(v) is np.ndarray and v.dtype == np.int32 and v.shape == (n,):
+        return np.ascontiguousarray(v)
+    return _arr(np.broadcast_to(v, (n,)), np.int32)
+
+
 class GpuSystem:
     """One simulation box on the GPU (handle of rgpu_system)."""
 
@@ -197,22 +225,22 @@ class GpuSystem:
     # ---- state ------------------------------------------------------------
     def set_adsorbates(self, xyz):
         xyz = _arr(np.asarray(xyz, float).reshape(-1, self.natom, 3), np.float64)
-        _check(load().rgpu_set_adsorbates(self.h, len(xyz), xyz.ctypes.data_as(_dp)))
+        _check(load().rgpu_set_adsorbates(self.h, len(xyz), _dptr(xyz)))
 
     def adsorbates(self) -> np.ndarray:
         n = C.c_int()
         _check(load().rgpu_get_adsorbates(self.h, C.byref(n), None, 0))
         out = np.zeros((max(n.value, 1), self.natom, 3))
-        _check(load().rgpu_get_adsorbates(self.h, C.byref(n), out.ctypes.data_as(_dp), out.shape[0]))
+        _check(load().rgpu_get_adsorbates(self.h, C.byref(n), _dptr(out), out.shape[0]))
         return out[: n.value]
 
     def update_molecule(self, m, xyz):
         x = _arr(xyz, np.float64)
-        _check(load().rgpu_update_molecule(self.h, C.c_int(m), x.ctypes.data_as(_dp)))
+        _check(load().rgpu_update_molecule(self.h, C.c_int(m), _dptr(x)))
 
     def insert_molecule(self, xyz):
         x = _arr(xyz, np.float64)
-        _check(load().rgpu_insert_molecule(self.h, x.ctypes.data_as(_dp)))
+        _check(load().rgpu_insert_molecule(self.h, _dptr(x)))
 
     def remove_molecule(self, m):
         _check(load().rgpu_remove_molecule(self.h, C.c_int(m)))
@@ -221,27 +249,26 @@ class GpuSystem:
     def bead_energies(self, xyz, atom, exclude, precision=RGPU_FP64) -> np.ndarray:
         x = _arr(np.asarray(xyz, float).reshape(-1, 3), np.float64)
         n = len(x)
-        a = _arr(np.broadcast_to(atom, (n,)), np.int32)
-        e = _arr(np.broadcast_to(exclude, (n,)), np.int32)
+        a, e = _per_bead(atom, n), _per_bead(exclude, n)
         out = np.zeros((n, 4))
-        _check(load().rgpu_bead_energies(self.h, C.c_int(precision), C.c_int(n), x.ctypes.data_as(_dp),
-                                         a.ctypes.data_as(_ip), e.ctypes.data_as(_ip), out.ctypes.data_as(_dp)))
+        _check(load().rgpu_bead_energies(self.h, C.c_int(precision), C.c_int(n), _dptr(x),
+                                         _iptr(a), _iptr(e), _dptr(out)))
         return out
 
     def move_difference(self, m, new_xyz, precision=RGPU_FP64):
         x = _arr(new_xyz, np.float64)
         out = np.zeros(4)
         ov = C.c_int()
-        _check(load().rgpu_move_energy_difference(self.h, C.c_int(precision), C.c_int(m), x.ctypes.data_as(_dp),
-                                                  out.ctypes.data_as(_dp), C.byref(ov)))
+        _check(load().rgpu_move_energy_difference(self.h, C.c_int(precision), C.c_int(m), _dptr(x),
+                                                  _dptr(out), C.byref(ov)))
         return bool(ov.value), out
 
     def ewald_difference(self, old_mol=-1, new_xyz=None, precision=RGPU_FP64):
         out = np.zeros(3)
         x = None if new_xyz is None else _arr(new_xyz, np.float64)
         _check(load().rgpu_ewald_fourier_difference(self.h, C.c_int(precision), C.c_int(old_mol),
-                                                    None if x is None else x.ctypes.data_as(_dp),
-                                                    out.ctypes.data_as(_dp)))
+                                                    None if x is None else _dptr(x),
+                                                    _dptr(out)))
         return out
 
     def ewald_accept(self):
@@ -249,7 +276,7 @@ class GpuSystem:
 
     def total_energy(self) -> np.ndarray:
         out = np.zeros(6)
-        _check(load().rgpu_total_energy(self.h, out.ctypes.data_as(_dp)))
+        _check(load().rgpu_total_energy(self.h, _dptr(out)))
         return out
 
     def set_grids(self, grid_ptrs, npts, size, shift, cell):
