@@ -139,13 +139,13 @@ __global__ void __launch_bounds__(32 * POINT_WARPS) k_points_fp64(const RgpuSys 
   }
 }
 
-/* As k_points_fp64 on the mixed path: one CTA per position and one warp per
- * unit of eval_plan's cut for POINT_MIXED_WARPS warps (framework chunks, then
- * adsorbate chunks), so that each FP32 sum runs over the same pairs in the
- * same order whatever the number of positions a call shares the GPU with.
- * Bound by the one warp that walks all tiles of a position when a call has
- * five positions or more. 64 positions in 4096 atoms: 48 us a call (137 us
- * with all units on one CTA). */
+/* As k_points_fp64 on the mixed path, whose FP32 sums run over the same pairs in
+ * the same order whatever the number of positions a call shares the GPU with:
+ * the units of eval_plan's cut for POINT_MIXED_WARPS warps (framework chunks,
+ * then adsorbate chunks), one warp's sum each. One CTA per position.
+ * k_points_mixed gives each unit a warp; it serves calls of up to four
+ * positions, whose framework is cut into chunks. From five positions on a
+ * position's framework is one unit (k_points_mixed_long). */
 __global__ void __launch_bounds__(64 * POINT_MIXED_WARPS) k_points_mixed(const RgpuSys *sysp, const int4 *ads, int nads,
                                                                         const __grid_constant__ RgpuPoints in,
                                                                         EvalPlan pl, int pair_check, int fw_grid,
@@ -207,6 +207,153 @@ __global__ void __launch_bounds__(64 * POINT_MIXED_WARPS) k_points_mixed(const R
   }
 }
 
+/* One framework unit per position, its pairs in the order of one warp's queue
+ * (ascending tiles and atoms; pair j is added by lane j mod 32) but found and
+ * formed by all warps: each culls and tests an eighth of the tiles into a list
+ * of its own, all threads form the lists' pair terms into one sequence, and
+ * one warp adds that up. A ninth warp takes the adsorbates meanwhile. A
+ * list that overflows sends the position through one warp's queue. Bound by the
+ * chain of steps. 64 positions in 4096 atoms: 23 us a call, 40 us with one warp
+ * walking all tiles of a position. */
+#define LONG_WARPS 8
+#define LONG_LIST 256          /* pairs of one warp; a sixteenth of the sphere's atoms at 0.09 / A^3 is 41 */
+
+struct LongSmem {
+  RgpuSys S;
+  BeadPos b;
+  float2 list[LONG_WARPS][LONG_LIST];   /* {r2, charge} */
+  unsigned char type[LONG_WARPS][LONG_LIST];
+  float2 term[LONG_WARPS * LONG_LIST];  /* {LJ, charge} of the sequence */
+  __align__(8) float queue[2 * RGPU_QUEUE_FLOATS];
+  int count[LONG_WARPS], ov[LONG_WARPS + 1];
+  double red[2][2];
+};
+
+template <bool TRI>
+__device__ __forceinline__ int long_list(const RgpuSys &S, int t0, int t1, const BeadPos &b, float2 *list,
+                                         unsigned char *type)
+{
+  const int lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15;
+  const unsigned below = (1u << lane) - 1u;
+  const float rc2 = S.rc2f;
+  int n = 0;
+  for (int tb = t0; tb < t1; tb += 32) {
+    bool vis = false;
+    int tn = 0;
+    if (tb + lane < t1) {
+      const TileRec tr = S.tiles[tb + lane];
+      tn = tr.c.w;
+      vis = tile_visible<TRI>(S, tr, b, rc2);
+    }
+    unsigned m = __ballot_sync(RGPU_FULL, vis);
+    while (m) {
+      const unsigned mm = m & (m - (unsigned)half);
+      m &= m - 1;
+      m &= m - 1;
+      const int mine = __ffs(mm) - 1;
+      const int nt = __shfl_sync(RGPU_FULL, tn, mine & 31);
+      const bool live = mine >= 0 && hl < nt;
+      int4 f = make_int4(0, 0, 0, 0);
+      if (live) f = S.fw32[(size_t)(tb + mine) * RGPU_TILE + hl];
+      float dx, dy, dz;
+      if (!TRI) {
+        dx = __int2float_rn(f.x - b.xi) * S.fix_scale[0];
+        dy = __int2float_rn(f.y - b.yi) * S.fix_scale[1];
+        dz = __int2float_rn(f.z - b.zi) * S.fix_scale[2];
+      } else {
+        rgpu_fix_to_cart_tri(S, f.x - b.xi, f.y - b.yi, f.z - b.zi, dx, dy, dz);
+      }
+      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      const bool in = live && r2 < rc2;
+      const unsigned bal = __ballot_sync(RGPU_FULL, in);
+      const int p = n + __popc(bal & below);
+      if (in && p < LONG_LIST) {
+        list[p] = make_float2(r2, __int_as_float(f.w));
+        type[p] = (unsigned char)(f.z & 3);
+      }
+      n += __popc(bal);
+    }
+  }
+  return n;
+}
+
+__global__ void __launch_bounds__(32 * (LONG_WARPS + 1)) k_points_mixed_long(const RgpuSys *sysp, const int4 *ads, int nads,
+                                                                            const __grid_constant__ RgpuPoints in,
+                                                                            int pair_check, double *out, int *ov)
+{
+  __shared__ LongSmem sm;
+  const RgpuSys &S = sm.S;
+  const int p = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  load_sys(&sm.S, sysp);
+  if (threadIdx.x == 0) bead_set(sm.b, S, in.xyz[p][0], in.xyz[p][1], in.xyz[p][2], in.atom[p], in.excl[p]);
+  __syncthreads();
+  const BeadPos &b = sm.b;
+  const bool check = p < pair_check;
+  float av = 0.0f, ac = 0.0f;
+  int o = 0, nin = 0, nch = 0, nvis = 0;
+  if (w < LONG_WARPS) {
+    const int t0 = S.ntile * w / LONG_WARPS, t1 = S.ntile * (w + 1) / LONG_WARPS;
+    const int n = S.triclinic ? long_list<true>(S, t0, t1, b, sm.list[w], sm.type[w])
+                              : long_list<false>(S, t0, t1, b, sm.list[w], sm.type[w]);
+    if (lane == 0) sm.count[w] = n;
+  } else if (nads > 0) {
+    float *mem = sm.queue + RGPU_QUEUE_FLOATS;
+    if (S.triclinic) unit_ads_mixed<true>(S, ads, b, 0, nads, b.excl, check, av, ac, o, nin, nch, nvis, mem);
+    else unit_ads_mixed<false>(S, ads, b, 0, nads, b.excl, check, av, ac, o, nin, nch, nvis, mem);
+  }
+  __syncthreads();
+  int n = 0, most = 0;
+  for (int q = 0; q < LONG_WARPS; q++) {
+    n += sm.count[q];
+    most = max(most, sm.count[q]);
+  }
+  const bool listed = most <= LONG_LIST;
+  if (listed && w < LONG_WARPS) {
+    const RgpuLJf *P = S.ljf_bf[b.atom];
+    const float qa = S.mol_qf[b.atom] * S.coulombf, alpha = S.alphaf, thr = (float)S.overlap;
+    const bool charged = S.fw_charged && qa != 0.0f;
+    for (int j = threadIdx.x; j < n; j += 32 * LONG_WARPS) {
+      int q = 0, i = j;
+      while (i >= sm.count[q]) i -= sm.count[q++];
+      const float2 e = sm.list[q][i];
+      float u = 0.0f, uc = 0.0f;
+      pair_mixed_queued(P, e.x, e.y, charged, qa, alpha, check, thr, u, uc, o, nch, sm.type[q][i]);
+      sm.term[j] = make_float2(u, uc);
+    }
+  }
+  if (listed) __syncthreads();
+  if (w == 0) {
+    if (listed) {
+#pragma unroll 4
+      for (int j = lane; j < n; j += 32) {
+        const float2 t = sm.term[j];
+        av += t.x;
+        ac += t.y;
+      }
+    } else if (S.triclinic) {
+      unit_tiles_mixed<true>(S, S.fw32, S.tiles, 0, S.ntile, b, check, av, ac, o, nin, nch, nvis, sm.queue);
+    } else {
+      unit_tiles_mixed<false>(S, S.fw32, S.tiles, 0, S.ntile, b, check, av, ac, o, nin, nch, nvis, sm.queue);
+    }
+  }
+  o = warp_or(o);
+  if (lane == 0) sm.ov[w] = o;
+  if (w == 0 || w == LONG_WARPS) {
+    const double ev = (double)warp_sum(av), eq = (double)warp_sum(ac);
+    if (lane == 0) {
+      sm.red[w != 0][0] = ev;
+      sm.red[w != 0][1] = eq;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int any = 0;
+    for (int q = 0; q <= LONG_WARPS; q++) any |= sm.ov[q];
+    for (int k = 0; k < 4; k++) out[4 * p + k] = sm.red[k >> 1][k & 1];
+    ov[p] = any;
+  }
+}
+
 /* ntile: the system's framework tiles (0 with the GRID framework model) */
 cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ads, int nads, const RgpuPoints &in, int P,
                                int ntile, int pair_check, int fw_grid, double *d_out, int *d_ov, cudaStream_t st)
@@ -214,6 +361,12 @@ cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ad
   if (P < 1 || P > RGPU_MAX_POS) return cudaErrorInvalidValue;
   if (mixed) {
     EvalPlan pl = eval_plan(P, ntile, nads, POINT_MIXED_WARPS, 8 * RGPU_MAX_POS, 2);
+    /* one framework unit a position and a tile for every warp: 23 us a call from
+     * 8 to 64 positions and 300 to 4096 atoms, 25 to 40 with a warp per unit */
+    if (pl.cf == 1 && pl.ca <= 1 && ntile >= LONG_WARPS) {
+      k_points_mixed_long<<<P, 32 * (LONG_WARPS + 1), 0, st>>>(d_sys, (const int4 *)d_ads, nads, in, pair_check, d_out, d_ov);
+      return cudaGetLastError();
+    }
     const int per = pl.cf + pl.ca;
     k_points_mixed<<<P, 32 * (per > 1 ? per : 1), 0, st>>>(d_sys, (const int4 *)d_ads, nads, in, pl, pair_check, fw_grid,
                                                          d_out, d_ov);

@@ -106,3 +106,25 @@ def test_totals_and_fourier_at_split_edges(cuda, atoms, nmol, kmax, tri):
     totals(np.concatenate([moved, extra[None]]))
     g.remove_molecule(0)
     totals(np.concatenate([extra[None], moved[1:]]))
+
+
+@pytest.mark.parametrize("atoms", [128, 4800])
+def test_mixed_lists_and_their_overflow(cuda, atoms):
+    """The mixed kernel's pair lists from a tile per warp on, and a framework so dense (0.34 atoms per cubic
+    Angstrom) that a warp's list overflows and one warp walks the tiles. Random atoms overlap the beads, so the bound
+    is the sensitivity of FP32 distances: r^2 within 3e-7 (three rounded products, coordinates of 2e-8 A at
+    r > 0.3 A), 6 times that for r^-12, some 5 roundings of the term and its sum: 5e-6 of the absolute terms."""
+    s = co2_box(16, False)
+    rng = np.random.default_rng(atoms)
+    s = dataclasses.replace(s, unit_cell=np.array([24.1, 24.1, 24.1]), frac=np.round(rng.random((atoms, 3)), 12),
+                            uc_types=["Sifw"] * (atoms // 2) + ["Ofw"] * (atoms - atoms // 2),
+                            uc_charges=np.round(rng.uniform(-1, 1, atoms), 8))
+    g = native.GpuSystem(s, maxmol=4)
+    o = O.Oracle.from_system(s, maxmol=4)
+    xyz, atom = rng.uniform(0.0, 24.1, (9, 3)), rng.integers(0, 3, 9)
+    t, q = s.molecule_types(), s.molecule.charges()
+    scale = np.array([o.point_abs(int(t[a]), float(q[a]), x, -1) for a, x in zip(atom, xyz)])
+    ref, got = (g.bead_energies(xyz, atom, -1, p) for p in (native.RGPU_FP64, native.RGPU_MIXED))
+    near = np.max(np.abs(ref), axis=1) < 1e15      # a pair within about 0.3 A gives more
+    assert near.sum() >= 3
+    assert np.all(np.abs(got - ref)[near] <= 5e-6 * scale[near] + 1e-6)
