@@ -779,6 +779,8 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   h.sk_fw = s->sk_fw;
   h.sk_ads = s->sk_ads;
   h.ads_xyz = s->ads_xyz;
+  h.rec32 = s->rec32;
+  h.rec64 = s->rec64;
   h.nmol = s->nmol;
   h.energy = s->energy;
   h.step = s->step;
@@ -1072,6 +1074,8 @@ static bool grid_geom_set(rgpu_system *s, int which, RgpuGridGeom &g, const int 
     g.size[c] = size[c];
     g.shift[c] = shift[c];
     g.cell[c] = cell[c];
+    g.icell[c] = 1.0 / cell[c];
+    g.scale[c] = npts[c] / size[c];
   }
   if (!s->h.triclinic) return grid_covers_cell(npts, size, shift, cell);
   g.tri = 1;
@@ -2007,7 +2011,6 @@ extern "C" int rgpu_engine_set_adsorbates(rgpu_engine *e, const int *nmol, const
   int max_nk = 0;
   for (int i = 0; i < n; i++) {
     rgpu_system *s = e->sys[i];
-    CK(rgpu_records_launch(s->d_sys, nmol[i] * s->d.natom, -1, s->rec32, s->rec64, e->st));
     s->records_stale = 0;
     max_nk = std::max(max_nk, s->h.nk);
   }

@@ -96,8 +96,10 @@ size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int fwd_items, int tiles,
  * spread over threads (placing positions, adding up CTAs' sums) is done by all
  * of them between barriers, which cost some 500 cycles. Code now 120 to 270
  * KB. Measured (upload, moves, states read back): 64 mixed CO2 boxes, 1000
- * moves each, 21.9 ms (27.4 before); one FP64 CO2 box, 200 moves, 3.28 ms
- * (4.27); 32 hexane boxes over grids, 100 moves, 4.29 ms (4.42). */
+ * moves each, 21.5 ms (27.2 before); one FP64 CO2 box, 200 moves, 3.26 ms
+ * (4.30); 32 hexane boxes over grids, 100 moves, 3.97 ms (4.45; 4.29 with the
+ * bend angles of a growth, its uniforms, the next bead's frames and the
+ * trials' LJ all formed by warp 0 or on its way). */
 #define RGPU_COLD __noinline__
 
 /* floor(2^32 / n) + 1 (less one for powers of two: 2^32 / n) for 2 <= n <= 64, 0
@@ -165,7 +167,6 @@ struct Ctl {
   /* flexible chains: chosen bead positions of the configuration being grown
    * or retraced, intramolecular energy */
   double cp[RGPU_MAX_ATOMS][3];
-  double ub[2][RGPU_MAX_TRIALS];  /* bonded energies of a bead's trials, by bead parity */
   /* a retrace's beads: trial weight sum, the old bead's host VDW, adsorbate
    * VDW, intramolecular LJ and bonded energy, any valid trial */
   double rb[RGPU_MAX_ATOMS][6];
@@ -191,6 +192,16 @@ struct Ctl {
 };
 static_assert(sizeof(Stage) % 16 == 0, "stages are 16-byte aligned");
 
+/* what is kept for a flexible chain's growth, in place of a rigid molecule's
+ * orientation trials */
+struct Growth {
+  double ub[2][RGPU_MAX_TRIALS];  /* bonded energies of a bead's trials, by bead parity */
+  double frame[RGPU_MAX_TRIALS][9];   /* the next bead's frame, should this trial be chosen (chain_frame) */
+  double lj[RGPU_MAX_TRIALS];  /* intramolecular LJ of the current bead's trials (beads 4..) */
+  double sel[3][RGPU_MAX_ATOMS];   /* uniforms that choose among a growth's trials, by bead, of three steps */
+  double theta[3][RGPU_MAX_ATOMS];   /* bend angles of a growth's beads, of three steps */
+};
+
 /* The part of shared memory whose size does not depend on the systems, at its
  * start: the bookkeeping reaches it with addresses known to the compiler,
  * without pointers (which, in functions of their own, would be generic ones:
@@ -205,7 +216,10 @@ struct __align__(256) Fixed {
   double4 tot[RGPU_MAX_POS];       /* the cluster's, of the stage */
   EwSite sites[2][2 * RGPU_MAX_ATOMS];   /* by sites buffer */
   double red[2 * RGPU_MAX_WARPS];
-  double rot[3][2][RGPU_MAX_TRIALS][4];  /* quaternions of the orientation trials (new, retrace), of three steps */
+  union {
+    double rot[3][2][RGPU_MAX_TRIALS][4];  /* quaternions of the orientation trials (new, retrace), of three steps */
+    Growth gr;
+  };
   uint64_t step0;                  /* first MC step of the launch */
   unsigned ads, ang;               /* offsets of the adsorbate records and of the chain trial trigonometry
                                     * ([2][RGPU_ANG_DOUBLES]: of a growth and of a retrace stage) */
@@ -332,8 +346,10 @@ __device__ __forceinline__ void share(int n, int r, int c, int &lo, int &hi)
 __device__ __forceinline__ bool has_ewald(const RgpuSys &S) { return S.ewald && S.mol_charged; }
 
 /* ------------------------------------------------------------------------ */
-/* Random numbers, move type, rotation of a displacement and quaternions
- * of the orientation trials of MC step `step`, into buffer db, by
+__device__ double chain_ref_theta(const RgpuSys &S, int i, int stage, uint64_t step, int lane, const double (*old)[3]);
+
+/* Random numbers, move type, rotation of a displacement, quaternions of the
+ * orientation trials and bend angles of a growth of MC step `step`, into buffer db, by
  * threads t0, t0 + nt, .... All of it depends on the step alone. The warps
  * that wait for warp 0's bookkeeping draw it two steps ahead (a step's tables
  * have to be visible when warp 0 starts it, in the same section in which it
@@ -346,14 +362,16 @@ __device__ RGPU_COLD void draw_step(Build<MIXED, FLEX> E, uint64_t step, int db,
   /* thread i < nr: block i of the table; nr + j, j < 16: orientation trial j;
    * j < 32: retrace orientation j - 16 of a reinsertion; j = 32: the move */
   const int nr = RGPU_RND / 2;
+  const bool chain = FLEX && S.flexible;   /* j = 33..36: the choices among a growth's trials */
 #pragma unroll 1
-  for (int i = t0; i < nr + 33; i += nt) {
+  for (int i = t0; i < nr + (chain ? 37 : 33); i += nt) {
     const int j = i - nr, t = j & 15, old = j >> 4;
     const uint32_t slot = (old ? SLOT_ORIENT_OLD : SLOT_ORIENT) + 4 * t;
-    double2 u = cold_uniforms(S, step, j < 0 ? (uint32_t)i : 0u);
-    if (j < 0) {
-      C.rnd[db][2 * i] = u.x;
-      C.rnd[db][2 * i + 1] = u.y;
+    double2 u = cold_uniforms(S, step, j < 0 ? (uint32_t)i : (j > 32 ? (RGPU_SLOT_CHAIN_SEL >> 1) + j - 33 : 0u));
+    if (j < 0 || j > 32) {
+      double *r = j < 0 ? &C.rnd[db][2 * i] : &fx().gr.sel[db][2 * (j - 33)];
+      r[0] = u.x;
+      r[1] = u.y;
       continue;
     }
     int mv = 0;
@@ -371,9 +389,22 @@ __device__ RGPU_COLD void draw_step(Build<MIXED, FLEX> E, uint64_t step, int db,
     const double2 v = cold_uniforms(S, step, (slot >> 1) + 1);
     random_quaternion(u.x, u.y, v.x, fx().rot[db][old][t]);
   }
+  if (chain && S.chain_scheme == 0) {
+    /* the bend angles of a growth's beads, one warp each */
+    __syncwarp();
+    const double u0 = cold_uniforms(S, step, 0u).x;
+    int mv = 0;
+    while (mv < 5 && u0 >= S.cum[mv]) mv++;
+    if (mv == 2 || mv >= 4)
+      for (int i = 2 + (t0 >> 5); i < S.natom; i += nt >> 5) {
+        const double th = chain_ref_theta(S, i, 0, step, threadIdx.x & 31, nullptr);
+        if ((threadIdx.x & 31) == 0) fx().gr.theta[db][i] = th;
+      }
+  }
 }
 
-static_assert(SLOT_VNEW % 2 == 0 && SLOT_MOVE == 0 && SLOT_ORIENT % 2 == 0 && SLOT_ORIENT_OLD % 2 == 0,
+static_assert(SLOT_VNEW % 2 == 0 && SLOT_MOVE == 0 && SLOT_ORIENT % 2 == 0 && SLOT_ORIENT_OLD % 2 == 0 &&
+                  RGPU_SLOT_CHAIN_SEL % 2 == 0,
               "draw_step takes the first uniform of a block");
 
 /* ------------------------------------------------------------------------ */
@@ -476,7 +507,13 @@ __device__ __forceinline__ void place(Build<MIXED, FLEX> E, const Stage &g, int 
     if (j < g.k) {
       a = g.ci;
       excl = g.mv == 4 ? m : -1;
-      chain_position(E, step, 0, a, j, C.cp, fx_ang(), p);
+      if (a >= 2) {
+        /* in the frame that the last bead's choice left */
+        const double *t = fx_ang() + RGPU_ANG_STRIDE * ((a - 2) * RGPU_MAX_TRIALS + j);
+        chain_place_frame(fx().gr.frame[C.sel], C.cp[a - 1], S.bond, t[0], t[1], t[2], t[3], p);
+      } else {
+        chain_position(E, step, 0, a, j, C.cp, fx_ang(), p);
+      }
     } else {
       /* retrace trials: bead a of the group, trial t in growth order; trial
        * 0 of each bead is the old bead */
@@ -589,6 +626,11 @@ __device__ __forceinline__ void eval_stage(Eng<MIXED, FLEX> &E, const Stage &g)
         if (p < g.check && v >= S.overlap) C.ovf[E.xb] = 1;
       }
     }
+  }
+  if (FLEX && g.ph == PH_GROW && g.ci >= 4 && w == nw - 1 && lane < g.k) {
+    /* the trials' LJ with the chain, for warp 0's choice */
+    const double p[3] = {fx().pos[lane].x, fx().pos[lane].y, fx().pos[lane].z};
+    fx().gr.lj[lane] = chain_intra_lj(S, C.cp, g.ci, p);
   }
   if (g.P) {
     E.sc.ovf = &C.ovf[E.xb];
@@ -1360,7 +1402,7 @@ __device__ __noinline__ void chain_ref_trial(const RgpuSys &S, int i, int stage,
  * table. */
 template <int MIXED, bool FLEX>
 __device__ __forceinline__ void chain_angles_table(Build<MIXED, FLEX> E, uint64_t step, int stage, double *tab,
-                                                   const double (*old)[3])
+                                                   const double (*old)[3], const double *ahead)
 {
   const RgpuSys &S = fx().S;
   const int na = S.natom, nt = S.ntrial;
@@ -1369,14 +1411,19 @@ __device__ __forceinline__ void chain_angles_table(Build<MIXED, FLEX> E, uint64_
   const int gw = fx().rank * nw + (threadIdx.x >> 5), ngw = nw * fx().csize;   /* warp of the cluster */
   const int per = S.chain_scheme == 0 ? 1 : 4;                           /* tasks a warp takes at once */
   if (S.chain_scheme == 0) {
-    /* each bead's bend angle once (one warp per bead, in every CTA), then
-     * one warp per (bead, trial); the angles sit after the table */
-    double *theta = tab + RGPU_ANG_TABLE;
-    for (int i = 2 + (threadIdx.x >> 5); i < na; i += nw) {
-      const double th = chain_ref_theta(S, i, stage, step, lane, old);
-      if (lane == 0) theta[i] = th;
+    /* each bead's bend angle once (a retrace's here, one warp per bead, in every
+     * CTA; a growth's was drawn ahead), then one warp per (bead, trial); a
+     * retrace's angles sit after the table */
+    const double *theta = ahead;
+    if (old) {
+      double *th = tab + RGPU_ANG_TABLE;
+      theta = th;
+      for (int i = 2 + (threadIdx.x >> 5); i < na; i += nw) {
+        const double v = chain_ref_theta(S, i, stage, step, lane, old);
+        if (lane == 0) th[i] = v;
+      }
+      __syncthreads();
     }
-    __syncthreads();
     for (int task = gw; task < ntask; task += ngw) {
       const int i = 2 + task / nt, t = task % nt;
       chain_ref_trial<(MIXED != 0)>(S, i, stage, t, step, lane, old, theta[i],
@@ -1534,7 +1581,7 @@ __device__ RGPU_COLD void chain_tables(Build<MIXED, FLEX> E, const Stage &g)
       if (threadIdx.x < fx().S.natom) atom_xyz(E, g.m, threadIdx.x, x[threadIdx.x]);
       __syncthreads();          /* the old configuration, read by the table */
     }
-    chain_angles_table(E, step, old ? 1 : 0, fx_ang() + t * RGPU_ANG_DOUBLES, old ? x : nullptr);
+    chain_angles_table(E, step, old ? 1 : 0, fx_ang() + t * RGPU_ANG_DOUBLES, old ? x : nullptr, fx().gr.theta[g.buf]);
   }
 }
 
@@ -1607,8 +1654,7 @@ __device__ __forceinline__ bool end_grow(Build<MIXED, FLEX> E, const Stage &g)
   const double r[4] = {rt.x, rt.y, rt.z, rt.w};
   const BeadPos &q = fx().pos[lane];
   if (lane < k) {
-    const double p[3] = {q.x, q.y, q.z};
-    lj = chain_intra_lj(S, C.cp, i, p);
+    if (i >= 4) lj = fx().gr.lj[lane];
     ov = r[0] >= S.overlap || r[1] >= S.overlap || r[2] >= S.overlap || r[3] >= S.overlap || lj >= S.overlap;
     bf = -S.beta * (r[0] + r[2] + lj);
   }
@@ -1618,7 +1664,7 @@ __device__ __forceinline__ bool end_grow(Build<MIXED, FLEX> E, const Stage &g)
   const double cum = warp_scan(w), wsum = __shfl_sync(RGPU_FULL, cum, 31);
   int sel = 0;
   /* SelectTrialPosition (src/cbmc.c:563-599) on the weights themselves */
-  if (any) sel = select_trial(w, cum, k, rgpu_uniform(S.seed, S.sys_id, fx().step0 + (uint64_t)cur().it, RGPU_SLOT_CHAIN_SEL + i));
+  if (any) sel = select_trial(w, cum, k, fx().gr.sel[g.buf][i]);
   const double hv = __shfl_sync(RGPU_FULL, r[0], sel), av = __shfl_sync(RGPU_FULL, r[2], sel);
   const double ljs = __shfl_sync(RGPU_FULL, lj, sel);
   /* with the chosen trial's torsion Rosenbluth factor (src/cbmc.c:2793; 1
@@ -1633,7 +1679,7 @@ __device__ __forceinline__ bool end_grow(Build<MIXED, FLEX> E, const Stage &g)
     C.cp[i][2] = q.z;
   }
   if (lane == 0) {
-    if (i - 1 >= 2) C.uintra += C.ub[(i - 1) & 1][C.sel];   /* the last bead's bonded energy (warp 1) */
+    if (i - 1 >= 2) C.uintra += fx().gr.ub[(i - 1) & 1][C.sel];   /* the last bead's bonded energy (warp 1) */
     C.rosen = rosen;
     C.u[0] += hv;
     C.u[2] += av;
@@ -1729,7 +1775,7 @@ __device__ __forceinline__ void end_chain(Build<MIXED, FLEX> E, int buf)
 {
   Ctl &C = fx().C;
   const int last = fx().S.natom - 1;
-  if (last >= 2 && threadIdx.x == 0) C.uintra += C.ub[last & 1][C.sel];
+  if (last >= 2 && threadIdx.x == 0) C.uintra += fx().gr.ub[last & 1][C.sel];
   __syncwarp();
   if (cur().mv == 4) accept_reinsert_chain(E, buf);
   else accept_swap_chain(E, buf);
@@ -2063,10 +2109,18 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
            * energies of this bead's trials (warp 0 writes only C.cp[ci]) */
           if (g.r1 > g.r0) retrace_book(B, g.r0, g.r1, g.k, C.co, fx_ang() + RGPU_ANG_DOUBLES, 1);
           const int t = threadIdx.x - 32;
+          /* warp 2 (warp 1 of a block of two): the next bead's frame for each of
+           * this bead's trials */
+          const int f = t - (blockDim.x > 64 ? 32 : 0);
+          if (g.ci >= 1 && f >= 0 && f < g.k) {
+            const BeadPos &q = fx().pos[f];
+            const double p[3] = {q.x, q.y, q.z};
+            chain_frame(g.ci >= 2 ? C.cp[g.ci - 2] : nullptr, C.cp[g.ci - 1], p, fx().gr.frame[f]);
+          }
           if (g.ci >= 2 && t < g.k) {
             const BeadPos &q = fx().pos[t];
             const double p[3] = {q.x, q.y, q.z};
-            C.ub[g.ci & 1][t] = chain_bonded_energy(S, C.cp, g.ci, p);
+            fx().gr.ub[g.ci & 1][t] = chain_bonded_energy(S, C.cp, g.ci, p);
           }
         }
         if (g.db >= 0) draw_step(B, g.dstep, g.db, threadIdx.x - 32, blockDim.x - 32);
@@ -2170,6 +2224,7 @@ __global__ void k_gather_states(const RgpuSys *systems, const unsigned long long
   for (int i = threadIdx.x; i < n; i += blockDim.x) xd[i] = S.ads_xyz[i];
 }
 
+/* with the per-call records of the positions */
 __global__ void k_scatter_positions(const RgpuSys *systems, const unsigned long long *off, const unsigned char *buf)
 {
   const RgpuSys &S = systems[blockIdx.x];
@@ -2178,6 +2233,17 @@ __global__ void k_scatter_positions(const RgpuSys *systems, const unsigned long 
   const double *xs = (const double *)(src + sizeof(RgpuState));
   for (int i = threadIdx.x; i < nmol * S.natom * 3; i += blockDim.x) S.ads_xyz[i] = xs[i];
   if (threadIdx.x == 0) *S.nmol = nmol;
+  const int na = S.natom;
+  for (int i = threadIdx.x; i < nmol * na; i += blockDim.x) {
+    const int m = i / na, a = i - m * na;
+    const double x = xs[3 * i], y = xs[3 * i + 1], z = xs[3 * i + 2];
+    int xi, yi, zi;
+    rgpu_fix3(S, x, y, z, xi, yi, zi);
+    S.rec32[i] = make_int4(xi, yi, zi, m * 16 + a);
+    AdsRec64 r;
+    r.x = x; r.y = y; r.z = z; r.tag = m * 16 + a;
+    ((AdsRec64 *)S.rec64)[i] = r;
+  }
 }
 
 cudaError_t rgpu_gather_states_launch(const RgpuSys *d_systems, int n, const unsigned long long *d_off,

@@ -99,6 +99,10 @@ __host__ __device__ inline double chain_cos_dihedral(const double *a, const doub
 __host__ __device__ inline void chain_place_trig(const double *a, const double *b, const double *c, double L,
                                                  double ct, double st, double cp, double sp, double *out);
 
+__host__ __device__ inline void chain_frame(const double *a, const double *b, const double *c, double *F);
+__host__ __device__ inline void chain_place_frame(const double *F, const double *c, double L, double ct, double st,
+                                                  double cp, double sp, double *out);
+
 __host__ __device__ inline void chain_place(const double *a, const double *b, const double *c, double L, double theta,
                                             double phi, double *out)
 {
@@ -108,6 +112,14 @@ __host__ __device__ inline void chain_place(const double *a, const double *b, co
 /* chain_place with cos/sin of theta (ct, st) and of phi (cp, sp) given */
 __host__ __device__ inline void chain_place_trig(const double *a, const double *b, const double *c, double L,
                                                  double ct, double st, double cp, double sp, double *out)
+{
+  double F[9];
+  chain_frame(a, b, c, F);
+  chain_place_frame(F, c, L, ct, st, cp, sp, out);
+}
+
+/* the frame {b-c direction, m, n} of a bead placed after a, b, c */
+__host__ __device__ inline void chain_frame(const double *a, const double *b, const double *c, double *F)
 {
   double bc[3] = {c[0] - b[0], c[1] - b[1], c[2] - b[2]};
   double nb = sqrt(bc[0] * bc[0] + bc[1] * bc[1] + bc[2] * bc[2]);
@@ -127,8 +139,18 @@ __host__ __device__ inline void chain_place_trig(const double *a, const double *
   const double nn = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
   n[0] /= nn; n[1] /= nn; n[2] /= nn;
   const double m[3] = {n[1] * bc[2] - n[2] * bc[1], n[2] * bc[0] - n[0] * bc[2], n[0] * bc[1] - n[1] * bc[0]};
+  for (int k = 0; k < 3; k++) {
+    F[k] = bc[k];
+    F[3 + k] = m[k];
+    F[6 + k] = n[k];
+  }
+}
+
+__host__ __device__ inline void chain_place_frame(const double *F, const double *c, double L, double ct, double st,
+                                                  double cp, double sp, double *out)
+{
   const double dx = -L * ct, dy = L * st * cp, dz = L * st * sp;
-  for (int k = 0; k < 3; k++) out[k] = c[k] + dx * bc[k] + dy * m[k] + dz * n[k];
+  for (int k = 0; k < 3; k++) out[k] = c[k] + dx * F[k] + dy * F[3 + k] + dz * F[6 + k];
 }
 
 /* bonded energy (bend + torsion) that bead i adds to beads 0..i-1 */

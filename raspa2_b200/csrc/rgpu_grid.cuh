@@ -13,7 +13,8 @@
 
 #include "rgpu_types.h"
 
-/* the point wrapped into the unit cell the grid spans: per axis in a
+/* the point wrapped into the unit cell the grid spans (a point at half a cell
+ * may round either way: both wrap to the same place): per axis in a
  * rectangular cell (src/grids.c:995-1002), through the fractional
  * coordinates in a triclinic one (:1004-1021) */
 __device__ __forceinline__ void rgpu_grid_wrap(const RgpuGridGeom &ip, const double *xyz, double *pw)
@@ -22,7 +23,7 @@ __device__ __forceinline__ void rgpu_grid_wrap(const RgpuGridGeom &ip, const dou
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       double p = xyz[c];
-      p -= ip.cell[c] * rgpu_nint(p / ip.cell[c]);
+      p -= ip.cell[c] * rgpu_round(p * ip.icell[c]);
       if (p < 0.0) p += ip.cell[c];
       pw[c] = p;
     }
@@ -33,7 +34,7 @@ __device__ __forceinline__ void rgpu_grid_wrap(const RgpuGridGeom &ip, const dou
 #pragma unroll
   for (int r = 0; r < 3; r++) {
     f[r] = __ldg(v + 3 * r) * xyz[0] + __ldg(v + 3 * r + 1) * xyz[1] + __ldg(v + 3 * r + 2) * xyz[2];
-    f[r] -= rgpu_nint(f[r]);
+    f[r] -= rgpu_round(f[r]);
     if (f[r] < 0.0) f[r] += 1.0;
   }
 #pragma unroll
@@ -61,7 +62,7 @@ __device__ __forceinline__ double rgpu_grid_value(const float *grid, const RgpuG
   rgpu_grid_wrap(ip, xyz, pw);
   for (int c = 0; c < 3; c++) {
     const double p = pw[c];
-    const double s = ((p - ip.shift[c]) / ip.size[c]) * (double)ip.npts[c];
+    const double s = (p - ip.shift[c]) * ip.scale[c];
     /* a point on the upper cell face (p == cell after wrapping) uses the last
      * grid cell at r = 1, so the 2x2x2 corner block stays inside the grid */
     i0[c] = min(max((int)s, 0), ip.npts[c] - 1);
@@ -120,7 +121,7 @@ __device__ __forceinline__ double rgpu_grid_value8(const float *grid, const Rgpu
     rgpu_grid_wrap(ip, xyz, pw);
     for (int c = 0; c < 3; c++) {
       const double p = pw[c];
-      const double s = ((p - ip.shift[c]) / ip.size[c]) * (double)ip.npts[c];
+      const double s = (p - ip.shift[c]) * ip.scale[c];
       i0[c] = min(max((int)s, 0), ip.npts[c] - 1);
       r[c] = s - i0[c];
     }

@@ -128,6 +128,7 @@ typedef struct {
   int npts[3];
   int tri;
   double size[3], shift[3], cell[3];
+  double icell[3], scale[3];  /* 1 / cell, npts / size */
   const double *uc;
 } RgpuGridGeom;
 
@@ -208,6 +209,8 @@ typedef struct RgpuSys {
   const double2 *sk_fw;       /* [nk] */
   double2 *sk_ads;            /* [nk] */
   double *ads_xyz;            /* [maxmol*natom*3] authoritative positions */
+  int4 *rec32;                /* the per-call adsorbate records of these, fixed point and FP64 */
+  void *rec64;
   int *nmol;                  /* [1] */
   double *energy;             /* [RGPU_NE] running totals (inside the RgpuState block) */
   unsigned long long *step;   /* [4], see RgpuState.step */

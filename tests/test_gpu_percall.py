@@ -128,3 +128,28 @@ def test_mixed_lists_and_their_overflow(cuda, atoms):
     near = np.max(np.abs(ref), axis=1) < 1e15      # a pair within about 0.3 A gives more
     assert near.sum() >= 3
     assert np.all(np.abs(got - ref)[near] <= 5e-6 * scale[near] + 1e-6)
+
+
+@pytest.mark.parametrize("tri", [False, True])
+def test_energies_after_a_batched_upload(cuda, tri):
+    """A batched upload leaves the records that per-call energies read: the same bits as after uploads system by
+    system, for no molecule, one, and more atoms than a block has threads."""
+    s = co2_box(96, tri)
+    rng = np.random.default_rng(7)
+    counts = [0, 1, 86, 200]
+    mols = [molecules(rng, s, n) for n in counts]
+    xyz = s.box_point(rng.random((24, 3)))
+    atom, excl = rng.integers(0, 3, 24), np.full(24, -1)
+    got = []
+    for batched in (False, True):
+        gs = [native.GpuSystem(s, maxmol=256, stream_id=i) for i in range(len(counts))]
+        e = native.Engine(gs, precision=native.RGPU_MIXED, threads=256, cluster=2)
+        if batched:
+            for g in gs:
+                g.set_adsorbates(molecules(rng, s, 40))
+            e.set_adsorbates(mols)
+        else:
+            for g, x in zip(gs, mols):
+                g.set_adsorbates(x)
+        got.append([g.bead_energies(xyz, atom, excl, p) for g in gs for p in (native.RGPU_FP64, native.RGPU_MIXED)])
+    np.testing.assert_array_equal(np.array(got[0]), np.array(got[1]))
