@@ -97,9 +97,9 @@ size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int fwd_items, int tiles,
  * of them between barriers, which cost some 500 cycles. Code now 120 to 270
  * KB. Measured (upload, moves, states read back): 64 mixed CO2 boxes, 1000
  * moves each, 21.5 ms (27.2 before); one FP64 CO2 box, 200 moves, 3.26 ms
- * (4.30); 32 hexane boxes over grids, 100 moves, 3.97 ms (4.45; 4.29 with the
- * bend angles of a growth, its uniforms, the next bead's frames and the
- * trials' LJ all formed by warp 0 or on its way). */
+ * (4.30); 32 hexane boxes over grids, 100 moves, 3.89 ms (4.43; 4.29 with the
+ * bend angles of a growth, its uniforms, the next bead's frames, the trials'
+ * LJ and the next stage's description all formed by warp 0 or on its way). */
 #define RGPU_COLD __noinline__
 
 /* floor(2^32 / n) + 1 (less one for powers of two: 2^32 / n) for 2 <= n <= 64, 0
@@ -1588,14 +1588,13 @@ __device__ RGPU_COLD void chain_tables(Build<MIXED, FLEX> E, const Stage &g)
 /* Stage for bead i of a growth (k trials), with
  * the retrace beads from r0 on that ride along (r0 = natom: none) */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void grow_stage(Build<MIXED, FLEX> E, int i, int k, int r0)
+__device__ __forceinline__ void grow_stage(Build<MIXED, FLEX> E, Stage &n, const Stage &c, int i, int k, int r0)
 {
   const RgpuSys &S = fx().S;
   int r1 = r0, rP = 0;
   if (r0 < S.natom) r1 = retrace_group_end(r0, S.natom, S.ntrial_first, S.ntrial, RGPU_MAX_POS - k, rP);
-  next_stage(E, PH_GROW, k + rP, 0, 0);
-  if (threadIdx.x == 0) {
-    Stage &n = next_of();
+  fill_stage(E, n, c, PH_GROW, k + rP, 0, 0);
+  if ((threadIdx.x & 31) == 0) {
     n.ci = i;
     n.k = k;
     n.r0 = r0;
@@ -1637,7 +1636,7 @@ __device__ __forceinline__ void end_table(Build<MIXED, FLEX> E)
     retrace_stage(E, 0);
     return;
   }
-  grow_stage(E, 0, S.ntrial_first, mv == 4 ? 0 : S.natom);
+  grow_stage(E, next_of(), cur(), 0, S.ntrial_first, mv == 4 ? 0 : S.natom);
 }
 
 /* warp 0, after the trials of bead g.ci: returns whether the step is done
@@ -1647,7 +1646,7 @@ __device__ __forceinline__ bool end_grow(Build<MIXED, FLEX> E, const Stage &g)
 {
   RgpuSys &S = fx().S;
   Ctl &C = fx().C;
-  const int na = S.natom, i = g.ci, k = g.k, lane = threadIdx.x;
+  const int i = g.ci, k = g.k, lane = threadIdx.x;
   double lj = 0.0, bf = 0.0;
   int ov = 0;
   const double4 rt = fx().tot[lane < k ? lane : 0];
@@ -1688,13 +1687,34 @@ __device__ __forceinline__ bool end_grow(Build<MIXED, FLEX> E, const Stage &g)
     if (fail) C.cnt[RGPU_CNT_OVERLAP]++;
   }
   __syncwarp();
-  if (fail) return true;
-  if (i + 1 < na) {
-    grow_stage(E, i + 1, S.ntrial, g.r1);
-  } else {
-    next_stage(E, PH_CHAINEND, 0, 0, 0);
+  return fail;
+}
+
+/* what the other warps do while warp 0 chooses among the trials of bead g.ci:
+ * the bookkeeping of a riding retrace group, the frame that each trial would
+ * give the next bead, the trials' bonded energies (warp 0 writes only
+ * C.cp[ci]), the stage that follows a growth that did not fail */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ void beside_grow(Build<MIXED, FLEX> E, Stage &n, const Stage &g)
+{
+  const RgpuSys &S = fx().S;
+  Ctl &C = fx().C;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, i = g.ci;
+  if (g.r1 > g.r0) retrace_book(E, g.r0, g.r1, g.k, C.co, fx_ang() + RGPU_ANG_DOUBLES, 1);
+  /* a warp each, as far as the block has them (warp 1 describes the next step) */
+  if (w == (nw > 2 ? 2 : 1) && i >= 1 && lane < g.k) {
+    const double p[3] = {fx().pos[lane].x, fx().pos[lane].y, fx().pos[lane].z};
+    chain_frame(i >= 2 ? C.cp[i - 2] : nullptr, C.cp[i - 1], p, fx().gr.frame[lane]);
   }
-  return false;
+  if (w == (nw > 3 ? 3 : 1) && i >= 2 && lane < g.k) {
+    const double p[3] = {fx().pos[lane].x, fx().pos[lane].y, fx().pos[lane].z};
+    fx().gr.ub[i & 1][lane] = chain_bonded_energy(S, C.cp, i, p);
+  }
+  if (w == (nw > 4 ? 4 : 1)) {
+    __syncwarp();
+    if (i + 1 < S.natom) grow_stage(E, n, g, i + 1, S.ntrial, g.r1);
+    else fill_stage(E, n, g, PH_CHAINEND, 0, 0, 0);
+  }
 }
 
 /* Acceptance of a chain insertion, deletion or Widom sample
@@ -2104,26 +2124,8 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
         /* warp 1: the next step's first stage, should this stage end its step */
         if (threadIdx.x < 64 && g.ph != PH_TABLE)
           start_step(B, C.st[stage_after(c, 2)], g, g.it + 1, g.buf == 2 ? 0 : g.buf + 1, nsteps, step_end);
-        if (FLEX && g.ph == PH_GROW) {
-          /* a riding retrace group's bookkeeping; then warp 1: the bonded
-           * energies of this bead's trials (warp 0 writes only C.cp[ci]) */
-          if (g.r1 > g.r0) retrace_book(B, g.r0, g.r1, g.k, C.co, fx_ang() + RGPU_ANG_DOUBLES, 1);
-          const int t = threadIdx.x - 32;
-          /* warp 2 (warp 1 of a block of two): the next bead's frame for each of
-           * this bead's trials */
-          const int f = t - (blockDim.x > 64 ? 32 : 0);
-          if (g.ci >= 1 && f >= 0 && f < g.k) {
-            const BeadPos &q = fx().pos[f];
-            const double p[3] = {q.x, q.y, q.z};
-            chain_frame(g.ci >= 2 ? C.cp[g.ci - 2] : nullptr, C.cp[g.ci - 1], p, fx().gr.frame[f]);
-          }
-          if (g.ci >= 2 && t < g.k) {
-            const BeadPos &q = fx().pos[t];
-            const double p[3] = {q.x, q.y, q.z};
-            fx().gr.ub[g.ci & 1][t] = chain_bonded_energy(S, C.cp, g.ci, p);
-          }
-        }
-        if (g.db >= 0) draw_step(B, g.dstep, g.db, threadIdx.x - 32, blockDim.x - 32);
+        if (FLEX && g.ph == PH_GROW) beside_grow(B, C.st[stage_after(c, 1)], g);
+        if (g.db >= 0) draw_step(B, g.dstep, g.db, blockDim.x - 1 - threadIdx.x, blockDim.x - 32);
       }
     }
     const long long it = C.it;
