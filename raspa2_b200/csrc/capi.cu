@@ -752,7 +752,7 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   ALLOC(s->kfactor, sizeof(double) * nk1);
   ALLOC(s->sk_fw, sizeof(double2) * nk1);
   ALLOC(s->sk_ads, sizeof(double2) * nk1);
-  ALLOC(s->ds, sizeof(double2) * nk1);
+  ALLOC(s->ds, sizeof(double2) * 2 * nk1);   /* of per-call differences; of an engine's moves */
   ALLOC(s->ads_xyz, sizeof(double) * 3 * nads);
   ALLOC(s->state, sizeof(RgpuState));
   s->nmol = &s->state->nmol;
@@ -778,6 +778,7 @@ extern "C" int rgpu_system_create(rgpu_system **out, const rgpu_system_desc *d)
   h.kfactor = s->kfactor;
   h.sk_fw = s->sk_fw;
   h.sk_ads = s->sk_ads;
+  h.ds = s->ds + nk1;
   h.ads_xyz = s->ads_xyz;
   h.rec32 = s->rec32;
   h.rec64 = s->rec64;

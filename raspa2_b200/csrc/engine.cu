@@ -96,8 +96,9 @@ size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int fwd_items, int tiles,
  * spread over threads (placing positions, adding up CTAs' sums) is done by all
  * of them between barriers, which cost some 500 cycles. Code now 120 to 270
  * KB. Measured (upload, moves, states read back): 64 mixed CO2 boxes, 1000
- * moves each, 21.5 ms (27.2 before); one FP64 CO2 box, 200 moves, 3.26 ms
- * (4.30); 32 hexane boxes over grids, 100 moves, 3.89 ms (4.43; 4.29 with the
+ * moves each, 20.9 ms (27.2 before; 21.5 with
+ * dS(k) formed again on acceptance); one FP64 CO2 box, 200 moves, 3.21 ms
+ * (4.30); 32 hexane boxes over grids, 100 moves, 3.86 ms (4.43; 4.29 with the
  * bend angles of a growth, its uniforms, the next bead's frames, the trials'
  * LJ and the next stage's description all formed by warp 0 or on its way). */
 #define RGPU_COLD __noinline__
@@ -115,8 +116,8 @@ static __constant__ unsigned c_magic[66] = {0, 0, M8(2), M8(10), M8(18), M8(26),
 struct __align__(16) Stage {
   int ph;                     /* PH_*: what the stage evaluates, and what warp 0 does with it */
   int P, check;               /* bead positions to evaluate, how many of them test single pairs for overlap */
-  int ns, xs;                 /* Ewald sites to sum (0: none); sites buffer of these, or of the latest ones */
-  int ap, xa;                 /* accepted sites still to be added to S_ads(k), in sites buffer xa (0: none) */
+  int ns;                     /* Ewald sites to sum (0: none) */
+  int ap;                     /* the last sites summed are still to be added to S_ads(k) */
   int db;                     /* buffer to draw step dstep's random numbers into (-1: none) */
   unsigned long long dstep;
   int sample;                 /* the step before ended: its state enters the ensemble sums */
@@ -176,7 +177,7 @@ struct Ctl {
   double ew[2];               /* the cluster's, of the stage */
   int nmol;
   int fail;
-  int accept;                 /* accepted Ewald sites (0: none) */
+  int accept;                 /* the last Ewald sites summed were accepted */
   int sel;
   int nads;                   /* adsorbate atoms = nmol * natom */
   int status;                 /* RGPU_ERR_* bits */
@@ -214,7 +215,7 @@ struct __align__(256) Fixed {
   double4 part[2][RGPU_MAX_POS];   /* this CTA's sums {host VDW, host real, adsorbate VDW, adsorbate real} of each
                                     * position, by buffer */
   double4 tot[RGPU_MAX_POS];       /* the cluster's, of the stage */
-  EwSite sites[2][2 * RGPU_MAX_ATOMS];   /* by sites buffer */
+  EwSite sites[2 * RGPU_MAX_ATOMS];
   double red[2 * RGPU_MAX_WARPS];
   union {
     double rot[3][2][RGPU_MAX_TRIALS][4];  /* quaternions of the orientation trials (new, retrace), of three steps */
@@ -563,7 +564,7 @@ __device__ __forceinline__ void place(Build<MIXED, FLEX> E, const Stage &g, int 
   bead_set(b, S, p[0], p[1], p[2], a, excl);
   if (!site) fx().pos[j] = b;
   if (g.ns && (site || ph == PH_DISP)) {
-    EwSite &t = fx().sites[g.xs][j];
+    EwSite &t = fx().sites[j];
     t.b = b;
     t.q = q;
   }
@@ -579,7 +580,7 @@ __device__ __forceinline__ void place(Build<MIXED, FLEX> E, const Stage &g, int 
  * The Ewald work follows the pair units and fills their tail (with a fixed
  * share per warp a stage waited for the warps that had two pair units before
  * theirs). On the mixed path it needs no phase table; the other paths build one
- * per stage, after the pending update has used the last. */
+ * per stage. */
 template <int MIXED, bool FLEX>
 __device__ __forceinline__ void eval_stage(Eng<MIXED, FLEX> &E, const Stage &g)
 {
@@ -588,16 +589,10 @@ __device__ __forceinline__ void eval_stage(Eng<MIXED, FLEX> &E, const Stage &g)
   cg::cluster_group cl = cg::this_cluster();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const long long t0 = clock64();
-  const EwSite *sites = fx().sites[g.xs], *acc = fx().sites[g.xa & 1];
-  if (MIXED != 1) {
-    if (g.ap) {
-      ewald_apply_share<MIXED>(S, E.tab, E.kw, acc, g.ap, E.k0, E.k1, w);
-      if (g.ns) __syncthreads();
-    }
-    if (g.ns) {
-      ewald_phases<MIXED>(S, sites, g.ns, E.tab, E.kw);
-      __syncthreads();
-    }
+  const EwSite *sites = fx().sites;
+  if (MIXED != 1 && g.ns) {
+    ewald_phases<MIXED>(S, sites, g.ns, E.tab, E.kw);
+    __syncthreads();
   }
   if (g.ns && threadIdx.x == 0) {
     C.work[0] += (unsigned long long)(E.k1 - E.k0) * g.ns;
@@ -640,7 +635,7 @@ __device__ __forceinline__ void eval_stage(Eng<MIXED, FLEX> &E, const Stage &g)
     const int pl = g.plan[E.rank];
     eval_units<MIXED>(S, E.sl, fx().pos, g.P, g.check, E.sc, pl & 0xffff, pl >> 16, g.mf, g.ma);
   }
-  if (g.ns || (MIXED == 1 && g.ap)) {
+  if (g.ns || g.ap) {
     /* the shares of the wave vectors, one per warp of the block, taken as the
      * warps run out of pair units; the last to finish adds them up in order */
     for (;;) {
@@ -648,9 +643,8 @@ __device__ __forceinline__ void eval_stage(Eng<MIXED, FLEX> &E, const Stage &g)
       if (lane == 0) u = atomicAdd(&C.nextk, 1);
       u = __shfl_sync(RGPU_FULL, u, 0);
       if (u >= nw) break;
-      if (MIXED == 1 && g.ap) ewald_apply_share<MIXED>(S, E.tab, E.kw, acc, g.ap, E.k0, E.k1, u);
+      ewald_share<MIXED>(S, E.tab, E.kw, sites, g.ns, g.ap, E.k0, E.k1, u, fx().red);
       if (!g.ns) continue;
-      ewald_energy_share<MIXED>(S, E.tab, E.kw, sites, g.ns, E.k0, E.k1, u, fx().red);
       int d = 0;
       if (lane == 0) {
         __threadfence_block();
@@ -740,8 +734,7 @@ __device__ __forceinline__ int stage_after(int c, int n) { return c + n >= 3 ? c
 __device__ __forceinline__ const Stage &cur() { return fx().C.st[fx().C.cur]; }
 
 /* Describes stage n, which follows stage c: what it evaluates, and the chunks
- * of a position in every CTA (lane q: CTA q). ns > 0: its Ewald sites take the
- * buffer that the last sites, whose S(k) update may be pending, do not use. */
+ * of a position in every CTA (lane q: CTA q). */
 template <int MIXED, bool FLEX>
 __device__ RGPU_COLD void fill_stage(Build<MIXED, FLEX> E, Stage &n, const Stage &c, int ph, int P, int check, int ns)
 {
@@ -772,7 +765,6 @@ __device__ RGPU_COLD void fill_stage(Build<MIXED, FLEX> E, Stage &n, const Stage
     n.P = P;
     n.check = check;
     n.ns = ns;
-    n.xs = ns ? c.xs ^ 1 : c.xs;
     n.db = -1;
     n.first = 0;
     n.k = n.rP = 0;
@@ -796,9 +788,9 @@ __device__ __forceinline__ void next_stage(Build<MIXED, FLEX> E, int ph, int P, 
 /* an accepted move's sites are added to S_ads(k) in the next stage (end_stage
  * passes them on) */
 template <int MIXED, bool FLEX>
-__device__ __forceinline__ void accept_sites(Build<MIXED, FLEX> E, int ns)
+__device__ __forceinline__ void accept_sites(Build<MIXED, FLEX> E)
 {
-  if (has_ewald(fx().S) && threadIdx.x == 0) fx().C.accept = ns;
+  if (has_ewald(fx().S) && threadIdx.x == 0) fx().C.accept = 1;
 }
 
 __device__ RGPU_COLD double cold_exp(double x) { return exp(x); }
@@ -939,7 +931,7 @@ __device__ __forceinline__ void end_displace(Build<MIXED, FLEX> E, int buf)
       const double p[3] = {fx().pos[lane].x, fx().pos[lane].y, fx().pos[lane].z};
       atom_store(E, cur().m, lane, p);
     }
-    accept_sites(E, 2 * na);
+    accept_sites(E);
   }
 }
 
@@ -1004,7 +996,7 @@ __device__ RGPU_COLD void accept_swap(Build<MIXED, FLEX> E, int buf)
         atom_store(E, m, threadIdx.x, p);
       }
     }
-    accept_sites(E, na);
+    accept_sites(E);
   }
 }
 
@@ -1120,7 +1112,7 @@ __device__ RGPU_COLD void accept_reinsert(Build<MIXED, FLEX> E, int buf)
       chosen_atom(E, threadIdx.x, p);
       atom_store(E, cur().m, threadIdx.x, p);
     }
-    accept_sites(E, 2 * na);
+    accept_sites(E);
   }
 }
 
@@ -1935,7 +1927,6 @@ __device__ RGPU_COLD void end_stage(Build<MIXED, FLEX> E, int c, long long nstep
   if (threadIdx.x == 0) {
     Stage &n = C.st[nx];
     n.ap = C.accept;
-    n.xa = g.xs;
     n.sample = done && fx().step0 + (uint64_t)g.it >= avg0;
     if (done) C.it = g.it + 1;
     C.which = nx;
@@ -2016,7 +2007,6 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
       C.cur = 0;
       C.which = 0;
       C.accept = 0;
-      C.st[2].xs = 0;
       for (int k = 0; k < RGPU_NSUM; k++) C.sums[k] = 0.0;
       C.nmol = *S.nmol;
       C.nads = C.nmol * S.natom;
@@ -2109,7 +2099,7 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
         eval_stage(E, g);
       } else {
         if (g.ap)
-          ewald_apply_share<MIXED>(S, E.tab, E.kw, fx().sites[g.xa & 1], g.ap, E.k0, E.k1, threadIdx.x >> 5);
+          ewald_share<MIXED>(S, E.tab, E.kw, nullptr, 0, true, E.k0, E.k1, threadIdx.x >> 5, nullptr);
         if (g.ph == PH_END) break;
         if (FLEX && g.ph == PH_TABLE) chain_tables(B, g);
         __syncthreads();          /* also: every thread knows the stage before warp 0 names the next */

@@ -1137,43 +1137,41 @@ __device__ __forceinline__ double2 ewald_dS(const typename PhaseT<MIXED>::T *tab
   }
 }
 
-/* The energy change over share u of wave vectors [k0, k1): those of thread
- * 32 u + lane of blockDim.x that stride through them; its {e_ads, e_host} go
- * to red[2u], red[2u+1]. Warp-wide. */
+/* Share u of wave vectors [k0, k1): those of thread 32 u + lane of blockDim.x
+ * that stride through them. Warp-wide.
+ * apply: S_ads(k) += dS(k) of the last sites summed (AcceptEwaldAdsorbateMove,
+ * src/ewald.c:11732), from S.ds, so the stored sums are those the accepted
+ * energy was computed with. Forming dS(k) again instead took 6 sites' phases a
+ * wave vector, half of the Ewald work of an accepted displacement.
+ * Then, ns > 0: dS(k) of the sites, to S.ds, and the energy change; the
+ * share's {e_ads, e_host} go to red[2u], red[2u+1]. */
 template <int MIXED>
-__device__ __forceinline__ void ewald_energy_share(const RgpuSys &S, const typename PhaseT<MIXED>::T *tab, int kw,
-                                                   const EwSite *sites, int ns, int k0, int k1, int u, double *red)
+__device__ __forceinline__ void ewald_share(const RgpuSys &S, const typename PhaseT<MIXED>::T *tab, int kw,
+                                            const EwSite *sites, int ns, bool apply, int k0, int k1, int u, double *red)
 {
   double ea = 0.0, eh = 0.0;
 #pragma unroll 1
   for (int k = k0 + 32 * u + (threadIdx.x & 31); k < k1; k += blockDim.x) {
-    double2 d = ewald_dS<MIXED>(tab, kw, sites, ns, S.kvec[k]);
     double2 so = S.sk_ads[k];
-    double2 sf = S.sk_fw[k];
-    double kf = S.kfactor[k];
+    if (apply) {
+      const double2 d = S.ds[k];
+      so = make_double2(so.x + d.x, so.y + d.y);
+      S.sk_ads[k] = so;
+    }
+    if (!ns) continue;
+    const double2 d = ewald_dS<MIXED>(tab, kw, sites, ns, S.kvec[k]);
+    S.ds[k] = d;
+    const double2 sf = S.sk_fw[k];
+    const double kf = S.kfactor[k];
     ea += kf * (2.0 * (so.x * d.x + so.y * d.y) + d.x * d.x + d.y * d.y);
     eh += kf * (sf.x * d.x + sf.y * d.y);
   }
+  if (!ns) return;
   ea = warp_sum(ea);
   eh = warp_sum(eh);
   if ((threadIdx.x & 31) == 0) {
     red[2 * u] = ea;
     red[2 * u + 1] = eh;
-  }
-}
-
-/* S_ads(k) += dS(k) (AcceptEwaldAdsorbateMove, src/ewald.c:11732) over share
- * u of wave vectors [k0, k1). The same ewald_dS call as in the energy sum, so
- * the stored sums are those the accepted energy was computed with. */
-template <int MIXED>
-__device__ __forceinline__ void ewald_apply_share(const RgpuSys &S, const typename PhaseT<MIXED>::T *tab, int kw,
-                                                  const EwSite *sites, int ns, int k0, int k1, int u)
-{
-#pragma unroll 1
-  for (int k = k0 + 32 * u + (threadIdx.x & 31); k < k1; k += blockDim.x) {
-    double2 d = ewald_dS<MIXED>(tab, kw, sites, ns, S.kvec[k]);
-    double2 so = S.sk_ads[k];
-    S.sk_ads[k] = make_double2(so.x + d.x, so.y + d.y);
   }
 }
 

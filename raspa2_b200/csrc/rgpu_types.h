@@ -208,6 +208,7 @@ typedef struct RgpuSys {
   const double *kfactor;      /* [nk] */
   const double2 *sk_fw;       /* [nk] */
   double2 *sk_ads;            /* [nk] */
+  double2 *ds;                /* [nk] dS(k) of an engine's last Ewald sum */
   double *ads_xyz;            /* [maxmol*natom*3] authoritative positions */
   int4 *rec32;                /* the per-call adsorbate records of these, fixed point and FP64 */
   void *rec64;
