@@ -346,7 +346,7 @@ cudaError_t rgpu_grid_interp_launch(const float *d_grid, const int npts[3], cons
     ip.shift[c] = shift[c];
     ip.cell[c] = cell[c];
     ip.icell[c] = 1.0 / cell[c];
-    ip.scale[c] = npts[c] / size[c];
+    ip.isize[c] = 1.0 / size[c];
   }
   if (n <= 0) return cudaSuccess;
   k_grid_interp<<<(n + INTERP_THREADS - 1) / INTERP_THREADS, INTERP_THREADS, 0, st>>>(d_grid, ip, n, d_xyz, d_out);

@@ -128,7 +128,7 @@ typedef struct {
   int npts[3];
   int tri;
   double size[3], shift[3], cell[3];
-  double icell[3], scale[3];  /* 1 / cell, npts / size */
+  double icell[3], isize[3];  /* 1 / cell, 1 / size */
   const double *uc;
 } RgpuGridGeom;
 

@@ -127,3 +127,25 @@ def test_interpolate_across_stage_edges(cuda, n):
                           for i in range(0, n, 8192)])
     for g in got:
         np.testing.assert_array_equal(g, ref)
+
+
+@pytest.mark.parametrize("cell", [10.0, 13.7])
+def test_lookups_at_half_cells(cuda, cell):
+    """Points at multiples of half a cell and next to them, where the nearest image is a tie: the value at the
+    wrapped point, which is in the cell already (within the rounding of the wrap, a few ulp of 4 cells, times the
+    slopes of a random grid of a dozen points a side)."""
+    import torch
+    npts, size, shift = np.array([7, 9, 11], np.int32), np.full(3, cell), np.zeros(3)
+    g = torch.rand(8, 10, 12, 8, device="cuda")
+    g[-1], g[:, -1], g[:, :, -1] = g[0], g[:, 0], g[:, :, 0]    # periodic: a point may round onto either face
+    g[-1] = g[0]
+    grid = g.contiguous()
+    half = np.concatenate([np.arange(-8, 9) * (0.5 * cell), np.nextafter(np.arange(-8, 9) * (0.5 * cell), 0.0)])
+    xyz = np.stack(np.meshgrid(half, half, half[::3]), -1).reshape(-1, 3)
+    n = np.trunc(xyz / cell + np.where(xyz >= 0.0, 0.5, -0.5))
+    wrapped = xyz - cell * n
+    wrapped = np.where(wrapped < 0.0, wrapped + cell, wrapped)
+    torch.cuda.synchronize()
+    look = [native.grid_interpolate(grid.data_ptr(), npts, size, shift, size, x) for x in (xyz, wrapped)]
+    scale = np.abs(look[1]).max()
+    assert np.all(np.abs(look[0] - look[1]) <= 1e-12 * scale)
