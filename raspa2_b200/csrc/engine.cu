@@ -98,7 +98,7 @@ size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int fwd_items, int tiles,
  * KB. Measured (upload, moves, states read back): 64 mixed CO2 boxes, 1000
  * moves each, 20.9 ms (27.2 before; 21.5 with
  * dS(k) formed again on acceptance); one FP64 CO2 box, 200 moves, 3.21 ms
- * (4.30); 32 hexane boxes over grids, 100 moves, 3.86 ms (4.43; 4.29 with the
+ * (4.30); 32 hexane boxes over grids, 100 moves, 3.88 ms (4.43; 4.29 with the
  * bend angles of a growth, its uniforms, the next bead's frames, the trials'
  * LJ and the next stage's description all formed by warp 0 or on its way). */
 #define RGPU_COLD __noinline__

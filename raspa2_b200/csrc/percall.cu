@@ -65,9 +65,11 @@ __device__ __forceinline__ void grid_terms(const RgpuSys &S, const BeadPos &b, i
  * unit_tiles_fp64, and the sums meet in the first CTA's shared memory in rank
  * and warp order. What bounds it is the chain of one warp (descriptor load,
  * cull, two or three tile passes, one queue evaluation), not arithmetic.
- * Measured, whole call from Python: 20 positions in a 1536-atom CO2 box 34 us,
- * 139 us with one CTA of 8 warps walking all atoms of all positions; one
- * position in 3456 uncharged atoms 29 us (46 us). */
+ * Measured, whole call from Python: 20 positions in a 1536-atom CO2 box 23.5 us
+ * (the kernel 12.8, cold, under the profiler), 139 us with one CTA of 8 warps
+ * walking all atoms of all positions; one position in 3456 uncharged atoms 18.9
+ * us (kernel 9.2), 46 us before. Of each, some 10 us went with the binding's
+ * buffer pointers, the rest with this kernel and its launch. */
 __global__ void __launch_bounds__(32 * POINT_WARPS) k_points_fp64(const RgpuSys *sysp, const AdsRec64 *ads, int nads,
                                                                  const __grid_constant__ RgpuPoints in, int pair_check,
                                                                  int fw_grid, double *out, int *ov)
@@ -213,8 +215,9 @@ __global__ void __launch_bounds__(64 * POINT_MIXED_WARPS) k_points_mixed(const R
  * of its own, all threads form the lists' pair terms into one sequence, and
  * one warp adds that up. A ninth warp takes the adsorbates meanwhile. A
  * list that overflows sends the position through one warp's queue. Bound by the
- * chain of steps. 64 positions in 4096 atoms: 23 us a call, 40 us with one warp
- * walking all tiles of a position. */
+ * chain of steps. 64 positions in 4096 atoms: 26 us a call from Python (the
+ * kernel 16.7, cold, under the profiler), 40 us with one warp walking all tiles
+ * of a position. */
 #define LONG_WARPS 8
 #define LONG_LIST 256          /* pairs of one warp; a sixteenth of the sphere's atoms at 0.09 / A^3 is 41 */
 
@@ -401,7 +404,9 @@ cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ad
  * VDW, adsorbate real, exclusion} of its atoms and molecules in out[5 c ..]
  * (mapped host memory). Each CTA takes every gridDim-th atom, a warp per
  * quarter of the framework tiles and of the adsorbate records, so that a
- * loaded box fills the GPU in one launch; bound by FP64 pair arithmetic. */
+ * loaded box fills the GPU in one launch. 408 atoms in 4096: 21.7 us under the
+ * profiler, cold, a warp's chain of tile passes with the FP64 pipe 15 % busy (4.5
+ * ms in seven launches of one CTA before). */
 #define TOTAL_WARPS 4
 
 __global__ void __launch_bounds__(32 * TOTAL_WARPS) k_total_pairs(const RgpuSys *sysp, const AdsRec64 *ads, int nads,
@@ -483,9 +488,12 @@ cudaError_t rgpu_total_pairs_launch(const RgpuSys *d_sys, const void *d_ads, int
  * three shared-memory reads and 10 FMAs instead of a sincospi. The atoms are
  * cut into SK_PARTS parts (every SK_PARTS-th table of atoms), which the CTAs of a
  * cluster share; S(k) is the sum of the parts' sums in order, so it has the
- * same bits however many CTAs a kernel gives to it. Bound by FP64 instructions where atoms are many, else by the table.
- * Measured: 408 atoms, 2600 wave vectors 9 us (103 us with one sincospi per
- * pair and one thread looping over all atoms). */
+ * same bits however many CTAs a kernel gives to it.
+ * Bound by latency (the table and its barriers, one atom after the other): the
+ * FP64 pipe is 13 to 19 % busy. Measured under the profiler, cold: 408 atoms,
+ * about 2600 wave vectors 15.6 us, the 4096 charges of a framework 94 us, once
+ * a system (103 us and more with one sincospi per pair and one thread looping
+ * over all atoms). */
 #define SK_THREADS 256
 #define SK_ATOMS 16
 #define SK_KMAX 20             /* rgpu_system_create's limit on kmax */
@@ -656,7 +664,8 @@ cudaError_t rgpu_upload_sk_launch(const RgpuSys *d_systems, int n, int max_nk, c
  * into d_ds (for a later accept) and {e_ads, e_host} into out (mapped host
  * memory). One cluster of CTAs splits the wave vectors; each CTA builds the
  * (small) phase tables of the FP64 path for itself. Bound by latency: the
- * descriptor, the table, one or two wave vectors a thread, two reductions. */
+ * descriptor, the table, one or two wave vectors a thread, two reductions (11.4
+ * us for a displaced CO2 under the profiler, cold; 14 with one CTA). */
 #define DELTA_CLUSTER 8
 
 template <int MIXED>

@@ -598,8 +598,9 @@ __device__ __forceinline__ void unit_tiles_cc64(const RgpuSys &S, const int4 *fw
 }
 
 /* framework tiles [t0, t1) for bead b, FP32 path (warp-wide); TRI: the
- * box is triclinic (S.triclinic). mem: the warp's queue. Issue-bound (about
- * 45 instructions a pass of two tiles, 90 per 32 queued pairs). */
+ * box is triclinic (S.triclinic). mem: the warp's queue. Bound by
+ * instruction issue: a batched engine's step fills half of all issue slots,
+ * nearly all of them in its evaluations. */
 template <bool TRI>
 __device__ __forceinline__ void unit_tiles_mixed(const RgpuSys &S, const int4 *fw, const TileRec *tiles, int t0, int t1,
                                                  const BeadPos &b, bool check, float &av, float &ac, int &ov,
