@@ -678,9 +678,9 @@ __device__ __forceinline__ void pair_fp64_queued(const RgpuSys &S, const double4
   if (r2 < S.rc2) {
     nin++;
     const RgpuLJ P = S.lj_bf[b.atom][entry & 3];
-    double ri = 0.0, ir2;
+    double ir2;
     if (charged) {
-      ri = rsqrt(r2);
+      const double ri = rsqrt(r2);
       ir2 = ri * ri;
     } else {
       ir2 = 1.0 / r2;
@@ -692,7 +692,9 @@ __device__ __forceinline__ void pair_fp64_queued(const RgpuSys &S, const double4
     if (check && u >= S.overlap) ov = 1;
     if (charged) {
       nch++;
-      const double uc = qa * f.w * (erfc(S.alpha * (r2 * ri)) * ri);
+      /* r by the square root: on an atom (r2 = 0) erfc(0) / 0 is infinite, r2 * rsqrt(r2) would be NaN */
+      const double r = sqrt(r2);
+      const double uc = qa * f.w * (erfc(S.alpha * r) / r);
       ac += uc;
       if (check && uc >= S.overlap) ov = 1;
     }

@@ -153,3 +153,28 @@ def test_energies_after_a_batched_upload(cuda, tri):
                 g.set_adsorbates(x)
         got.append([g.bead_energies(xyz, atom, excl, p) for g in gs for p in (native.RGPU_FP64, native.RGPU_MIXED)])
     np.testing.assert_array_equal(np.array(got[0]), np.array(got[1]))
+
+
+@pytest.mark.parametrize("tri", [False, True])
+def test_bead_on_a_charged_framework_atom(cuda, tri):
+    """A bead exactly on a framework atom: the real-space charge energy is infinite with the sign of the charges'
+    product, and a molecule on a like charge overlaps, also where the atom's type has no LJ (its LJ term, zero
+    times infinity, is NaN)."""
+    s = co2_box(16, tri)
+    rng = np.random.default_rng(3)
+    q = np.round(rng.uniform(0.2, 1.0, 16), 8) * np.where(np.arange(16) % 4 < 2, 1.0, -1.0)
+    s = dataclasses.replace(s, uc_types=["Sifw", "Dummy"] * 8, uc_charges=q - q.mean())
+    pos, _, fq = s.framework()
+    n = len(pos)
+    lj = np.array(s.uc_types)[:n] == "Sifw"
+    g = native.GpuSystem(s, maxmol=4)
+    atom = rng.integers(0, 3, n)
+    got = g.bead_energies(pos, atom, -1)
+    np.testing.assert_array_equal(got[:, 1], np.inf * np.sign(s.molecule.charges()[atom] * fq))
+    np.testing.assert_array_equal(got[lj, 0], np.inf)
+    # a molecule whose carbon (charge +0.7) sits on an atom, its oxygens on none
+    far = s.box_point(np.array([[0.5, 0.5, 0.5]])) + s.molecule.positions
+    g.set_adsorbates(far[None])
+    for k in range(n):
+        overlap, _ = g.move_difference(0, pos[k] + s.molecule.positions - s.molecule.positions[1])
+        assert overlap == (bool(lj[k]) or fq[k] > 0), k
