@@ -122,8 +122,9 @@ struct __align__(16) Stage {
   unsigned long long dstep;
   int sample;                 /* the step before ended: its state enters the ensemble sums */
   int first;                  /* the first stage of a step: the move is counted */
-  /* the move: its type, molecule, whether a deletion takes one evaluation,
-   * the buffer of the step's random numbers, steps done in this launch */
+  /* the move: its type, molecule, whether a deletion or reinsertion has its
+   * retrace orientations evaluated with the first-bead trials, the buffer of
+   * the step's random numbers, steps done in this launch */
   int mv, m, one, buf;
   long long it;
   int ci, k;                  /* chains: bead of the growth and its trials */
@@ -136,7 +137,8 @@ enum {
   PH_END, PH_SKIP,            /* launch done; step without an evaluation */
   PH_DISP,                    /* translation, rotation */
   PH_SWAP1, PH_SWAP2, PH_SWAPEW,     /* rigid insertion, deletion, Widom: first bead, orientations, Ewald sum */
-  PH_REINS1, PH_REINS2, PH_REINSEW,  /* rigid reinsertion */
+  PH_REINS1, PH_REINSOLD, PH_REINS2, PH_REINSEW,  /* rigid reinsertion: first bead (and the old orientations), those
+                                                    * by themselves, new orientations, Ewald sum */
   PH_TABLE, PH_GROW, PH_RETRACE, PH_CHAINEND   /* flexible chains */
 };
 
@@ -545,7 +547,8 @@ __device__ __forceinline__ void place(Build<MIXED, FLEX> E, const Stage &g, int 
     atom_xyz(E, m, a, p);
   } else {
     const bool insert = ph <= PH_SWAPEW && g.mv != 3, second = ph == PH_SWAP2 || ph == PH_REINS2;
-    const int n1 = second ? 0 : (ph == PH_REINS1 ? nf + 1 : nf);   /* first-bead positions */
+    const bool reinsold = ph == PH_REINS1 || ph == PH_REINSOLD;
+    const int n1 = second || ph == PH_REINSOLD ? 0 : (reinsold ? nf + 1 : nf);   /* first-bead positions */
     if (insert) excl = -1;
     if (j < n1) {
       a = sb;
@@ -557,7 +560,7 @@ __device__ __forceinline__ void place(Build<MIXED, FLEX> E, const Stage &g, int 
       double o[3];
       if (second) { o[0] = C.first[0]; o[1] = C.first[1]; o[2] = C.first[2]; }
       else atom_xyz(E, m, sb, o);
-      a = orientation_bead(E, o, fx().rot[buf][ph == PH_REINS1], j - n1, insert || ph == PH_REINS2 ? -1 : m, p);
+      a = orientation_bead(E, o, fx().rot[buf][reinsold], j - n1, insert || ph == PH_REINS2 ? -1 : m, p);
     }
   }
   BeadPos b;
@@ -1082,8 +1085,9 @@ __device__ RGPU_COLD bool add_orientations(Build<MIXED, FLEX> E, bool grow, int 
  * nt - 1 fresh ones. Accepted with probability
  * exp(-beta dU_Fourier) W(new) / W(old).
  * Stage 1 holds the nf new first-bead trials, the old first bead and the
- * retrace orientations (all known up front); stage 2 the new orientations
- * around the chosen first bead; stage 3 the Ewald sum of both. */
+ * retrace orientations (all known up front), these in a stage of their own
+ * where they do not fit (RGPU_MAX_POS positions); stage 2 the new
+ * orientations around the chosen first bead; stage 3 the Ewald sum of both. */
 template <int MIXED, bool FLEX>
 __device__ RGPU_COLD void accept_reinsert(Build<MIXED, FLEX> E, int buf)
 {
@@ -1128,33 +1132,48 @@ __device__ RGPU_COLD bool grown_reinsert(Build<MIXED, FLEX> E, int buf)
   return true;
 }
 
+/* the retrace orientations (trial 0 = the old one) at positions off.. of the
+ * last evaluation complete the old configuration's weight and energies;
+ * returns whether none is valid */
+template <int MIXED, bool FLEX>
+__device__ RGPU_COLD bool old_orientations(Build<MIXED, FLEX> E, int off)
+{
+  Ctl &C = fx().C;
+  const int nt = fx().S.ntrial;
+  const Trials &b = C.tr[1];
+  cbmc_trials(E, off, nt, fx().S.natom - 1, false, false, 0.0, &C.tr[1]);
+  if (threadIdx.x < 4) C.uo[threadIdx.x] += b.e[threadIdx.x];
+  if (threadIdx.x == 0) {
+    C.rosen_old *= b.w_sum / (double)nt;
+    if (!b.any) C.cnt[RGPU_CNT_OVERLAP]++;
+  }
+  __syncwarp();
+  return !b.any;
+}
+
 template <int MIXED, bool FLEX>
 __device__ __forceinline__ bool end_reinsert1(Build<MIXED, FLEX> E, int buf)
 {
   RgpuSys &S = fx().S;
   Ctl &C = fx().C;
   const int na = S.natom, nf = S.ntrial_first, nt = S.ntrial, nb = na - 1;
-  const Trials &a = C.tr[0], &b = C.tr[1];
+  const Trials &a = C.tr[0];
   cbmc_trials(E, 0, nf, 1, true, true, C.rnd[buf][SLOT_FIRST_SELECT], &C.tr[0]);
   /* the old first bead */
   const double4 r = fx().tot[nf];
   const bool ovo = r.x >= S.overlap || r.y >= S.overlap || r.z >= S.overlap || r.w >= S.overlap;
   const double w_old1 = ovo ? 0.0 : cold_exp(-S.beta * (r.x + r.z));
-  /* the retrace orientations (trial 0 = the old one) */
-  if (na > 1) cbmc_trials(E, nf + 1, nt, nb, false, false, 0.0, &C.tr[1]);
   const double rosen = a.w_sum / (double)nf;
-  double rosen_old = (w_old1 + (a.w_sum - a.w_sel)) / (double)nf;
-  if (na > 1) rosen_old *= b.w_sum / (double)nt;
-  const bool fail = !a.any || rosen < 1e-150 || ovo || (na > 1 && !b.any);
+  const bool fail = !a.any || rosen < 1e-150 || ovo;
   if (threadIdx.x == 0) {
     const double ro[4] = {r.x, r.y, r.z, r.w};
     C.rosen = rosen;
-    C.rosen_old = rosen_old;
+    C.rosen_old = (w_old1 + (a.w_sum - a.w_sel)) / (double)nf;
     C.sel = a.sel;
 #pragma unroll 1
     for (int k = 0; k < 4; k++) {
       C.u[k] = a.e[k];
-      C.uo[k] = na > 1 ? ro[k] + b.e[k] : ro[k];
+      C.uo[k] = ro[k];
     }
     const BeadPos &p = fx().pos[a.sel];
     C.first[0] = p.x; C.first[1] = p.y; C.first[2] = p.z;
@@ -1163,7 +1182,19 @@ __device__ __forceinline__ bool end_reinsert1(Build<MIXED, FLEX> E, int buf)
   __syncwarp();
   if (fail) return true;
   if (na == 1) return grown_reinsert(E, buf);
-  next_stage(E, PH_REINS2, nt * nb, 0, 0);
+  const bool one = cur().one != 0;
+  if (one && old_orientations(E, nf + 1)) return true;
+  next_stage(E, one ? PH_REINS2 : PH_REINSOLD, nt * nb, 0, 0);
+  return false;
+}
+
+/* after retrace orientations in a stage of their own; returns whether the
+ * step is done */
+template <int MIXED, bool FLEX>
+__device__ __forceinline__ bool end_reinsert_old(Build<MIXED, FLEX> E)
+{
+  if (old_orientations(E, 0)) return true;
+  next_stage(E, PH_REINS2, fx().S.ntrial * (fx().S.natom - 1), 0, 0);
   return false;
 }
 
@@ -1852,8 +1883,9 @@ __device__ RGPU_COLD void start_step(Build<MIXED, FLEX> E, Stage &n, const Stage
   const Ctl &C = fx().C;
   const int na = S.natom, nf = S.ntrial_first, trials = S.ntrial * (na - 1);
   const int mv = C.mvn[buf], nmol = C.nmol;
+  const int first = mv == 4 ? nf + 1 : nf;   /* first-bead positions */
   const bool end = !(it < nsteps && fx().step0 + (uint64_t)it < step_end);
-  const bool ew = has_ewald(S), one = mv == 3 && nf + trials <= RGPU_MAX_POS;
+  const bool ew = has_ewald(S), one = (mv == 3 || mv == 4) && first + trials <= RGPU_MAX_POS;
   int ph, P = 0, check = 0, ns = 0, m = nmol;
   if (mv != 2 && mv != 5) {
     m = (int)(C.rnd[buf][SLOT_MOLECULE] * nmol);
@@ -1870,13 +1902,10 @@ __device__ RGPU_COLD void start_step(Build<MIXED, FLEX> E, Stage &n, const Stage
     ns = ew ? 2 * na : 0;
   } else if (FLEX && S.flexible) {
     ph = PH_TABLE;       /* the chain moves begin with a stage that draws the angle tables */
-  } else if (mv == 4) {
-    ph = PH_REINS1;
-    P = nf + 1 + trials;
   } else {
-    ph = PH_SWAP1;
-    P = one ? nf + trials : nf;
-    ns = one && ew ? na : 0;
+    ph = mv == 4 ? PH_REINS1 : PH_SWAP1;
+    P = one ? first + trials : first;
+    ns = mv == 3 && one && ew ? na : 0;
   }
   fill_stage(E, n, c, ph, P, check, ns);
   if ((threadIdx.x & 31) == 0) {
@@ -1912,6 +1941,7 @@ __device__ RGPU_COLD void end_stage(Build<MIXED, FLEX> E, int c, long long nstep
   else if (ph == PH_SWAP2) done = add_orientations(E, g.mv != 3, buf) || grown_swap(E, buf);
   else if (ph == PH_SWAPEW) accept_swap(E, buf);
   else if (ph == PH_REINS1) done = end_reinsert1(E, buf);
+  else if (ph == PH_REINSOLD) done = end_reinsert_old(E);
   else if (ph == PH_REINS2) done = add_orientations(E, true, buf) || grown_reinsert(E, buf);
   else if (ph == PH_REINSEW) accept_reinsert(E, buf);
   else if (FLEX && ph == PH_TABLE) { end_table(E); done = false; }

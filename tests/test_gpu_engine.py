@@ -271,3 +271,47 @@ def test_mixed_running_totals_within_1e6_on_batched_boxes(cuda):
         ref = np.asarray(g.total_energy())
         worst = max(worst, abs(np.sum(st["energy"][:6]) - ref.sum()) / abs(ref.sum()))
     assert worst <= 1e-6, worst
+
+
+RIGID_BEADS = ["O_co2", "C_co2", "O_co2", "CH4_sp3", "CH4_sp3", "O_co2", "C_co2", "O_co2"]
+
+
+def rigid_cluster_system(natom, nf, nt):
+    """A rigid molecule of natom beads about its second one, with nf first-bead and nt orientation trials, in the
+    tiny CO2 framework; reinsertion the most frequent move."""
+    import dataclasses
+    s = systems.tiny_co2_system(seed=7)
+    rng = np.random.default_rng(natom)
+    u = rng.normal(size=(natom, 3))
+    x = 0.9 * u / np.linalg.norm(u, axis=1, keepdims=True)
+    x[1] = 0.0
+    mol = systems.Molecule("cluster", RIGID_BEADS[:natom], x, 1, True)
+    return dataclasses.replace(s, molecule=mol, trials_first_bead=nf, trials=nt, pressure=1e6,
+                               moves=systems.MoveMix(translation=0.5, rotation=0.5, swap_insert=1.0, swap_delete=0.5,
+                                                     reinsertion=2.0, widom=0.2))
+
+
+# first-stage positions nf + 1 + nt * (natom - 1): 64 (the most of one evaluation), 65, 73, 81
+@pytest.mark.parametrize("natom,nf,nt,cluster", [(4, 15, 16, 2), (4, 16, 16, 1), (8, 9, 9, 2), (5, 16, 16, 3)])
+def test_reinsertion_of_more_trials_than_one_evaluation(cuda, natom, nf, nt, cluster):
+    """Where a reinsertion's first-bead trials and old orientations do not fit one evaluation, the old orientations
+    take one of their own; the FP64 engine follows the oracle's trajectory, and the mixed engine's running energies
+    agree with a recomputation."""
+    s = rigid_cluster_system(natom, nf, nt)
+    empty = np.zeros((0, natom, 3))
+    n = 400
+    g, st = engine_run(s, empty, n, native.RGPU_FP64, cluster=cluster)
+    o, ost = oracle_run(s, empty, n)
+    assert st["status"] == 0
+    np.testing.assert_array_equal(st["counters"][0:4], np.array(ost.attempts[:4]))
+    np.testing.assert_array_equal(st["counters"][4:8], np.array(ost.accepted[:4]))
+    assert st["counters"][18] == ost.attempts[4] > 50
+    assert st["counters"][19] == ost.accepted[4] > 0
+    assert st["nmol"] == o.nmol > 0
+    np.testing.assert_allclose(g.adsorbates(), o.molecules(), rtol=0, atol=1e-10)
+    np.testing.assert_allclose(st["energy"][:6], np.array(ost.u), rtol=1e-9, atol=1e-6)
+    g, st = engine_run(s, empty, n, native.RGPU_MIXED, cluster=cluster)
+    assert st["status"] == 0 and st["counters"][19] > 0
+    e = g.total_energy()
+    kT = units.K_B * s.temperature
+    assert np.all(np.abs(st["energy"][:6] - e) <= 1e-5 * np.maximum(np.abs(e), kT) * max(1.0, st["counters"][4:8].sum() / 100))
