@@ -678,14 +678,9 @@ __device__ __forceinline__ void pair_fp64_queued(const RgpuSys &S, const double4
   if (r2 < S.rc2) {
     nin++;
     const RgpuLJ P = S.lj_bf[b.atom][entry & 3];
-    double ir2;
-    if (charged) {
-      const double ri = rsqrt(r2);
-      ir2 = ri * ri;
-    } else {
-      ir2 = 1.0 / r2;
-    }
-    double s6 = P.sig2 * ir2;
+    /* one rounded quotient: its error counts six times in r^-12, and rsqrt(r2)
+     * squared (or 1 / r2) times sigma^2 doubled that of the whole term */
+    double s6 = P.sig2 / r2;
     s6 = s6 * s6 * s6;
     const double u = P.eps4 * (s6 * (s6 - 1.0)) - P.shift;
     av += u;

@@ -178,3 +178,26 @@ def test_bead_on_a_charged_framework_atom(cuda, tri):
     for k in range(n):
         overlap, _ = g.move_difference(0, pos[k] + s.molecule.positions - s.molecule.positions[1])
         assert overlap == (bool(lj[k]) or fq[k] > 0), k
+
+
+@pytest.mark.parametrize("charged", [False, True])
+def test_fp64_lj_rounding(cuda, charged):
+    """LJ of one pair at exactly representable distances against extended precision. With one rounded quotient
+    sigma^2 / r^2 the r^-12 term collects at most 13 units of u = 2^-53 (6 from the quotient, 2 + 2 from the products
+    of s^6, 3 from the rest) and, roundings being independent with an rms of 0.43 u, 2.9 u rms; one more rounding of
+    1 / r^2 makes that 3.9 u, so 3.3 u tells them apart (4096 pairs give it to 2 %)."""
+    s = co2_box(16, False)
+    s = dataclasses.replace(s, unit_cell=np.array([32.0, 32.0, 32.0]), frac=np.full((1, 3), 0.25), uc_types=["Sifw"],
+                            uc_charges=np.array([0.5 if charged else 0.0]))
+    g = native.GpuSystem(s, maxmol=4)
+    rng = np.random.default_rng(11)
+    d = rng.normal(size=(4096, 3))
+    d *= rng.uniform(0.8, 1.6, (4096, 1)) / np.linalg.norm(d, axis=1, keepdims=True)
+    d = np.round(d * 4096) / 4096          # r^2 is exact
+    got = g.bead_energies(8.0 + d, 0, -1)[:, 0].astype(np.longdouble)
+    eps, sig2, shift = (t[s.molecule_types()[0], systems.TYPE_ORDER.index("Sifw")] for t in s.lj_tables())
+    s6 = (np.longdouble(sig2) / np.sum(d.astype(np.longdouble) ** 2, axis=1)) ** 3
+    ref = 4 * np.longdouble(eps) * (s6 * (s6 - 1)) - np.longdouble(shift)
+    err = (got - ref) / ref * 2.0 ** 53
+    assert np.max(np.abs(err)) <= 13 * 1.05          # s^6 >= 21: (2 s^6 - 1) / (s^6 - 1) is within 5 % of 2
+    assert np.sqrt(np.mean(err ** 2)) <= 3.3
