@@ -209,7 +209,10 @@ int rgpu_grid_build_coulomb(rgpu_system *sys, const int npts[3], const double si
  * reading the device grid; cell = the unit-cell lengths the grid spans.
  * The same lookup serves a Coulomb grid (InterpolateCoulombGrid,
  * src/grids.c:1200-1295, before the multiplication by the bead charge): its
- * capped points hold 2e7, below the VDW lookup's 1e10 corner test. */
+ * capped points hold 2e7, below the VDW lookup's 1e10 corner test. The
+ * library keeps 4 MB of host memory, mapped for the device, from the first
+ * call on (one block per process; calls that overlap allocate instead); it
+ * may be called again after cudaDeviceReset. */
 int rgpu_grid_interpolate(const float *d_grid, const int npts[3], const double size[3], const double shift[3],
                           const double cell[3], int n, const double *xyz, double *out);
 

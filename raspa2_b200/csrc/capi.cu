@@ -1449,7 +1449,10 @@ extern "C" int rgpu_grid_file_path(char *buf, size_t n, const char *raspa_dir, c
  * buffers of its own. Pageable copies of 100 k points (2.4 MB in, 0.8 MB out)
  * alone took 1.5 ms; copied into this in LOOKUP_CHUNK pieces, each looked up
  * while the next is copied, the whole call takes 0.31 ms
- * (1.64 with the copies). */
+ * (1.64 with the copies). The pages are the library's own and registered with
+ * the runtime: cudaDeviceReset undoes the registration, not the memory, so
+ * each call asks whether it still stands (under 1 us) and registers again
+ * where it does not. */
 #define LOOKUP_POINTS 131072
 #define LOOKUP_CHUNK 16384
 
@@ -1458,12 +1461,29 @@ struct LookupStage {
   double xyz[3 * LOOKUP_POINTS];
   double out[LOOKUP_POINTS];
 };
+static_assert(sizeof(LookupStage) % 4096 == 0, "whole pages");
 struct LookupHolder {
   std::mutex mu;
-  LookupStage *p = nullptr;
+  LookupStage *host = nullptr;
+  /* the stage as the device sees it; nullptr: none to be had */
+  LookupStage *device()
+  {
+    if (!host) host = (LookupStage *)aligned_alloc(4096, sizeof(LookupStage));
+    if (!host) return nullptr;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer)
+      return (LookupStage *)at.devicePointer;
+    void *d = nullptr;
+    if (cudaHostRegister(host, sizeof(LookupStage), cudaHostRegisterMapped | cudaHostRegisterPortable) == cudaSuccess &&
+        cudaHostGetDevicePointer(&d, host, 0) == cudaSuccess)
+      return (LookupStage *)d;
+    cudaGetLastError();
+    return nullptr;
+  }
   ~LookupHolder()
   {
-    if (p) cudaFreeHost(p);
+    if (host) cudaHostUnregister(host);
+    free(host);
   }
 };
 LookupHolder g_lookup;
@@ -1479,21 +1499,16 @@ extern "C" int rgpu_grid_interpolate(const float *d_grid, const int npts[3], con
   if (!grid_covers_cell(npts, size, shift, cell)) return fail(RGPU_E_INVALID, "grid does not cover the cell");
   if (n == 0) return RGPU_SUCCESS;
   std::unique_lock<std::mutex> lock(g_lookup.mu, std::try_to_lock);
-  if (lock.owns_lock() && !g_lookup.p) {
-    if (cudaHostAlloc((void **)&g_lookup.p, sizeof(LookupStage), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      g_lookup.p = nullptr;
-    }
-  }
-  if (lock.owns_lock() && g_lookup.p) {
-    LookupStage *g = g_lookup.p;
+  LookupStage *d = lock.owns_lock() ? g_lookup.device() : nullptr;
+  if (d) {
+    LookupStage *g = g_lookup.host;
     for (int base = 0; base < n; base += LOOKUP_POINTS) {
       const int m = std::min(LOOKUP_POINTS, n - base);
       cudaError_t e = cudaSuccess;
       for (int c = 0; c < m && e == cudaSuccess; c += LOOKUP_CHUNK) {
         const int k = std::min(LOOKUP_CHUNK, m - c);
         memcpy(g->xyz + 3 * (size_t)c, xyz + 3 * ((size_t)base + c), sizeof(double) * 3 * k);
-        e = rgpu_grid_interp_launch(d_grid, npts, size, shift, cell, k, g->xyz + 3 * (size_t)c, g->out + c, 0);
+        e = rgpu_grid_interp_launch(d_grid, npts, size, shift, cell, k, d->xyz + 3 * (size_t)c, d->out + c, 0);
       }
       /* wait before the stage is read or used again, also after an error */
       const cudaError_t w = cudaStreamSynchronize(0);

@@ -149,3 +149,48 @@ def test_lookups_at_half_cells(cuda, cell):
     look = [native.grid_interpolate(grid.data_ptr(), npts, size, shift, size, x) for x in (xyz, wrapped)]
     scale = np.abs(look[1]).max()
     assert np.all(np.abs(look[0] - look[1]) <= 1e-12 * scale)
+
+
+def test_lookup_after_a_device_reset(cuda):
+    """Lookups in a process of their own, before and after cudaDeviceReset (which undoes the mapping of the staging
+    memory): the same bits, and those of this process."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import ctypes as C, sys
+import numpy as np
+from raspa2_b200 import native
+rt = C.CDLL("libcudart.so.12")
+native.load()
+rng = np.random.default_rng(5)
+grid = rng.normal(size=9 * 8 * 7 * 8).astype(np.float32)
+xyz = rng.uniform(-9.0, 20.0, (40000, 3))
+def lookup():
+    d = C.c_void_p()
+    assert rt.cudaMalloc(C.byref(d), C.c_size_t(grid.nbytes)) == 0
+    assert rt.cudaMemcpy(d, grid.ctypes.data_as(C.c_void_p), C.c_size_t(grid.nbytes), 1) == 0
+    size = np.array([10.0, 9.0, 8.0])
+    return native.grid_interpolate(d.value, [8, 7, 6], size, np.zeros(3), size, xyz)
+a = lookup()
+assert np.array_equal(lookup(), a)
+for _ in range(2):
+    assert rt.cudaDeviceReset() == 0
+    assert np.array_equal(lookup(), a)
+np.save(sys.argv[1], a)
+"""
+    import tempfile
+
+    import torch
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    with tempfile.TemporaryDirectory() as tmp:
+        f = os.path.join(tmp, "a.npy")
+        p = subprocess.run([sys.executable, "-c", code, f], cwd=root, capture_output=True, text=True, timeout=120,
+                           env=dict(os.environ, PYTHONPATH=root))
+        assert p.returncode == 0, p.stdout + p.stderr
+        a = np.load(f)
+    rng = np.random.default_rng(5)
+    grid = torch.from_numpy(rng.normal(size=9 * 8 * 7 * 8).astype(np.float32)).cuda()
+    size = np.array([10.0, 9.0, 8.0])
+    got = native.grid_interpolate(grid.data_ptr(), [8, 7, 6], size, np.zeros(3), size, rng.uniform(-9.0, 20.0, (40000, 3)))
+    np.testing.assert_array_equal(got, a)
