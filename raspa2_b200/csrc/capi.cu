@@ -1502,12 +1502,12 @@ extern "C" int rgpu_grid_interpolate(const float *d_grid, const int npts[3], con
   LookupStage *d = lock.owns_lock() ? g_lookup.device() : nullptr;
   if (d) {
     LookupStage *g = g_lookup.host;
-    for (int base = 0; base < n; base += LOOKUP_POINTS) {
-      const int m = std::min(LOOKUP_POINTS, n - base);
+    for (size_t base = 0; base < (size_t)n; base += LOOKUP_POINTS) {
+      const int m = (int)std::min((size_t)LOOKUP_POINTS, (size_t)n - base);
       cudaError_t e = cudaSuccess;
       for (int c = 0; c < m && e == cudaSuccess; c += LOOKUP_CHUNK) {
         const int k = std::min(LOOKUP_CHUNK, m - c);
-        memcpy(g->xyz + 3 * (size_t)c, xyz + 3 * ((size_t)base + c), sizeof(double) * 3 * k);
+        memcpy(g->xyz + 3 * (size_t)c, xyz + 3 * (base + c), sizeof(double) * 3 * k);
         e = rgpu_grid_interp_launch(d_grid, npts, size, shift, cell, k, d->xyz + 3 * (size_t)c, d->out + c, 0);
       }
       /* wait before the stage is read or used again, also after an error */

@@ -12,7 +12,7 @@ static struct { char *p; size_t n; } mapped[RANGES];
 int fake_launches;       /* launches asked for */
 int fake_fail_launch;    /* launches return an error */
 int fake_syncs, fake_host_allocs;
-/* 1: every launch is a grid lookup, done as out[i] = x of position i; fake_stray counts those whose
+/* 1: every launch is a grid lookup, done as out[i] = x of position i + 1; fake_stray counts those whose
  * positions or results lie outside the mapped ranges (and are left out) */
 int fake_lookup, fake_stray;
 
@@ -122,7 +122,7 @@ static cudaError_t launch(void **args)
     double *out = *(double **)args[4];
     if (map_find(x, sizeof(double) * 3 * n) < 0 || map_find(out, sizeof(double) * n) < 0) fake_stray++;
     else
-      for (int i = 0; i < n; i++) out[i] = x[3 * i];
+      for (int i = 0; i < n; i++) out[i] = x[3 * i] + 1.0;
   }
   return cudaSuccess;
 }

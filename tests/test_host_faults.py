@@ -53,7 +53,38 @@ def test_lookup_after_a_device_reset(fake):
         value("fake_lookup").value = 1
         x = np.arange(3 * 20000.0).reshape(-1, 3)
         for _ in range(3):
-            assert np.array_equal(lookup(x), x[:, 0])
+            assert np.array_equal(lookup(x), x[:, 0] + 1.0)
             fake.fake_reset()
         assert value("fake_stray").value == 0
+    """)
+
+
+def test_lookup_of_as_many_points_as_an_int_counts(fake):
+    """2^31 - 1 positions, the largest count the call takes: every chunk is looked up once and none after the last.
+    The arrays are addresses (51 and 17 GB) over a page of zeros and a block of 2^21 results."""
+    child(fake, """
+        import os
+        libc = C.CDLL(None, use_errno=True)
+        libc.mmap.restype = C.c_void_p
+        libc.mmap.argtypes = [C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_int, C.c_long]
+        libc.madvise.argtypes = [C.c_void_p, C.c_size_t, C.c_int]
+        def addresses(size, prot):                     # private, anonymous, no reserve
+            at = libc.mmap(None, size, prot, 0x4022, -1, 0)
+            assert at != C.c_void_p(-1).value
+            return at
+        n, k = 2 ** 31 - 1, 2 ** 21
+        x = addresses(24 * 2 ** 31, 1)
+        libc.madvise(x, 24 * 2 ** 31, 14)              # the large page of zeros, where there is one
+        out = addresses(8 * 2 ** 31, 0)
+        fd = os.memfd_create("results")
+        os.ftruncate(fd, 8 * k)
+        for o in range(0, 8 * 2 ** 31, 8 * k):
+            assert libc.mmap(out + o, 8 * k, 3, 0x11, fd, 0) == out + o    # shared, fixed
+        value("fake_lookup").value = 1
+        size, npts, zero = (C.c_double * 3)(*cell), (C.c_int * 3)(1, 1, 1), (C.c_double * 3)()
+        rc = native.load().rgpu_grid_interpolate(C.c_void_p(d_grid), npts, size, zero, size, C.c_int(n), C.c_void_p(x),
+                                                 C.c_void_p(out))
+        assert rc == 0 and value("fake_stray").value == 0
+        assert value("fake_launches").value == 2 ** 31 // 16384
+        assert np.array_equal(np.ctypeslib.as_array(C.cast(out, C.POINTER(C.c_double)), (k,)), np.ones(k))
     """)
