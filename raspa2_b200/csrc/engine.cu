@@ -655,6 +655,7 @@ __device__ __forceinline__ void eval_stage(Eng<MIXED, FLEX> &E, const Stage &g)
         __threadfence_block();
       }
       if (__shfl_sync(RGPU_FULL, d, 0) == nw - 1) {
+        __syncwarp();           /* lane 0's fences before the other lanes' reads of the shares */
         const double ea = warp_sum(lane < nw ? fx().red[2 * lane] : 0.0), eh = warp_sum(lane < nw ? fx().red[2 * lane + 1] : 0.0);
         if (lane == 0) {
           C.ewt[E.xb][0] = ea;

@@ -1014,7 +1014,10 @@ __device__ __forceinline__ void eval_units(const RgpuSys &S, const EvalSlice &sl
       __threadfence_block();
     }
     if (__shfl_sync(RGPU_FULL, d, 0) == per - 1) {
-      /* the position's last unit: lane k < 4 adds up term k */
+      /* the position's last unit: lane k < 4 adds up term k. The barrier
+       * orders the other warps' sums, which lane 0's fences have made visible
+       * to it, before the other lanes' reads; the shuffle does not. */
+      __syncwarp();
       if (lane < 4) {
         const double *t = (const double *)(sc.u + p * per) + (lane & 1);
         const int c0 = lane < 2 ? 0 : cf, c1 = lane < 2 ? cf : per;

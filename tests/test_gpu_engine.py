@@ -315,3 +315,15 @@ def test_reinsertion_of_more_trials_than_one_evaluation(cuda, natom, nf, nt, clu
     e = g.total_energy()
     kT = units.K_B * s.temperature
     assert np.all(np.abs(st["energy"][:6] - e) <= 1e-5 * np.maximum(np.abs(e), kT) * max(1.0, st["counters"][4:8].sum() / 100))
+
+
+@pytest.mark.parametrize("precision,threads", [(native.RGPU_FP64, 512), (native.RGPU_MIXED, 1024),
+                                               (native.RGPU_MIXED_CC64, 512)])
+def test_repeated_runs_have_the_same_bits(cuda, precision, threads):
+    """The units of a position and the shares of the wave vectors are summed by whichever warp finishes last: with
+    many warps to a CTA, and so a different one each time, repeated runs have the same bits."""
+    s = systems.co2_system(seed=21, n_atoms=512, cell=20.0, kmax=5)
+    runs = [engine_run(s, np.zeros((0, 3, 3)), 400, precision, threads=threads, cluster=1)[1] for _ in range(4)]
+    for st in runs[1:]:
+        np.testing.assert_array_equal(st["energy"], runs[0]["energy"])
+        np.testing.assert_array_equal(st["counters"][:15], runs[0]["counters"][:15])
