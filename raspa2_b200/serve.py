@@ -87,14 +87,14 @@ def system_footprint_bytes(s: systems.System, maxmol: int) -> int:
     """Device memory of one system as rgpu_system_create allocates it, plus
     the engine's per-system descriptor."""
     nfw = s.n_framework()
-    ntile = (nfw + 31) // 32 + 8
+    ntile = (nfw + 15) // 16
     nk = len(systems.kvector_indices(s.kmax)) if s.ewald else 1
     nads = maxmol * s.molecule.n_atoms
-    io_n = max(64, nfw, nads)
-    b = nfw * 32 + ntile * (32 * 16 + 32)          # fw64, fw32, tiles
-    b += nk * (4 + 8 + 16 * 3)                     # kvec, kfactor, S_fw, S_ads, dS
+    b = nfw * (32 + 24 + 8)                        # fw64, framework as given for S_fw(k)
+    b += ntile * (16 * (16 + 32) + 32)             # fixed-point and FP64 atoms by tile, tiles
+    b += nk * (4 + 8 + 16 * 4)                     # kvec, kfactor, S_fw, S_ads, two dS
     b += nads * (24 + 16 + 32)                     # positions, records
-    b += io_n * 32 + 64 * (32 + 12) + 4096         # per-call scratch, descriptor, state
+    b += 16384                                     # descriptor here and in the engine, state, cell matrices
     return int(b)
 
 

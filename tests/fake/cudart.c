@@ -12,6 +12,7 @@ static struct { char *p; size_t n; } mapped[RANGES];
 int fake_launches;       /* launches asked for */
 int fake_fail_launch;    /* launches return an error */
 int fake_syncs, fake_host_allocs;
+long long fake_device_bytes;   /* device memory asked for */
 /* 1: every launch is a grid lookup, done as out[i] = x of position i + 1; fake_stray counts those whose
  * positions or results lie outside the mapped ranges (and are left out) */
 int fake_lookup, fake_stray;
@@ -55,7 +56,12 @@ cudaError_t cudaDeviceSynchronize(void) { fake_syncs++; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) { (void)f; *s = (cudaStream_t)1; return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { (void)s; return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; fake_syncs++; return cudaSuccess; }
-cudaError_t cudaMalloc(void **p, size_t n) { *p = calloc(1, n); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaMalloc(void **p, size_t n)
+{
+  fake_device_bytes += (long long)n;
+  *p = calloc(1, n);
+  return *p ? cudaSuccess : cudaErrorMemoryAllocation;
+}
 cudaError_t cudaFree(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, enum cudaMemcpyKind k)
 {

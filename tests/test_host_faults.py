@@ -88,3 +88,23 @@ def test_lookup_of_as_many_points_as_an_int_counts(fake):
         assert value("fake_launches").value == 2 ** 31 // 16384
         assert np.array_equal(np.ctypeslib.as_array(C.cast(out, C.POINTER(C.c_double)), (k,)), np.ones(k))
     """)
+
+
+def test_footprint_is_what_a_system_allocates(fake):
+    """The serving front end's estimate of a job's device memory covers what rgpu_system_create and the engine's
+    descriptor take, and is not much above it."""
+    child(fake, """
+        import dataclasses
+        from raspa2_b200 import serve
+        co2 = systems.co2_system(seed=21, n_atoms=1536, cell=25.8, kmax=8, layout="uniform")
+        for s, maxmol in ((systems.tiny_co2_system(), 8), (co2, 64), (co2, 512), (systems.methane_system(seed=3), 512),
+                          (dataclasses.replace(co2, unit_cells=np.array([3, 2, 2])), 100),
+                          (dataclasses.replace(systems.tiny_co2_system(), cell_angles=(80.0, 95.0, 100.0),
+                                               unit_cell=np.array([29.0, 28.0, 30.0])), 20)):
+            n = C.c_longlong.in_dll(fake, "fake_device_bytes")
+            n.value = 0
+            g = native.GpuSystem(s, maxmol=maxmol)
+            e = native.Engine([g], threads=256, cluster=1)
+            got = serve.system_footprint_bytes(s, maxmol)
+            assert n.value <= got <= 1.05 * n.value + 16384, (s.name, n.value, got)
+    """)
