@@ -838,7 +838,8 @@ extern "C" int rgpu_set_adsorbates(rgpu_system *s, int nmol, const double *xyz)
   s->net_ads = nmol * s->h.mol_charge;
   s->pending_dq = 0.0;
   if (n) CK(cudaMemcpyAsync(s->ads_xyz, s->h_xyz.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
-  CK(rgpu_records_launch(s->d_sys, nmol * s->d.natom, nmol, s->rec32, s->rec64, s->st));
+  if (n) CK(rgpu_records_launch(s->d_sys, nmol * s->d.natom, nmol, s->rec32, s->rec64, s->st));
+  else CK(cudaMemsetAsync(s->nmol, 0, sizeof(int), s->st));
   s->records_stale = 0;
   CK(rgpu_structure_factor_launch(s->d_sys, s->ads_xyz, nullptr, nmol * s->d.natom, s->h.nk, s->sk_ads, s->st));
   CK(cudaStreamSynchronize(s->st));
@@ -1192,7 +1193,7 @@ extern "C" int rgpu_total_energy(rgpu_system *s, double *out)
   CK(rgpu_total_pairs_launch(s->d_sys, s->rec64, nads, s->fw_model == RGPU_FRAMEWORK_GRID, s->h_call->total, &ctas, s->st));
   if (fourier)
     CK(rgpu_ads_fourier_launch(s->d_sys, s->ads_xyz, nads, h.nk, s->sk_ads, s->h_call->fourier, &blocks, s->st));
-  CK(cudaStreamSynchronize(s->st));
+  if (ctas || blocks) CK(cudaStreamSynchronize(s->st));
   double hv = 0, hc = 0, av = 0, ac = 0, ex = 0, hf = 0, af = 0;
   for (int c = 0; c < ctas; c++) {
     const double *t = s->h_call->total + 5 * c;

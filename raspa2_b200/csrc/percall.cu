@@ -619,6 +619,7 @@ static cudaError_t sk_launch(const RgpuSys *d_sys, const double *d_xyz, const do
                              double *d_out, cudaStream_t st)
 {
   if (nk <= 0) return cudaSuccess;
+  if (n <= 0 && !d_out) return cudaMemsetAsync(d_sk, 0, sizeof(double2) * (size_t)nk, st);
   const int blocks = (nk + SK_THREADS - 1) / SK_THREADS;
   /* CTAs that share the atoms of a block of wave vectors: a table's worth of
    * atoms each, as long as all CTAs run at once (148 SMs, 2 CTAs each) */

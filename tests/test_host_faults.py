@@ -108,3 +108,19 @@ def test_footprint_is_what_a_system_allocates(fake):
             got = serve.system_footprint_bytes(s, maxmol)
             assert n.value <= got <= 1.05 * n.value + 16384, (s.name, n.value, got)
     """)
+
+
+def test_empty_configurations_launch_no_kernel(fake):
+    """No molecule: an upload is two memsets, and an uncharged system's total energy neither launches nor waits."""
+    child(fake, """
+        for s in (systems.tiny_co2_system(), systems.methane_system(seed=3)):
+            g = native.GpuSystem(s, maxmol=8)
+            na = s.molecule.n_atoms
+            g.set_adsorbates(np.ones((3, na, 3)))
+            n = value("fake_launches").value
+            g.set_adsorbates(np.zeros((0, na, 3)))
+            assert value("fake_launches").value == n
+            syncs = value("fake_syncs").value
+            g.total_energy()
+            assert s.ewald or (value("fake_launches").value, value("fake_syncs").value) == (n, syncs)
+    """)
