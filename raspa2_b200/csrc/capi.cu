@@ -859,17 +859,18 @@ extern "C" int rgpu_get_adsorbates(rgpu_system *s, int *nmol, double *xyz, int c
   return RGPU_SUCCESS;
 }
 
-/* puts xyz in molecule slot m (none for m < 0) and the molecule count h_nmol
- * on the device, with the slot's records */
-static int write_molecule(rgpu_system *s, int m, const double *xyz)
+/* puts xyz in molecule slot m (none for m < 0), with its records, and sets
+ * the molecule count; the host's copy follows once that is on its way */
+static int write_molecule(rgpu_system *s, int m, int nmol, const double *xyz)
 {
   const int na = s->d.natom;
   RgpuSites in;
-  if (m >= 0) {
-    memcpy(&s->h_xyz[(size_t)m * na * 3], xyz, sizeof(double) * 3 * na);
-    memcpy(in.xyz, xyz, sizeof(double) * 3 * na);
-  }
-  CK(rgpu_set_molecule_launch(s->d_sys, in, m, s->h_nmol, s->rec32, s->rec64, s->st));
+  if (m >= 0) memcpy(in.xyz, xyz, sizeof(double) * 3 * na);
+  CK(rgpu_set_molecule_launch(s->d_sys, in, m, nmol, s->rec32, s->rec64, s->st));
+  s->h_xyz.resize((size_t)std::max(nmol, s->h_nmol) * na * 3);
+  if (m >= 0) memcpy(&s->h_xyz[(size_t)m * na * 3], in.xyz, sizeof(double) * 3 * na);
+  s->h_xyz.resize((size_t)nmol * na * 3);
+  s->h_nmol = nmol;
   return RGPU_SUCCESS;
 }
 
@@ -879,7 +880,7 @@ extern "C" int rgpu_update_molecule(rgpu_system *s, int m, const double *xyz)
   int rc = refresh_from_device(s);
   if (rc) return rc;
   if (m < 0 || m >= s->h_nmol) return fail(RGPU_E_INVALID, "molecule %d", m);
-  return write_molecule(s, m, xyz);
+  return write_molecule(s, m, s->h_nmol, xyz);
 }
 
 extern "C" int rgpu_insert_molecule(rgpu_system *s, const double *xyz)
@@ -888,9 +889,7 @@ extern "C" int rgpu_insert_molecule(rgpu_system *s, const double *xyz)
   int rc = refresh_from_device(s);
   if (rc) return rc;
   if (s->h_nmol >= s->d.maxmol) return fail(RGPU_E_CAPACITY, "maxmol %d reached", s->d.maxmol);
-  s->h_xyz.resize((size_t)(s->h_nmol + 1) * s->d.natom * 3);
-  s->h_nmol++;
-  rc = write_molecule(s, s->h_nmol - 1, xyz);
+  rc = write_molecule(s, s->h_nmol, s->h_nmol + 1, xyz);
   if (rc) return rc;
   CK(cudaStreamSynchronize(s->st));
   return RGPU_SUCCESS;
@@ -902,13 +901,9 @@ extern "C" int rgpu_remove_molecule(rgpu_system *s, int m)
   int rc = refresh_from_device(s);
   if (rc) return rc;
   if (m < 0 || m >= s->h_nmol) return fail(RGPU_E_INVALID, "molecule %d", m);
-  const int na = s->d.natom, last = s->h_nmol - 1;
-  double x[3 * RGPU_MAX_ATOMS];
-  memcpy(x, &s->h_xyz[(size_t)last * na * 3], sizeof(double) * 3 * na);
-  s->h_nmol--;
-  rc = write_molecule(s, m != last ? m : -1, x);
+  const int last = s->h_nmol - 1;
+  rc = write_molecule(s, m != last ? m : -1, last, &s->h_xyz[(size_t)last * s->d.natom * 3]);
   if (rc) return rc;
-  s->h_xyz.resize((size_t)s->h_nmol * na * 3);
   CK(cudaStreamSynchronize(s->st));
   return RGPU_SUCCESS;
 }

@@ -40,7 +40,13 @@ void fake_reset(void) { memset(mapped, 0, sizeof mapped); }
 
 cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+static cudaError_t last = cudaSuccess;
+cudaError_t cudaGetLastError(void)
+{
+  const cudaError_t e = last;
+  last = cudaSuccess;
+  return e;
+}
 cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int d)
 {
   (void)d;
@@ -120,7 +126,7 @@ cudaError_t cudaHostGetDevicePointer(void **d, void *p, unsigned f)
 static cudaError_t launch(void **args)
 {
   fake_launches++;
-  if (fake_fail_launch) return cudaErrorLaunchFailure;
+  if (fake_fail_launch) return last = cudaErrorLaunchFailure;
   if (fake_lookup) {
     /* (grid, geometry, n, positions, results) */
     const int n = *(int *)args[2];

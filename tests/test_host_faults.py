@@ -124,3 +124,30 @@ def test_empty_configurations_launch_no_kernel(fake):
             g.total_energy()
             assert s.ewald or (value("fake_launches").value, value("fake_syncs").value) == (n, syncs)
     """)
+
+
+def test_failed_molecule_updates_change_nothing(fake):
+    """Where the launch that writes a molecule to the device fails, the host's copy of the configuration stays as the
+    device's."""
+    child(fake, """
+        s = systems.tiny_co2_system()
+        g = native.GpuSystem(s, maxmol=8)
+        x = np.random.default_rng(1).uniform(0.0, 20.0, (5, 3, 3))
+        g.set_adsorbates(x)
+        value("fake_fail_launch").value = 1
+        for call in (lambda: g.insert_molecule(x[0] + 1.0), lambda: g.remove_molecule(1), lambda: g.remove_molecule(4),
+                     lambda: g.update_molecule(2, x[2] + 1.0)):
+            try:
+                call()
+            except native.NativeError:
+                pass
+            else:
+                assert False, "no error"
+            assert np.array_equal(g.adsorbates(), x)
+        value("fake_fail_launch").value = 0
+        g.insert_molecule(x[0] + 1.0)
+        g.update_molecule(2, x[2] + 1.0)
+        g.remove_molecule(1)
+        g.remove_molecule(4)
+        assert np.array_equal(g.adsorbates(), np.stack([x[0], x[0] + 1.0, x[2] + 1.0, x[3]]))
+    """)
