@@ -87,7 +87,7 @@ struct rgpu_system {
     double e[4 * RGPU_MAX_POS];
     int ov[RGPU_MAX_POS];
     double total[5 * RGPU_TOTAL_CTAS];
-    double fourier[2 * 128];   /* blocks of 256 wave vectors; kmax <= 20 has under 20000 */
+    double fourier[2 * RGPU_FOURIER_BLOCKS];
   } *h_call;
   /* host mirrors */
   RgpuState h_state;          /* initial state at creation; last state read */

@@ -650,6 +650,7 @@ cudaError_t rgpu_ads_fourier_launch(const RgpuSys *d_sys, const double *d_xyz, i
                                     int *blocks, cudaStream_t st)
 {
   *blocks = (nk + SK_THREADS - 1) / SK_THREADS;
+  if (*blocks > RGPU_FOURIER_BLOCKS) return cudaErrorInvalidValue;
   return sk_launch(d_sys, d_xyz, nullptr, n, nk, d_sk, d_out, st);
 }
 

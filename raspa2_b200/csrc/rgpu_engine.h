@@ -26,7 +26,8 @@ cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ad
 cudaError_t rgpu_total_pairs_launch(const RgpuSys *d_sys, const void *d_ads, int nads, int fw_grid, double *d_out,
                                     int *ctas, cudaStream_t st);
 /* S_ads(k) of n adsorbate atoms into d_sk, and the Fourier sums into
- * d_out[2 * *blocks], *blocks = (nk + 255) / 256 */
+ * d_out[2 * *blocks], *blocks = (nk + 255) / 256; an error where that
+ * exceeds RGPU_FOURIER_BLOCKS */
 cudaError_t rgpu_ads_fourier_launch(const RgpuSys *d_sys, const double *d_xyz, int n, int nk, double2 *d_sk, double *d_out,
                                     int *blocks, cudaStream_t st);
 cudaError_t rgpu_ewald_delta_launch(int mixed, const RgpuSys *d_sys, const RgpuSites &in, int ns, int nk, double2 *d_ds,

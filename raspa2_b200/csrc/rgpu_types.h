@@ -119,6 +119,8 @@ typedef struct {
 } RgpuSites;
 
 #define RGPU_TOTAL_CTAS 592    /* CTAs of a total-energy evaluation: 4 on each of 148 SMs */
+#define RGPU_FOURIER_BLOCKS 128 /* most blocks of 256 wave vectors of a Fourier sum; the 20004 of kmax 20, the largest
+                                * accepted, take 79 */
 
 /* geometry of an energy grid: npts cells per axis over `size` from `shift`,
  * spanning a unit cell of lengths `cell`; a triclinic unit cell (tri = 1)

@@ -201,3 +201,19 @@ def test_fp64_lj_rounding(cuda, charged):
     err = (got - ref) / ref * 2.0 ** 53
     assert np.max(np.abs(err)) <= 13 * 1.05          # s^6 >= 21: (2 s^6 - 1) / (s^6 - 1) is within 5 % of 2
     assert np.sqrt(np.mean(err ** 2)) <= 3.3
+
+
+def test_total_energy_with_the_most_wave_vectors(cuda):
+    """kmax 20, the largest accepted: 20004 wave vectors in 79 of the 128 blocks that a call's results have room
+    for (the bounds of the totals above)."""
+    s = dataclasses.replace(co2_box(16, False), kmax=(20, 20, 20))
+    assert s.n_kvectors() == 20004 <= 128 * 256
+    rng = np.random.default_rng(20)
+    mols = molecules(rng, s, 12)
+    g = native.GpuSystem(s, maxmol=16)
+    g.set_adsorbates(mols)
+    o = O.Oracle.from_system(s, maxmol=16)
+    o.set_molecules(mols)
+    ref, e = np.array(o.total_energy())[:6], np.asarray(g.total_energy())
+    size = np.abs(np.array(o.ewald_delta_abs(new=mols[0])))[:2].max() * 13 ** 2
+    assert np.all(np.abs(e - ref)[4:] <= 1e-9 * np.abs(ref[4:]) + 1e-12 * size + 1e-7), (e, ref)
