@@ -11,6 +11,7 @@
 #ifndef RGPU_GRID_CUH
 #define RGPU_GRID_CUH
 
+#include "rgpu_quotient.h"
 #include "rgpu_types.h"
 
 /* the point wrapped into the unit cell the grid spans (a point at half a cell
@@ -41,15 +42,11 @@ __device__ __forceinline__ void rgpu_grid_wrap(const RgpuGridGeom &ip, const dou
   for (int r = 0; r < 3; r++) pw[r] = __ldg(m + 3 * r) * f[0] + __ldg(m + 3 * r + 1) * f[1] + __ldg(m + 3 * r + 2) * f[2];
 }
 
-/* p along axis c in grid cells: ((p - shift) / size) * npts, the quotient from
- * the rounded reciprocal with one residual correction (Markstein, "Computation
- * of elementary functions on the IBM RISC System/6000 processor", 1990), which
- * rounds as the division does at a third of its instructions. (One product
+/* p along axis c in grid cells: ((p - shift) / size) * npts. (One product
  * with npts / size had up to six times the error in the looked-up energy.) */
 __device__ __forceinline__ double rgpu_grid_coord(const RgpuGridGeom &ip, int c, double p)
 {
-  const double x = p - ip.shift[c], q = x * ip.isize[c];
-  return fma(fma(-q, ip.size[c], x), ip.isize[c], q) * (double)ip.npts[c];
+  return rgpu_quotient(p - ip.shift[c], ip.size[c], ip.isize[c]) * (double)ip.npts[c];
 }
 
 /* Cubic Hermite basis on [0,1]: {p0, p1, slope0, slope1} */
