@@ -1443,9 +1443,8 @@ extern "C" int rgpu_grid_file_path(char *buf, size_t n, const char *raspa_dir, c
  * One per process, made at the first call and given back when the library is
  * unloaded; a call that finds it in use by another thread goes through device
  * buffers of its own. Pageable copies of 100 k points (2.4 MB in, 0.8 MB out)
- * alone took 1.5 ms; copied into this in LOOKUP_CHUNK pieces, each looked up
- * while the next is copied, the whole call takes 0.31 ms
- * (1.64 with the copies). The pages are the library's own and registered with
+ * alone took 1.5 ms and more; copied into this in LOOKUP_CHUNK pieces, each
+ * looked up while the next is copied, the whole call takes 0.30 ms. The pages are the library's own and registered with
  * the runtime: cudaDeviceReset undoes the registration, not the memory, so
  * each call asks whether it still stands (under 1 us) and registers again
  * where it does not. */

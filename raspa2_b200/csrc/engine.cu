@@ -95,12 +95,9 @@ size_t rgpu_engine_smem_bytes(int mixed, int fw_items, int fwd_items, int tiles,
  * more than once beside it is a function of its own; and the work that can be
  * spread over threads (placing positions, adding up CTAs' sums) is done by all
  * of them between barriers, which cost some 500 cycles. Code now 120 to 270
- * KB. Measured (upload, moves, states read back): 64 mixed CO2 boxes, 1000
- * moves each, 20.9 ms (27.2 before; 21.5 with
- * dS(k) formed again on acceptance); one FP64 CO2 box, 200 moves, 3.21 ms
- * (4.30); 32 hexane boxes over grids, 100 moves, 3.88 ms (4.43; 4.29 with the
- * bend angles of a growth, its uniforms, the next bead's frames, the trials'
- * LJ and the next stage's description all formed by warp 0 or on its way). */
+ * KB. Measured (upload, moves, states read back), before and after: 64 mixed
+ * CO2 boxes, 1000 moves each, 27.3 and 21.0 ms; one FP64 CO2 box, 200 moves,
+ * 4.25 and 3.36 ms; 32 hexane boxes over grids, 100 moves, 4.45 and 3.87 ms. */
 #define RGPU_COLD __noinline__
 
 /* floor(2^32 / n) + 1 (less one for powers of two: 2^32 / n) for 2 <= n <= 64, 0
@@ -1574,9 +1571,10 @@ __device__ __forceinline__ void retrace_combine(Ctl &C, int i0, int i1, int nf, 
  * of sum w / trials), the chosen beads (cp), their host and adsorbate VDW
  * (u[0], u[2]) and the intramolecular energy (uintra: bonded + LJ).
  *
- * Growth: one stage per bead. Warp 0 selects a trial; meanwhile warp 1
- * computes every trial's bonded energy, the chosen
- * one's being added in the next stage.
+ * Growth: one stage per bead. Warp 0 selects a trial; meanwhile other warps
+ * form what each trial would need if chosen (beside_grow): the next bead's
+ * frame, the bonded energy (the chosen one's is added in the next stage) and
+ * the next stage's description.
  *
  * Retrace: the beads it "chooses" are the old ones, known before anything is
  * evaluated, so the trial sets of several beads are placed together and
@@ -1702,7 +1700,7 @@ __device__ __forceinline__ bool end_grow(Build<MIXED, FLEX> E, const Stage &g)
     C.cp[i][2] = q.z;
   }
   if (lane == 0) {
-    if (i - 1 >= 2) C.uintra += fx().gr.ub[(i - 1) & 1][C.sel];   /* the last bead's bonded energy (warp 1) */
+    if (i - 1 >= 2) C.uintra += fx().gr.ub[(i - 1) & 1][C.sel];   /* the last bead's bonded energy (beside_grow) */
     C.rosen = rosen;
     C.u[0] += hv;
     C.u[2] += av;
@@ -1999,9 +1997,9 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 512) rgpu_engine_kernel(RgpuSys 
     E.csize = csize;
     E.xb = 0;
     E.sc.u = fx().u;
-    E.sc.qr2 = (float *)(smem + L.q);
-    E.sc.qq = E.sc.qr2 + nwarps * (MIXED == 2 ? 128 : 64);
-    E.sc.qt = MIXED ? (int *)(E.sc.qq + nwarps * 64) : (int *)(smem + L.q);
+    E.sc.qr2 = MIXED ? (float *)(smem + L.q) : nullptr;
+    E.sc.qq = MIXED == 2 ? E.sc.qr2 + nwarps * 128 : nullptr;
+    E.sc.qt = MIXED == 2 ? (int *)(E.sc.qq + nwarps * 64) : (MIXED ? nullptr : (int *)(smem + L.q));
     E.tab = (typename PhaseT<MIXED>::T *)(smem + L.tab);
     E.kw = kw;
     Ctl &C = fx().C;

@@ -163,9 +163,9 @@ __device__ __forceinline__ int grid_stage(const RgpuSys &S, const GridParams &gp
  * its erfc = exp(-x^2) erfcx(x) shares. 64 and 80 registers keep 32 and 24
  * warps on an SM; with the compiler's choice (94, 116) there were 16 and the
  * dependent FP64 instructions left the pipe half idle. 102^3 points over 4096
- * atoms in a 40 A cell, LJ: 2.28 ms, 12.9 TFLOP/s at 60 FLOP a pair inside the
- * cut-off (5.78 ms with a rounding per pair and axis and four divisions; 3.06
- * at 94 registers). 78^3 points over 1536 atoms, Coulomb: 4.02 ms (6.76; 4.71).
+ * atoms in a 40 A cell, LJ: 2.27 ms, 12.9 TFLOP/s at 60 FLOP a pair inside the
+ * cut-off (5.77 ms with a rounding per pair and axis and four divisions; 3.06
+ * at 94 registers). 78^3 points over 1536 atoms, Coulomb: 4.01 ms (6.77; 4.71).
  * IMAGES: every image of an atom within reach of the tile is, along each cell
  * vector, its nearest to the tile's centre or the next one
  * (cutoff + tile radius below every perpendicular width); all of those within

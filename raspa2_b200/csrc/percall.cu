@@ -65,11 +65,10 @@ __device__ __forceinline__ void grid_terms(const RgpuSys &S, const BeadPos &b, i
  * unit_tiles_fp64, and the sums meet in the first CTA's shared memory in rank
  * and warp order. What bounds it is the chain of one warp (descriptor load,
  * cull, two or three tile passes, one queue evaluation), not arithmetic.
- * Measured, whole call from Python: 20 positions in a 1536-atom CO2 box 23.5 us
- * (the kernel 12.8, cold, under the profiler), 139 us with one CTA of 8 warps
- * walking all atoms of all positions; one position in 3456 uncharged atoms 18.9
- * us (kernel 9.2), 46 us before. Of each, some 10 us went with the binding's
- * buffer pointers, the rest with this kernel and its launch. */
+ * Measured, whole call from Python: 20 positions in a 1536-atom CO2 box 25 us
+ * (the kernel 13.8, cold, under the profiler; 140 us a call with one CTA of 8
+ * warps walking all atoms of all positions); one position in 3456 uncharged
+ * atoms 20 us (kernel 9.0; 47 us). */
 __global__ void __launch_bounds__(32 * POINT_WARPS) k_points_fp64(const RgpuSys *sysp, const AdsRec64 *ads, int nads,
                                                                  const __grid_constant__ RgpuPoints in, int pair_check,
                                                                  int fw_grid, double *out, int *ov)
@@ -215,11 +214,11 @@ __global__ void __launch_bounds__(64 * POINT_MIXED_WARPS) k_points_mixed(const R
  * of its own, all threads form the lists' pair terms into one sequence, and
  * one warp adds that up. A ninth warp takes the adsorbates meanwhile. A
  * list that overflows sends the position through one warp's queue. Bound by the
- * chain of steps. 64 positions in 4096 atoms: 26 us a call from Python (the
- * kernel 16.7, cold, under the profiler), 40 us with one warp walking all tiles
+ * chain of steps. 64 positions in 4096 atoms: 27 us a call from Python (the
+ * kernel 17.4, cold, under the profiler), 40 us with one warp walking all tiles
  * of a position. */
 #define LONG_WARPS 8
-#define LONG_LIST 256          /* pairs of one warp; a sixteenth of the sphere's atoms at 0.09 / A^3 is 41 */
+#define LONG_LIST 256          /* pairs of one warp; an eighth of a 12 A sphere's atoms at 0.09 / A^3 is 81 */
 
 struct LongSmem {
   RgpuSys S;
@@ -364,8 +363,8 @@ cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ad
   if (P < 1 || P > RGPU_MAX_POS) return cudaErrorInvalidValue;
   if (mixed) {
     EvalPlan pl = eval_plan(P, ntile, nads, POINT_MIXED_WARPS, 8 * RGPU_MAX_POS, 2);
-    /* one framework unit a position and a tile for every warp: 23 us a call from
-     * 8 to 64 positions and 300 to 4096 atoms, 25 to 40 with a warp per unit */
+    /* one framework unit a position and a tile for every warp: from 300 to 4096
+     * atoms 23 to 27 us a call of 8 to 64 positions, 25 to 40 with a warp per unit */
     if (pl.cf == 1 && pl.ca <= 1 && ntile >= LONG_WARPS) {
       k_points_mixed_long<<<P, 32 * (LONG_WARPS + 1), 0, st>>>(d_sys, (const int4 *)d_ads, nads, in, pair_check, d_out, d_ov);
       return cudaGetLastError();
@@ -404,7 +403,7 @@ cudaError_t rgpu_points_launch(int mixed, const RgpuSys *d_sys, const void *d_ad
  * VDW, adsorbate real, exclusion} of its atoms and molecules in out[5 c ..]
  * (mapped host memory). Each CTA takes every gridDim-th atom, a warp per
  * quarter of the framework tiles and of the adsorbate records, so that a
- * loaded box fills the GPU in one launch. 408 atoms in 4096: 21.7 us under the
+ * loaded box fills the GPU in one launch. 408 atoms in 4096: 22.9 us under the
  * profiler, cold, a warp's chain of tile passes with the FP64 pipe 15 % busy (4.5
  * ms in seven launches of one CTA before). */
 #define TOTAL_WARPS 4
