@@ -818,11 +818,13 @@ __device__ __forceinline__ double warp_scan(double v)
 
 /* SelectTrialPosition (src/cbmc.c:563-599) among the weights w of lanes < n,
  * cum their sums up to each lane: the first trial whose cumulative weight
- * reaches u times their sum */
+ * reaches u times their sum; trial 0 where that is zero or NaN (weights that
+ * all underflow, or overflow and cancel), as the reference's loop takes it */
 __device__ __forceinline__ int select_trial(double w, double cum, int n, double u)
 {
   const int lane = threadIdx.x & 31;
   const double target = u * __shfl_sync(RGPU_FULL, cum, 31);
+  if (!(target > 0.0)) return 0;
   const unsigned hit = __ballot_sync(RGPU_FULL, lane < n && w > 0.0 && !(cum < target));
   return hit ? __ffs(hit) - 1 : n - 1;
 }

@@ -115,3 +115,26 @@ def test_grid_loading_matches_direct_sums(cuda):
     a, b = loads[False], loads[True]
     se = np.hypot(a.std(ddof=1), b.std(ddof=1)) / np.sqrt(nrep)
     assert abs(a.mean() - b.mean()) <= 4.0 * se, (a.mean(), b.mean(), se)
+
+
+@pytest.mark.parametrize("seed,overlaps,accepted", [(2, 147, [2, 0, 2, 0]), (5, 166, [6, 1, 3, 0]),
+                                                    (6, 171, [2, 10, 4, 0])])
+def test_trial_selection_where_weights_leave_the_range(cuda, seed, overlaps, accepted):
+    """Grids too coarse for their framework interpolate to wells so deep that a bead's weights are infinite and the
+    next bead's all zero: trial 0 is chosen there, as the reference's loop over the cumulative weights chooses it, and
+    the growth goes on with a weight that is not a number. Which trial is chosen shows in the growths that fail later;
+    the counts are those of an engine that selected by that loop."""
+    import dataclasses
+    s = systems.co2_system(seed=seed, n_atoms=700, cell=25.0, kmax=1, layout="uniform", dmin=1.2, pressure=1e6)
+    s = dataclasses.replace(s, molecule=systems.HEXANE, ewald=False, uc_charges=np.zeros(len(s.uc_types)), trials=2,
+                            trials_first_bead=14, moves=systems.MoveMix(0.5, 0.5, 1.0, 0.3, 0.3, 1.0))
+    g = native.GpuSystem(s, maxmol=48, seed=777, stream_id=seed)
+    g.set_adsorbates(np.zeros((0, 6, 3)))
+    g.use_energy_grids(0.8)
+    e = native.Engine([g], precision=native.RGPU_FP64, threads=256, cluster=2)
+    e.run(300)
+    e.sync()
+    st = g.state()
+    assert st["status"] == 2          # a non-finite energy reached an acceptance test
+    assert st["counters"][9] == overlaps
+    assert st["counters"][4:8].tolist() == accepted
